@@ -109,7 +109,7 @@ __global__ void paged_decode_kernel(const __nv_bfloat16* __restrict__ q, const v
 //   P V      lane = pair (D 64) or quad (D 128) of output columns: the probabilities of the chunk go through shared
 //            memory, each V row is read as one conflict-free line and every lane updates its G x E accumulators.
 // The warps' partial results are merged in shared memory and written in the (normalised output, max, sum) form that
-// the merge kernel below combines across splits.  bf16 caches only (e4m3 stays on the kernel above); block_size must
+// the merge kernel below combines across splits.  bf16 caches only; block_size must
 // divide 32 or be a multiple of it.
 constexpr int kPdWarps = 4;
 constexpr int kPdMaxG = 8;
@@ -348,6 +348,52 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4],
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// End of a CTA of the tensor-core decode kernels: shared memory (the tile area: every requested copy has been waited for) takes
+// the four warps' maxima, sums and outputs, [warps][16], [warps][16] and [warps][16][D] floats; the last one is returned.
+__device__ __forceinline__ float* pd_row_sums(uint8_t* smem, int warp, int lane, bool ok, float m_lo, float m_hi, float l_lo, float l_hi) {
+  const int g = lane >> 2;
+  l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
+  l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
+  l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);
+  l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
+  __syncthreads();
+  float* red_m = reinterpret_cast<float*>(smem);
+  float* red_l = red_m + kPdWarps * kPdMmaMaxG;
+  if ((lane & 3) == 0) {
+    red_m[warp * kPdMmaMaxG + g] = ok ? m_lo : -INFINITY;
+    red_l[warp * kPdMmaMaxG + g] = ok ? l_lo : 0.f;
+    red_m[warp * kPdMmaMaxG + g + 8] = ok ? m_hi : -INFINITY;
+    red_l[warp * kPdMmaMaxG + g + 8] = ok ? l_hi : 0.f;
+  }
+  return red_l + kPdWarps * kPdMmaMaxG;
+}
+// part: the group's rows [G][splits][D + 2]; out_scale multiplies the outputs.
+template <int D>
+__device__ __forceinline__ void pd_write_partial(uint8_t* smem, float* part, int G, int splits, int sp, float out_scale) {
+  const float* red_m = reinterpret_cast<const float*>(smem);
+  const float* red_l = red_m + kPdWarps * kPdMmaMaxG;
+  const float* red_o = red_l + kPdWarps * kPdMmaMaxG;
+  __syncthreads();
+  for (int i = threadIdx.x; i < G * D; i += blockDim.x) {
+    const int gg = i / D, d = i % D;
+    float gm = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < kPdWarps; ++w) gm = fmaxf(gm, red_m[w * kPdMmaMaxG + gg]);
+    float lsum = 0.f, o = 0.f;
+#pragma unroll
+    for (int w = 0; w < kPdWarps; ++w) {
+      const float mw = red_m[w * kPdMmaMaxG + gg];
+      if (mw == -INFINITY) continue;
+      const float a = __expf(mw - gm);
+      lsum += red_l[w * kPdMmaMaxG + gg] * a;
+      o += red_o[(w * kPdMmaMaxG + gg) * D + d] * a;
+    }
+    float* out = part + ((long long)gg * splits + sp) * (D + 2);
+    out[d] = lsum > 0.f ? o / lsum * out_scale : 0.f;
+    if (d == 0) { out[D] = gm; out[D + 1] = lsum; }
+  }
+}
+
 // tmK / tmV: the caches seen as [num_blocks * Hkv * block_size rows, D] bf16, box 64 columns x min(block_size, 32) rows,
 // 128-byte swizzle.  block_size is a multiple of 8 and divides 32 or is a multiple of it.
 template <int D>
@@ -533,20 +579,7 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     __syncwarp();            // every lane is done with this stage before lane 0 requests into it again
   }
   // ---- merge the four warps (the tile area is free now: every requested copy has been waited for), write the partial result
-  l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
-  l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
-  l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);
-  l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
-  __syncthreads();
-  float* red_m = reinterpret_cast<float*>(pd_smem);                 // [warps][16]
-  float* red_l = red_m + kPdWarps * kPdMmaMaxG;                      // [warps][16]
-  float* red_o = red_l + kPdWarps * kPdMmaMaxG;                      // [warps][16][D]
-  if (qd == 0) {
-    red_m[warp * kPdMmaMaxG + g] = ok ? m_lo : -INFINITY;
-    red_l[warp * kPdMmaMaxG + g] = ok ? l_lo : 0.f;
-    red_m[warp * kPdMmaMaxG + g + 8] = ok ? m_hi : -INFINITY;
-    red_l[warp * kPdMmaMaxG + g + 8] = ok ? l_hi : 0.f;
-  }
+  float* red_o = pd_row_sums(pd_smem, warp, lane, ok, m_lo, m_hi, l_lo, l_hi);
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt) {
     float* lo = red_o + (warp * kPdMmaMaxG + g) * D + nt * 8 + qd * 2;
@@ -554,25 +587,265 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     *reinterpret_cast<float2*>(lo) = make_float2(oacc[nt][0], oacc[nt][1]);
     *reinterpret_cast<float2*>(hi) = make_float2(oacc[nt][2], oacc[nt][3]);
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < G * D; i += blockDim.x) {
-    const int gg = i / D, d = i % D;
-    float gm = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < kPdWarps; ++w) gm = fmaxf(gm, red_m[w * kPdMmaMaxG + gg]);
-    float lsum = 0.f, o = 0.f;
-#pragma unroll
-    for (int w = 0; w < kPdWarps; ++w) {
-      const float mw = red_m[w * kPdMmaMaxG + gg];
-      if (mw == -INFINITY) continue;
-      const float a = __expf(mw - gm);
-      lsum += red_l[w * kPdMmaMaxG + gg] * a;
-      o += red_o[(w * kPdMmaMaxG + gg) * D + d] * a;
-    }
-    float* out = part + (((long long)s * Hq + hkv * G + gg) * splits + sp) * (D + 2);
-    out[d] = lsum > 0.f ? o / lsum : 0.f;
-    if (d == 0) { out[D] = gm; out[D + 1] = lsum; }
+  pd_write_partial<D>(pd_smem, part + ((long long)s * Hq + hkv * G) * splits * (D + 2), G, splits, sp, 1.f);
+}
+
+// The same split of the work for e4m3 caches.  What was a warp per query head that walked the keys one at a time (968 us for 8
+// sequences of 4500 to 9000 tokens, 8 KV heads of 128 and 4 query heads each, where the cache streams in 18 us) reads every byte once for
+// the whole group.  8-bit keys and values are exact as fp16 operands (one conversion for two of them):
+//   scores   a lane takes 16 contiguous bytes of a key row, which are its fragments of four instructions when the columns of
+//            the query are permuted alike; the query's rows are scaled by a power of two so that fp16 holds all of their bits;
+//   P V      ldmatrix transposes pairs of bytes, so that a lane gets two neighbouring columns of two neighbouring keys; even and odd
+//            columns go to instructions of their own.  The softmax weights stay at 32-bit precision: 2^14 p is the sum of two fp16
+//            parts, each with an instruction of its own.
+template <int D>
+struct PdF8Cfg {
+  static constexpr int kStages = (D == 64) ? 4 : 3;
+  static constexpr int kTileBytes = 32 * D;                               // 32 keys of K (or V)
+  static constexpr int kWarpBytes = kStages * 2 * kTileBytes;
+  static constexpr int kOffBar = kPdWarps * kWarpBytes;
+  static constexpr int kSmemBytes = kOffBar + kPdWarps * kStages * 8 + 16 + 1024;   // + slack to align the tiles to 1024 bytes
+  static_assert(kOffBar >= kPdWarps * kPdMmaMaxG * (D + 2) * 4, "the reduction at the end reuses the tile area");
+};
+constexpr float kPdWeightScale = 16384.f;   // weights are at most 1: the largest fp16 part is 2^14, the smallest 2^-24 stands for 2^-38
+
+__device__ __forceinline__ void mma_f16_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// Two e4m3 values (low byte first) -> fp16 pair, exactly.
+__device__ __forceinline__ uint32_t e4m3x2_to_f16x2(uint32_t two) {
+  const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(__nv_fp8x2_storage_t(two), __NV_E4M3);
+  return uint32_t(h.x) | (uint32_t(h.y) << 16);
+}
+__device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
+  const __half2 v = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+// x = hi + lo as two fp16 pairs.
+__device__ __forceinline__ void split_f16x2(float x0, float x1, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(x0, x1);
+  const float2 f = __half22float2(h);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = pack_f16x2(x0 - f.x, x1 - f.y);
+}
+
+// tmK / tmV: the caches seen as [num_blocks * Hkv * block_size rows, D] bytes, box D columns x min(block_size, 32) rows; rows of 128
+// bytes arrive with the 128-byte swizzle, rows of 64 as they are.
+template <int D>
+__global__ void __launch_bounds__(kPdWarps * 32)
+paged_decode_f8_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+                       const __nv_bfloat16* __restrict__ q, const int* __restrict__ block_tables,
+                       const int* __restrict__ context_lens, float* __restrict__ part, int S, int Hq, int Hkv, int block_size,
+                       int max_blocks, int splits, float scale, float v_scale, int window, int* status) {
+  using Cfg = PdF8Cfg<D>;
+  constexpr int ST = Cfg::kStages;
+  constexpr int KS = D / 16;     // k-steps of the score product
+  constexpr int NU = D / 16;     // 16-byte units of a value row
+  extern __shared__ uint8_t pd_raw[];
+  uint8_t* pd_smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(pd_raw) + 1023) & ~uintptr_t(1023));
+  const int G = Hq / Hkv;
+  const int sp = blockIdx.x % splits;
+  const int hkv = (blockIdx.x / splits) % Hkv;
+  const int s = blockIdx.x / (splits * Hkv);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, qd = lane & 3;
+  uint8_t* my_tiles = pd_smem + warp * Cfg::kWarpBytes;
+  const uint32_t bar0 = smem_u32(pd_smem + Cfg::kOffBar) + warp * ST * 8;
+  __shared__ int abort_s, drain_s;
+  if (threadIdx.x == 0) { abort_s = 0; drain_s = 0; }
+  if (lane == 0) {
+    for (int st = 0; st < ST; ++st) mbar_init(bar0 + 8u * st, 1);
+    fence_barrier_init();
+    fence_proxy_async();
   }
+  // offset of 16-byte unit u of row r inside a tile
+  auto unit = [](int r, int u) { return D == 128 ? r * 128 + ((u ^ (r & 7)) << 4) : r * 64 + (u << 4); };
+  // A fragments of the query block, columns permuted: step kk = 4 h + r takes columns 64 h + 16 qd + 4 r + {0 .. 3}.  Rows = heads of the
+  // group (g and g + 8), zero past G, scaled by a power of two to a largest value in [2^14, 2^15).
+  uint32_t qa[KS][4];
+  float scale_lo, scale_hi;
+  {
+    uint2 raw[2][KS];
+    float top[2] = {0.f, 0.f};
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const bool there = g + 8 * half < G;
+      const __nv_bfloat16* row = q + ((long long)s * Hq + hkv * G + (there ? g + 8 * half : 0)) * D + qd * 16;
+#pragma unroll
+      for (int kk = 0; kk < KS; ++kk) {
+        raw[half][kk] = there ? *reinterpret_cast<const uint2*>(row + (kk >> 2) * 64 + (kk & 3) * 4) : make_uint2(0u, 0u);
+        const float2 a = unpack_bf16x2(raw[half][kk].x), b = unpack_bf16x2(raw[half][kk].y);
+        top[half] = fmaxf(top[half], fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y))));
+      }
+      top[half] = fmaxf(top[half], __shfl_xor_sync(0xffffffffu, top[half], 1));
+      top[half] = fmaxf(top[half], __shfl_xor_sync(0xffffffffu, top[half], 2));
+      // (a row of zeros or with an infinity stays as it is)
+      const int e = top[half] > 0.f && top[half] <= 3.4e38f ? max(-120, min(100, 14 - ilogbf(top[half]))) : 0;
+      const float up = ldexpf(1.f, e);
+      (half ? scale_hi : scale_lo) = scale * ldexpf(1.f, -e);
+#pragma unroll
+      for (int kk = 0; kk < KS; ++kk) {
+        const float2 a = unpack_bf16x2(raw[half][kk].x), b = unpack_bf16x2(raw[half][kk].y);
+        qa[kk][half] = pack_f16x2(a.x * up, a.y * up);
+        qa[kk][2 + half] = pack_f16x2(b.x * up, b.y * up);
+      }
+    }
+  }
+  __syncthreads();
+  volatile int* abort_flag = &abort_s;
+  const int ctx = context_lens[s];
+  const int lo = window > 0 ? max(0, ctx - window) : 0;              // first visible key
+  const int base = lo & ~31;                                         // chunks start on multiples of 32 keys
+  const int per = ((ctx - base + splits - 1) / splits + 31) / 32 * 32;      // whole 32-key chunks per split
+  const int t0 = base + sp * per, t1 = min(ctx, t0 + per);
+  const int* bt = block_tables + (long long)s * max_blocks;
+  const int n_chunks = t1 > t0 ? (t1 - t0 + 31) / 32 : 0;
+  const int my_n = n_chunks > warp ? (n_chunks - warp + kPdWarps - 1) / kPdWarps : 0;   // chunks warp, warp + 4, ...
+  const int run = block_size < 32 ? block_size : 32;                 // rows per tensor copy
+
+  auto request = [&](int i) {
+    const int c0 = t0 + (warp + i * kPdWarps) * 32;
+    const uint32_t bar = bar0 + 8u * (i % ST);
+    const uint32_t kt = smem_u32(my_tiles + (i % ST) * 2 * Cfg::kTileBytes);
+    const int last_row = ((t1 - 1) / block_size + 1) * block_size;   // end of the last block holding a live key
+    const int r_end = min(c0 + 32, last_row);
+    mbar_expect_tx(bar, uint32_t(2 * (r_end - c0) * D));
+    for (int r = c0; r < r_end; r += run) {
+      const int row = (bt[r / block_size] * Hkv + hkv) * block_size + r % block_size;
+      tma_load_2d(kt + (r - c0) * D, &tmK, bar, 0, row);
+      tma_load_2d(kt + Cfg::kTileBytes + (r - c0) * D, &tmV, bar, 0, row);
+    }
+  };
+
+  float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.f, l_hi = 0.f;   // l: this lane's share of the row sums
+  float oacc[NU][2][4];                                               // [unit][even / odd column][fragment]
+#pragma unroll
+  for (int u = 0; u < NU; ++u)
+#pragma unroll
+    for (int r = 0; r < 8; ++r) oacc[u][r >> 2][r & 3] = 0.f;
+
+  if (lane == 0)
+    for (int i = 0; i < ST - 1 && i < my_n; ++i) request(i);
+  bool ok = true;
+  const int lj = lane >> 3, lr = lane & 7;   // ldmatrix: this lane addresses row lr of matrix lj
+  for (int i = 0; i < my_n; ++i) {
+    if (lane == 0 && i + ST - 1 < my_n) request(i + ST - 1);      // its stage was consumed in iteration i - 1
+    ok = __all_sync(0xffffffffu, mbar_wait(bar0 + 8u * (i % ST), uint32_t(i / ST) & 1u, abort_flag, status, kStatusTimeoutFull));
+    if (!ok) {
+      // a copy never arrived: give the other requested stages one more bounded wait each, so that no copy of this
+      // warp is still writing shared memory when the CTA leaves, then drop out (the result of the CTA is discarded)
+      for (int r = i + 1; r < my_n && r < i + ST; ++r)
+        mbar_wait(bar0 + 8u * (r % ST), uint32_t(r / ST) & 1u, &drain_s, status, kStatusTimeoutFull);
+      break;
+    }
+    const int c0 = t0 + (warp + i * kPdWarps) * 32;
+    uint8_t* kt = my_tiles + (i % ST) * 2 * Cfg::kTileBytes;
+    uint8_t* vt = kt + Cfg::kTileBytes;
+    const uint32_t vt_addr = smem_u32(vt);
+    const int nk = min(32, t1 - c0);
+    if (nk < 32 || c0 < lo) {
+      // rows past the context or before the window may hold anything: zero them in V so that their zero weights do not meet a NaN
+      if (lane >= nk || c0 + lane < lo) {
+#pragma unroll
+        for (int u = 0; u < NU; ++u) *reinterpret_cast<uint4*>(vt + lane * D + u * 16) = make_uint4(0u, 0u, 0u, 0u);
+      }
+      __syncwarp();
+    }
+    // ---- S = Q K^T: four blocks of 8 keys
+    float sacc[4][4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+#pragma unroll
+      for (int r = 0; r < 4; ++r) sacc[t][r] = 0.f;
+#pragma unroll
+      for (int h = 0; h < D / 64; ++h) {
+        const uint4 w = *reinterpret_cast<const uint4*>(kt + unit(t * 8 + g, h * 4 + qd));
+        const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          mma_f16_16816(sacc[t], qa[h * 4 + r], e4m3x2_to_f16x2(ww[r] & 0xffffu), e4m3x2_to_f16x2(ww[r] >> 16));
+      }
+    }
+    // ---- online softmax: this lane holds columns t * 8 + qd * 2 + {0, 1} of rows g (registers 0, 1) and g + 8 (2, 3)
+    float mx_lo = -INFINITY, mx_hi = -INFINITY;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int col = t * 8 + qd * 2 + e;
+        const bool live = col < nk && c0 + col >= lo;
+        sacc[t][e] = live ? sacc[t][e] * scale_lo : -INFINITY;
+        sacc[t][2 + e] = live ? sacc[t][2 + e] * scale_hi : -INFINITY;
+        mx_lo = fmaxf(mx_lo, sacc[t][e]);
+        mx_hi = fmaxf(mx_hi, sacc[t][2 + e]);
+      }
+    }
+    mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 1));
+    mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 2));
+    mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1));
+    mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
+    const float nm_lo = fmaxf(m_lo, mx_lo), nm_hi = fmaxf(m_hi, mx_hi);
+    const float a_lo = (m_lo == -INFINITY) ? 0.f : __expf(m_lo - nm_lo);
+    const float a_hi = (m_hi == -INFINITY) ? 0.f : __expf(m_hi - nm_hi);
+    m_lo = nm_lo; m_hi = nm_hi;
+    float ps_lo = 0.f, ps_hi = 0.f;
+    uint32_t ph[2][4], pl[2][4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const float p0 = __expf(sacc[t][0] - nm_lo), p1 = __expf(sacc[t][1] - nm_lo);
+      const float p2 = __expf(sacc[t][2] - nm_hi), p3 = __expf(sacc[t][3] - nm_hi);
+      ps_lo += p0 + p1;
+      ps_hi += p2 + p3;
+      const int at = (t & 1) * 2;                            // keys 16 ks + 8 (t & 1) + ..: registers 0 / 2 rows g, 1 / 3 rows g + 8
+      split_f16x2(p0 * kPdWeightScale, p1 * kPdWeightScale, ph[t >> 1][at], pl[t >> 1][at]);
+      split_f16x2(p2 * kPdWeightScale, p3 * kPdWeightScale, ph[t >> 1][at + 1], pl[t >> 1][at + 1]);
+    }
+    l_lo = l_lo * a_lo + ps_lo;
+    l_hi = l_hi * a_hi + ps_hi;
+#pragma unroll
+    for (int u = 0; u < NU; ++u)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        oacc[u][e][0] *= a_lo; oacc[u][e][1] *= a_lo;
+        oacc[u][e][2] *= a_hi; oacc[u][e][3] *= a_hi;
+      }
+    // ---- O += P V: two steps of 16 keys
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks) {
+      const int key = ks * 16 + (lj & 1) * 8 + lr;
+#pragma unroll
+      for (int u2 = 0; u2 < NU / 2; ++u2) {
+        uint32_t b[2][2];                                    // [unit][keys 0 .. 7 / 8 .. 15 of the step]
+        ldsm_x4_trans(vt_addr + unit(key, u2 * 2 + (lj >> 1)), b[0][0], b[0][1], b[1][0], b[1][1]);
+#pragma unroll
+        for (int uu = 0; uu < 2; ++uu) {
+          uint32_t ev[2], od[2];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const uint32_t ka = e4m3x2_to_f16x2(b[uu][h] & 0xffffu), kb = e4m3x2_to_f16x2(b[uu][h] >> 16);
+            ev[h] = __byte_perm(ka, kb, 0x5410);
+            od[h] = __byte_perm(ka, kb, 0x7632);
+          }
+          mma_f16_16816(oacc[u2 * 2 + uu][0], ph[ks], ev[0], ev[1]);
+          mma_f16_16816(oacc[u2 * 2 + uu][1], ph[ks], od[0], od[1]);
+          mma_f16_16816(oacc[u2 * 2 + uu][0], pl[ks], ev[0], ev[1]);
+          mma_f16_16816(oacc[u2 * 2 + uu][1], pl[ks], od[0], od[1]);
+        }
+      }
+    }
+    __syncwarp();            // every lane is done with this stage before lane 0 requests into it again
+  }
+  float* red_o = pd_row_sums(pd_smem, warp, lane, ok, m_lo, m_hi, l_lo, l_hi);
+#pragma unroll
+  for (int u = 0; u < NU; ++u) {
+    float* at = red_o + (warp * kPdMmaMaxG + g) * D + u * 16 + qd * 4;
+    *reinterpret_cast<float4*>(at) = make_float4(oacc[u][0][0], oacc[u][1][0], oacc[u][0][1], oacc[u][1][1]);
+    *reinterpret_cast<float4*>(at + 8 * D) = make_float4(oacc[u][0][2], oacc[u][1][2], oacc[u][0][3], oacc[u][1][3]);
+  }
+  pd_write_partial<D>(pd_smem, part + ((long long)s * Hq + hkv * G) * splits * (D + 2), G, splits, sp, v_scale / kPdWeightScale);
 }
 
 template <int D>
@@ -662,24 +935,28 @@ int lt_paged_decode_window(const void* q, const void* k_cache, const void* v_cac
   const int G = Hq / Hkv;
   const bool bs_ok = block_size > 0 && (32 % block_size == 0 || block_size % 32 == 0);
   const bool aligned = (reinterpret_cast<uintptr_t>(k_cache) & 15) == 0 && (reinterpret_cast<uintptr_t>(v_cache) & 15) == 0;
-  if (!kv_fp8 && G <= kPdMmaMaxG && bs_ok && block_size % 8 == 0 && num_blocks > 0 && aligned &&
-      (long long)num_blocks * Hkv * block_size < (1ll << 31)) {
-    // bf16 caches in blocks of 8 keys or more: tiles by TMA in the swizzled layout, scores and P V on mma.sync
+  if (G <= kPdMmaMaxG && bs_ok && block_size % 8 == 0 && num_blocks > 0 && aligned && (long long)num_blocks * Hkv * block_size < (1ll << 31)) {
+    // caches in blocks of 8 keys or more: tiles by TMA, scores and P V on mma.sync
     const int ctas = S * Hkv * splits;
+    const uint64_t rows = uint64_t(num_blocks) * Hkv * block_size;
+    const uint32_t run = block_size < 32 ? block_size : 32;
+    const int bytes = kv_fp8 ? 1 : 2;
+    CUtensorMap tmK, tmV;
+    int r = encode_tmap_2d(&tmK, k_cache, bytes, D, rows, uint64_t(D) * bytes, kv_fp8 ? D : 64, run, !kv_fp8 || D == 128);
+    if (r == 0) r = encode_tmap_2d(&tmV, v_cache, bytes, D, rows, uint64_t(D) * bytes, kv_fp8 ? D : 64, run, !kv_fp8 || D == 128);
+    if (r) return r > 0 ? 1000 + r : r;
+    int* status = device_status_word();
     static bool configured_mma = false;
     if (!configured_mma) {
+      LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_f8_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdF8Cfg<64>::kSmemBytes));
+      LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_f8_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdF8Cfg<128>::kSmemBytes));
       LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdMmaCfg<64>::kSmemBytes));
       LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdMmaCfg<128>::kSmemBytes));
       configured_mma = true;
     }
-    const uint64_t rows = uint64_t(num_blocks) * Hkv * block_size;
-    const uint32_t run = block_size < 32 ? block_size : 32;
-    CUtensorMap tmK, tmV;
-    int r = encode_tmap_2d(&tmK, k_cache, 2, D, rows, uint64_t(D) * 2, 64, run, 1);
-    if (r == 0) r = encode_tmap_2d(&tmV, v_cache, 2, D, rows, uint64_t(D) * 2, 64, run, 1);
-    if (r) return r > 0 ? 1000 + r : r;
-    int* status = device_status_word();
-    if (D == 64) paged_decode_mma_kernel<64><<<ctas, kPdWarps * 32, PdMmaCfg<64>::kSmemBytes, st>>>(tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale, window, status);
+    if (kv_fp8 && D == 64) paged_decode_f8_kernel<64><<<ctas, kPdWarps * 32, PdF8Cfg<64>::kSmemBytes, st>>>(tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale * k_scale, v_scale, window, status);
+    else if (kv_fp8) paged_decode_f8_kernel<128><<<ctas, kPdWarps * 32, PdF8Cfg<128>::kSmemBytes, st>>>(tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale * k_scale, v_scale, window, status);
+    else if (D == 64) paged_decode_mma_kernel<64><<<ctas, kPdWarps * 32, PdMmaCfg<64>::kSmemBytes, st>>>(tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale, window, status);
     else paged_decode_mma_kernel<128><<<ctas, kPdWarps * 32, PdMmaCfg<128>::kSmemBytes, st>>>(tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale, window, status);
   } else if (!kv_fp8 && window == 0 && G <= kPdMaxG && bs_ok && (reinterpret_cast<uintptr_t>(k_cache) & 15) == 0 && (reinterpret_cast<uintptr_t>(v_cache) & 15) == 0) {
     // bf16 caches: every K / V byte is read once for the whole group of query heads, through a shared-memory pipeline

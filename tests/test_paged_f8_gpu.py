@@ -1,0 +1,72 @@
+"""Decode attention over e4m3 caches on the tensor-core kernel, against 64-bit arithmetic over sizes at the edges of its chunks, copies,
+groups and splits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def reference(q, kc, vc, tables, ctx, bs, scale, ks, vs, window):
+    S, H, D = q.shape
+    G = kc.shape[1]
+    out = torch.zeros(S, H, D, dtype=torch.float64, device=q.device)
+    for s in range(S):
+        n = int(ctx[s])
+        lo = max(0, n - window) if window else 0
+        if n == lo:
+            continue
+        at = torch.arange(lo, n, device=q.device)
+        k = kc[tables[s].long()[at // bs], :, at % bs].double() * ks                 # [keys, G, D]
+        v = vc[tables[s].long()[at // bs], :, at % bs].double() * vs
+        k, v = k.repeat_interleave(H // G, 1), v.repeat_interleave(H // G, 1)
+        p = torch.softmax(torch.einsum("hd,khd->hk", q[s].double(), k) * scale, -1)
+        out[s] = torch.einsum("hk,khd->hd", p, v)
+    return out
+
+
+@pytest.mark.parametrize("D,H,G,bs,window,contexts,splits", [
+    (64, 8, 8, 8, 0, [1, 31, 32, 33], 1),
+    (128, 8, 2, 16, 0, [1, 127, 128, 129, 1000], 3),
+    (128, 32, 2, 32, 0, [4095, 17], 8),                  # 16 query heads to a key head
+    (64, 12, 4, 64, 0, [63, 64, 65, 700], 2),            # blocks longer than a chunk, 3 heads to a key head
+    (128, 16, 4, 16, 100, [5, 99, 100, 101, 131, 2000], 4),
+    (64, 4, 4, 16, 33, [32, 33, 34, 500], 1),
+])
+def test_e4m3_decode_against_64_bits(D, H, G, bs, window, contexts, splits):
+    from litetorch_b200.ops import kernels as K
+    torch.manual_seed(D + H + bs)
+    S, ks, vs = len(contexts), 0.05, 0.07
+    width = (max(contexts) + bs - 1) // bs + 1
+    n_blocks = S * width
+    kc, vc = (torch.randn(n_blocks, G, bs, D, device="cuda").mul_(20).to(torch.float8_e4m3fn) for _ in range(2))
+    tables = torch.randperm(n_blocks, device="cuda").int().view(S, width).contiguous()
+    q = torch.randn(S, H, D, device="cuda").to(torch.bfloat16)
+    q[0, 0] *= 1e-6                                       # a head far below fp16's range as it stands, and one above it
+    q[0, -1] *= 1e6
+    ctx = torch.tensor(contexts, dtype=torch.int32, device="cuda")
+    # what lies past a sequence's end, or before its window, must not matter
+    for s, n in enumerate(contexts):
+        rows = list(range(n, width * bs)) + (list(range(0, n - window)) if window else [])
+        for r in rows:
+            for t in (kc, vc):
+                t.view(torch.uint8)[tables[s, r // bs].long(), :, r % bs] = 0x7F      # NaN
+    out = K.paged_decode(q, kc, vc, tables, ctx, bs, splits, D ** -0.5, ks, vs, window=window)
+    ref = reference(q, kc, vc, tables, ctx, bs, D ** -0.5, ks, vs, window)
+    assert torch.isfinite(out).all()
+    # the result is rounded to bf16 (2^-9); scores of the row times 1e6 are in the millions, where 32-bit products are off by up to
+    # 2^-24 of them times the length of the dot product, so that row may weigh two keys of nearly equal score differently: left out
+    keep = torch.ones(S, H, dtype=torch.bool, device="cuda")
+    keep[0, -1] = False
+    err = (out.double() - ref)[keep].abs().max()
+    assert err <= 2 ** -8 * ref[keep].abs().max(), float(err)
+    assert K.status_fetch() == 0
+
+
+def test_e4m3_decode_propagates_nan_keys():
+    """A NaN inside the context is not hidden by the conversion of 8-bit values."""
+    from litetorch_b200.ops import kernels as K
+    kc, vc = (torch.randn(4, 1, 16, 64, device="cuda").to(torch.float8_e4m3fn) for _ in range(2))
+    vc.view(torch.uint8)[1, 0, 3, 5] = 0x7F
+    q = torch.randn(1, 2, 64, device="cuda").to(torch.bfloat16)
+    out = K.paged_decode(q, kc, vc, torch.arange(4, device="cuda").int().view(1, 4), torch.tensor([60], dtype=torch.int32, device="cuda"), 16, 1, 0.125)
+    assert torch.isnan(out[0, :, 5]).all() and torch.isfinite(out[0, :, 6]).all()
