@@ -61,6 +61,18 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
 
+// True in one lane of a converged warp.  Code behind it is known to the compiler to run in a single thread, so that operands of
+// tcgen05 and TMA instructions stay in uniform registers; behind `lane == 0` each is moved there first.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t on;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(on));
+  return on != 0;
+}
+
 // ----------------------------------------------------------------------------------------------
 // mbarrier
 // ----------------------------------------------------------------------------------------------

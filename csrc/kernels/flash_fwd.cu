@@ -4,27 +4,42 @@
 // buffers), runs a row-softmax kernel and a second batched GEMM, has no causal mask and ignores the number
 // of KV heads (src/backend/gpu_native/nn/flash_attention.cu:188-299).  This kernel never leaves the chip:
 //
-//   warp 0    TMA producer: Q tile once, K/V tiles double-buffered (128-byte swizzle, mbarrier tx)
-//   warp 1    MMA issuer:   S_j = Q K_j^T  (tcgen05.mma, 128x128xD, S double-buffered in TMEM)
-//                           O  += P_j V_j  (A = P_j from shared memory, B = V_j as an N-major operand)
-//   warps 2-5 softmax:      one query row per thread (TMEM lane = row): tcgen05.ld S, online max / sum in
-//                           the exp2 domain, P_j written to shared memory in the swizzled operand layout.
+//   warp 0    TMA producer: Q tile once, K and V blocks through one ring (128-byte swizzle, mbarrier tx)
+//   warp 1    MMA issuer:   S_j = Q K_j^T  (tcgen05.mma, scores of block j + 1 issued before the softmax of block j is done)
+//                           O  += P_j V_j  (A = P_j from tensor memory, B = V_j as an N-major operand)
+//   warps 2-5 softmax:      one query row per thread (TMEM lane = row): tcgen05.ld of the whole row into registers, maximum,
+//                           exponentials, P_j as bf16 back into tensor memory.
 // The running maximum is updated lazily: O in TMEM is rescaled only when a row's maximum grew by more
 // than 2^8, which keeps exp2 arguments bounded and makes the rescale (tcgen05.ld/st of O) rare.
-// Query / key size D and value size DV may differ, and KV blocks may be 64 keys where a 128-key block of the larger size does
-// not fit in shared memory.  SHARED: the last 64 columns of a key are the same for all heads (a rotated part beside the
+//
+// What bounds it: the exponentials, 16 a clock and SM (1024 clocks for 128 x 128 scores against 256 (D 64) or 512 (D 128) of MMA), and
+// the softmax warps' waits around them.  So a CTA has a single query tile and half of an SM's tensor memory, shared memory and
+// registers: two CTAs run side by side, one's exponentials under the other's loads, waits, start and end.  (Two tiles in one CTA, as
+// two heads of a KV head, read K and V half as often but were slower or equal: 168 against 146 us for D 64, 4 x 2048 tokens, 32
+// heads, and 56 against 33 us where their fewer CTAs end in an empty wave.)  Scores are read from tensor memory once, P never
+// goes through shared memory, scale, sum and conversion work on pairs, and the body for blocks that every row sees whole
+// holds no tests: with a test per score, most of the time went into branches and instruction fetches.
+// Measured against the kernel before it (four softmax warps to either parity of key blocks, P through shared memory, one CTA an SM), causal,
+// 32 heads, L2 flushed: D 64, 4 x 2048 tokens 363 -> 136 us; D 64, 4096 tokens 299 -> 122; D 128, 8192 tokens 1177 -> 474 (1160 TFLOP/s);
+// D 128, 1337 queries on 5437 keys 301 -> 155.  Left: 1.3 to 1.5 times the exponentials' time in the loop, and 3 to 5 us a CTA of
+// start, masked blocks and end.
+// Query / key size D and value size DV may differ.  SHARED: the last 64 columns of a key are the same for all heads (a rotated part beside the
 // heads' own unrotated ones) and come from a tensor of their own, so that keys are never put together in memory.
 // Output: O [B, Tq, Hq, D] bf16 and the natural-log LSE [B, Hq, Tq] fp32 for the backward pass.
 #include "lt_cuda.h"
 #include "common/host.h"
 #include "common/ptx.cuh"
 
+#include <type_traits>
+
 namespace lt {
 
 constexpr int kFaBlockQ = 128;
-constexpr int kFaBlockKV = 128;
-constexpr int kFaThreads = 352;          // warp 0 producer, warp 1 PV MMA issuer, warps 2-9 softmax, warp 10 score MMA issuer
-constexpr int kFaSoftmaxThreads = 256;   // two warps per TMEM lane quarter, 64 score columns each
+constexpr int kFaShardRows = 128;        // context-parallel shards are whole numbers of query tiles and key blocks
+constexpr int kFaThreads = 192;          // warp 0 producer, warp 1 MMA issuer, warps 2-5 softmax
+// Keys of a block: two score buffers of 64 columns leave room for 128 columns of O.  With O of 64 columns one buffer of 128 beside
+// its weights fits, and larger blocks wait less often.
+constexpr int fa_block_kv(int dv) { return dv == 64 ? 128 : 64; }
 
 struct FlashFwdParams {
   __nv_bfloat16* O;
@@ -59,61 +74,73 @@ __device__ __forceinline__ float ex2_approx_f(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float y;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  return y;
+}
+// Two floats in a register pair; one instruction works on both.
+__device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
+  uint64_t y;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(a), "f"(b));
+  return y;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t x, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x));
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t y;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(y) : "l"(a), "l"(b), "l"(c));
+  return y;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+  uint64_t y;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(y) : "l"(a), "l"(b));
+  return y;
+}
 
+// Shared memory: the query tile, then a ring that K and V blocks go through in turn.
 template <int D, int DV, int BKV>
 struct FaFwdCfg {
   static constexpr int kQBytes = kFaBlockQ * D * 2;
   static constexpr int kKBytes = BKV * D * 2;
   static constexpr int kVBytes = BKV * DV * 2;
-  static constexpr int kPBytes = kFaBlockQ * BKV * 2;
-  static constexpr int kOffQ = 0;
-  static constexpr int kOffK = kQBytes;
-  static constexpr int kOffV = kOffK + 2 * kKBytes;
-  static constexpr int kOffP = kOffV + 2 * kVBytes;
-  static constexpr int kOffBar = kOffP + 2 * kPBytes;
-  static constexpr int kOffSeg = kOffBar + 224;               // KvSeg table (16 entries) + block count
-  static constexpr int kOffX = kOffSeg + kFaMaxSegs * 16 + 16;                 // row statistics exchanged between the two column halves
-  static constexpr int kNeeded = kOffX + 2 * 2 * 128 * 4;     // [parity][half][128] floats
-  // 1 KB of slack for the 1024-byte alignment where it fits under the 227 KB limit; the kernel checks at run time
-  // that the aligned layout lies inside the allocation and reports kStatusBadArgument otherwise.
-  static constexpr int kSmemBytes = (kNeeded + 1024 <= 232448) ? kNeeded + 1024 : 232448;
-  static constexpr int kTmemCols = 512;
-  // Score buffers of BKV columns beside the two output accumulators: three where tensor memory has room (head_dim 64, or
-  // 64-key blocks), so that S of block j+2 is computed while the softmax of blocks j and j+1 is still reading theirs; else two.
-  static constexpr int kSBufs = (512 - 2 * DV) / BKV < 3 ? (512 - 2 * DV) / BKV : 3;
-  static constexpr int kColS = 0;
-  static constexpr int kColO = kSBufs * BKV;   // two accumulators of DV columns (KV blocks of even / odd index)
-  static_assert(kNeeded <= 232448 && kSBufs >= 2, "does not fit");
+  static constexpr int kSlotBytes = kKBytes > kVBytes ? kKBytes : kVBytes;
+  static constexpr int kFit = (113 * 1024 - 2560 - kQBytes) / kSlotBytes;     // two CTAs share an SM
+  static constexpr int kSlots = kFit < 4 ? kFit : 4;
+  static constexpr int kOffRing = kQBytes;
+  static constexpr int kOffBar = kOffRing + kSlots * kSlotBytes;
+  static constexpr int kOffSeg = kOffBar + 160;                               // KvSeg table (16 entries) + block count
+  static constexpr int kSmemBytes = kOffSeg + kFaMaxSegs * 16 + 16 + 1024;    // 1 KB for the 1024-byte alignment
+  // 256 columns of tensor memory.  With 64-key blocks two score buffers fit beside O; the softmax weights P (two bf16 a column)
+  // go over their own scores, which the threads have in registers by then, and the next scores into the other buffer.  With
+  // 128-key blocks (head size 64) P has columns of its own, and the next scores are made as soon as these have been read.
+  static constexpr bool kTwoS = 2 * BKV + DV <= 256;
+  static constexpr int kColP = kTwoS ? 0 : BKV;      // from the score buffer's first column
+  static constexpr int kColO = 256 - DV;
+  static constexpr int kTmemCols = 256;
+  static_assert(kSlots >= 2 && (kTwoS || BKV + BKV / 2 + DV <= 256), "does not fit");
 };
 
 template <int D, int DV, int BKV, bool SHARED>
-__global__ void __launch_bounds__(kFaThreads, 1)
+__global__ void __launch_bounds__(kFaThreads, 2)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ KvMaps maps, const FlashFwdParams p) {
   using Cfg = FaFwdCfg<D, DV, BKV>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t sbase = smem_u32(smem);
-  if (int(smem - smem_raw) + Cfg::kNeeded > Cfg::kSmemBytes) {  // uniform for the whole grid
-    if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, int(kStatusBadArgument));
-    return;
-  }
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kOffBar);
   const uint32_t bb = smem_u32(bars);
-  // barrier map
   const uint32_t q_full = bb;
-  auto k_full = [&](int s) { return bb + 8u * (1 + s); };
-  auto v_full = [&](int s) { return bb + 8u * (3 + s); };
-  auto k_empty = [&](int s) { return bb + 8u * (5 + s); };
-  auto v_empty = [&](int s) { return bb + 8u * (7 + s); };
-  auto s_full = [&](int s) { return bb + 8u * (9 + s); };    // up to three
-  auto p_full = [&](int s) { return bb + 8u * (12 + s); };
-  auto p_empty = [&](int s) { return bb + 8u * (14 + s); };
-  const uint32_t o_full = bb + 8u * 16;
-  // x_bar(quarter): both warps of a TMEM lane quarter have published their partial row statistics
-  auto x_bar = [&](int qtr) { return bb + 8u * (17 + qtr); };
-  auto s_free = [&](int sb) { return bb + 8u * (21 + sb); };   // the group's four warps have read score buffer sb
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 24);
-  float* xmax = reinterpret_cast<float*>(smem + Cfg::kOffX);  // [2 (rendezvous parity)][2 (half)][128]
+  auto full = [&](int i) { return bb + 8u * (1 + i); };      // ring slots, up to four
+  auto empty = [&](int i) { return bb + 8u * (5 + i); };
+  // One barrier for blocks of either parity: with two score buffers the softmax and the MMA issuer may be a block ahead of each
+  // other, and a phase bit tells only neighbouring phases of one barrier apart.
+  auto s_full = [&](int j) { return bb + 8u * (9 + (j & 1)); };    // scores of block j are in tensor memory
+  auto p_full = [&](int j) { return bb + 8u * (11 + (j & 1)); };   // its softmax weights are
+  auto o_full = [&](int j) { return bb + 8u * (13 + (j & 1)); };   // its PV product has been added
+  const uint32_t s_free = bb + 8u * 15;                            // scores have been read (only where P has columns of its own)
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -175,28 +202,14 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
     for (int i = ns; i < kFaMaxSegs; ++i) segs[i] = KvSeg{0, 0, 0, 0};
     *n_blocks_s = total;
-  }
-  __syncthreads();
-  const int n_blocks = *n_blocks_s;
-  // block j of the schedule -> (owner rank, first local key row, global position of its first key)
-  auto locate = [&](int j, int& owner, int& kv0, int& kbase) {
-    int sidx = 0;
-    while (sidx < kFaMaxSegs - 1 && j >= segs[sidx].n) { j -= segs[sidx].n; ++sidx; }
-    owner = segs[sidx].owner;
-    kv0 = segs[sidx].kv0 + j * BKV;
-    kbase = segs[sidx].kbase + j * BKV;
-  };
-
-  if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(k_full(s), 1); mbar_init(v_full(s), 1);
-      mbar_init(k_empty(s), 1); mbar_init(v_empty(s), 1);
-      mbar_init(p_full(s), kFaSoftmaxThreads / 64); mbar_init(p_empty(s), 1);
+    for (int j = 0; j < 2; ++j) {
+      mbar_init(s_full(j), 1);
+      mbar_init(p_full(j), 4);
+      mbar_init(o_full(j), 1);
     }
-    for (int s = 0; s < Cfg::kSBufs; ++s) { mbar_init(s_full(s), 1); mbar_init(s_free(s), kFaSoftmaxThreads / 64); }
-    mbar_init(o_full, 1);
-    for (int qtr = 0; qtr < 4; ++qtr) mbar_init(x_bar(qtr), 2);
+    mbar_init(s_free, 4);
+    for (int i = 0; i < Cfg::kSlots; ++i) { mbar_init(full(i), 1); mbar_init(empty(i), 1); }
     *abort_flag = 0;
     fence_barrier_init();
     fence_proxy_async();
@@ -210,186 +223,184 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  const int n_blocks = *n_blocks_s;
+  // block j of the schedule -> (owner rank, first local key row, global position of its first key)
+  auto locate = [&](int j, int& owner, int& kv0, int& kbase) {
+    int sidx = 0;
+    if (p.cp_world > 1)
+      while (sidx < kFaMaxSegs - 1 && j >= segs[sidx].n) { j -= segs[sidx].n; ++sidx; }
+    owner = segs[sidx].owner;
+    kv0 = segs[sidx].kv0 + j * BKV;
+    kbase = segs[sidx].kbase + j * BKV;
+  };
+  // K and V blocks in the order in which they go through the ring: K0, K1, V0, K2, V1, ...
+  auto k_seq = [](int j) { return j == 0 ? 0 : 2 * j - 1; };
+  auto v_seq = [&](int j) { return j + 1 < n_blocks ? 2 * j + 2 : 2 * j + 1; };
 
   if (warp == 0) {
     // ---------------------------------------------------------------- producer
-    if (lane == 0 && n_blocks > 0) {
-      mbar_expect_tx(q_full, Cfg::kQBytes);
-#pragma unroll
-      for (int c = 0; c < D / 64; ++c)
-        tma_load_4d(sbase + Cfg::kOffQ + c * (kFaBlockQ * 128), &tmQ, q_full, c * 64, h, q0, b);
-      // K runs one block ahead of V: the wait for a free V stage (the PV product two blocks back) must not hold up
-      // the K tile that the next score product needs.
-      auto load_k = [&](int j) -> bool {
-        const int s = j & 1;
+    if (n_blocks > 0 && elect_one()) {
+      auto load = [&](int i, int j, bool is_k) -> bool {
+        const int s = i % Cfg::kSlots;
         int owner, kv0, kbase;
         locate(j, owner, kv0, kbase);
-        if (!mbar_wait(k_empty(s), ((j >> 1) & 1) ^ 1u, abort_flag, p.status, kStatusTimeoutEmpty)) return false;
-        mbar_expect_tx(k_full(s), Cfg::kKBytes);
+        if (!mbar_wait(empty(s), (uint32_t(i / Cfg::kSlots) & 1u) ^ 1u, abort_flag, p.status, kStatusTimeoutEmpty)) return false;
+        const uint32_t dst = sbase + Cfg::kOffRing + s * Cfg::kSlotBytes;
+        mbar_expect_tx(full(s), is_k ? Cfg::kKBytes : Cfg::kVBytes);
+        if (is_k) {
 #pragma unroll
-        for (int c = 0; c < D / 64; ++c)
-          if (SHARED && c == D / 64 - 1)
-            tma_load_4d(sbase + Cfg::kOffK + s * Cfg::kKBytes + c * (BKV * 128), &maps.k[1], k_full(s), 0, 0, kv0, b);
-          else
-            tma_load_4d(sbase + Cfg::kOffK + s * Cfg::kKBytes + c * (BKV * 128), &maps.k[owner], k_full(s), c * 64, hkv, kv0, b);
+          for (int c = 0; c < D / 64; ++c)
+            if (SHARED && c == D / 64 - 1)
+              tma_load_4d(dst + c * (BKV * 128), &maps.k[1], full(s), 0, 0, kv0, b);
+            else
+              tma_load_4d(dst + c * (BKV * 128), &maps.k[owner], full(s), c * 64, hkv, kv0, b);
+        } else {
+#pragma unroll
+          for (int c = 0; c < DV / 64; ++c) tma_load_4d(dst + c * (BKV * 128), &maps.v[owner], full(s), c * 64, hkv, kv0, b);
+        }
         return true;
       };
-      bool okp = load_k(0);
-      for (int j = 0; okp && j < n_blocks; ++j) {
-        if (j + 1 < n_blocks && !load_k(j + 1)) break;
-        const int s = j & 1;
-        int owner, kv0, kbase;
-        locate(j, owner, kv0, kbase);
-        if (!mbar_wait(v_empty(s), ((j >> 1) & 1) ^ 1u, abort_flag, p.status, kStatusTimeoutEmpty)) break;
-        mbar_expect_tx(v_full(s), Cfg::kVBytes);
+      mbar_expect_tx(q_full, Cfg::kQBytes);
 #pragma unroll
-        for (int c = 0; c < DV / 64; ++c)
-          tma_load_4d(sbase + Cfg::kOffV + s * Cfg::kVBytes + c * (BKV * 128), &maps.v[owner], v_full(s), c * 64, hkv,
-                      kv0, b);
+      for (int c = 0; c < D / 64; ++c) tma_load_4d(sbase + c * (kFaBlockQ * 128), &tmQ, q_full, c * 64, h, q0, b);
+      bool ok = load(0, 0, true);
+      for (int j = 0; ok && j < n_blocks; ++j) {
+        if (j + 1 < n_blocks) ok = load(k_seq(j + 1), j + 1, true);
+        ok = ok && load(v_seq(j), j, false);
       }
     }
-  } else if (warp == 10) {
-    // ---------------------------------------------------------------- score MMA issuer (S = Q K^T)
-    // Issuing a tcgen05.mma costs its thread on the order of a hundred cycles whatever the tile width, so the twelve
-    // MMAs of a KV block are split over two issuing threads: this one runs the score products as far ahead as the
-    // score buffers allow, warp 1 runs the PV products.
-    if (lane == 0 && n_blocks > 0) {
+  } else if (warp == 1) {
+    // ---------------------------------------------------------------- MMA issuer: S = Q K^T, O += P V
+    if (n_blocks > 0 && elect_one()) {
       constexpr uint32_t idesc_s = make_idesc_f16(kFaBlockQ, BKV, 1, 0, 0);
-      const uint64_t q_desc = make_smem_desc_sw128(sbase + Cfg::kOffQ, 16, 1024);
-      const uint64_t k_desc0 = make_smem_desc_sw128(sbase + Cfg::kOffK, 16, 1024);
-      const uint64_t k_desc1 = make_smem_desc_sw128(sbase + Cfg::kOffK + Cfg::kKBytes, 16, 1024);
-      bool ok = mbar_wait(q_full, 0, abort_flag, p.status, kStatusTimeoutFull);
-      for (int j = 0; ok && j < n_blocks; ++j) {
-        const int s = j & 1;                 // K stage
-        const int sb = j % Cfg::kSBufs;      // score buffer, last read by the softmax of block j - kSBufs
-        if (!mbar_wait(k_full(s), (j >> 1) & 1, abort_flag, p.status, kStatusTimeoutFull)) break;
-        if (j >= Cfg::kSBufs &&
-            !mbar_wait(s_free(sb), uint32_t(j / Cfg::kSBufs - 1) & 1u, abort_flag, p.status, kStatusTimeoutTmemEmpty)) break;
-        tc_fence_after();
-        const uint64_t kd = s ? k_desc1 : k_desc0;
-        const uint32_t d_s = tmem_base + Cfg::kColS + sb * BKV;
+      constexpr uint32_t idesc_o = make_idesc_f16(kFaBlockQ, DV, 1, 0, 1);
+      auto wait_ring = [&](int i) {
+        return mbar_wait(full(i % Cfg::kSlots), uint32_t(i / Cfg::kSlots) & 1u, abort_flag, p.status, kStatusTimeoutFull);
+      };
+      const uint64_t q_desc = make_smem_desc_sw128(sbase, 16, 1024);
+      const uint64_t k_desc = make_smem_desc_sw128(sbase + Cfg::kOffRing, 16, 1024);
+      const uint64_t v_desc = make_smem_desc_sw128(sbase + Cfg::kOffRing, BKV * 128, 1024);
+      auto scores = [&](int j) {
+        const int slot = k_seq(j) % Cfg::kSlots;
+        const uint64_t kd = k_desc + uint64_t(slot * (Cfg::kSlotBytes >> 4));
+        const uint32_t d = tmem_base + (Cfg::kTwoS ? (j & 1) * BKV : 0);
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
           const uint64_t q_off = uint64_t(((k / 4) * (kFaBlockQ * 128) + (k % 4) * 32) >> 4);   // 16-byte units
           const uint64_t k_off = uint64_t(((k / 4) * (BKV * 128) + (k % 4) * 32) >> 4);
-          umma_f16_ss(d_s, q_desc + q_off, kd + k_off, idesc_s, k > 0 ? 1u : 0u);
+          umma_f16_ss(d, q_desc + q_off, kd + k_off, idesc_s, k > 0 ? 1u : 0u);
         }
-        umma_commit(k_empty(s));
-        umma_commit(s_full(sb));
-      }
-    }
-  } else if (warp == 1) {
-    // ---------------------------------------------------------------- PV MMA issuer (O_g += P V)
-    if (lane == 0 && n_blocks > 0) {
-      constexpr uint32_t idesc_o = make_idesc_f16(kFaBlockQ, DV, 1, 0, 1);
-      uint64_t v_desc[2], p_desc[2];
+        umma_commit(s_full(j));
+        umma_commit(empty(slot));
+      };
+      auto values = [&](int j) {
+        const int slot = v_seq(j) % Cfg::kSlots;
+        const uint64_t vd = v_desc + uint64_t(slot * (Cfg::kSlotBytes >> 4));
+        const uint32_t a = tmem_base + (Cfg::kTwoS ? (j & 1) * BKV : 0) + Cfg::kColP;
 #pragma unroll
-      for (int st = 0; st < 2; ++st) {
-        v_desc[st] = make_smem_desc_sw128(sbase + Cfg::kOffV + st * Cfg::kVBytes, BKV * 128, 1024);
-        p_desc[st] = make_smem_desc_sw128(sbase + Cfg::kOffP + st * Cfg::kPBytes, 16, 1024);
-      }
-      const bool trm = p.trace != nullptr && blockIdx.z == 0 && h == 0 && b == 0;
-      long long tm[3] = {0, 0, 0};
-      bool ok = true;
+        for (int k = 0; k < BKV / 16; ++k)
+          umma_f16_ts(tmem_base + Cfg::kColO, a + k * 8, vd + uint64_t((k * (16 * 128)) >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+        umma_commit(o_full(j));
+        umma_commit(empty(slot));
+      };
+      bool ok = wait_ring(0) && mbar_wait(q_full, 0, abort_flag, p.status, kStatusTimeoutFull);
+      if (ok) scores(0);
       for (int j = 0; ok && j < n_blocks; ++j) {
-        const int s = j & 1;
-        const uint32_t par = (j >> 1) & 1;
-        long long c0 = trm ? clock64() : 0;
-        if (!mbar_wait(p_full(s), par, abort_flag, p.status, kStatusTimeoutTmemFull)) { ok = false; break; }
-        if (trm) { const long long c1 = clock64(); tm[1] += c1 - c0; c0 = c1; }   // waiting for P
-        if (!mbar_wait(v_full(s), par, abort_flag, p.status, kStatusTimeoutFull)) { ok = false; break; }
-        if (trm) { const long long c1 = clock64(); tm[2] += c1 - c0; c0 = c1; }   // waiting for V
-        tc_fence_after();
-        const uint64_t pd = s ? p_desc[1] : p_desc[0];
-        const uint64_t vd = s ? v_desc[1] : v_desc[0];
-        const uint32_t d_o = tmem_base + Cfg::kColO + s * DV;
-#pragma unroll
-        for (int k = 0; k < BKV / 16; ++k) {
-          const uint64_t a_off = uint64_t(((k / 4) * (128 * 128) + (k % 4) * 32) >> 4);
-          const uint64_t b_off = uint64_t((k * (16 * 128)) >> 4);
-          umma_f16_ss(d_o, pd + a_off, vd + b_off, idesc_o, (j > 1 || k > 0) ? 1u : 0u);
+        if (j + 1 < n_blocks) {
+          // Two buffers: the other one held the weights of block j - 1, whose product was issued before and so reads them first.
+          ok = wait_ring(k_seq(j + 1)) &&
+               (Cfg::kTwoS || mbar_wait(s_free, uint32_t(j) & 1u, abort_flag, p.status, kStatusTimeoutTmemEmpty));
+          if (!ok) break;
+          tc_fence_after();
+          scores(j + 1);
         }
-        umma_commit(v_empty(s));
-        umma_commit(p_empty(s));
-        if (j == n_blocks - 1) umma_commit(o_full);
-        if (trm) { const long long c1 = clock64(); tm[0] += c1 - c0; c0 = c1; }   // issuing the PV MMAs
+        ok = wait_ring(v_seq(j)) && mbar_wait(p_full(j), uint32_t(j >> 1) & 1u, abort_flag, p.status, kStatusTimeoutTmemFull);
+        if (!ok) break;
+        tc_fence_after();
+        values(j);
       }
-      if (trm) { p.trace[8] = tm[0]; p.trace[9] = tm[1]; p.trace[10] = tm[2]; p.trace[11] = n_blocks; }
     }
-  } else if (warp < 10) {
-    // ---------------------------------------------------------------- softmax + epilogue
-    // Two independent groups of four warps: group g takes the KV blocks of parity g (score buffer g, P buffer g) and
-    // keeps its own running maximum, row sum and output accumulator O_g, so a thread owns a whole score row of its
-    // block (no exchange of row statistics between warps) and the softmax of block j+1 overlaps that of block j.
-    // The two accumulators are merged once, at the end.
+  } else {
+    // ---------------------------------------------------------------- softmax + epilogue: one query row per thread
     const int quarter = warp & 3;          // TMEM lanes this warp may touch
-    const int grp = (warp - 2) >> 2;       // which blocks (and, in the epilogue, which half of the output columns)
     const int row = quarter * 32 + lane;
     const int q_idx = q0 + row;
-    const uint32_t lane_base = uint32_t(quarter * 32) << 16;
-    const uint32_t o_mine = tmem_base + lane_base + Cfg::kColO + grp * DV;
+    const uint32_t tm = tmem_base + (uint32_t(quarter * 32) << 16);
+    const uint32_t o_mine = tm + Cfg::kColO;
+    const float scale = p.scale_log2;
     float m_used = 0.f, l = 0.f;
     bool seen = false;   // this row has met a visible key (with a window, whole blocks may lie before it)
     bool ok = true;
-    const bool tr = p.trace != nullptr && blockIdx.z == 0 && h == 0 && b == 0 && warp == 2 && lane == 0;
-    long long tc[6] = {0, 0, 0, 0, 0, 0};
-    int tn = 0;
-    for (int j = grp; j < n_blocks; j += 2) {
-      long long c0 = tr ? clock64() : 0;
-      ++tn;
-      const uint32_t par = (j >> 1) & 1;
-      const int sb = j % Cfg::kSBufs;
-      ok = __all_sync(0xffffffffu, mbar_wait(s_full(sb), uint32_t(j / Cfg::kSBufs) & 1u, abort_flag, p.status,
-                                             kStatusTimeoutTmemFull));
+    const bool tr = p.trace != nullptr && blockIdx.z == 0 && h == 0 && b == 0 && threadIdx.x == 64;
+    long long waited = 0, t0 = tr ? clock64() : 0;
+    for (int j = 0; j < n_blocks; ++j) {
+      const long long c0 = tr ? clock64() : 0;
+      ok = __all_sync(0xffffffffu, mbar_wait(s_full(j), uint32_t(j >> 1) & 1u, abort_flag, p.status, kStatusTimeoutTmemFull));
       if (!ok) break;
-      if (tr) { const long long c1 = clock64(); tc[0] += c1 - c0; c0 = c1; }   // waiting for S
+      if (tr) waited += clock64() - c0;
       tc_fence_after();
+      const uint32_t s_mine = tm + (Cfg::kTwoS ? (j & 1) * BKV : 0);
+      uint32_t r[BKV / 32][32];
+#pragma unroll
+      for (int c = 0; c < BKV / 32; ++c) tmem_ld_32x32(s_mine + c * 32, r[c]);
       int owner, kv0b, kbase;
       locate(j, owner, kv0b, kbase);
-      // last visible column of this 128-key block for this row: causal position and end of the rank's keys
+      // last visible column of this block for this row: causal position and end of the rank's keys
       int limit = p.Tk - 1 - kv0b;
       if (p.causal) limit = min(limit, q_base + row - kbase);
       const int lower = p.window > 0 ? q_base + row - kbase - p.window + 1 : 0;   // first visible column
-      const uint32_t s_mine = tmem_base + lane_base + Cfg::kColS + sb * BKV;
-      // pass 1: row maximum (the scores are read from tensor memory twice, 64 columns at a time, instead of
-      // holding all 128 in registers)
-      float mx = -INFINITY;
-#pragma unroll 1
-      for (int hh = 0; hh < BKV / 64; ++hh) {
-        uint32_t r[2][32];
-        tmem_ld_32x32(s_mine + hh * 64, r[0]);
-        tmem_ld_32x32(s_mine + hh * 64 + 32, r[1]);
-        tmem_ld_wait();
-        if (limit >= hh * 64 + 63 && lower <= hh * 64) {
+      // columns of a 32-key chunk that this row sees; chunks that no row of the warp sees are skipped
+      auto visible = [&](int c) {
+        const int lo = max(lower - c * 32, 0), hi = min(limit - c * 32, 31);
+        return hi < lo ? 0u : (0xffffffffu >> (31 - hi)) & (0xffffffffu << lo);
+      };
+      const bool whole = __all_sync(0xffffffffu, limit >= BKV - 1 && lower <= 0);
+      tmem_ld_wait();
+      if constexpr (!Cfg::kTwoS) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(s_free);
+      }
+      float mx;
+      if (whole) {
+        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-          for (int c = 0; c < 2; ++c)
+        for (int c = 0; c < BKV / 32; ++c)
 #pragma unroll
-            for (int i = 0; i < 32; ++i) mx = fmaxf(mx, __uint_as_float(r[c][i]));
-        } else {
+          for (int i = 0; i < 32; i += 8)
 #pragma unroll
-          for (int c = 0; c < 2; ++c)
+            for (int u = 0; u < 4; ++u) m4[u] = max3(m4[u], __uint_as_float(r[c][i + u]), __uint_as_float(r[c][i + u + 4]));
+        mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+      } else {
+        mx = -INFINITY;
 #pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (hh * 64 + c * 32 + i <= limit && hh * 64 + c * 32 + i >= lower) mx = fmaxf(mx, __uint_as_float(r[c][i]));
+        for (int c = 0; c < BKV / 32; ++c) {
+          const uint32_t vis = visible(c);
+          if (__any_sync(0xffffffffu, vis != 0u)) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) mx = fmaxf(mx, (vis >> i) & 1u ? __uint_as_float(r[c][i]) : -INFINITY);
+          }
         }
       }
-      if (tr) { const long long c1 = clock64(); tc[1] += c1 - c0; c0 = c1; }   // pass 1 (row maximum)
-      const float m_blk = mx * p.scale_log2;
+      const float m_blk = mx * scale;
       if (!seen) {
-        // nothing accumulated for this row yet (its P entries were zero): take the block's maximum as it is
+        // nothing accumulated for this row yet (its weights were zero): take the block's maximum as it is
         m_used = (m_blk == -INFINITY) ? 0.f : m_blk;
         seen = m_blk != -INFINITY;
       }
-      if (j != grp) {
+      if (j > 0) {
         const float m_new = fmaxf(m_used, m_blk);
-        const bool need = (m_new - m_used > 8.f);
-        if (__any_sync(0xffffffffu, need)) {
-          // O_g must be complete up to this group's previous block before it is rescaled.
-          ok = __all_sync(0xffffffffu, mbar_wait(p_empty(grp), par ^ 1u, abort_flag, p.status, kStatusTimeoutTmemEmpty));
+        const bool need = m_new - m_used > 8.f;
+        const bool any = __any_sync(0xffffffffu, need);
+        if (!Cfg::kTwoS || any) {
+          // the product of the block before has read its weights and is in O
+          ok = __all_sync(0xffffffffu, mbar_wait(o_full(j - 1), uint32_t((j - 1) >> 1) & 1u, abort_flag, p.status, kStatusTimeoutTmemEmpty));
           if (!ok) break;
           tc_fence_after();
+        }
+        if (any) {
           const float alpha = need ? ex2_approx_f(m_used - m_new) : 1.f;
-#pragma unroll
+#pragma unroll 1
           for (int c = 0; c < DV / 16; ++c) {
             uint32_t o[16];
             tmem_ld_32x16(o_mine + c * 16, o);
@@ -403,119 +414,82 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           if (need) m_used = m_new;
         }
       }
-      if (tr) { const long long c1 = clock64(); tc[2] += c1 - c0; c0 = c1; }   // rescale of O (rare)
-      // P buffer g is free once this group's previous PV has been executed.
-      ok = __all_sync(0xffffffffu, mbar_wait(p_empty(grp), par ^ 1u, abort_flag, p.status, kStatusTimeoutTmemEmpty));
-      if (!ok) break;
-      if (tr) { const long long c1 = clock64(); tc[3] += c1 - c0; c0 = c1; }   // waiting for the P buffer
-      // pass 2: exponentials, row sum, bf16 P into the swizzled operand tile (64 keys = one 128-byte row chunk)
-      float sum = 0.f;
-      uint8_t* prow = smem + Cfg::kOffP + grp * Cfg::kPBytes + (row >> 3) * 1024 + (row & 7) * 128;
-#pragma unroll 1
-      for (int hh = 0; hh < BKV / 64; ++hh) {
-        uint32_t r[2][32];
-        tmem_ld_32x32(s_mine + hh * 64, r[0]);
-        tmem_ld_32x32(s_mine + hh * 64 + 32, r[1]);
-        tmem_ld_wait();
-        const bool full_vis = (limit >= hh * 64 + 63 && lower <= hh * 64);
+      // exponentials two at a time, row sum, weights as bf16 into tensor memory
+      const uint64_t scale2 = pack_f32x2(scale, scale), minus2 = pack_f32x2(-m_used, -m_used);
+      uint64_t sum2[2] = {0ull, 0ull};
+      auto weights = [&](auto masked) {
 #pragma unroll
-        for (int c = 0; c < 2; ++c)
+        for (int c = 0; c < BKV / 32; ++c) {
+          uint32_t w[16];
+          const uint32_t vis = decltype(masked)::value ? visible(c) : ~0u;
+          if (decltype(masked)::value && !__any_sync(0xffffffffu, vis != 0u)) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            float pv = ex2_approx_f(fmaf(__uint_as_float(r[c][i]), p.scale_log2, -m_used));
-            if (!full_vis && (hh * 64 + c * 32 + i > limit || hh * 64 + c * 32 + i < lower)) pv = 0.f;
-            sum += pv;
-            r[c][i] = __float_as_uint(pv);
+            for (int i = 0; i < 16; ++i) w[i] = 0u;
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              float e0, e1;
+              unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[c][2 * i]), __uint_as_float(r[c][2 * i + 1])), scale2, minus2), e0, e1);
+              e0 = ex2_approx_f(e0);
+              e1 = ex2_approx_f(e1);
+              if constexpr (decltype(masked)::value) {
+                e0 = (vis >> (2 * i)) & 1u ? e0 : 0.f;
+                e1 = (vis >> (2 * i + 1)) & 1u ? e1 : 0.f;
+              }
+              sum2[i & 1] = add_f32x2(sum2[i & 1], pack_f32x2(e0, e1));
+              w[i] = pack_bf16x2(e0, e1);
+            }
           }
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            uint4 w;
-            w.x = pack_bf16x2(__uint_as_float(r[c][u * 8 + 0]), __uint_as_float(r[c][u * 8 + 1]));
-            w.y = pack_bf16x2(__uint_as_float(r[c][u * 8 + 2]), __uint_as_float(r[c][u * 8 + 3]));
-            w.z = pack_bf16x2(__uint_as_float(r[c][u * 8 + 4]), __uint_as_float(r[c][u * 8 + 5]));
-            w.w = pack_bf16x2(__uint_as_float(r[c][u * 8 + 6]), __uint_as_float(r[c][u * 8 + 7]));
-            const int unit = (c * 4 + u) ^ (row & 7);  // 16-byte unit inside the 128-byte row of key chunk hh
-            *reinterpret_cast<uint4*>(prow + hh * (128 * 128) + unit * 16) = w;
-          }
+          tmem_st_32x16(s_mine + Cfg::kColP + c * 16, w);
         }
-      }
-      l += sum;
-      fence_proxy_async();
+      };
+      // two bodies: a test inside would be a branch per pair of keys
+      if (whole) weights(std::false_type{});
+      else weights(std::true_type{});
+      float s0, s1;
+      unpack_f32x2(add_f32x2(sum2[0], sum2[1]), s0, s1);
+      l += s0 + s1;
+      tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) {   // one arrival per warp of the group
-        mbar_arrive(s_free(sb));
-        mbar_arrive(p_full(grp));
-      }
-      if (tr) { const long long c1 = clock64(); tc[4] += c1 - c0; c0 = c1; }   // pass 2 (exp, P stores, fence, arrive)
+      if (lane == 0) mbar_arrive(p_full(j));   // one arrival per warp
     }
     if (tr) {
-      for (int i = 0; i < 5; ++i) p.trace[i] = tc[i];
-      p.trace[15] = tn;
+      p.trace[0] = waited;              // waiting for scores
+      p.trace[4] = clock64() - t0;      // the whole loop
+      p.trace[15] = n_blocks;
     }
     if (ok && n_blocks > 0) {
-      ok = __all_sync(0xffffffffu, mbar_wait(o_full, 0, abort_flag, p.status, kStatusTimeoutTmemFull));
-    }
-    // merge the two groups: exchange (maximum, row sum) with the warp of the other group on the same lane quarter
-    const bool mine_used = n_blocks > grp, other_used = n_blocks > (grp ^ 1);
-    float m_o = 0.f, l_o = 0.f;
-    if (ok) {
-      xmax[(grp * 2 + 0) * 128 + row] = m_used;
-      xmax[(grp * 2 + 1) * 128 + row] = l;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(x_bar(quarter));
-      ok = __all_sync(0xffffffffu, mbar_wait(x_bar(quarter), 0, abort_flag, p.status, kStatusTimeoutLocalFlag));
-      if (ok) {
-        m_o = xmax[((grp ^ 1) * 2 + 0) * 128 + row];
-        l_o = xmax[((grp ^ 1) * 2 + 1) * 128 + row];
-      }
+      ok = __all_sync(0xffffffffu, mbar_wait(o_full(n_blocks - 1), uint32_t((n_blocks - 1) >> 1) & 1u, abort_flag, p.status, kStatusTimeoutTmemFull));
+      tc_fence_after();
     }
     if (ok) {
-      float m_all = m_used, a_mine = 1.f, a_other = 0.f;
-      if (mine_used && other_used && l > 0.f && l_o > 0.f) {
-        m_all = fmaxf(m_used, m_o);
-        a_mine = ex2_approx_f(m_used - m_all);
-        a_other = ex2_approx_f(m_o - m_all);
-      } else if (other_used && !(mine_used && l > 0.f)) {     // only the other group met a visible key of this row
-        m_all = m_o; a_mine = 0.f; a_other = 1.f;
-      }
-      const float l_all = (mine_used ? l * a_mine : 0.f) + (other_used ? l_o * a_other : 0.f);
-      const float inv_l = (l_all > 0.f) ? 1.f / l_all : 0.f;
-      const float w_mine = a_mine * inv_l, w_other = a_other * inv_l;
-      if (n_blocks > 0) tc_fence_after();
+      const float inv_l = (l > 0.f) ? 1.f / l : 0.f;
       __nv_bfloat16* orow = p.O + (long long)b * p.so_b + (long long)q_idx * p.so_t + (long long)h * DV;
-      const uint32_t o_other = tmem_base + lane_base + Cfg::kColO + (grp ^ 1) * DV;
-      // this warp writes output columns [grp * DV / 2, (grp + 1) * DV / 2) of its 32 rows
 #pragma unroll 1
-      for (int c = grp * (DV / 32); c < (grp + 1) * (DV / 32); ++c) {
-        uint32_t o[16], o2[16];
-        if (mine_used) tmem_ld_32x16(o_mine + c * 16, o);
-        if (other_used) tmem_ld_32x16(o_other + c * 16, o2);
-        if (mine_used || other_used) tmem_ld_wait();
-        float v[16];
+      for (int c = 0; c < DV / 32; ++c) {
+        uint32_t o[32];
+        if (n_blocks > 0) {
+          tmem_ld_32x32(o_mine + c * 32, o);
+          tmem_ld_wait();
+        } else {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          float acc = 0.f;
-          if (mine_used) acc = __uint_as_float(o[i]) * w_mine;
-          if (other_used) acc = fmaf(__uint_as_float(o2[i]), w_other, acc);
-          v[i] = acc;
+          for (int i = 0; i < 32; ++i) o[i] = 0u;
         }
         if (q_idx < p.Tq) {
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
+          for (int u = 0; u < 4; ++u) {
             uint4 w;
-            w.x = pack_bf16x2(v[u * 8 + 0], v[u * 8 + 1]);
-            w.y = pack_bf16x2(v[u * 8 + 2], v[u * 8 + 3]);
-            w.z = pack_bf16x2(v[u * 8 + 4], v[u * 8 + 5]);
-            w.w = pack_bf16x2(v[u * 8 + 6], v[u * 8 + 7]);
-            *reinterpret_cast<uint4*>(orow + c * 16 + u * 8) = w;
+            w.x = pack_bf16x2(__uint_as_float(o[u * 8 + 0]) * inv_l, __uint_as_float(o[u * 8 + 1]) * inv_l);
+            w.y = pack_bf16x2(__uint_as_float(o[u * 8 + 2]) * inv_l, __uint_as_float(o[u * 8 + 3]) * inv_l);
+            w.z = pack_bf16x2(__uint_as_float(o[u * 8 + 4]) * inv_l, __uint_as_float(o[u * 8 + 5]) * inv_l);
+            w.w = pack_bf16x2(__uint_as_float(o[u * 8 + 6]) * inv_l, __uint_as_float(o[u * 8 + 7]) * inv_l);
+            *reinterpret_cast<uint4*>(orow + c * 32 + u * 8) = w;
           }
         }
       }
-      if (grp == 0 && q_idx < p.Tq)
-        p.lse[((long long)b * p.Hq + h) * p.Tq + q_idx] = (l_all > 0.f) ? (m_all + log2f(l_all)) * 0.6931471805599453f : -INFINITY;
+      if (q_idx < p.Tq)
+        p.lse[((long long)b * p.Hq + h) * p.Tq + q_idx] = (l > 0.f) ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
     }
   }
 
@@ -533,7 +507,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
 static long long* g_fwd_trace = nullptr;
 
-template <int D, int DV = D, int BKV = kFaBlockKV, bool SHARED = false>
+template <int D, int DV, int BKV, bool SHARED = false>
 static int launch_flash_fwd(const CUtensorMap& tq, const KvMaps& maps, const FlashFwdParams& p, cudaStream_t st) {
   using Cfg = FaFwdCfg<D, DV, BKV>;
   static bool configured = false;
@@ -554,8 +528,8 @@ static int flash_fwd_common(const void* q, const void* const* k_ptrs, const void
                             int causal, int cp_world, int cp_rank, int zigzag, int window, void* stream) {
   if (window < 0 || (window > 0 && (!causal || cp_world != 1))) return -int(kStatusBadArgument);
   if ((D != 64 && D != 128) || Hq % Hkv != 0 || cp_world < 1 || cp_world > kFaMaxRanks) return -int(kStatusBadArgument);
-  if (cp_world > 1 && zigzag && ((Tq / 2) % kFaBlockQ != 0 || (Tk / 2) % kFaBlockKV != 0)) return -int(kStatusBadArgument);
-  if (cp_world > 1 && !zigzag && (Tq % kFaBlockQ != 0 || Tk % kFaBlockKV != 0)) return -int(kStatusBadArgument);
+  if (cp_world > 1 && zigzag && ((Tq / 2) % kFaBlockQ != 0 || (Tk / 2) % kFaShardRows != 0)) return -int(kStatusBadArgument);
+  if (cp_world > 1 && !zigzag && (Tq % kFaBlockQ != 0 || Tk % kFaShardRows != 0)) return -int(kStatusBadArgument);
   if (B == 0 || Tq == 0) return 0;
   CUtensorMap tq;
   KvMaps maps;
@@ -564,10 +538,10 @@ static int flash_fwd_common(const void* q, const void* const* k_ptrs, const void
   for (int i = 0; i < kFaMaxRanks; ++i) {
     const int src = i < cp_world ? i : 0;
     r = encode_tmap_4d(&maps.k[i], k_ptrs[src], 2, D, Hkv, Tk, B, (uint64_t)D * 2, (uint64_t)sk_t * 2, (uint64_t)sk_b * 2, 64, 1,
-                       kFaBlockKV, 1, 1);
+                       fa_block_kv(D), 1, 1);
     if (r) return 2000 + r;
     r = encode_tmap_4d(&maps.v[i], v_ptrs[src], 2, D, Hkv, Tk, B, (uint64_t)D * 2, (uint64_t)sv_t * 2, (uint64_t)sv_b * 2, 64, 1,
-                       kFaBlockKV, 1, 1);
+                       fa_block_kv(D), 1, 1);
     if (r) return 3000 + r;
   }
   FlashFwdParams p{};
@@ -582,7 +556,7 @@ static int flash_fwd_common(const void* q, const void* const* k_ptrs, const void
   p.status = device_status_word();
   p.trace = g_fwd_trace;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  return D == 64 ? launch_flash_fwd<64>(tq, maps, p, st) : launch_flash_fwd<128>(tq, maps, p, st);
+  return D == 64 ? launch_flash_fwd<64, 64, 128>(tq, maps, p, st) : launch_flash_fwd<128, 128, 64>(tq, maps, p, st);
 }
 
 // One sequence whose keys are [the head's own columns | 64 columns shared by all heads].
@@ -592,7 +566,7 @@ static int flash_fwd_shared(const void* q, const void* k, const void* k_shared, 
   const bool wide = D == 192 && DV == 128, mid = D == 128 && (DV == 64 || DV == 128);
   if ((!wide && !mid) || H < 1 || Tk < Tq || window < 0) return -int(kStatusBadArgument);
   if (Tq == 0) return 0;
-  const int block_kv = wide ? 64 : kFaBlockKV, dk = D - 64;
+  const int block_kv = fa_block_kv(DV), dk = D - 64;
   // one batch entry: its stride is never used, but has to be a valid one
   auto map = [&](CUtensorMap* m, const void* base, int cols, int heads, int rows, long long pitch, int box_rows) {
     return encode_tmap_4d(m, base, 2, cols, heads, rows, 1, (uint64_t)cols * 2, (uint64_t)pitch * 2, (uint64_t)pitch * rows * 2, 64, 1,
@@ -619,7 +593,7 @@ static int flash_fwd_shared(const void* q, const void* k, const void* k_shared, 
   p.window = window;
   p.status = device_status_word();
   if (wide) return launch_flash_fwd<192, 128, 64, true>(tq, maps, p, st);
-  return DV == 64 ? launch_flash_fwd<128, 64, kFaBlockKV, true>(tq, maps, p, st) : launch_flash_fwd<128, 128, kFaBlockKV, true>(tq, maps, p, st);
+  return DV == 64 ? launch_flash_fwd<128, 64, 128, true>(tq, maps, p, st) : launch_flash_fwd<128, 128, 64, true>(tq, maps, p, st);
 }
 
 }  // namespace lt
