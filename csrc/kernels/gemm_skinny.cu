@@ -22,6 +22,7 @@
 #include "common/host.h"
 #include "common/ptx.cuh"
 #include "common/scalar.cuh"
+#include "weight_stream.h"
 
 #include <atomic>
 #include <map>
@@ -361,6 +362,8 @@ int lt_gemm_skinny_bf16(const void* x, long long ldx, const void* w, long long l
   p.residual = static_cast<const __nv_bfloat16*>(residual); p.ldr = ldr;
   p.M = M; p.N = N; p.K = K;
   if (M < 1 || M > 128 || !skinny_ok(p)) return -int(kStatusBadArgument);
+  const StreamProduct s{p.x, ldx, p.w, ldw, p.y, ldy, p.residual, ldr, M, N, K, 0};
+  if (stream_takes(s)) return launch_stream(s, static_cast<cudaStream_t>(stream));
   return skinny_by_rows<kSkPlain, false>(p, M, 1, static_cast<cudaStream_t>(stream));
 }
 
@@ -373,6 +376,8 @@ int lt_gemm_skinny_glu(const void* x, long long ldx, const void* w, void* y, int
   p.y = static_cast<__nv_bfloat16*>(y); p.ldy = N;
   p.M = M; p.N = N; p.K = K; p.act = act;
   if (M < 1 || M > 128 || act < 1 || act > 2 || !skinny_ok(p)) return -int(kStatusBadArgument);
+  const StreamProduct s{p.x, ldx, p.w, K, p.y, N, nullptr, 0, M, N, K, act};
+  if (stream_takes(s)) return launch_stream(s, static_cast<cudaStream_t>(stream));
   return skinny_by_rows<kSkPlain, true>(p, M, 1, static_cast<cudaStream_t>(stream));
 }
 

@@ -1,0 +1,65 @@
+"""Products of a few rows with a weight matrix, over sizes at the edges of tiles, stages and row blocks, against 64-bit arithmetic."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def bound(ref, mag, K):
+    """Rounding to bf16 (2^-8 of the result), and of every 32-bit addition, which a tensor core may cut off (2^-23 of the sum of sizes each)."""
+    return 2.0 ** -8 * ref.abs() + (K + 16) * 2.0 ** -23 * mag + 1e-30
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 8), (1, 17, 2056), (2, 2367, 64), (3, 2369, 72), (8, 4737, 136), (8, 9473, 520), (7, 31, 14336), (8, 20001, 64)])
+def test_gemv_rows(M, N, K):
+    from litetorch_b200.ops import kernels as KK
+    torch.manual_seed(N + K)
+    x, w, r = (torch.randn(*s, device="cuda").bfloat16() for s in ((M, K), (N, K), (M, N)))
+    for res in (None, r):
+        y = KK.gemm(x, w, residual=res)
+        ref = x.double() @ w.double().t() + (0 if res is None else res.double())
+        mag = x.double().abs() @ w.double().abs().t() + (0 if res is None else res.double().abs())
+        assert ((y.double() - ref).abs() <= bound(ref, mag, K)).all()
+    assert torch.equal(KK.gemm(x, w, residual=r), y)
+    assert KK.status_fetch() == 0
+
+
+@pytest.mark.parametrize("M", [9, 16, 17, 32, 33, 64, 65])
+@pytest.mark.parametrize("N,K", [(8, 32), (2368, 96), (2376, 64), (4736, 544), (4744, 2048), (9480, 128), (28672, 64)])
+def test_skinny_rows(M, N, K):
+    from litetorch_b200.ops import kernels as KK
+    torch.manual_seed(M + N + K)
+    x, w, r = (torch.randn(*s, device="cuda").bfloat16() for s in ((M, K), (N, K), (M, N)))
+    y = KK.gemm(x, w, residual=r)
+    ref = x.double() @ w.double().t() + r.double()
+    assert ((y.double() - ref).abs() <= bound(ref, x.double().abs() @ w.double().abs().t() + r.double().abs(), K)).all()
+    assert KK.status_fetch() == 0
+
+
+@pytest.mark.parametrize("act", ["gelu", "silu"])
+@pytest.mark.parametrize("M,F,K", [(1, 8, 32), (8, 1184, 64), (9, 1192, 96), (16, 2376, 64), (17, 520, 544), (32, 5632, 64), (64, 1000, 96)])
+def test_gated(M, F, K, act):
+    from litetorch_b200.ops import kernels as KK
+    torch.manual_seed(M + F)
+    x, gu = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(2 * F, K, device="cuda") * K ** -0.5).bfloat16()
+    down = torch.eye(F, device="cuda").bfloat16()                     # hands the gated values through
+    y = KK.glu_mlp(x, gu, down, act)
+    g, u = (x.double() @ gu.double().t()).chunk(2, -1)
+    a = torch.nn.functional.silu(g) if act == "silu" else torch.nn.functional.gelu(g, approximate="tanh")
+    mag = (x.double().abs() @ gu.double().abs().t())
+    slack = (K + 16) * 2.0 ** -23 * 1.2 * (mag[:, :F] * u.abs() + mag[:, F:] * a.abs())      # both factors' sums; the slopes of the activations are below 1.2
+    assert ((y.double() - a * u).abs() <= 2.0 ** -7 * (a * u).abs() + slack + 1e-5 * u.abs()).all()
+    assert KK.status_fetch() == 0
+
+
+def test_rows_that_overlap():
+    """Expanded and sliding views take the general kernels."""
+    from litetorch_b200.ops import kernels as KK
+    torch.manual_seed(0)
+    base = torch.randn(4096, device="cuda").bfloat16()
+    x = base[:256].expand(4, 256)                                     # pitch 0
+    w = base.as_strided((64, 256), (8, 1))                            # pitch below the row's length
+    plain = torch.randn(64, 256, device="cuda").bfloat16()
+    for a, b in ((x, plain), (plain[:4], w), (x, w)):
+        ref = a.double() @ b.double().t()
+        assert ((KK.gemm(a, b).double() - ref).abs() <= bound(ref, a.double().abs() @ b.double().abs().t(), 256)).all()
