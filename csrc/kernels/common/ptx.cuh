@@ -464,6 +464,30 @@ __device__ __forceinline__ float2 unpack_bf16x2(uint32_t u) {
   __nv_bfloat162 v = *reinterpret_cast<__nv_bfloat162*>(&u);
   return __bfloat1622float2(v);
 }
+// Two floats in a register pair; one instruction works on both.
+__device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
+  uint64_t y;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(a), "f"(b));
+  return y;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t x, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x));
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t y;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(y) : "l"(a), "l"(b), "l"(c));
+  return y;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+  uint64_t y;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(y) : "l"(a), "l"(b));
+  return y;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+  uint64_t y;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(y) : "l"(a), "l"(b));
+  return y;
+}
 __device__ __forceinline__ float gelu_tanh(float x) {
   const float k0 = 0.7978845608028654f, k1 = 0.044715f;
   float u = k0 * (x + k1 * x * x * x);

@@ -12,15 +12,25 @@
 //   dV += P^T dO_i      dK += dS^T Q_i                (A read M-major from the same P / dS tiles)
 //   dQ_i = dS K         -> red.global.add into an fp32 accumulator, converted to bf16 by a last kernel
 //
+// What bounds it: a serial chain.  S and dP, their exponentials (1024 clocks for 128 x 128 on one SM's special function units, about
+// 2100 with the loads from tensor memory and the stores around them), and, with head_dim 128, dQ, which shares tensor memory with dP and
+// shared memory with P and dS.  So what need not be on the chain is not: four warps of their own take dQ from tensor memory to the
+// accumulator under the next block's products; Q is loaded a block ahead, and dV is the first product of a block, which frees dO for
+// the next load and P for the first half of dQ; P and dS are made in registers before their tiles are waited for.
+// Measured with the pre-pass and the conversion, causal, L2 flushed, against one set of warps doing both parts: D 128, 8192 tokens, 32 / 8
+// heads 2191 -> 1711 us (7700 -> 6000 clocks a block; 40 MMAs take 2560); D 64, 4 x 2048 tokens, 32 / 4 heads 359 -> 325 us (3690 -> 3400).
+//
 // delta = rowsum(O * dO) comes from a small pre-pass.  All waits are bounded (see common/ptx.cuh).
 #include "lt_cuda.h"
 #include "common/host.h"
 #include "common/ptx.cuh"
 
+#include <type_traits>
+
 namespace lt {
 
 constexpr int kFbBlock = 128;
-constexpr int kFbThreads = 384;   // warp 0 producer, warps 1 / 10 / 11 MMA issuers (S,dP / dV,dK / dQ), warps 2-9 compute
+constexpr int kFbThreads = 512;   // warp 0 producer, warps 1 / 10 MMA issuers (S, dP / dQ, dV, dK), warps 2-9 compute, 12-15 write dQ
 constexpr int kFbComputeThreads = 256;
 
 constexpr int kFbMaxRanks = 8;
@@ -41,7 +51,6 @@ struct FlashBwdParams {
   // Optional phase timing (nullptr: off): the CTA of key block 0 / head 0 / batch 0 adds the SM cycles its compute
   // warp 2 and its MMA thread spend in each phase to trace[0..15] and counts iterations in trace[15].
   long long* trace;
-  int dbg;   // timing experiments only (results are wrong when non-zero): 1 = no bulk reduction, 2 = no staging either
 };
 
 struct QMaps {
@@ -57,35 +66,31 @@ template <int D>
 struct FaBwdCfg {
   static constexpr int kTile = kFbBlock * D * 2;          // one 128 x D bf16 tile
   static constexpr int kPTile = kFbBlock * kFbBlock * 2;  // 128 x 128 bf16
-  static constexpr int kStages = (D == 64) ? 2 : 1;       // Q / dO buffering
+  // Q is loaded a block ahead; dO too where there is room, else as soon as dV has been added (before dK and dQ).
+  static constexpr int kQStages = 2, kDoStages = (D == 64) ? 2 : 1;
   static constexpr int kOffK = 0;
   static constexpr int kOffV = kTile;
   static constexpr int kOffQ = 2 * kTile;
-  static constexpr int kOffDO = kOffQ + kStages * kTile;
-  static constexpr int kOffP = kOffDO + kStages * kTile;
+  static constexpr int kOffDO = kOffQ + kQStages * kTile;
+  static constexpr int kOffP = kOffDO + kDoStages * kTile;
   static constexpr int kOffDS = kOffP + kPTile;
   static constexpr int kOffBar = kOffDS + kPTile;
-  static constexpr int kOffSeg = kOffBar + 128;
-  // dQ tiles staged for TMA reductions into the fp32 accumulator (head_dim 64 only: with head_dim 128 shared memory
-  // is full and the rows go out as red.global.add).  One 32-row x 32-column fp32 tile (4 KB, 128-byte swizzle) per
-  // compute warp, reduced into global memory by ONE cp.reduce.async.bulk.tensor per warp and iteration: the copy
-  // engine does the atomics, not the LSU, and it is given few, large operations.
-  static constexpr bool kBulkDq = true;
+  static constexpr int kOffSeg = kOffBar + 192;
+  // dQ tiles are staged in shared memory for TMA reductions into the fp32 accumulator: boxes of 32 rows x 32 columns (4 KB, 128-byte
+  // swizzle), D / 32 to each of the four writing warps.  The copy engine does the atomics, not the LSU, and it is given few, large
+  // operations.
   static constexpr int kDqTile = 32 * 128;                 // one 32-row x 32-column fp32 box
-  static constexpr int kDqBoxes = D / 64;                  // boxes per warp: its 32 rows x D / 2 columns
+  static constexpr int kDqBoxes = D / 32;                  // boxes per warp: its 32 rows
   // head_dim 64: a staging area of its own.  head_dim 128: shared memory is full, so the staging area IS the P and dS
-  // tiles (64 KB, free between the MMAs of one iteration and the exp phase of the next); a barrier among the compute
-  // warps keeps the next exp phase from overwriting tiles a reduction is still reading.
+  // tiles (free between the MMAs of one iteration and the stores of the next): columns 0 .. 63 in the P tile, which is free first.
   static constexpr bool kStageAliasesP = (D != 64);
   static constexpr int kOffDqStage = kStageAliasesP ? kOffP : ((kOffSeg + kFbMaxSegs * 16 + 16 + 1023) / 1024) * 1024;
-  static constexpr int kSmemBytes = (kStageAliasesP ? kOffSeg + kFbMaxSegs * 16 + 16
-                                                    : kOffDqStage + (kFbComputeThreads / 32) * kDqTile) + 1024;
+  static constexpr int kSmemBytes = (kStageAliasesP ? kOffSeg + kFbMaxSegs * 16 + 16 : kOffDqStage + 4 * kDqBoxes * kDqTile) + 1024;
+  static_assert(kSmemBytes <= 232448, "does not fit");
   static constexpr int kColS = 0, kColDP = 128, kColDV = 256, kColDK = 256 + D;
-  static constexpr int kColDQ = (D == 64) ? 384 : 0;  // D == 64: two buffers (384, 448); D == 128: aliases S
-  // D == 64: dQ of iteration i is read one iteration later, right after S / dP of iteration i+1 arrive, when the
-  // tensor pipe is idle (a tcgen05.ld issued while MMAs are queued waits behind them) and off the critical chain.
-  static constexpr bool kDeferDq = (D == 64);
-  static constexpr bool kDqAliasesS = (D != 64);
+  static constexpr int kColDQ = (D == 64) ? 384 : kColDP;  // D == 64: two buffers (384, 448); D == 128: over dP, which has been read by then
+  static constexpr bool kTwoDq = (D == 64);
+  static constexpr bool kDqOverDp = (D != 64);
 };
 
 // delta[b,h,t] = sum_d O * dO ; D/8 threads per (b,t,h) row, 16 bytes each.
@@ -154,6 +159,7 @@ __device__ __forceinline__ void tma_reduce_add_4d(const CUtensorMap* m, uint32_t
                ::"l"(reinterpret_cast<uint64_t>(m)), "r"(smem_src), "r"(x), "r"(h), "r"(t), "r"(b) : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
@@ -162,27 +168,28 @@ __global__ void __launch_bounds__(kFbThreads, 1)
 flash_bwd_kernel(const __grid_constant__ QMaps qm, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDQ, const FlashBwdParams p) {
   using Cfg = FaBwdCfg<D>;
-  constexpr int ST = Cfg::kStages;
+  constexpr int QS = Cfg::kQStages, DS = Cfg::kDoStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t sbase = smem_u32(smem);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kOffBar);
   const uint32_t bb = smem_u32(bars);
   const uint32_t kv_full = bb;
-  auto qdo_full = [&](int s) { return bb + 8u * (1 + s); };
-  auto qdo_empty = [&](int s) { return bb + 8u * (3 + s); };
-  const uint32_t sdp_full = bb + 8u * 5;   // S and dP are in TMEM
-  const uint32_t sdp_free = bb + 8u * 6;   // compute warps have read S and dP (one arrival per warp)
-  const uint32_t pds_full = bb + 8u * 7;   // P and dS are in shared memory (one arrival per warp)
-  const uint32_t pds_empty = bb + 8u * 8;  // the three MMAs that read P / dS have executed
-  const uint32_t dq_full = bb + 8u * 9;    // dQ_i is in TMEM
-  const uint32_t dq_free = bb + 8u * 10;   // compute warps have read dQ_i (one arrival per warp)
-  const uint32_t dkv_full = bb + 8u * 11;  // all MMAs done
-  const uint32_t dq_free1 = bb + 8u * 12;  // second dQ buffer (deferred-dQ flow)
-  const uint32_t stg_free = bb + 8u * 13;  // every compute warp's dQ reduction has finished reading shared memory
-  const uint32_t dq_full1 = bb + 8u * 14;  // dQ of odd iterations (deferred-dQ flow: one barrier per dQ buffer, so a
-                                           // waiter can never be overtaken by two completions)
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 15);
+  auto q_full = [&](int i) { return bb + 8u * (1 + i); };
+  auto q_empty = [&](int i) { return bb + 8u * (3 + i); };
+  auto do_full = [&](int i) { return bb + 8u * (5 + i); };
+  auto do_empty = [&](int i) { return bb + 8u * (7 + i); };
+  const uint32_t sdp_full = bb + 8u * 9;    // S and dP are in TMEM
+  const uint32_t sdp_free = bb + 8u * 10;   // compute warps have read S and dP (one arrival per warp)
+  const uint32_t pds_full = bb + 8u * 11;   // P and dS are in shared memory (one arrival per warp)
+  const uint32_t ds_empty = bb + 8u * 12;   // the MMAs that read dS have executed
+  auto dq_full = [&](int i) { return bb + 8u * (13 + i); };   // dQ is in TMEM (one barrier per dQ buffer, so a waiter can never be
+  auto dq_free = [&](int i) { return bb + 8u * (15 + i); };   // overtaken by two completions); the writing warps have read it
+  const uint32_t dkv_full = bb + 8u * 17;   // all MMAs done
+  const uint32_t p_empty = bb + 8u * 18;    // the MMAs that read P have executed
+  const uint32_t stg_p = bb + 8u * 19;      // dQ reductions have finished reading what they staged in the P tile
+  const uint32_t stg_ds = bb + 8u * 20;     // ... and in the dS tile
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 21);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -238,7 +245,15 @@ flash_bwd_kernel(const __grid_constant__ QMaps qm, const __grid_constant__ CUten
   __syncthreads();
   const int per_head = *per_head_s;
   const int n_iter = per_head * G;
+  const bool single = p.cp_world == 1;                    // a single run, kept in registers
+  const int first_q0 = segs[0].q0, first_qbase = segs[0].qbase;
   auto locate = [&](int j, int& owner, int& q0, int& qbase) {
+    if (single) {
+      owner = 0;
+      q0 = first_q0 + j * kFbBlock;
+      qbase = first_qbase + j * kFbBlock;
+      return;
+    }
     int sidx = 0;
     while (sidx < kFbMaxSegs - 1 && j >= segs[sidx].n) { j -= segs[sidx].n; ++sidx; }
     owner = segs[sidx].owner;
@@ -248,12 +263,15 @@ flash_bwd_kernel(const __grid_constant__ QMaps qm, const __grid_constant__ CUten
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
-    for (int s = 0; s < 2; ++s) { mbar_init(qdo_full(s), 1); mbar_init(qdo_empty(s), 1); }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(q_full(i), 1); mbar_init(q_empty(i), 1);
+      mbar_init(do_full(i), 1); mbar_init(do_empty(i), 1);
+      mbar_init(dq_full(i), 1); mbar_init(dq_free(i), 4);
+    }
     mbar_init(sdp_full, 1); mbar_init(sdp_free, kFbComputeThreads / 32);
-    mbar_init(pds_full, kFbComputeThreads / 32); mbar_init(pds_empty, 2);   // the dV/dK and the dQ issuer release P / dS
-    mbar_init(dq_full, 1); mbar_init(dq_full1, 1); mbar_init(dq_free, kFbComputeThreads / 32); mbar_init(dq_free1, kFbComputeThreads / 32);
-    mbar_init(stg_free, kFbComputeThreads / 32);
-    mbar_init(dkv_full, 2);   // the dV/dK and the dQ issuer have drained
+    mbar_init(pds_full, kFbComputeThreads / 32); mbar_init(ds_empty, 1);
+    mbar_init(p_empty, 1); mbar_init(stg_p, 4); mbar_init(stg_ds, 4);
+    mbar_init(dkv_full, 1);
     *abort_flag = 0;
     fence_barrier_init();
     fence_proxy_async();
@@ -271,7 +289,7 @@ flash_bwd_kernel(const __grid_constant__ QMaps qm, const __grid_constant__ CUten
 
   if (warp == 0) {
     // ---------------------------------------------------------------- producer
-    if (lane == 0 && n_iter > 0) {
+    if (n_iter > 0 && elect_one()) {
       mbar_expect_tx(kv_full, 2 * Cfg::kTile);
 #pragma unroll
       for (int c = 0; c < D / 64; ++c) {
@@ -279,123 +297,179 @@ flash_bwd_kernel(const __grid_constant__ QMaps qm, const __grid_constant__ CUten
         tma_load_4d(sbase + Cfg::kOffV + c * (kFbBlock * 128), &tmV, kv_full, c * 64, hkv, kv0, b);
       }
       for (int it = 0; it < n_iter; ++it) {
-        const int s = it % ST;
-        const uint32_t par = (it / ST) & 1;
+        const int qs = it % QS, ds = it % DS;
         const int h = hkv * G + it / per_head;
         int owner, q0, qbase;
         locate(it % per_head, owner, q0, qbase);
-        if (!mbar_wait(qdo_empty(s), par ^ 1u, abort_flag, p.status, kStatusTimeoutEmpty)) break;
-        mbar_expect_tx(qdo_full(s), 2 * Cfg::kTile);
+        if (!mbar_wait(q_empty(qs), (uint32_t(it / QS) & 1u) ^ 1u, abort_flag, p.status, kStatusTimeoutEmpty)) break;
+        mbar_expect_tx(q_full(qs), Cfg::kTile);
 #pragma unroll
-        for (int c = 0; c < D / 64; ++c) {
-          tma_load_4d(sbase + Cfg::kOffQ + s * Cfg::kTile + c * (kFbBlock * 128), &qm.q[owner], qdo_full(s), c * 64, h, q0, b);
-          tma_load_4d(sbase + Cfg::kOffDO + s * Cfg::kTile + c * (kFbBlock * 128), &qm.d_o[owner], qdo_full(s), c * 64, h, q0, b);
-        }
+        for (int c = 0; c < D / 64; ++c)
+          tma_load_4d(sbase + Cfg::kOffQ + qs * Cfg::kTile + c * (kFbBlock * 128), &qm.q[owner], q_full(qs), c * 64, h, q0, b);
+        if (!mbar_wait(do_empty(ds), (uint32_t(it / DS) & 1u) ^ 1u, abort_flag, p.status, kStatusTimeoutEmpty)) break;
+        mbar_expect_tx(do_full(ds), Cfg::kTile);
+#pragma unroll
+        for (int c = 0; c < D / 64; ++c)
+          tma_load_4d(sbase + Cfg::kOffDO + ds * Cfg::kTile + c * (kFbBlock * 128), &qm.d_o[owner], do_full(ds), c * 64, h, q0, b);
       }
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- first MMA issuer: S = Q K^T, dP = dO V^T
     // (as far ahead as the S / dP columns of tensor memory allow: they are free once the compute warps have loaded them)
-    if (lane == 0 && n_iter > 0) {
+    if (n_iter > 0 && elect_one()) {
       constexpr uint32_t idesc_sd = make_idesc_f16(128, 128, 1, 0, 0);  // S, dP: A K-major, B K-major
       bool ok = mbar_wait(kv_full, 0, abort_flag, p.status, kStatusTimeoutFull);
-      const uint32_t ka = sbase + Cfg::kOffK, va = sbase + Cfg::kOffV;
+      // descriptors advance by 16-byte units: only their address field changes
+      const uint64_t k_desc = make_smem_desc_sw128(sbase + Cfg::kOffK, 16, 1024), v_desc = make_smem_desc_sw128(sbase + Cfg::kOffV, 16, 1024);
+      const uint64_t q_desc = make_smem_desc_sw128(sbase + Cfg::kOffQ, 16, 1024), do_desc = make_smem_desc_sw128(sbase + Cfg::kOffDO, 16, 1024);
       const bool tr = p.trace != nullptr && kv_blk == 0 && hkv == 0 && b == 0;
       long long tm[4] = {0, 0, 0, 0};
       for (int it = 0; ok && it < n_iter; ++it) {
-        const int s = it % ST;
-        const uint32_t par = (it / ST) & 1;
+        const int qs = it % QS, ds = it % DS;
         const uint32_t ipar = it & 1;
-        const uint32_t qa = sbase + Cfg::kOffQ + s * Cfg::kTile;
-        const uint32_t doa = sbase + Cfg::kOffDO + s * Cfg::kTile;
+        const uint64_t qd = q_desc + uint64_t(qs * (Cfg::kTile >> 4)), dod = do_desc + uint64_t(ds * (Cfg::kTile >> 4));
         long long c0 = tr ? clock64() : 0;
-        if (!mbar_wait(qdo_full(s), par, abort_flag, p.status, kStatusTimeoutFull)) { ok = false; break; }
+        if (!mbar_wait(q_full(qs), uint32_t(it / QS) & 1u, abort_flag, p.status, kStatusTimeoutFull)) { ok = false; break; }
         if (tr) { const long long c1 = clock64(); tm[0] += c1 - c0; c0 = c1; }
         if (!mbar_wait(sdp_free, ipar ^ 1u, abort_flag, p.status, kStatusTimeoutTmemEmpty)) { ok = false; break; }
         if (tr) { const long long c1 = clock64(); tm[1] += c1 - c0; c0 = c1; }
-        if (Cfg::kDqAliasesS) {
-          if (!mbar_wait(dq_free, ipar ^ 1u, abort_flag, p.status, kStatusTimeoutTmemEmpty)) { ok = false; break; }
-        }
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off = (k / 4) * (128 * 128) + (k % 4) * 32;
-          umma_f16_ss(tmem_base + Cfg::kColS, make_smem_desc_sw128(qa + off, 16, 1024),
-                      make_smem_desc_sw128(ka + off, 16, 1024), idesc_sd, k > 0 ? 1u : 0u);
+          const uint64_t off = ((k / 4) * (128 * 128) + (k % 4) * 32) >> 4;
+          umma_f16_ss(tmem_base + Cfg::kColS, qd + off, k_desc + off, idesc_sd, k > 0 ? 1u : 0u);
         }
+        if (Cfg::kDqOverDp && !mbar_wait(dq_free(0), ipar ^ 1u, abort_flag, p.status, kStatusTimeoutTmemEmpty)) { ok = false; break; }
+        if (!mbar_wait(do_full(ds), uint32_t(it / DS) & 1u, abort_flag, p.status, kStatusTimeoutFull)) { ok = false; break; }
+        if (tr) { const long long c1 = clock64(); tm[2] += c1 - c0; c0 = c1; }
+        tc_fence_after();
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off = (k / 4) * (128 * 128) + (k % 4) * 32;
-          umma_f16_ss(tmem_base + Cfg::kColDP, make_smem_desc_sw128(doa + off, 16, 1024),
-                      make_smem_desc_sw128(va + off, 16, 1024), idesc_sd, k > 0 ? 1u : 0u);
+          const uint64_t off = ((k / 4) * (128 * 128) + (k % 4) * 32) >> 4;
+          umma_f16_ss(tmem_base + Cfg::kColDP, dod + off, v_desc + off, idesc_sd, k > 0 ? 1u : 0u);
         }
         umma_commit(sdp_full);
       }
       if (tr) {
-        // MMA thread: wait for Q/dO, for S/dP to be read, for P/dS
+        // MMA thread: wait for Q, for S / dP (and dQ) to be read, for dO
         p.trace[8] = tm[0]; p.trace[9] = tm[1]; p.trace[10] = tm[2];
       }
     }
-  } else if (warp == 11) {
-    // ---------------------------------------------------------------- third MMA issuer: dQ_i = dS K
-    if (lane == 0 && n_iter > 0) {
-      constexpr uint32_t idesc_dq = make_idesc_f16(128, D, 1, 0, 1);    // A K-major, B N-major
-      const uint32_t ka = sbase + Cfg::kOffK, dsa = sbase + Cfg::kOffDS;
-      bool ok = mbar_wait(kv_full, 0, abort_flag, p.status, kStatusTimeoutFull);
-      for (int it = 0; ok && it < n_iter; ++it) {
-        const uint32_t ipar = it & 1;
-        if (!mbar_wait(pds_full, ipar, abort_flag, p.status, kStatusTimeoutTmemFull)) break;
-        if (!Cfg::kDqAliasesS) {
-          // dQ buffer it & 1 was last used by iteration it - 2
-          if (!mbar_wait((it & 1) ? dq_free1 : dq_free, ((uint32_t(it) >> 1) & 1u) ^ 1u, abort_flag, p.status,
-                         kStatusTimeoutTmemEmpty)) break;
-        }
-        tc_fence_after();
-#pragma unroll
-        for (int k = 0; k < kFbBlock / 16; ++k) {   // K dimension = the 128 keys
-          const uint64_t adesc = make_smem_desc_sw128(dsa + (k / 4) * (128 * 128) + (k % 4) * 32, 16, 1024);
-          const uint64_t bdesc = make_smem_desc_sw128(ka + k * (16 * 128), 128 * 128, 1024);
-          umma_f16_ss(tmem_base + Cfg::kColDQ + (Cfg::kDeferDq ? (it & 1) * D : 0), adesc, bdesc, idesc_dq, k > 0 ? 1u : 0u);
-        }
-        umma_commit(pds_empty);
-        umma_commit((Cfg::kDeferDq && (it & 1)) ? dq_full1 : dq_full);
-        if (it == n_iter - 1) umma_commit(dkv_full);
-      }
-    }
   } else if (warp == 10) {
-    // ---------------------------------------------------------------- second MMA issuer: dV += P^T dO, dK += dS^T Q
-    // Issuing a tcgen05.mma costs its thread on the order of a hundred cycles whatever the tile width, and in this
-    // kernel the issue time sits on the critical chain (the exp phase of the next iteration waits for all of them):
-    // the 16 dV / dK MMAs of an iteration go out from this thread while warp 1 issues dQ and the next S / dP.
-    if (lane == 0 && n_iter > 0) {
+    // ---------------------------------------------------------------- second MMA issuer: dV += P^T dO, dQ = dS K, dK += dS^T Q
+    // dV frees dO and P, which the next block's loads and dQ's way out wait for; dQ is read and written out while the tensor core
+    // works on dK, and the next dP needs its columns.
+    if (n_iter > 0 && elect_one()) {
       constexpr uint32_t idesc_kv = make_idesc_f16(128, D, 1, 1, 1);    // A M-major, B N-major
-      const uint32_t pa = sbase + Cfg::kOffP, dsa = sbase + Cfg::kOffDS;
+      constexpr uint32_t idesc_dq = make_idesc_f16(128, D, 1, 0, 1);    // A K-major, B N-major
+      const uint64_t dsq_desc = make_smem_desc_sw128(sbase + Cfg::kOffDS, 16, 1024), k_desc = make_smem_desc_sw128(sbase + Cfg::kOffK, 128 * 128, 1024);
+      const uint64_t p_desc = make_smem_desc_sw128(sbase + Cfg::kOffP, 128 * 128, 1024), ds_desc = make_smem_desc_sw128(sbase + Cfg::kOffDS, 128 * 128, 1024);
+      const uint64_t q_desc = make_smem_desc_sw128(sbase + Cfg::kOffQ, 128 * 128, 1024), do_desc = make_smem_desc_sw128(sbase + Cfg::kOffDO, 128 * 128, 1024);
       for (int it = 0; it < n_iter; ++it) {
-        const int s = it % ST;
+        const int qs = it % QS, ds = it % DS;
         const uint32_t ipar = it & 1;
-        const uint32_t qa = sbase + Cfg::kOffQ + s * Cfg::kTile;
-        const uint32_t doa = sbase + Cfg::kOffDO + s * Cfg::kTile;
+        const uint64_t qd = q_desc + uint64_t(qs * (Cfg::kTile >> 4)), dod = do_desc + uint64_t(ds * (Cfg::kTile >> 4));
         // P / dS ready implies Q / dO of this stage are in shared memory (S and dP were computed from them)
         if (!mbar_wait(pds_full, ipar, abort_flag, p.status, kStatusTimeoutTmemFull)) break;
+        // two buffers: this one was last used by iteration it - 2; over dP: the scores of this iteration waited for it
+        if (Cfg::kTwoDq && !mbar_wait(dq_free(it & 1), ((uint32_t(it) >> 1) & 1u) ^ 1u, abort_flag, p.status, kStatusTimeoutTmemEmpty)) break;
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < kFbBlock / 16; ++k) {   // K dimension = the 128 query rows, 16 rows per instruction
-          const uint32_t koff = k * (16 * 128);
-          umma_f16_ss(tmem_base + Cfg::kColDV, make_smem_desc_sw128(pa + koff, 128 * 128, 1024),
-                      make_smem_desc_sw128(doa + koff, 128 * 128, 1024), idesc_kv, (it > 0 || k > 0) ? 1u : 0u);
+          const uint64_t koff = k * (16 * 128) >> 4;
+          umma_f16_ss(tmem_base + Cfg::kColDV, p_desc + koff, dod + koff, idesc_kv, (it > 0 || k > 0) ? 1u : 0u);
         }
+        umma_commit(do_empty(ds));
+        umma_commit(p_empty);
+#pragma unroll
+        for (int k = 0; k < kFbBlock / 16; ++k)   // K dimension = the 128 keys
+          umma_f16_ss(tmem_base + Cfg::kColDQ + (Cfg::kTwoDq ? (it & 1) * D : 0), dsq_desc + uint64_t(((k / 4) * (128 * 128) + (k % 4) * 32) >> 4),
+                      k_desc + uint64_t(k * (16 * 128) >> 4), idesc_dq, k > 0 ? 1u : 0u);
+        umma_commit(dq_full(Cfg::kTwoDq ? it & 1 : 0));
 #pragma unroll
         for (int k = 0; k < kFbBlock / 16; ++k) {
-          const uint32_t koff = k * (16 * 128);
-          umma_f16_ss(tmem_base + Cfg::kColDK, make_smem_desc_sw128(dsa + koff, 128 * 128, 1024),
-                      make_smem_desc_sw128(qa + koff, 128 * 128, 1024), idesc_kv, (it > 0 || k > 0) ? 1u : 0u);
+          const uint64_t koff = k * (16 * 128) >> 4;
+          umma_f16_ss(tmem_base + Cfg::kColDK, ds_desc + koff, qd + koff, idesc_kv, (it > 0 || k > 0) ? 1u : 0u);
         }
-        umma_commit(qdo_empty(s));
-        umma_commit(pds_empty);
+        umma_commit(q_empty(qs));
+        umma_commit(ds_empty);
         if (it == n_iter - 1) umma_commit(dkv_full);
       }
     }
-  } else {
+  } else if (warp >= 12) {
+    // ---------------------------------------------------------------- dQ: tensor memory -> shared memory -> added to the accumulator
+    const int quarter = warp & 3;
+    const uint32_t lane_base = uint32_t(quarter * 32) << 16;
+    uint8_t* tile = smem + Cfg::kOffDqStage + quarter * (2 * Cfg::kDqTile);
+    bool ok = true, pending = false;   // pending: a reduction that reads the staging area may be in flight
+    int hh = 0, jj = 0;
+    for (int it = 0; it < n_iter; ++it) {
+      const int buf = Cfg::kTwoDq ? it & 1 : 0;
+      const int h = hkv * G + hh;
+      int owner, q0, qbase;
+      locate(jj, owner, q0, qbase);
+      if (++jj == per_head) { jj = 0; ++hh; }
+      ok = __all_sync(0xffffffffu, mbar_wait(dq_full(buf), uint32_t(Cfg::kTwoDq ? it >> 1 : it) & 1u, abort_flag, p.status, kStatusTimeoutTmemFull));
+      if (!ok) break;
+      tc_fence_after();
+      const bool local = owner == p.cp_rank;
+      const int q_idx = q0 + quarter * 32 + lane;
+      float* dq_row = (p.cp_world == 1 ? p.dq_acc[0] : p.dq_acc[owner]) + (((long long)b * p.Tq + q_idx) * p.Hq + h) * D;
+#pragma unroll
+      for (int half = 0; half < D / 64; ++half) {
+        uint32_t dq[2][32];
+        tmem_ld_32x32(tmem_base + lane_base + Cfg::kColDQ + buf * D + half * 64, dq[0]);
+        tmem_ld_32x32(tmem_base + lane_base + Cfg::kColDQ + buf * D + half * 64 + 32, dq[1]);
+        tmem_ld_wait();
+        if (half == D / 64 - 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(dq_free(buf));
+        }
+        if (local) {
+          uint8_t* to = tile + half * Cfg::kPTile;
+          if (Cfg::kStageAliasesP) {
+            // the staging area is the P, then the dS tile: the MMAs of this iteration must be done with it
+            ok = __all_sync(0xffffffffu, mbar_wait(half == 0 ? p_empty : ds_empty, uint32_t(it) & 1u, abort_flag, p.status, kStatusTimeoutTmemEmpty));
+            if (!ok) break;
+          } else {
+            if (pending && lane == 0) bulk_wait_read0();
+            __syncwarp();
+          }
+#pragma unroll
+          for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int u = 0; u < 8; ++u)   // row `lane` of the box, 16-byte units swizzled like the tensor map expects
+              *reinterpret_cast<uint4*>(to + x * Cfg::kDqTile + lane * 128 + ((u ^ (lane & 7)) * 16)) =
+                  make_uint4(dq[x][u * 4], dq[x][u * 4 + 1], dq[x][u * 4 + 2], dq[x][u * 4 + 3]);
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) {
+#pragma unroll
+            for (int x = 0; x < 2; ++x)   // rows past Tq are clipped by the copy engine
+              tma_reduce_add_4d(&tmDQ, smem_u32(to + x * Cfg::kDqTile), half * 64 + x * 32, h, q0 + quarter * 32, b);
+            bulk_commit();
+          }
+          pending = true;
+        } else if (q_idx < p.Tq) {
+#pragma unroll
+          for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              red_add_v4(dq_row + half * 64 + x * 32 + u * 4, __uint_as_float(dq[x][u * 4]), __uint_as_float(dq[x][u * 4 + 1]),
+                         __uint_as_float(dq[x][u * 4 + 2]), __uint_as_float(dq[x][u * 4 + 3]));
+        }
+      }
+      if (!ok) break;
+      if (Cfg::kStageAliasesP && lane == 0) {
+        bulk_wait_read1();
+        mbar_arrive(stg_p);
+        bulk_wait_read0();
+        mbar_arrive(stg_ds);
+      }
+    }
+    if (pending && lane == 0) bulk_wait_all0();   // shared memory must outlive the reductions that read it
+  } else if (warp < 10) {
     // ---------------------------------------------------------------- compute warps
     // Two warps share each TMEM lane quarter (a warp may only touch lanes 32*(warp%4)..+31); they split the columns.
     const int quarter = warp & 3;
@@ -407,93 +481,29 @@ flash_bwd_kernel(const __grid_constant__ QMaps qm, const __grid_constant__ CUten
     long long tc[6] = {0, 0, 0, 0, 0, 0};
     // Row statistics are fetched one iteration ahead (the global-load latency is off the chain); the position of an
     // iteration (query head, block within the head) is advanced with counters, not divisions.
-    const bool single = (p.cp_world == 1);
-    const float* lse0 = p.lse[0];
-    const float* delta0 = p.delta[0];
-    float* dq0 = p.dq_acc[0];
+    const long long stat0 = ((long long)b * p.Hq + hkv * G) * p.Tq;      // of this KV head's first query head
+    const float* lse0 = p.lse[0] + stat0;
+    const float* delta0 = p.delta[0] + stat0;
     auto fetch_stats = [&](int hh, int jj, float& lse_raw, float& dl) {
       lse_raw = 0.f; dl = 0.f;
       if (hh >= G) return;
-      const int h = hkv * G + hh;
       int owner, q0, qbase;
       locate(jj, owner, q0, qbase);
       const int q_idx = q0 + row;
       if (q_idx < p.Tq) {
-        const long long si = ((long long)b * p.Hq + h) * p.Tq + q_idx;
+        const int at = hh * p.Tq + q_idx;
         // (indexing the pointer arrays of the kernel parameters with a run-time rank makes the compiler copy them to
         // local memory: the single-rank case reads element 0 directly)
-        lse_raw = single ? lse0[si] : p.lse[owner][si];
-        dl = single ? delta0[si] : p.delta[owner][si];
+        lse_raw = single ? lse0[at] : p.lse[owner][stat0 + at];
+        dl = single ? delta0[at] : p.delta[owner][stat0 + at];
       }
     };
     float lse_next, dlt_next;
     int hh_next = 0, jj_next = 0;   // position of the iteration whose statistics are in lse_next / dlt_next
     fetch_stats(n_iter > 0 ? 0 : G, 0, lse_next, dlt_next);
-    bool dq_pending = false;   // this thread has a bulk reduction in flight that reads its staging piece
-    // This warp's 32 x (D / 2) piece of one dQ tile: TMEM -> registers -> global accumulator; the TMEM buffer is
-    // released as soon as the values are in registers.
-    auto emit_dq = [&](int buf, float* dq_row, bool valid, bool local, int h_, int q0_) {
-      if (Cfg::kBulkDq && local) {
-        uint8_t* tile = smem + Cfg::kOffDqStage + (warp - 2) * (Cfg::kDqBoxes * Cfg::kDqTile);
-        if (!Cfg::kStageAliasesP && dq_pending) {   // the previous reduction has finished reading the tile
-          if (lane == 0) bulk_wait_read0();
-          __syncwarp();
-        }
-#pragma unroll
-        for (int bx = 0; bx < Cfg::kDqBoxes; ++bx) {
-          uint32_t dq[32];
-          tmem_ld_32x32(tmem_base + lane_base + Cfg::kColDQ + buf * D + (half * Cfg::kDqBoxes + bx) * 32, dq);
-          tmem_ld_wait();
-          if (bx == Cfg::kDqBoxes - 1) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(buf ? dq_free1 : dq_free);
-          }
-          if (p.dbg >= 2) continue;
-#pragma unroll
-          for (int u = 0; u < 8; ++u)   // row `lane` of the box, 16-byte units swizzled like the tensor map expects
-            *reinterpret_cast<uint4*>(tile + bx * Cfg::kDqTile + lane * 128 + ((u ^ (lane & 7)) * 16)) =
-                make_uint4(dq[u * 4], dq[u * 4 + 1], dq[u * 4 + 2], dq[u * 4 + 3]);
-        }
-        if (p.dbg >= 2) return;
-        fence_proxy_async();
-        __syncwarp();
-        dq_pending = false;
-        if (p.dbg == 0) {
-          if (lane == 0) {
-#pragma unroll
-            for (int bx = 0; bx < Cfg::kDqBoxes; ++bx)   // rows past Tq are clipped by the copy engine
-              tma_reduce_add_4d(&tmDQ, smem_u32(tile + bx * Cfg::kDqTile), (half * Cfg::kDqBoxes + bx) * 32, h_,
-                                q0_ + quarter * 32, b);
-            bulk_commit();
-          }
-          dq_pending = true;
-        }
-      } else {
-#pragma unroll 1
-        for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
-          uint32_t dq[32];
-          tmem_ld_32x32(tmem_base + lane_base + Cfg::kColDQ + buf * D + c * 32, dq);
-          tmem_ld_wait();
-          if (valid) {
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-              red_add_v4(dq_row + c * 32 + u * 4, __uint_as_float(dq[u * 4]), __uint_as_float(dq[u * 4 + 1]),
-                         __uint_as_float(dq[u * 4 + 2]), __uint_as_float(dq[u * 4 + 3]));
-          }
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(buf ? dq_free1 : dq_free);
-      }
-    };
-    float* prev_row = nullptr;   // deferred-dQ flow: where the previous iteration's dQ row goes
-    bool prev_valid = false, prev_local = true;
-    int prev_h = 0, prev_q0 = 0;
     for (int it = 0; it < n_iter; ++it) {
       long long c0 = tr ? clock64() : 0;
       const uint32_t ipar = it & 1;
-      const int h = hkv * G + hh_next;
       int owner, q0, qbase;
       locate(jj_next, owner, q0, qbase);
       const int q_idx = q0 + row;
@@ -507,109 +517,75 @@ flash_bwd_kernel(const __grid_constant__ QMaps qm, const __grid_constant__ CUten
       ok = __all_sync(0xffffffffu, mbar_wait(sdp_full, ipar, abort_flag, p.status, kStatusTimeoutTmemFull));
       if (!ok) break;
       if (tr) { const long long c1 = clock64(); tc[1] += c1 - c0; c0 = c1; }   // waiting for S / dP
-      // P / dS tiles are free once the MMAs of the previous iteration have executed.
-      ok = __all_sync(0xffffffffu, mbar_wait(pds_empty, ipar ^ 1u, abort_flag, p.status, kStatusTimeoutTmemEmpty));
-      if (!ok) break;
-      if (Cfg::kStageAliasesP && it > 0) {
-        // ... and once every warp's dQ reduction of the previous iteration has finished reading them
-        if (lane == 0) {
-          if (dq_pending) bulk_wait_read0();
-          mbar_arrive(stg_free);
-        }
-        ok = __all_sync(0xffffffffu, mbar_wait(stg_free, uint32_t(it - 1) & 1u, abort_flag, p.status, kStatusTimeoutLocalFlag));
-        if (!ok) break;
-      }
-      if (tr) { const long long c1 = clock64(); tc[2] += c1 - c0; c0 = c1; }   // waiting for the P / dS tiles
       tc_fence_after();
-      uint8_t* prow = smem + Cfg::kOffP + (row >> 3) * 1024 + (row & 7) * 128;
-      uint8_t* dsrow = smem + Cfg::kOffDS + (row >> 3) * 1024 + (row & 7) * 128;
-#pragma unroll 1
-      for (int c = 2 * half; c < 2 * half + 2; ++c) {
-        uint32_t sv[32], dp[32];
-        tmem_ld_32x32(tmem_base + lane_base + Cfg::kColS + c * 32, sv);
-        tmem_ld_32x32(tmem_base + lane_base + Cfg::kColDP + c * 32, dp);
+      const bool live = q_valid && lse2 != -INFINITY;
+      const float dlt_s = dlt * p.scale;
+      const uint64_t c2 = pack_f32x2(p.scale_log2, p.scale_log2), l2 = pack_f32x2(-lse2, -lse2);
+      const uint64_t s2 = pack_f32x2(p.scale, p.scale), d2 = pack_f32x2(-dlt_s, -dlt_s);
+      uint8_t* prow = smem + Cfg::kOffP + (row >> 3) * 1024 + (row & 7) * 128 + half * (128 * 128);
+      uint8_t* dsrow = smem + Cfg::kOffDS + (row >> 3) * 1024 + (row & 7) * 128 + half * (128 * 128);
+      uint32_t dw[32];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t sv[32], dp[32], pw[16];
+        tmem_ld_32x32(tmem_base + lane_base + Cfg::kColS + (2 * half + c) * 32, sv);
+        tmem_ld_32x32(tmem_base + lane_base + Cfg::kColDP + (2 * half + c) * 32, dp);
         tmem_ld_wait();
-        if (c == 2 * half + 1) {   // S / dP are in registers: the next iteration's score products may overwrite them
+        if (c == 1) {   // S / dP are in registers: the next iteration's score products may overwrite them
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(sdp_free);
         }
-        const bool live = q_valid && lse2 != -INFINITY;
-        const float dlt_s = dlt * p.scale;
-        if (live && kv0 + c * 32 + 31 <= limit) {   // every column of the chunk is visible: no per-element test
+        auto weights = [&](auto masked) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const float pv = ex2_approx(fmaf(__uint_as_float(sv[i]), p.scale_log2, -lse2));
-            const float ds = pv * fmaf(__uint_as_float(dp[i]), p.scale, -dlt_s);
-            sv[i] = __float_as_uint(pv);
-            dp[i] = __float_as_uint(ds);
+          for (int i = 0; i < 16; ++i) {
+            float e0, e1, g0, g1;
+            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), c2, l2), e0, e1);
+            e0 = ex2_approx(e0);
+            e1 = ex2_approx(e1);
+            if constexpr (decltype(masked)::value) {
+              const int kv_idx = kv0 + (2 * half + c) * 32 + 2 * i;
+              e0 = live && kv_idx <= limit ? e0 : 0.f;
+              e1 = live && kv_idx + 1 <= limit ? e1 : 0.f;
+            }
+            unpack_f32x2(mul_f32x2(pack_f32x2(e0, e1), fma_f32x2(pack_f32x2(__uint_as_float(dp[2 * i]), __uint_as_float(dp[2 * i + 1])), s2, d2)), g0, g1);
+            pw[i] = pack_bf16x2(e0, e1);
+            dw[c * 16 + i] = pack_bf16x2(g0, g1);
           }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int kv_idx = kv0 + c * 32 + i;
-            float pv = 0.f;
-            if (live && kv_idx <= limit) pv = ex2_approx(fmaf(__uint_as_float(sv[i]), p.scale_log2, -lse2));
-            const float ds = pv * fmaf(__uint_as_float(dp[i]), p.scale, -dlt_s);
-            sv[i] = __float_as_uint(pv);
-            dp[i] = __float_as_uint(ds);
-          }
+        };
+        // every column of the chunk is visible to every row of the warp: no per-element test
+        if (__all_sync(0xffffffffu, live && kv0 + (2 * half + c) * 32 + 31 <= limit)) weights(std::false_type{});
+        else weights(std::true_type{});
+        if (c == 0) {
+          if (tr) { const long long c1 = clock64(); tc[3] += c1 - c0; c0 = c1; }
+          // The tiles are waited for only when there is something to store: they are free once the MMAs of the previous iteration have
+          // executed and, where dQ is staged there, its reductions have finished reading.
+          ok = __all_sync(0xffffffffu, mbar_wait(p_empty, ipar ^ 1u, abort_flag, p.status, kStatusTimeoutTmemEmpty));
+          if (ok && Cfg::kStageAliasesP && it > 0)
+            ok = __all_sync(0xffffffffu, mbar_wait(stg_p, uint32_t(it - 1) & 1u, abort_flag, p.status, kStatusTimeoutLocalFlag));
+          if (!ok) break;
+          if (tr) { const long long c1 = clock64(); tc[2] += c1 - c0; c0 = c1; }   // waiting for the P tile
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          uint4 w, z;
-          w.x = pack_bf16x2(__uint_as_float(sv[u * 8 + 0]), __uint_as_float(sv[u * 8 + 1]));
-          w.y = pack_bf16x2(__uint_as_float(sv[u * 8 + 2]), __uint_as_float(sv[u * 8 + 3]));
-          w.z = pack_bf16x2(__uint_as_float(sv[u * 8 + 4]), __uint_as_float(sv[u * 8 + 5]));
-          w.w = pack_bf16x2(__uint_as_float(sv[u * 8 + 6]), __uint_as_float(sv[u * 8 + 7]));
-          z.x = pack_bf16x2(__uint_as_float(dp[u * 8 + 0]), __uint_as_float(dp[u * 8 + 1]));
-          z.y = pack_bf16x2(__uint_as_float(dp[u * 8 + 2]), __uint_as_float(dp[u * 8 + 3]));
-          z.z = pack_bf16x2(__uint_as_float(dp[u * 8 + 4]), __uint_as_float(dp[u * 8 + 5]));
-          z.w = pack_bf16x2(__uint_as_float(dp[u * 8 + 6]), __uint_as_float(dp[u * 8 + 7]));
-          const int col16 = c * 4 + u;
-          const int chunk = col16 >> 3;
-          const int unit = (col16 & 7) ^ (row & 7);
-          *reinterpret_cast<uint4*>(prow + chunk * (128 * 128) + unit * 16) = w;
-          *reinterpret_cast<uint4*>(dsrow + chunk * (128 * 128) + unit * 16) = z;
-        }
+        for (int u = 0; u < 4; ++u)
+          *reinterpret_cast<uint4*>(prow + ((c * 4 + u) ^ (row & 7)) * 16) = make_uint4(pw[u * 4], pw[u * 4 + 1], pw[u * 4 + 2], pw[u * 4 + 3]);
       }
+      if (!ok) break;
+      if (tr) { const long long c1 = clock64(); tc[3] += c1 - c0; c0 = c1; }
+      ok = __all_sync(0xffffffffu, mbar_wait(ds_empty, ipar ^ 1u, abort_flag, p.status, kStatusTimeoutTmemEmpty));
+      if (ok && Cfg::kStageAliasesP && it > 0)
+        ok = __all_sync(0xffffffffu, mbar_wait(stg_ds, uint32_t(it - 1) & 1u, abort_flag, p.status, kStatusTimeoutLocalFlag));
+      if (!ok) break;
+      if (tr) { const long long c1 = clock64(); tc[4] += c1 - c0; c0 = c1; }   // waiting for the dS tile
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        *reinterpret_cast<uint4*>(dsrow + (u ^ (row & 7)) * 16) = make_uint4(dw[u * 4], dw[u * 4 + 1], dw[u * 4 + 2], dw[u * 4 + 3]);
       // one arrival per warp: 256 same-address arrivals on a shared-memory barrier serialise
       tc_fence_before();
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(pds_full);
       if (tr) { const long long c1 = clock64(); tc[3] += c1 - c0; c0 = c1; }   // exp / dS / stores to shared memory
-      if (Cfg::kDeferDq) {
-        // While the tensor core works on dV / dK / dQ of this iteration and S / dP of the next, write out dQ of the
-        // PREVIOUS iteration: it is complete (S / dP of this iteration were committed after it), and its transfer
-        // TMEM -> registers -> shared memory -> TMA reduction is off the critical chain here.
-        if (it > 0) {
-          ok = __all_sync(0xffffffffu, mbar_wait(((it - 1) & 1) ? dq_full1 : dq_full, (uint32_t(it - 1) >> 1) & 1u, abort_flag,
-                                                 p.status, kStatusTimeoutTmemFull));
-          if (!ok) break;
-          tc_fence_after();
-          emit_dq((it - 1) & 1, prev_row, prev_valid, prev_local, prev_h, prev_q0);
-          if (tr) { const long long c1 = clock64(); tc[5] += c1 - c0; c0 = c1; }
-        }
-        prev_row = (single ? dq0 : p.dq_acc[owner]) + (((long long)b * p.Tq + q_idx) * p.Hq + h) * D;
-        prev_valid = q_valid;
-        prev_local = (owner == p.cp_rank);
-        prev_h = h; prev_q0 = q0;
-        continue;
-      }
-      // dQ_i
-      ok = __all_sync(0xffffffffu, mbar_wait(dq_full, ipar, abort_flag, p.status, kStatusTimeoutTmemFull));
-      if (!ok) break;
-      if (tr) { const long long c1 = clock64(); tc[4] += c1 - c0; c0 = c1; }   // waiting for dQ
-      if (Cfg::kStageAliasesP) {
-        // the staging area is the P / dS tiles: the dV / dK MMAs of the other issuer must be done with them too
-        ok = __all_sync(0xffffffffu, mbar_wait(pds_empty, ipar, abort_flag, p.status, kStatusTimeoutTmemEmpty));
-        if (!ok) break;
-      }
-      tc_fence_after();
-      emit_dq(0, (single ? dq0 : p.dq_acc[owner]) + (((long long)b * p.Tq + q_idx) * p.Hq + h) * D, q_valid,
-              owner == p.cp_rank, h, q0);
-      if (tr) { const long long c1 = clock64(); tc[5] += c1 - c0; c0 = c1; }   // dQ read + reduction
     }
     if (tr) {
       for (int i = 0; i < 6; ++i) p.trace[i] = tc[i];
@@ -617,11 +593,6 @@ flash_bwd_kernel(const __grid_constant__ QMaps qm, const __grid_constant__ CUten
     }
     // ---------------------------------------------------------------- dK / dV epilogue (row = key index)
     if (ok && n_iter > 0) ok = __all_sync(0xffffffffu, mbar_wait(dkv_full, 0, abort_flag, p.status, kStatusTimeoutTmemFull));
-    if (Cfg::kDeferDq && ok && n_iter > 0) {
-      tc_fence_after();
-      emit_dq((n_iter - 1) & 1, prev_row, prev_valid, prev_local, prev_h, prev_q0);   // dQ of the last iteration
-    }
-    if (dq_pending && lane == 0) bulk_wait_all0();   // shared memory must outlive the reductions that read it
     if (ok) {
       if (n_iter > 0) tc_fence_after();
       const int kv_idx = kv0 + row;
@@ -751,7 +722,6 @@ static int bwd_main(const void* const* q_ptrs, const void* k, const void* v, con
   p.causal = causal;
   p.status = device_status_word();
   p.trace = g_bwd_trace;
-  p.dbg = 0;
   // fp32 dQ accumulator of this rank, [B, Tq, Hq, D]: boxes of 32 rows x 32 columns (128 bytes, swizzled)
   CUtensorMap tdq;
   r = encode_tmap_4d(&tdq, dq_acc_ptrs[cp_rank], 4, D, Hq, Tq, B, (uint64_t)D * 4, (uint64_t)Hq * D * 4,

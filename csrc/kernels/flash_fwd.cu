@@ -79,26 +79,6 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
   return y;
 }
-// Two floats in a register pair; one instruction works on both.
-__device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
-  uint64_t y;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(a), "f"(b));
-  return y;
-}
-__device__ __forceinline__ void unpack_f32x2(uint64_t x, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x));
-}
-__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t y;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(y) : "l"(a), "l"(b), "l"(c));
-  return y;
-}
-__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
-  uint64_t y;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(y) : "l"(a), "l"(b));
-  return y;
-}
-
 // Shared memory: the query tile, then a ring that K and V blocks go through in turn.
 template <int D, int DV, int BKV>
 struct FaFwdCfg {
