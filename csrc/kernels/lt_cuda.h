@@ -258,6 +258,8 @@ int lt_kv_append(const void* k_new, const void* v_new, void* k_cache, void* v_ca
 // ---- pointwise.cu: RoPE, SwiGLU, GELU, embedding, casts, axpby
 int lt_rope(void* x, const float* cos_t, const float* sin_t, const int* pos, long long rows, int T, int heads, int hd,
             long long row_stride, int backward, void* stream);
+int lt_rope_append(void* qkv, long long ld, const float* cos_t, const float* sin_t, const int* pos, const int* slots, void* q_out, void* k_cache,
+                   void* v_cache, long long rows, int Hq, int Hkv, int hd, int block_size, int kv_fp8, float k_scale, float v_scale, void* stream);
 int lt_swiglu_fwd(const void* gu, void* h, long long M, int F, void* stream);
 int lt_clamped_glu(int fp32, const void* gu, void* h, long long M, int F, float limit, float slope, void* stream);
 int lt_act_glu(int fp32, const void* gu, void* h, long long M, int F, int act, const int* live, int block_rows, void* stream);

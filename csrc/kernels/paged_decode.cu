@@ -13,6 +13,7 @@
 
 #include "common/host.h"
 #include "common/ptx.cuh"
+#include "common/scalar.cuh"
 
 namespace lt {
 
@@ -855,20 +856,33 @@ __global__ void paged_decode_merge_kernel(const float* __restrict__ part, __nv_b
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
   constexpr int E = D / 32;
+  // A lane reads maximum and sum of one split, so that their loads are under way together, as are then those of the outputs (one split
+  // after another: 5.4 us for 32 rows of 16 splits, two thirds of them waiting).
+  const float* p0 = part + (long long)row * splits * (D + 2);
   float gm = -INFINITY;
-  for (int sp = 0; sp < splits; ++sp) gm = fmaxf(gm, part[((long long)row * splits + sp) * (D + 2) + D]);
+  for (int sp = lane; sp < splits; sp += 32) gm = fmaxf(gm, p0[(long long)sp * (D + 2) + D]);
+  gm = warp_max(gm);
   float wsum = 0.f, acc[E];
 #pragma unroll
   for (int i = 0; i < E; ++i) acc[i] = 0.f;
-  for (int sp = 0; sp < splits; ++sp) {
-    const float* p = part + ((long long)row * splits + sp) * (D + 2);
-    const float l = p[D + 1];
-    if (l <= 0.f) continue;
-    const float w = l * __expf(p[D] - gm);
+  for (int s0 = 0; s0 < splits; s0 += 32) {
+    const float* p = p0 + (long long)s0 * (D + 2);
+    const int n = min(32, splits - s0);
+    float w = 0.f;
+    if (lane < n) {
+      const float l = p[(long long)lane * (D + 2) + D + 1];
+      if (!(l <= 0.f)) w = l * __expf(p[(long long)lane * (D + 2) + D] - gm);
+    }
     wsum += w;
+#pragma unroll 8
+    for (int j = 0; j < n; ++j) {
+      const float wj = __shfl_sync(0xffffffffu, w, j);
+      // a split without keys has outputs of zero
 #pragma unroll
-    for (int i = 0; i < E; ++i) acc[i] += w * p[lane * E + i];
+      for (int i = 0; i < E; ++i) acc[i] += wj * p[(long long)j * (D + 2) + lane * E + i];
+    }
   }
+  wsum = warp_sum(wsum);
   float inv = wsum > 0.f ? 1.f / wsum : 0.f;
   if (gate) inv /= 1.f + expf(-__bfloat162float(gate[(row / Hq) * ldg + row % Hq]));     // times sigmoid(gate) of this head
 #pragma unroll

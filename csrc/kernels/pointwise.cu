@@ -7,6 +7,8 @@
 // The reference has no SiLU/SwiGLU; it is added because the Llama-style configurations need it.
 // Every kernel moves 16 bytes per thread per access and grid-strides.
 #include "lt_cuda.h"
+
+#include <cuda_fp8.h>
 #include "common/host.h"
 #include "common/ptx.cuh"
 #include "common/scalar.cuh"
@@ -54,6 +56,55 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restri
       o[2 * j + 1] = f[2 * j] * s[j] + f[2 * j + 1] * c[j];
     }
     st8(p, o);
+  }
+}
+
+// Rotation of queries and keys and the write of keys and values into a paged cache, in one pass over the rows [q | k | v] of a product.
+// Queries go to q_out, packed, or stay where they are (q_out nullptr: keys are then rotated in place too, for a prompt's own attention).
+// A launch for each of these (two rotations, two or three copies, the write) took 9 to 16 us a layer of a decode step, this one 2.
+template <bool FP8>
+__global__ void rope_append_kernel(__nv_bfloat16* __restrict__ qkv, long long ld, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                                   const int* __restrict__ pos, const int* __restrict__ slots, __nv_bfloat16* __restrict__ q_out,
+                                   void* __restrict__ k_cache, void* __restrict__ v_cache, long long rows, int Hq, int Hkv, int hd, int block_size,
+                                   float k_inv, float v_inv) {
+  const int vph = hd / 8, heads = Hq + 2 * Hkv;
+  const long long total = rows * heads * vph;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const int v = int(i % vph);
+    const int h = int((i / vph) % heads);
+    const long long r = i / ((long long)vph * heads);
+    __nv_bfloat16* p = qkv + r * ld + (long long)h * hd + v * 8;
+    float f[8];
+    ld8(p, f);
+    if (h < Hq + Hkv) {
+      const int t = pos[r];
+      const float4 c4 = *reinterpret_cast<const float4*>(cos_t + (long long)t * (hd / 2) + v * 4);
+      const float4 s4 = *reinterpret_cast<const float4*>(sin_t + (long long)t * (hd / 2) + v * 4);
+      const float c[4] = {c4.x, c4.y, c4.z, c4.w}, s[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float a = f[2 * j], b = f[2 * j + 1];
+        f[2 * j] = a * c[j] - b * s[j];
+        f[2 * j + 1] = a * s[j] + b * c[j];
+      }
+      if (h < Hq && q_out) st8(q_out + (r * Hq + h) * (long long)hd + v * 8, f);
+      else if (!q_out) st8(p, f);
+      if (h < Hq) continue;
+    }
+    const int slot = slots[r];
+    if (slot < 0) continue;
+    const bool is_k = h < Hq + Hkv;
+    const int g = h - Hq - (is_k ? 0 : Hkv);
+    const long long dst = (((long long)(slot / block_size) * Hkv + g) * block_size + slot % block_size) * hd + v * 8;
+    if (FP8) {
+      uint8_t out[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)   // what is cached is the value as 16 bits hold it
+        out[j] = __nv_fp8_e4m3(__bfloat162float(__float2bfloat16(f[j])) * (is_k ? k_inv : v_inv)).__x;
+      *reinterpret_cast<uint2*>(static_cast<uint8_t*>(is_k ? k_cache : v_cache) + dst) = *reinterpret_cast<const uint2*>(out);
+    } else {
+      st8(static_cast<__nv_bfloat16*>(is_k ? k_cache : v_cache) + dst, f);
+    }
   }
 }
 
@@ -290,6 +341,27 @@ int lt_rope(void* x, const float* cos_t, const float* sin_t, const int* pos, lon
   if (work == 0) return 0;
   rope_kernel<<<grid_for(work, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<__nv_bfloat16*>(x), cos_t, sin_t, pos, rows, T, heads, hd, row_stride, backward ? -1.f : 1.f);
+  LT_LAUNCH_CHECK();
+  return 0;
+}
+
+// qkv: rows [Hq | Hkv | Hkv heads of hd] at pitch ld; pos, slots [rows] int32; q_out [rows, Hq, hd] or nullptr; caches as in
+// lt_kv_append.  hd and ld are multiples of 8, qkv, q_out and the caches 16-byte aligned.
+int lt_rope_append(void* qkv, long long ld, const float* cos_t, const float* sin_t, const int* pos, const int* slots, void* q_out, void* k_cache,
+                   void* v_cache, long long rows, int Hq, int Hkv, int hd, int block_size, int kv_fp8, float k_scale, float v_scale, void* stream) {
+  using namespace lt;
+  if (hd % 8 != 0 || ld % 8 != 0 || block_size < 1 ||
+      ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15))
+    return -int(kStatusBadArgument);
+  const long long work = rows * (Hq + 2 * Hkv) * (hd / 8);
+  if (work == 0) return 0;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  auto X = static_cast<__nv_bfloat16*>(qkv);
+  auto Q = static_cast<__nv_bfloat16*>(q_out);
+  if (kv_fp8)
+    rope_append_kernel<true><<<grid_for(work, 256), 256, 0, st>>>(X, ld, cos_t, sin_t, pos, slots, Q, k_cache, v_cache, rows, Hq, Hkv, hd, block_size, 1.f / k_scale, 1.f / v_scale);
+  else
+    rope_append_kernel<false><<<grid_for(work, 256), 256, 0, st>>>(X, ld, cos_t, sin_t, pos, slots, Q, k_cache, v_cache, rows, Hq, Hkv, hd, block_size, 1.f, 1.f);
   LT_LAUNCH_CHECK();
   return 0;
 }

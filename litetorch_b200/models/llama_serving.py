@@ -45,7 +45,9 @@ class LlamaKVModel(ServingModel):
             self._index = PrefixCache()
 
     # ------------------------------------------------------------------ shared layer body
-    def _layers(self, x, positions, attend):
+    def _layers(self, x, positions, slots, attend, in_place: bool):
+        """attend(i, q, k, v) of rotated queries; k and v are those of the rows, rotated only if `in_place`: a pass that reads the cache
+        alone has its queries packed instead."""
         e, cfg, w, K = self.e, self.e.cfg, self.e.w, self.e.K
         Hq, Hkv, hd = cfg.n_heads, cfg.n_kv_heads, cfg.head_dim
         n = x.shape[0]
@@ -53,15 +55,15 @@ class LlamaKVModel(ServingModel):
             p = "layers.%d." % i
             h, _, _, _ = K.norm_fwd(x, w.p(p + "attn_norm"), eps=cfg.rms_eps)
             qkv = K.gemm(h, w.p(p + "wqkv"))
-            K.rope_(qkv, e.cos, e.sin, 1, Hq, hd, col_offset=0, positions=positions)
-            K.rope_(qkv, e.cos, e.sin, 1, Hkv, hd, col_offset=Hq * hd, positions=positions)
-            q = qkv[:, :Hq * hd].view(n, Hq, hd)
+            q = K.rope_append(qkv, e.cos, e.sin, positions, slots, Hq, Hkv, hd, self.cache.k[i], self.cache.v[i], self.block_size, self.cache.fp8,
+                              self.cache.k_scale, self.cache.v_scale, in_place=in_place)
             k = qkv[:, Hq * hd:(Hq + Hkv) * hd].view(n, Hkv, hd)
             v = qkv[:, (Hq + Hkv) * hd:].view(n, Hkv, hd)
             o = attend(i, q, k, v)
             x1 = K.gemm(o.reshape(n, Hq * hd), w.p(p + "wo"), residual=x)
             h2, _, _, _ = K.norm_fwd(x1, w.p(p + "mlp_norm"), eps=cfg.rms_eps)
-            hm = K.swiglu_fwd(K.gemm(h2, w.p(p + "w_gu")))
+            # gates in the product's epilogue, except in prompts of wide models: a long K loop hides the separate pass
+            hm = K.glu_rows(h2, w.p(p + "w_gu"), "silu") if n <= 128 or cfg.d_model <= 2048 else K.swiglu_fwd(K.gemm(h2, w.p(p + "w_gu")))
             x = K.gemm(hm, w.p(p + "w_down"), residual=x1)
         return x
 
@@ -157,7 +159,6 @@ class LlamaKVModel(ServingModel):
         blocks = torch.tensor(list(block_ids[:nb]), dtype=torch.int64, device=dev) if start > 0 else None
 
         def attend(i, q, k, v):
-            self.cache.append(i, k.contiguous(), v.contiguous(), slots)
             if start == 0:
                 o, _ = K.flash_fwd(q.unsqueeze(0), k.unsqueeze(0), v.unsqueeze(0), causal=True)
                 return o[0]
@@ -168,10 +169,10 @@ class LlamaKVModel(ServingModel):
             if self.cache.fp8:
                 kc = (kc.float() * self.cache.k_scale).to(q.dtype)
                 vc = (vc.float() * self.cache.v_scale).to(q.dtype)
-            o, _ = K.flash_fwd(q.unsqueeze(0), kc.contiguous().unsqueeze(0), vc.contiguous().unsqueeze(0), causal=True)
+            o, _ = K.flash_fwd(q.unsqueeze(0), kc.unsqueeze(0), vc.unsqueeze(0), causal=True)
             return o[0]
 
-        return self._layers(K.embedding_fwd(tok, e.w.p("embed")), pos, attend)
+        return self._layers(K.embedding_fwd(tok, e.w.p("embed")), pos, slots, attend, start == 0)
 
     # ------------------------------------------------------------------ one token for every running sequence
     def _decode_hidden(self, d: torch.Tensor, S: int, width: int) -> torch.Tensor:
@@ -184,8 +185,7 @@ class LlamaKVModel(ServingModel):
         splits = self.num_splits or self._splits_for(S * e.cfg.n_kv_heads, width * bs)
 
         def attend(i, q, k, v):
-            self.cache.append(i, k.contiguous(), v.contiguous(), slots)
-            return paged_attention(q.contiguous(), self.cache.k[i], self.cache.v[i], bt, ctx, bs, num_splits=splits,
+            return paged_attention(q, self.cache.k[i], self.cache.v[i], bt, ctx, bs, num_splits=splits,
                                    k_scale=self.cache.k_scale, v_scale=self.cache.v_scale)
 
-        return self._layers(K.embedding_fwd(tok, e.w.p("embed")), pos, attend)
+        return self._layers(K.embedding_fwd(tok, e.w.p("embed")), pos, slots, attend, False)

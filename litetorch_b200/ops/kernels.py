@@ -51,6 +51,7 @@ _SIGS = {
     "lt_set_wait_budget_cycles": [_ll, _ll],
     "lt_gemm_bf16": [_vp, _vp, _vp, _i, _i, _i, _ll, _ll, _ll, _i, _i, _i, _vp, _vp, _ll, _i, _i, _f, _i, _i, _vp],
     "lt_gemm_typed": [_i, _vp, _vp, _vp, _i, _i, _i, _ll, _ll, _ll, _i, _i, _i, _vp, _vp, _ll, _i, _i, _f, _vp],
+    "lt_rope_append": [_vp, _ll] + [_vp] * 7 + [_ll, _i, _i, _i, _i, _i, _f, _f, _vp],
     "lt_gemv_bf16": [_vp, _ll, _vp, _ll, _vp, _ll, _vp, _ll, _i, _i, _i, _vp],
     "lt_gemm_skinny_bf16": [_vp, _ll, _vp, _ll, _vp, _ll, _vp, _ll, _i, _i, _i, _vp],
     "lt_gemm_skinny_set_target": [_i, _i],
@@ -469,6 +470,19 @@ def rope_(x2d: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, T: int, heads
                         1 if backward else 0, _stream())
     _check(rc, "lt_rope")
     return x2d
+
+
+def rope_append(qkv, cos, sin, positions, slots, heads: int, kv_heads: int, head_dim: int, k_cache, v_cache, block_size: int, fp8: bool,
+                k_scale: float = 1.0, v_scale: float = 1.0, in_place: bool = False):
+    """Rows [q | k | v]: queries and keys are rotated, keys and values written to their cache slots.  Returns the queries [rows, heads,
+    head_dim]: packed, or (in_place) as a view of qkv, whose keys are then rotated too."""
+    n = qkv.shape[0]
+    q = qkv[:, :heads * head_dim].unflatten(1, (heads, head_dim)) if in_place else torch.empty((n, heads, head_dim), dtype=qkv.dtype, device=qkv.device)
+    rc = _fn("lt_rope_append")(qkv.data_ptr(), qkv.stride(0), cos.data_ptr(), sin.data_ptr(), positions.data_ptr(), slots.data_ptr(),
+                               None if in_place else q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), n, heads, kv_heads, head_dim, block_size,
+                               1 if fp8 else 0, float(k_scale), float(v_scale), _stream())
+    _check(rc, "lt_rope_append")
+    return q
 
 
 def swiglu_fwd(gu: torch.Tensor) -> torch.Tensor:
@@ -1139,18 +1153,23 @@ def gemm_staged(a, b, *, act: str = "", alpha: float = 1.0, block_n: int = 0):
     return y
 
 
-def glu_mlp(x, gu, down, act: str):
-    """down @ (act(gate @ x) * (up @ x)) with gu = [gate; up]; bf16 gates in the first product's epilogue."""
+def glu_rows(x, gu, act: str):
+    """act(gate @ x) * (up @ x) with gu = [gate; up]; bf16 gates in the product's epilogue."""
     M, Kd = x.shape
     F = gu.shape[0] // 2
     if x.dtype == torch.bfloat16 and 0 < M <= 128 and Kd % 32 == 0 and F % 8 == 0 and x.stride(0) % 8 == 0 and _aligned(x, gu):
         h = torch.empty((M, F), dtype=x.dtype, device=x.device)
         rc = _fn("lt_gemm_skinny_glu")(x.data_ptr(), x.stride(0), gu.data_ptr(), h.data_ptr(), M, F, Kd, _ACT[act], _stream())
         _check(rc, "lt_gemm_skinny_glu")
-        return linear(h, down)
+        return h
     if x.dtype == torch.bfloat16 and M > 128 and Kd % 8 == 0 and F % 8 == 0 and x.stride(0) % 8 == 0 and _aligned(x, gu):
-        return linear(gemm_staged(x, gu, act=act), down)
-    return linear(act_glu(linear(x, gu), act), down)
+        return gemm_staged(x, gu, act=act)
+    return act_glu(linear(x, gu), act)
+
+
+def glu_mlp(x, gu, down, act: str):
+    """down @ glu_rows(x)."""
+    return linear(glu_rows(x, gu, act), down)
 
 
 def moe_plan(logits, correction, top: int, block_rows: int, x=None):

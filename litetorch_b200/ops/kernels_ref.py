@@ -121,6 +121,19 @@ def rope_(x2d, cos, sin, T, heads, head_dim, *, col_offset=0, positions=None, ba
     return x2d
 
 
+def rope_append(qkv, cos, sin, positions, slots, heads, kv_heads, head_dim, k_cache, v_cache, block_size, fp8, k_scale=1.0, v_scale=1.0,
+                in_place=False):
+    n, D = qkv.shape[0], head_dim
+    x = qkv if in_place else qkv.clone()
+    rope_(x, cos, sin, 1, heads + kv_heads, D, positions=positions)
+    k, v = (x[:, a * D:(a + kv_heads) * D].view(n, kv_heads, D) for a in (heads, heads + kv_heads))
+    live = slots >= 0
+    blk, off = slots[live].long() // block_size, slots[live].long() % block_size
+    k_cache[blk, :, off] = (k.float() / k_scale if fp8 else k)[live].to(k_cache.dtype)
+    v_cache[blk, :, off] = (v.float() / v_scale if fp8 else v)[live].to(v_cache.dtype)
+    return x[:, :heads * D].unflatten(1, (heads, D))
+
+
 def swiglu_fwd(gu):
     F = gu.shape[1] // 2
     g, u = gu[:, :F].float(), gu[:, F:].float()
@@ -519,8 +532,12 @@ def act_glu(gu, act):
     return (_ACT[act](g) * u).to(gu.dtype)
 
 
+def glu_rows(x, gu, act):
+    return act_glu(linear(x, gu), act)
+
+
 def glu_mlp(x, gu, down, act):
-    return linear(act_glu(linear(x, gu), act), down)
+    return linear(glu_rows(x, gu, act), down)
 
 
 def moe_route(logits, correction, top):
