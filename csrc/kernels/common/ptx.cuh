@@ -61,6 +61,11 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
 
+// Programmatic dependent launch: a kernel says that the next one may start (a kernel that was not launched to do so ignores it), and the
+// next one waits for all of this one, and so for everything before it, ahead of its first access to what they read or write.
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // True in one lane of a converged warp.  Code behind it is known to the compiler to run in a single thread, so that operands of
 // tcgen05 and TMA instructions stay in uniform registers; behind `lane == 0` each is moved there first.
 __device__ __forceinline__ bool elect_one() {

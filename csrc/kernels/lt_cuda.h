@@ -112,6 +112,10 @@ int lt_gemm_staged(const void* A, const void* B, void* C, int M, int N, int K, l
 int lt_gemm_block_diag(const void* A, const void* B, float* C, int M, int blocks, int nb, int K, long long lda,
                        long long ldc, void* stream);
 
+// ---- weight_stream.cu
+int lt_weight_stream(const void* x, long long ldx, const void* w, long long ldw, void* y, long long ldy, const void* residual, long long ldr, int M,
+                     int N, int K, int act, int early, void* stream);
+
 // ---- gemv.cu: GEMV for 1-8 rows
 int lt_gemv_bf16(const void* x, long long ldx, const void* w, long long ldw, void* y, long long ldy,
                  const void* residual, long long ldr, int M, int N, int K, void* stream);

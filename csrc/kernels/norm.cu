@@ -55,6 +55,7 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
                 __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ sum_out, float* __restrict__ mean_out,
                 float* __restrict__ rstd_out, int M, int D, float eps) {
   __shared__ float red[32];
+  pdl_launch_dependents();   // a product behind this one may fetch its weights
   for (int row = blockIdx.x; row < M; row += gridDim.x) {
     const __nv_bfloat16* xr = x + (long long)row * D;
     const __nv_bfloat16* rr = res ? res + (long long)row * D : nullptr;

@@ -854,6 +854,7 @@ __global__ void paged_decode_merge_kernel(const float* __restrict__ part, __nv_b
                                           const __nv_bfloat16* __restrict__ gate, long long ldg, int Hq, int vdim) {
   const int row = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
+  pdl_launch_dependents();   // a product behind this one may fetch its weights
   if (row >= rows) return;
   constexpr int E = D / 32;
   // A lane reads maximum and sum of one split, so that their loads are under way together, as are then those of the outputs (one split

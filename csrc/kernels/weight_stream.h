@@ -20,6 +20,7 @@ struct StreamProduct {
   const __nv_bfloat16* residual;
   long long ldr;
   int M, N, K, act;
+  int early;   // the kernel starts under the one before it in the stream and fetches weights meanwhile, which that one must not write
 };
 // Rows of x or w that overlap (a pitch below K) are not taken.
 bool stream_takes(const StreamProduct& p);

@@ -54,23 +54,23 @@ class LlamaKVModel(ServingModel):
         for i in range(cfg.n_layers):
             p = "layers.%d." % i
             h, _, _, _ = K.norm_fwd(x, w.p(p + "attn_norm"), eps=cfg.rms_eps)
-            qkv = K.gemm(h, w.p(p + "wqkv"))
+            qkv = K.product_of_constants(h, w.p(p + "wqkv"))
             q = K.rope_append(qkv, e.cos, e.sin, positions, slots, Hq, Hkv, hd, self.cache.k[i], self.cache.v[i], self.block_size, self.cache.fp8,
                               self.cache.k_scale, self.cache.v_scale, in_place=in_place)
             k = qkv[:, Hq * hd:(Hq + Hkv) * hd].view(n, Hkv, hd)
             v = qkv[:, (Hq + Hkv) * hd:].view(n, Hkv, hd)
             o = attend(i, q, k, v)
-            x1 = K.gemm(o.reshape(n, Hq * hd), w.p(p + "wo"), residual=x)
+            x1 = K.product_of_constants(o.reshape(n, Hq * hd), w.p(p + "wo"), residual=x)
             h2, _, _, _ = K.norm_fwd(x1, w.p(p + "mlp_norm"), eps=cfg.rms_eps)
             # gates in the product's epilogue, except in prompts of wide models: a long K loop hides the separate pass
-            hm = K.glu_rows(h2, w.p(p + "w_gu"), "silu") if n <= 128 or cfg.d_model <= 2048 else K.swiglu_fwd(K.gemm(h2, w.p(p + "w_gu")))
-            x = K.gemm(hm, w.p(p + "w_down"), residual=x1)
+            hm = K.product_of_constants(h2, w.p(p + "w_gu"), act="silu") if n <= 128 or cfg.d_model <= 2048 else K.swiglu_fwd(K.gemm(h2, w.p(p + "w_gu")))
+            x = K.product_of_constants(hm, w.p(p + "w_down"), residual=x1)
         return x
 
     def _logits(self, hidden, rows=None):
         e, K = self.e, self.e.K
         hf, _, _, _ = K.norm_fwd(hidden if rows is None else hidden[rows], e.w.p("final_norm"), eps=e.cfg.rms_eps)
-        return K.gemm(hf, e.w.p("lm_head"))
+        return K.product_of_constants(hf, e.w.p("lm_head"))
 
     # ------------------------------------------------------------------ prompt chunks
     @torch.no_grad()

@@ -51,6 +51,7 @@ _SIGS = {
     "lt_set_wait_budget_cycles": [_ll, _ll],
     "lt_gemm_bf16": [_vp, _vp, _vp, _i, _i, _i, _ll, _ll, _ll, _i, _i, _i, _vp, _vp, _ll, _i, _i, _f, _i, _i, _vp],
     "lt_gemm_typed": [_i, _vp, _vp, _vp, _i, _i, _i, _ll, _ll, _ll, _i, _i, _i, _vp, _vp, _ll, _i, _i, _f, _vp],
+    "lt_weight_stream": [_vp, _ll] * 4 + [_i] * 5 + [_vp],
     "lt_rope_append": [_vp, _ll] + [_vp] * 7 + [_ll, _i, _i, _i, _i, _i, _f, _f, _vp],
     "lt_gemv_bf16": [_vp, _ll, _vp, _ll, _vp, _ll, _vp, _ll, _i, _i, _i, _vp],
     "lt_gemm_skinny_bf16": [_vp, _ll, _vp, _ll, _vp, _ll, _vp, _ll, _i, _i, _i, _vp],
@@ -470,6 +471,21 @@ def rope_(x2d: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, T: int, heads
                         1 if backward else 0, _stream())
     _check(rc, "lt_rope")
     return x2d
+
+
+def product_of_constants(x, w, residual=None, act: str = ""):
+    """x @ w^T (+ residual), or with `act` glu_rows(x, w), for weights that no kernel of the pass writes: with up to 64 rows the kernel starts
+    under the one before it and fetches weights meanwhile."""
+    M, Kd = x.shape
+    N = w.shape[0] // 2 if act else w.shape[0]
+    if (x.dtype == torch.bfloat16 and 0 < M <= 64 and Kd % 8 == 0 and x.stride(1) == 1 and w.is_contiguous() and x.stride(0) % 8 == 0 and x.stride(0) >= Kd
+            and _aligned(x, w)):
+        y = torch.empty((M, N), dtype=x.dtype, device=x.device)
+        rc = _fn("lt_weight_stream")(x.data_ptr(), x.stride(0), w.data_ptr(), Kd, y.data_ptr(), N, _p(residual),
+                                     residual.stride(0) if residual is not None else 0, M, N, Kd, _ACT[act] if act else 0, 1, _stream())
+        _check(rc, "lt_weight_stream")
+        return y
+    return glu_rows(x, w, act) if act else gemm(x, w, residual=residual)
 
 
 def rope_append(qkv, cos, sin, positions, slots, heads: int, kv_heads: int, head_dim: int, k_cache, v_cache, block_size: int, fp8: bool,

@@ -121,6 +121,10 @@ def rope_(x2d, cos, sin, T, heads, head_dim, *, col_offset=0, positions=None, ba
     return x2d
 
 
+def product_of_constants(x, w, residual=None, act=""):
+    return glu_rows(x, w, act) if act else gemm(x, w, residual=residual)
+
+
 def rope_append(qkv, cos, sin, positions, slots, heads, kv_heads, head_dim, k_cache, v_cache, block_size, fp8, k_scale=1.0, v_scale=1.0,
                 in_place=False):
     n, D = qkv.shape[0], head_dim

@@ -63,3 +63,36 @@ def test_rows_that_overlap():
     for a, b in ((x, plain), (plain[:4], w), (x, w)):
         ref = a.double() @ b.double().t()
         assert ((KK.gemm(a, b).double() - ref).abs() <= bound(ref, a.double().abs() @ b.double().abs().t(), 256)).all()
+
+
+@pytest.mark.parametrize("M", [1, 17, 64])
+def test_products_that_start_early(M):
+    """A chain of products behind norms and each other, recorded and replayed: the same as one after another, also when x has just been
+    overwritten."""
+    from litetorch_b200.ops import kernels as KK
+    torch.manual_seed(M)
+    W, F = 1024, 2816
+    x = torch.randn(M, W, device="cuda").bfloat16()
+    n = torch.ones(W, device="cuda").bfloat16()
+    ws = [tuple((torch.randn(*s, device="cuda") * s[1] ** -0.5).bfloat16() for s in ((W, W), (2 * F, W), (W, F))) for _ in range(4)]
+
+    def chain(x, product, gated):
+        for a, gu, down in ws:
+            x = product(KK.norm_fwd(x, n, eps=1e-5)[0], a, x)
+            x = product(gated(KK.norm_fwd(x, n, eps=1e-5)[0], gu), down, x)
+        return x
+
+    early = lambda x: chain(x, lambda h, w, r: KK.product_of_constants(h, w, residual=r), lambda h, w: KK.product_of_constants(h, w, act="silu"))  # noqa: E731
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        early(x)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        out = early(x)
+    for seed in range(5):
+        x.copy_(torch.randn(M, W, generator=torch.Generator().manual_seed(seed)).bfloat16())
+        graph.replay()
+        ref = chain(x.clone(), lambda h, w, r: KK.gemm(h, w, residual=r), lambda h, w: KK.glu_rows(h, w, "silu"))
+        assert torch.equal(out, ref)
+    assert KK.status_fetch() == 0
