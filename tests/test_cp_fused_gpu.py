@@ -69,3 +69,39 @@ def test_cp_flash_matches_full_attention(nproc):
     assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-3000:]
     res = json.loads([l for l in r.stdout.splitlines() if l.startswith("RESULT ")][-1][7:])
     assert res["status"] == 0 and res["worst_rel_err"] < 2.5e-2, res
+
+
+@pytest.mark.parametrize("world,zigzag,causal,D", [(2, True, True, 64), (2, True, True, 128), (3, False, True, 128), (2, False, False, 64), (4, True, True, 64),
+                                                   (4, True, True, 128)])
+def test_ranks_one_after_another_on_local_shards(world, zigzag, causal, D):
+    """The kernels of every rank on pointers to all shards, which here lie on one GPU: no kernel waits for another, so they can run in
+    turn.  Covers the walk over other ranks' segments and dQ's way into other ranks' accumulators."""
+    from litetorch_b200.ops import kernels as K
+    from litetorch_b200.parallel.cp import zigzag_merge, zigzag_split
+    torch.manual_seed(world * D)
+    B, T, H, G = 2, 256 * world, 4, 2
+    scale = D ** -0.5
+    full = [torch.randn(B, T, h, D, device="cuda").bfloat16() for h in (H, G, G, H)]
+    q, k, v, do = ([zigzag_split(t, r, world, 1) if zigzag else t.chunk(world, 1)[r].contiguous() for r in range(world)] for t in full)
+    ptrs = lambda ts: [t.data_ptr() for t in ts]  # noqa: E731
+    o, lse = zip(*(K.flash_fwd_cp(q[r], ptrs(k), ptrs(v), k[r], causal=causal, scale=scale, cp_world=world, cp_rank=r, zigzag=zigzag)
+                   for r in range(world)))
+    delta = [torch.empty_like(t) for t in lse]
+    acc = [torch.zeros(t.shape, device="cuda") for t in q]
+    dq, dk, dv = ([torch.empty_like(t) for t in ts] for ts in (q, k, v))
+    for phase in (0, 1, 2):
+        for r in range(world):
+            K.flash_bwd_cp(phase, q_ptrs=ptrs(q), k=k[r], v=v[r], o=o[r], do_ptrs=ptrs(do), lse_ptrs=ptrs(lse), delta_ptrs=ptrs(delta),
+                           dq_acc_ptrs=ptrs(acc), dq=dq[r], dk=dk[r], dv=dv[r], q_like=q[r], causal=causal, scale=scale, cp_world=world, cp_rank=r,
+                           zigzag=zigzag)
+    merge = (lambda ts: zigzag_merge(list(ts))) if zigzag else (lambda ts: torch.cat(list(ts), 1))
+    qf, kf, vf = (t.double().requires_grad_() for t in full[:3])
+    s = torch.einsum("bthd,bshd->bhts", qf, kf.repeat_interleave(H // G, 2)) * scale
+    if causal:
+        s = s.masked_fill(torch.ones(T, T, dtype=torch.bool, device="cuda").triu(1), -torch.inf)
+    of = torch.einsum("bhts,bshd->bthd", torch.softmax(s, -1), vf.repeat_interleave(H // G, 2))
+    of.backward(full[3].double())
+    # weights (twice in the backward pass) and results are rounded to bf16, 2^-9 each way: 0.3 % a rounding, three of them at most
+    for got, want in ((merge(o), of), (merge(dq), qf.grad), (merge(dk), kf.grad), (merge(dv), vf.grad)):
+        assert float((got.double() - want).norm() / want.norm()) < 0.009
+    assert K.status_fetch() == 0
