@@ -949,7 +949,9 @@ int lt_paged_decode_window(const void* q, const void* k_cache, const void* v_cac
                                                           block_size, max_blocks, splits, scale, k_scale, v_scale, window)
   const int G = Hq / Hkv;
   const bool bs_ok = block_size > 0 && (32 % block_size == 0 || block_size % 32 == 0);
-  const bool aligned = (reinterpret_cast<uintptr_t>(k_cache) & 15) == 0 && (reinterpret_cast<uintptr_t>(v_cache) & 15) == 0;
+  // (the tensor-core kernels read two query values at a time, for 8-bit caches four)
+  const bool aligned = (reinterpret_cast<uintptr_t>(k_cache) & 15) == 0 && (reinterpret_cast<uintptr_t>(v_cache) & 15) == 0 &&
+                       (reinterpret_cast<uintptr_t>(q) & (kv_fp8 ? 7 : 3)) == 0;
   if (G <= kPdMmaMaxG && bs_ok && block_size % 8 == 0 && num_blocks > 0 && aligned && (long long)num_blocks * Hkv * block_size < (1ll << 31)) {
     // caches in blocks of 8 keys or more: tiles by TMA, scores and P V on mma.sync
     const int ctas = S * Hkv * splits;

@@ -70,3 +70,21 @@ def test_e4m3_decode_propagates_nan_keys():
     q = torch.randn(1, 2, 64, device="cuda").to(torch.bfloat16)
     out = K.paged_decode(q, kc, vc, torch.arange(4, device="cuda").int().view(1, 4), torch.tensor([60], dtype=torch.int32, device="cuda"), 16, 1, 0.125)
     assert torch.isnan(out[0, :, 5]).all() and torch.isfinite(out[0, :, 6]).all()
+
+
+@pytest.mark.parametrize("fp8,D,bs,window", [(True, 64, 16, 0), (True, 128, 16, 40), (False, 128, 16, 0), (False, 64, 16, 33), (False, 64, 4, 0)])
+@pytest.mark.parametrize("at", [1, 2, 3, 4])
+def test_queries_at_any_address(fp8, D, bs, window, at):
+    """Queries that start at any element (a packed view into a larger tensor) go to a kernel that reads them as they lie."""
+    from litetorch_b200.ops import kernels as K
+    torch.manual_seed(at + D)
+    kc, vc = (torch.randn(12, 2, bs, D, device="cuda").to(torch.float8_e4m3fn if fp8 else torch.bfloat16) for _ in range(2))
+    tables = torch.randperm(12, device="cuda").int().view(2, 6).contiguous()
+    ctx = torch.tensor([6 * bs - 1, 2 * bs + 1], dtype=torch.int32, device="cuda")
+    room = torch.randn(2 * 8 * D + 8, device="cuda").to(torch.bfloat16)
+    q = room[at:at + 2 * 8 * D].view(2, 8, D)
+    out = K.paged_decode(q, kc, vc, tables, ctx, bs, 2, D ** -0.5, window=window)
+    ref = reference(q, kc, vc, tables, ctx, bs, D ** -0.5, 1.0, 1.0, window)
+    # 16-bit caches: weights and result are rounded to bf16 (2^-8 of the largest value each); 8-bit caches: the result alone
+    assert (out.double() - ref).abs().max() <= 2 ** -7 * ref.abs().max()
+    assert K.status_fetch() == 0
