@@ -749,9 +749,11 @@ paged_decode_f8_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     const int nk = min(32, t1 - c0);
     if (nk < 32 || c0 < lo) {
       // rows past the context or before the window may hold anything: zero them in V so that their zero weights do not meet a NaN
+      // (a window starts in a warp's first chunk, whose stage a later copy fills again: that copy has to come after these stores)
       if (lane >= nk || c0 + lane < lo) {
 #pragma unroll
         for (int u = 0; u < NU; ++u) *reinterpret_cast<uint4*>(vt + lane * D + u * 16) = make_uint4(0u, 0u, 0u, 0u);
+        fence_proxy_async();
       }
       __syncwarp();
     }

@@ -31,6 +31,8 @@ def reference(q, kc, vc, tables, ctx, bs, scale, ks, vs, window):
     (64, 12, 4, 64, 0, [63, 64, 65, 700], 2),            # blocks longer than a chunk, 3 heads to a key head
     (128, 16, 4, 16, 100, [5, 99, 100, 101, 131, 2000], 4),
     (64, 4, 4, 16, 33, [32, 33, 34, 500], 1),
+    (64, 4, 4, 16, 1701, [2011, 1702, 1718], 1),         # a window that starts inside a chunk, in a stage that is filled several times
+    (128, 8, 2, 32, 1701, [2011, 1719], 1),
 ])
 def test_e4m3_decode_against_64_bits(D, H, G, bs, window, contexts, splits):
     from litetorch_b200.ops import kernels as K
