@@ -478,8 +478,11 @@ def product_of_constants(x, w, residual=None, act: str = ""):
     under the one before it and fetches weights meanwhile."""
     M, Kd = x.shape
     N = w.shape[0] // 2 if act else w.shape[0]
-    if (x.dtype == torch.bfloat16 and 0 < M <= 64 and Kd % 8 == 0 and x.stride(1) == 1 and w.is_contiguous() and x.stride(0) % 8 == 0 and x.stride(0) >= Kd
-            and _aligned(x, w)):
+    assert x.dtype == w.dtype and w.dim() == 2 and w.shape[1] == Kd, "operands do not match: %s and %s" % (tuple(x.shape), tuple(w.shape))
+    assert x.stride(1) == 1 and w.stride(1) == 1 and (not act or (residual is None and w.shape[0] % 2 == 0))
+    if residual is not None:
+        assert residual.dtype == x.dtype and residual.shape == (M, N) and residual.stride(1) == 1
+    if x.dtype == torch.bfloat16 and 0 < M <= 64 and Kd % 8 == 0 and w.is_contiguous() and x.stride(0) % 8 == 0 and x.stride(0) >= Kd and _aligned(x, w):
         y = torch.empty((M, N), dtype=x.dtype, device=x.device)
         rc = _fn("lt_weight_stream")(x.data_ptr(), x.stride(0), w.data_ptr(), Kd, y.data_ptr(), N, _p(residual),
                                      residual.stride(0) if residual is not None else 0, M, N, Kd, _ACT[act] if act else 0, 1, _stream())
