@@ -496,6 +496,12 @@ def rope_append(qkv, cos, sin, positions, slots, heads: int, kv_heads: int, head
     """Rows [q | k | v]: queries and keys are rotated, keys and values written to their cache slots.  Returns the queries [rows, heads,
     head_dim]: packed, or (in_place) as a view of qkv, whose keys are then rotated too."""
     n = qkv.shape[0]
+    positions, slots = positions.to(torch.int32).contiguous(), slots.to(torch.int32).contiguous()
+    assert qkv.dtype == torch.bfloat16 and qkv.dim() == 2 and qkv.stride(1) == 1 and qkv.shape[1] >= (heads + 2 * kv_heads) * head_dim
+    assert positions.numel() == n and slots.numel() == n
+    assert all(t.dtype == torch.float32 and t.is_contiguous() and t.shape[-1] == head_dim // 2 for t in (cos, sin))
+    assert all(t.dtype == (torch.float8_e4m3fn if fp8 else torch.bfloat16) and t.is_contiguous() and t.shape[1:] == (kv_heads, block_size, head_dim)
+               for t in (k_cache, v_cache))
     q = qkv[:, :heads * head_dim].unflatten(1, (heads, head_dim)) if in_place else torch.empty((n, heads, head_dim), dtype=qkv.dtype, device=qkv.device)
     rc = _fn("lt_rope_append")(qkv.data_ptr(), qkv.stride(0), cos.data_ptr(), sin.data_ptr(), positions.data_ptr(), slots.data_ptr(),
                                None if in_place else q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), n, heads, kv_heads, head_dim, block_size,

@@ -25,7 +25,8 @@ def test_rope_append(n, H, G, D, bs, in_place, fp8):
     K.rope_(x, cos, sin, 1, G, D, col_offset=H * D, positions=pos)
     k, v = (x[:, a * D:(a + G) * D].reshape(n, G, D).contiguous() for a in (H, H + G))
     K.kv_append(k, v, *caches[0], slots, bs, fp8, 0.5, 0.25)
-    q = K.rope_append(y, cos, sin, pos, slots, H, G, D, *caches[1], bs, fp8, 0.5, 0.25, in_place=in_place)
+    wide, far = pos.long(), torch.stack([slots.long(), slots.long()], 1)[:, 0]           # other types and strides of whole numbers mean the same
+    q = K.rope_append(y, cos, sin, wide, far, H, G, D, *caches[1], bs, fp8, 0.5, 0.25, in_place=in_place)
     assert torch.equal(q, x[:, :H * D].reshape(n, H, D))
     assert torch.equal(y, x if in_place else qkv)
     for a, b in zip(*caches):
