@@ -97,7 +97,7 @@ __global__ void rope_append_kernel(__nv_bfloat16* __restrict__ qkv, long long ld
     const int g = h - Hq - (is_k ? 0 : Hkv);
     const long long dst = (((long long)(slot / block_size) * Hkv + g) * block_size + slot % block_size) * hd + v * 8;
     if (FP8) {
-      uint8_t out[8];
+      alignas(8) uint8_t out[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j)   // what is cached is the value as 16 bits hold it
         out[j] = __nv_fp8_e4m3(__bfloat162float(__float2bfloat16(f[j])) * (is_k ? k_inv : v_inv)).__x;
