@@ -362,7 +362,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           }
         }
       }
-      const float m_blk = mx * scale;
+      const float m_blk = mx == -INFINITY ? -INFINITY : mx * scale;   // a row that sees nothing here, whatever the scale
       if (!seen) {
         // nothing accumulated for this row yet (its weights were zero): take the block's maximum as it is
         m_used = (m_blk == -INFINITY) ? 0.f : m_blk;

@@ -61,14 +61,22 @@ def test_forward_against_64_bits(B, Tq, Tk, H, G, D, causal, window, grow):
     assert K.status_fetch() == 0
 
 
-def test_negative_and_zero_scale():
-    """Masked keys stay out whatever the sign of the scale."""
+@pytest.mark.parametrize("Tq,Tk,D,causal,window", [(200, 200, 64, True, 0), (200, 265, 64, True, 0), (200, 200, 128, True, 0), (300, 365, 128, True, 0),
+                                                   (300, 300, 64, True, 70), (300, 400, 128, True, 33), (100, 300, 128, False, 0)])
+@pytest.mark.parametrize("scale", [-0.05, 0.0])
+def test_negative_and_zero_scale(Tq, Tk, D, causal, window, scale):
+    """Masked keys stay out whatever the sign of the scale, also where a row sees nothing of a whole block."""
     from litetorch_b200.ops import kernels as K
     torch.manual_seed(0)
-    q, k, v = (torch.randn(1, 200, 2, 64, device="cuda").bfloat16() for _ in range(3))
-    for scale in (-0.05, 0.0):
-        o, _ = K.flash_fwd(q, k, v, causal=True, scale=scale)
-        for h in range(2):
-            s = (q[0, :, h].double() @ k[0, :, h].double().t() * scale).masked_fill(torch.ones(200, 200, device="cuda").triu(1).bool(), -torch.inf)
-            p = torch.softmax(s, -1)
-            assert ((o[0, :, h].double() - p @ v[0, :, h].double()).abs() <= 2.0 ** -7 * 1.01 * (p @ v[0, :, h].double().abs())).all()
+    q, k, v = (torch.randn(1, t, 2, D, device="cuda").bfloat16() for t in (Tq, Tk, Tk))
+    o, lse = K.flash_fwd(q, k, v, causal=causal, scale=scale, window=window)
+    gap = (torch.arange(Tq, device="cuda") + Tk - Tq)[:, None] - torch.arange(Tk, device="cuda")[None]
+    hidden = ((gap < 0) & causal) | ((gap >= window) if window else False)
+    for h in range(2):
+        s = (q[0, :, h].double() @ k[0, :, h].double().t() * scale).masked_fill(hidden, -torch.inf)
+        p = torch.softmax(s, -1)
+        # weights and result are rounded to bf16
+        assert ((o[0, :, h].double() - p @ v[0, :, h].double()).abs() <= 2.0 ** -7 * 1.01 * (p @ v[0, :, h].double().abs())).all()
+        # scores and the logarithm of their sum in 32 bits
+        assert ((lse[0, h].double() - torch.logsumexp(s, -1)).abs() <= 1e-5).all()
+    assert K.status_fetch() == 0
