@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace lt {
 
 // Device int that kernels write an error code to (0 = ok). One per device, created on first use.
@@ -31,6 +33,21 @@ int encode_tmap_4d(CUtensorMap* out, const void* base, int elem_bytes, uint64_t 
 // Every translation unit with bounded waits registers a function that stores the two wait budgets (SM cycles) into
 // its own device globals; lt_set_wait_budget_cycles() calls them all for the current device.
 void register_wait_budget_setter(int (*fn)(long long local_cycles, long long peer_cycles));
+
+// Work that is due once on every device, such as the opt-in to more than 48 KB of shared memory for a kernel, which belongs to the device that
+// is current.  Doing it twice is harmless: threads may race for it.
+class OncePerDevice {
+ public:
+  bool pending() const { return (done_.load(std::memory_order_acquire) & bit()) == 0; }
+  void finish() { done_.fetch_or(bit(), std::memory_order_release); }
+
+ private:
+  static uint64_t bit() {   // none: work stays due
+    int dev = -1;
+    return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 ? uint64_t(1) << dev : 0;
+  }
+  std::atomic<uint64_t> done_{0};
+};
 
 inline int cuda_ok(cudaError_t e) { return e == cudaSuccess ? 0 : int(e); }
 

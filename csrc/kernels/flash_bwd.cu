@@ -645,11 +645,11 @@ template <int D>
 static int launch_flash_bwd(const QMaps& qm, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdq,
                             const FlashBwdParams& p, cudaStream_t st) {
   using Cfg = FaBwdCfg<D>;
-  static bool configured = false;
+  static OncePerDevice configured;
   auto kern = flash_bwd_kernel<D>;
-  if (!configured) {
+  if (configured.pending()) {
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
-    configured = true;
+    configured.finish();
   }
   dim3 grid(p.Hkv, p.B, (p.Tk + kFbBlock - 1) / kFbBlock);
   kern<<<grid, kFbThreads, Cfg::kSmemBytes, st>>>(qm, tk, tv, tdq, p);

@@ -490,11 +490,11 @@ static long long* g_fwd_trace = nullptr;
 template <int D, int DV, int BKV, bool SHARED = false>
 static int launch_flash_fwd(const CUtensorMap& tq, const KvMaps& maps, const FlashFwdParams& p, cudaStream_t st) {
   using Cfg = FaFwdCfg<D, DV, BKV>;
-  static bool configured = false;
+  static OncePerDevice configured;
   auto kern = flash_fwd_kernel<D, DV, BKV, SHARED>;
-  if (!configured) {
+  if (configured.pending()) {
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
-    configured = true;
+    configured.finish();
   }
   dim3 grid(p.Hq, p.B, (p.Tq + kFaBlockQ - 1) / kFaBlockQ);
   kern<<<grid, kFaThreads, Cfg::kSmemBytes, st>>>(tq, maps, p);

@@ -366,11 +366,11 @@ template <int BLOCK_N, int A_MAJOR, int B_MAJOR>
 static int launch_ag_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, const GatherArgs& g,
                           const PrefetchArgs& pf, int grid, cudaStream_t st) {
   using Cfg = GemmCfg<BLOCK_N>;
-  static bool configured = false;
+  static OncePerDevice configured;
   auto kern = ag_gemm_kernel<BLOCK_N, A_MAJOR, B_MAJOR>;
-  if (!configured) {
+  if (configured.pending()) {
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
-    configured = true;
+    configured.finish();
   }
   kern<<<grid, kGemmThreads, Cfg::kSmemBytes, st>>>(tmA, tmB, p, g, pf);
   LT_LAUNCH_CHECK();
@@ -380,13 +380,13 @@ static int launch_ag_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const 
 template <int A_MAJOR, int B_MAJOR>
 static int launch_ag_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, const GatherArgs& g,
                                const PrefetchArgs& pf, int grid, cudaStream_t st) {
-  static bool configured = false;
+  static OncePerDevice configured;
   auto kern = ag_gemm_pair_kernel<A_MAJOR, B_MAJOR>;
   constexpr int kSmem = kPairSmemBytes > kGatherStages * kGatherStageBytes + 2048 ? kPairSmemBytes
                                                                                   : kGatherStages * kGatherStageBytes + 2048;
-  if (!configured) {
+  if (configured.pending()) {
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    configured = true;
+    configured.finish();
   }
   kern<<<grid, kGemmThreads, kSmem, st>>>(tmA, tmB, p, g, pf);
   LT_LAUNCH_CHECK();

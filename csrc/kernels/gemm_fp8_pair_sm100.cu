@@ -255,10 +255,10 @@ int lt_gemm_fp8_block_pair(const void* A8, const void* B8, void* C, int M, int N
   if (r) return 1000 + r;
   r = encode_tmap_2d(&tmB, B8, 1, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, kP8BlockK, 128, 1);
   if (r) return 2000 + r;
-  static bool configured = false;
-  if (!configured) {
+  static OncePerDevice configured;
+  if (configured.pending()) {
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(gemm_fp8_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kP8SmemBytes));
-    configured = true;
+    configured.finish();
   }
   int pairs = sm_count() / 2;
   if (pairs > p.num_tiles) pairs = p.num_tiles;

@@ -294,10 +294,10 @@ int lt_gemm_fp8_block(const void* A8, const void* B8, void* C, int M, int N, int
   if (r) return 1000 + r;
   r = encode_tmap_2d(&tmB, B8, 1, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, kF8BlockK, kF8BlockN, 1);
   if (r) return 2000 + r;
-  static bool configured = false;
-  if (!configured) {
+  static OncePerDevice configured;
+  if (configured.pending()) {
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(gemm_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kF8SmemBytes));
-    configured = true;
+    configured.finish();
   }
   int grid = sm_count();
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;

@@ -293,12 +293,12 @@ static bool get_skinny_ws(cudaStream_t st, SkinnyWs* out) {
 
 template <int MT, int MODE, bool GLU>
 static int launch_skinny(SkinnyParams p, int z, cudaStream_t st) {
-  static bool configured = false;
+  static OncePerDevice configured;
   constexpr int smem = 4 * MT * 16 * 32 * 4;
   auto kern = gemm_skinny_kernel<MT, MODE, GLU>;
-  if (!configured) {
+  if (configured.pending()) {
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    configured = true;
+    configured.finish();
   }
   const int sms = sm_count();
   const int cols = GLU ? kSkCols / 2 : kSkCols;

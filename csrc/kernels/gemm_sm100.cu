@@ -22,11 +22,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 template <int BLOCK_N, int A_MAJOR, int B_MAJOR, int MMA_KIND = 0>
 static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, int grid, cudaStream_t st) {
   using Cfg = GemmCfg<BLOCK_N>;
-  static bool configured = false;
+  static OncePerDevice configured;
   auto kern = gemm_bf16_kernel<BLOCK_N, A_MAJOR, B_MAJOR, MMA_KIND>;
-  if (!configured) {
+  if (configured.pending()) {
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
-    configured = true;
+    configured.finish();
   }
   kern<<<grid, kGemmThreads, Cfg::kSmemBytes, st>>>(tmA, tmB, p);
   LT_LAUNCH_CHECK();
@@ -41,11 +41,11 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 
 template <int A_MAJOR, int B_MAJOR, int MMA_KIND = 0>
 static int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, int grid, cudaStream_t st) {
-  static bool configured = false;
+  static OncePerDevice configured;
   auto kern = gemm_bf16_pair_kernel<A_MAJOR, B_MAJOR, MMA_KIND>;
-  if (!configured) {
+  if (configured.pending()) {
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes));
-    configured = true;
+    configured.finish();
   }
   kern<<<grid, kGemmThreads, kPairSmemBytes, st>>>(tmA, tmB, p);
   LT_LAUNCH_CHECK();
@@ -62,11 +62,11 @@ gemm_staged_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 template <int BLOCK_N, int EPI>
 static int launch_staged(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const GemmParams& p, int grid,
                          cudaStream_t st) {
-  static bool configured = false;
+  static OncePerDevice configured;
   auto kern = gemm_staged_kernel<BLOCK_N, EPI>;
-  if (!configured) {
+  if (configured.pending()) {
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<BLOCK_N>::kStagedSmemBytes));
-    configured = true;
+    configured.finish();
   }
   kern<<<grid, kGemmThreads, GemmCfg<BLOCK_N>::kStagedSmemBytes, st>>>(tmA, tmB, tmC, p);
   LT_LAUNCH_CHECK();
@@ -83,10 +83,10 @@ template <int BLOCK_N>
 static int launch_block_diag(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, int grid, cudaStream_t st) {
   using Cfg = GemmCfg<BLOCK_N>;
   auto kern = gemm_block_diag_kernel<BLOCK_N>;
-  static bool configured = false;
-  if (!configured) {
+  static OncePerDevice configured;
+  if (configured.pending()) {
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
-    configured = true;
+    configured.finish();
   }
   kern<<<grid, kGemmThreads, Cfg::kSmemBytes, st>>>(tmA, tmB, p);
   LT_LAUNCH_CHECK();

@@ -200,11 +200,11 @@ moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
 template <int BLOCK_N, int EPI>
 static int launch_grouped(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const GemmParams& p, const int* live,
                           int grid, cudaStream_t st) {
-  static bool configured = false;
+  static OncePerDevice configured;
   auto kern = moe_grouped_gemm_kernel<BLOCK_N, EPI>;
-  if (!configured) {
+  if (configured.pending()) {
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<BLOCK_N>::kStagedSmemBytes));
-    configured = true;
+    configured.finish();
   }
   kern<<<grid, kGemmThreads, GemmCfg<BLOCK_N>::kStagedSmemBytes, st>>>(tmA, tmB, tmC, p, live);
   LT_LAUNCH_CHECK();

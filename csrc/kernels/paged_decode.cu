@@ -965,13 +965,13 @@ int lt_paged_decode_window(const void* q, const void* k_cache, const void* v_cac
     if (r == 0) r = encode_tmap_2d(&tmV, v_cache, bytes, D, rows, uint64_t(D) * bytes, kv_fp8 ? D : 64, run, !kv_fp8 || D == 128);
     if (r) return r > 0 ? 1000 + r : r;
     int* status = device_status_word();
-    static bool configured_mma = false;
-    if (!configured_mma) {
+    static OncePerDevice configured_mma;
+    if (configured_mma.pending()) {
       LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_f8_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdF8Cfg<64>::kSmemBytes));
       LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_f8_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdF8Cfg<128>::kSmemBytes));
       LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdMmaCfg<64>::kSmemBytes));
       LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdMmaCfg<128>::kSmemBytes));
-      configured_mma = true;
+      configured_mma.finish();
     }
     if (kv_fp8 && D == 64) paged_decode_f8_kernel<64><<<ctas, kPdWarps * 32, PdF8Cfg<64>::kSmemBytes, st>>>(tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale * k_scale, v_scale, window, status);
     else if (kv_fp8) paged_decode_f8_kernel<128><<<ctas, kPdWarps * 32, PdF8Cfg<128>::kSmemBytes, st>>>(tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale * k_scale, v_scale, window, status);
@@ -982,11 +982,11 @@ int lt_paged_decode_window(const void* q, const void* k_cache, const void* v_cac
     const int ctas = S * Hkv * splits;
     auto KC = static_cast<const __nv_bfloat16*>(k_cache);
     auto VC = static_cast<const __nv_bfloat16*>(v_cache);
-    static bool configured = false;
-    if (!configured) {
+    static OncePerDevice configured;
+    if (configured.pending()) {
       LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_gqa_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdCfg<64>::kSmemBytes));
       LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_gqa_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdCfg<128>::kSmemBytes));
-      configured = true;
+      configured.finish();
     }
     int* status = device_status_word();
     if (D == 64) paged_decode_gqa_kernel<64><<<ctas, kPdWarps * 32, PdCfg<64>::kSmemBytes, st>>>(Q, KC, VC, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale, status);

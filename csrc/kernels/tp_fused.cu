@@ -128,11 +128,11 @@ template <int BLOCK_N, int A_MAJOR, int B_MAJOR>
 static int launch_gemm_rs(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, const RsArgs& a, int grid,
                           cudaStream_t st) {
   using Cfg = GemmCfg<BLOCK_N>;
-  static bool configured = false;
+  static OncePerDevice configured;
   auto kern = gemm_rs_kernel<BLOCK_N, A_MAJOR, B_MAJOR>;
-  if (!configured) {
+  if (configured.pending()) {
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
-    configured = true;
+    configured.finish();
   }
   kern<<<grid, kGemmThreads, Cfg::kSmemBytes, st>>>(tmA, tmB, p, a);
   LT_LAUNCH_CHECK();
@@ -151,11 +151,11 @@ gemm_rs_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 template <int A_MAJOR, int B_MAJOR>
 static int launch_gemm_rs_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, const RsArgs& a,
                                const ScatterMaps& sm, int grid, cudaStream_t st) {
-  static bool configured = false;
+  static OncePerDevice configured;
   auto kern = gemm_rs_pair_kernel<A_MAJOR, B_MAJOR>;
-  if (!configured) {
+  if (configured.pending()) {
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairScatterSmemBytes));
-    configured = true;
+    configured.finish();
   }
   kern<<<grid, kGemmThreads, kPairScatterSmemBytes, st>>>(tmA, tmB, p, a, sm);
   LT_LAUNCH_CHECK();

@@ -184,11 +184,11 @@ weight_stream_kernel(const __grid_constant__ CUtensorMap tw, const __grid_consta
 template <int XR, int R, bool GLU>
 static int launch_ws(const StreamProduct& p, cudaStream_t st) {
   using Cfg = WsCfg<XR, R>;
-  static bool configured = false;
+  static OncePerDevice configured;
   auto kern = weight_stream_kernel<XR, R, GLU>;
-  if (!configured) {
+  if (configured.pending()) {
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
-    configured = true;
+    configured.finish();
   }
   // As many tiles as CTAs, or a multiple of that, so that none ends in a round of a few tiles: tiles get as wide as that takes, and
   // the copies fetch that many rows.
