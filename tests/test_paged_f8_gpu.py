@@ -90,3 +90,24 @@ def test_queries_at_any_address(fp8, D, bs, window, at):
     # 16-bit caches: weights and result are rounded to bf16 (2^-8 of the largest value each); 8-bit caches: the result alone
     assert (out.double() - ref).abs().max() <= 2 ** -7 * ref.abs().max()
     assert K.status_fetch() == 0
+
+
+@pytest.mark.parametrize("D,n,splits", [(64, 4096, 1), (128, 16384, 1), (128, 16384, 32)])
+def test_partial_sums_in_32_bits(D, n, splits):
+    """The splits' outputs, as they go to the merge, over more chunks than a cut-off addition could take."""
+    from litetorch_b200.ops import kernels as K
+    torch.manual_seed(n)
+    H, G, bs = 8, 2, 16
+    kc, vc = (torch.randn(n // bs, G, bs, D, device="cuda").to(torch.float8_e4m3fn) for _ in range(2))
+    q, tables = torch.randn(1, H, D, device="cuda").bfloat16(), torch.randperm(n // bs, device="cuda").int().view(1, -1).contiguous()
+    ctx, part = torch.tensor([n], dtype=torch.int32, device="cuda"), torch.empty(H, splits, D + 2, device="cuda")
+    o = torch.empty(1, H, D, dtype=torch.bfloat16, device="cuda")
+    assert K._fn("lt_paged_decode")(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), tables.data_ptr(), ctx.data_ptr(), part.data_ptr(), o.data_ptr(), 1, H, G, D,
+                                    bs, n // bs, n // bs, splits, D ** -0.5, 1, 1.0, 1.0, K._stream()) == 0
+    p = part.double()
+    w = p[..., D + 1] * torch.exp(p[..., D] - p[..., D].amax(-1, keepdim=True))
+    out = (w[..., None] * p[..., :D]).sum(1) / w.sum(1, keepdim=True)
+    ref = reference(q, kc, vc, tables, ctx, bs, D ** -0.5, 1.0, 1.0, 0)[0]
+    # a warp adds up to n / 128 chunks, each addition rounded to 2^-24 of a sum that is at most some times the result's size (values of
+    # both signs), in either direction: (n / 128) ** 0.5 of them; scores of some units in 32 bits move weights by as much again
+    assert float((out - ref).norm() / ref.norm()) <= 2 * 2.0 ** -24 * (n / 128) ** 0.5 / 3 ** 0.5 + 3e-7
