@@ -31,6 +31,13 @@ __device__ __forceinline__ void ws_mma(float (&d)[4], uint32_t a0, uint32_t a1, 
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+// The same from zero.
+__device__ __forceinline__ void ws_mma_0(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
 __device__ __forceinline__ uint4 lds_16(uint32_t src) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(src) : "memory");
@@ -116,6 +123,10 @@ weight_stream_kernel(const __grid_constant__ CUtensorMap tw, const __grid_consta
     for (int i = 0; i < mine && ok; ++i) {
       ok = __all_sync(0xffffffffu, mbar_wait(bars + slot * 8, phase, abort_flag, status, kStatusTimeoutFull));
       if (!ok) break;
+      // The instruction cuts off what it adds to its accumulator.  With one block of rows, four of them start from zero for every stage and
+      // ordinary additions take the sums on (products of up to 8 rows were such additions throughout; 14336 deep, one result in a thousand came
+      // out a unit off in the 16 bits that leave, now one in ten thousand, as before).
+      float sum[MT == 1 ? R / 8 : 1][4];
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         const uint32_t from = (c ? from1 : from0) + slot * Cfg::kStage;
@@ -130,10 +141,22 @@ weight_stream_kernel(const __grid_constant__ CUtensorMap tw, const __grid_consta
           const uint4 wv = lds_16(from + f * 1024);
 #pragma unroll
           for (int m = 0; m < MT; ++m) {
-            ws_mma(acc[m][f], xv[m][0].x, xv[m][1].x, xv[m][0].y, xv[m][1].y, wv.x, wv.y);
-            ws_mma(acc[m][f], xv[m][0].z, xv[m][1].z, xv[m][0].w, xv[m][1].w, wv.z, wv.w);
+            if constexpr (MT == 1) {
+              if (c == 0) ws_mma_0(sum[f], xv[m][0].x, xv[m][1].x, xv[m][0].y, xv[m][1].y, wv.x, wv.y);
+              else ws_mma(sum[f], xv[m][0].x, xv[m][1].x, xv[m][0].y, xv[m][1].y, wv.x, wv.y);
+              ws_mma(sum[f], xv[m][0].z, xv[m][1].z, xv[m][0].w, xv[m][1].w, wv.z, wv.w);
+            } else {
+              ws_mma(acc[m][f], xv[m][0].x, xv[m][1].x, xv[m][0].y, xv[m][1].y, wv.x, wv.y);
+              ws_mma(acc[m][f], xv[m][0].z, xv[m][1].z, xv[m][0].w, xv[m][1].w, wv.z, wv.w);
+            }
           }
         }
+      }
+      if constexpr (MT == 1) {
+#pragma unroll
+        for (int f = 0; f < R / 8; ++f)
+#pragma unroll
+          for (int r = 0; r < 4; ++r) acc[0][f][r] += sum[f][r];
       }
       __syncwarp();
       load(true, true);

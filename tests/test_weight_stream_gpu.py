@@ -96,3 +96,19 @@ def test_products_that_start_early(M):
         ref = chain(x.clone(), lambda h, w, r: KK.gemm(h, w, residual=r), lambda h, w: KK.glu_rows(h, w, "silu"))
         assert torch.equal(out, ref)
     assert KK.status_fetch() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 4096, 14336), (8, 1024, 14336), (3, 2048, 5632), (8, 28672, 4096)])
+def test_few_rows_add_in_32_bits(M, N, K):
+    """Sums of one sign: what every addition cuts off would add up."""
+    from litetorch_b200.ops import kernels as KK
+    torch.manual_seed(N + K)
+    x, w = torch.randn(M, K, device="cuda").abs().bfloat16(), (torch.randn(N, K, device="cuda").abs() * K ** -0.5).bfloat16()
+    y = KK.gemm(x, w)
+    ref = x.double() @ w.double().t()
+    ulp = torch.exp2(torch.floor(torch.log2(ref)) - 7)
+    # beyond half a unit of the 16-bit result by as much as the 32-bit sum was off.  A stage's four instructions cut off up to 2^-23 of its
+    # part each (2^-23 of the whole, at most, as parts add up); then come K / 512 + 8 rounded additions, 2^-24 each at most, in either
+    # direction: three standard deviations (2^-24 / sqrt 3 each) of them
+    slack = 4 * 2.0 ** -23 + 3 * (K / 512 + 8) ** 0.5 * 2.0 ** -24 / 3 ** 0.5
+    assert (((y.double() - ref).abs() - 0.5 * ulp) / ref).max() <= slack
