@@ -112,3 +112,19 @@ def test_few_rows_add_in_32_bits(M, N, K):
     # direction: three standard deviations (2^-24 / sqrt 3 each) of them
     slack = 4 * 2.0 ** -23 + 3 * (K / 512 + 8) ** 0.5 * 2.0 ** -24 / 3 ** 0.5
     assert (((y.double() - ref).abs() - 0.5 * ulp) / ref).max() <= slack
+
+
+@pytest.mark.parametrize("M", [1, 8, 20, 64, 100, 200])
+def test_silu_of_far_negative_gates(M):
+    """Gates between -88.8 and -87.3, where the sigmoid's divisor passes 2^126."""
+    from litetorch_b200.ops import kernels as KK
+    K, F = 64, 256
+    x = torch.zeros(M, K, device="cuda").bfloat16()
+    x[:, 0], x[:, 1] = 1.0, 2.0 ** 100
+    gu = torch.zeros(2 * F, K, device="cuda").bfloat16()
+    gu[:F, 0] = torch.linspace(-88.5, -86.0, F, device="cuda").bfloat16()
+    gu[F:, 1] = 1.0
+    y = KK.glu_rows(x, gu, "silu").double()
+    ref = torch.nn.functional.silu(gu[:F, 0].double())[None].expand(M, F) * 2.0 ** 100
+    # __expf of 88 is off by 88 2^-23 (its argument is multiplied by log2 e in 32 bits) and a little; the result is rounded to bf16
+    assert ((y - ref).abs() <= (2.0 ** -8 + 88 * 2.0 ** -22) * ref.abs()).all()
