@@ -1,4 +1,6 @@
-// Weight-streaming GEMM for 9 to 128 rows (decode with a batch of sequences): y[M, N] = x[M, K] @ W[N, K]^T (+ residual).
+// Weight-streaming GEMM for 65 to 128 rows (decode with a large batch of sequences): y[M, N] = x[M, K] @ W[N, K]^T (+ residual); up to 64
+// rows weight_stream.cu does it, but for rows that overlap in memory, which come here too.  Batches of products and rows grouped by
+// expert (below) are done here whatever their rows.
 //
 // With this few rows the multiplication is bound by reading W once (a 1.1B model's weights stream in 0.3 ms), but a
 // 128-row tcgen05 tile wastes most of its rows and, worse, a 2048-column output gives a persistent tile kernel 8 or 16
@@ -325,9 +327,11 @@ static int launch_skinny(SkinnyParams p, int z, cudaStream_t st) {
 
 template <int MODE, bool GLU>
 static int skinny_by_rows(const SkinnyParams& p, int rows, int z, cudaStream_t st) {
-  if (rows <= 16) return launch_skinny<1, MODE, GLU>(p, z, st);
-  if (rows <= 32) return launch_skinny<2, MODE, GLU>(p, z, st);
-  if (rows <= 64) return launch_skinny<4, MODE, GLU>(p, z, st);
+  if constexpr (MODE != kSkPlain) {   // plain: only rows that overlap are fewer than 65
+    if (rows <= 16) return launch_skinny<1, MODE, GLU>(p, z, st);
+    if (rows <= 32) return launch_skinny<2, MODE, GLU>(p, z, st);
+    if (rows <= 64) return launch_skinny<4, MODE, GLU>(p, z, st);
+  }
   if constexpr (MODE == kSkGrouped) return -int(kStatusBadArgument);
   else return launch_skinny<8, MODE, GLU>(p, z, st);
 }

@@ -84,7 +84,7 @@ int lt_gemm_fp8_block(const void* A8, const void* B8, void* C, int M, int N, int
                       int max_ctas, void* stream);
 int lt_quant_fp8_1x128(const void* x, long long ldx, void* q, long long ldq, void* scale_t, int M, int K, void* stream);
 
-// ---- gemm_skinny.cu: weight-streaming GEMM for 9-128 rows
+// ---- gemm_skinny.cu: weight-streaming GEMM for 65-128 rows (fewer: weight_stream.cu, but for rows that overlap)
 int lt_gemm_skinny_set_target(int ctas_per_sm, int min_chunks_per_warp);
 int lt_gemm_skinny_bf16(const void* x, long long ldx, const void* w, long long ldw, void* y, long long ldy,
                         const void* residual, long long ldr, int M, int N, int K, void* stream);

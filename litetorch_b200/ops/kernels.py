@@ -220,7 +220,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_major: int = 0, b_major: int = 0
     if (a_major == 0 and b_major == 0 and a.shape[0] <= 8 and out is None and out_dtype == torch.bfloat16 and bias is None and act == 0
             and alpha == 1.0 and a.shape[1] % 8 == 0 and a.stride(0) % 8 == 0 and b.stride(0) % 8 == 0 and a.shape[0] > 0
             and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0):
-        # a handful of rows (decode): the weight-streaming kernel, one warp per output column
+        # a handful of rows (decode): the weight-streaming kernel
         M, Kd = a.shape
         N = b.shape[0]
         y = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
@@ -235,7 +235,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_major: int = 0, b_major: int = 0
                                  and out.stride(0) % 2 == 0 and out.data_ptr() % 4 == 0))
             and (residual is None or (residual.dtype == torch.bfloat16 and residual.shape == (a.shape[0], b.shape[0])
                                       and residual.stride(1) == 1 and residual.stride(0) % 2 == 0 and residual.data_ptr() % 4 == 0))):
-        # 9 to 128 rows (decode with a batch of sequences): the weight-streaming tensor-core kernel
+        # 9 to 128 rows (decode with a batch of sequences): the weight-streaming kernels
         M, Kd = a.shape
         N = b.shape[0]
         y = out if out is not None else torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
@@ -337,7 +337,7 @@ def gemm_set_tail_split(enable: bool):
 
 
 def gemm_skinny_set_target(ctas_per_sm: int = 1, min_chunks_per_warp: int = 16):
-    """Tuning of the 9-128-row weight-streaming GEMM on narrow outputs: CTAs per SM that its K split aims for and the
+    """Tuning of the 65-128-row weight-streaming GEMM on narrow outputs: CTAs per SM that its K split aims for and the
     fewest 32-element chunks of K a warp keeps (defaults 1 and 16: K is split from 8192 on)."""
     _fn("lt_gemm_skinny_set_target")(int(ctas_per_sm), int(min_chunks_per_warp))
 

@@ -128,3 +128,43 @@ def test_silu_of_far_negative_gates(M):
     ref = torch.nn.functional.silu(gu[:F, 0].double())[None].expand(M, F) * 2.0 ** 100
     # __expf of 88 is off by 88 2^-23 (its argument is multiplied by log2 e in 32 bits) and a little; the result is rounded to bf16
     assert ((y - ref).abs() <= (2.0 ** -8 + 88 * 2.0 ** -22) * ref.abs()).all()
+
+
+@pytest.mark.parametrize("M", [65, 79, 81, 113, 127, 128])
+@pytest.mark.parametrize("N,K", [(8, 8192), (40, 16416), (2056, 8224), (2048, 544), (1000, 14336)])
+def test_split_of_k_beyond_64_rows(M, N, K):
+    """K over several CTAs of a column group, as it is by default and as far as it goes; plain and gated."""
+    from litetorch_b200.ops import kernels as KK
+    torch.manual_seed(M + N + K)
+    x, w, r = (torch.randn(*s, device="cuda").bfloat16() for s in ((M, K), (N, K), (M, N)))
+    ref = x.double() @ w.double().t()
+    mag = x.double().abs() @ w.double().abs().t()
+    gated = torch.nn.functional.silu(ref[:, :N // 2]) * ref[:, N // 2:]
+    room = (K + 16) * 2.0 ** -23 * 1.2 * (mag[:, :N // 2] * ref[:, N // 2:].abs() + mag[:, N // 2:] * ref[:, :N // 2].abs())    # as in test_gated
+    for target in ((1, 16), (8, 1)):
+        KK.gemm_skinny_set_target(*target)
+        try:
+            y, again, g = KK.gemm(x, w, residual=r), KK.gemm(x, w, residual=r), KK.glu_rows(x, w, "silu")
+        finally:
+            KK.gemm_skinny_set_target()
+        assert torch.equal(y, again)
+        assert ((y.double() - ref - r.double()).abs() <= bound(ref + r.double(), mag + r.double().abs(), K)).all()
+        assert ((g.double() - gated).abs() <= 2.0 ** -7 * gated.abs() + room + 1e-5 * ref[:, N // 2:].abs()).all()
+    assert KK.status_fetch() == 0
+
+
+@pytest.mark.parametrize("M", [9, 17, 64, 65])
+def test_more_rows_that_overlap(M):
+    from litetorch_b200.ops import kernels as KK
+    torch.manual_seed(M)
+    base = torch.randn(4096, device="cuda").bfloat16()
+    x, w = base.as_strided((M, 256), (8, 1)), (torch.randn(48, 256, device="cuda") / 16).bfloat16()
+    ref, mag = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    assert ((KK.gemm(x, w).double() - ref).abs() <= bound(ref, mag, 256)).all()
+    v = base.as_strided((48, 256), (8, 1))
+    rv, mv = w[:1].expand(M, 256).double() @ v.double().t(), w[:1].expand(M, 256).double().abs() @ v.double().abs().t()
+    assert ((KK.gemm(w[:1].expand(M, 256), v).double() - rv).abs() <= bound(rv, mv, 256)).all()
+    a, u = ref.chunk(2, -1)
+    want = torch.nn.functional.silu(a) * u
+    assert ((KK.glu_rows(x, w, "silu").double() - want).abs() <= 2.0 ** -7 * want.abs() + 1e-3).all()
+    assert KK.status_fetch() == 0
