@@ -4,10 +4,10 @@ the split-K paged attention kernel, greedy sampling on the device.
 `LlamaKVModel` is the model side of `serving.ServingScheduler.step`: the native scheduler (admission, block tables,
 chunked prefill within a token budget, completion) hands it prompt chunks and the running sequences' newest tokens
 together with their block tables, and gets next tokens back.  Nothing is recomputed: every token's K and V are
-written once (`lt_kv_append`) and read by the attention of later tokens (`lt_paged_decode`, `lt_flash_fwd` for a
+written once (`lt_rope_append`, with the rotation of queries and keys) and read by the attention of later tokens (`lt_paged_decode`, `lt_flash_fwd` for a
 prompt chunk).  The reference's counterparts: ContinuousBatchingScheduler::step and its block tables
 (src/llm/continuous_batching.cpp:20-197), paged attention (src/ops/attention.cpp:351-477) and flash-decoding
-(src/ops/flash_decoding.cpp:13-115); its cache is never filled, here `PagedKVCache.append` is the write path.
+(src/ops/flash_decoding.cpp:13-115); its cache is never filled.
 """
 from __future__ import annotations
 
@@ -169,7 +169,8 @@ class LlamaKVModel(ServingModel):
             if self.cache.fp8:
                 kc = (kc.float() * self.cache.k_scale).to(q.dtype)
                 vc = (vc.float() * self.cache.v_scale).to(q.dtype)
-            o, _ = K.flash_fwd(q.unsqueeze(0), kc.unsqueeze(0), vc.unsqueeze(0), causal=True)
+            # (a single block is not copied by the reshape: its heads lie a block apart, and attention takes them side by side)
+            o, _ = K.flash_fwd(q.unsqueeze(0), kc.contiguous().unsqueeze(0), vc.contiguous().unsqueeze(0), causal=True)
             return o[0]
 
         return self._layers(K.embedding_fwd(tok, e.w.p("embed")), pos, slots, attend, start == 0)
