@@ -148,11 +148,6 @@ __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float 
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
-// Asynchronous bulk reduction shared -> global: global[i] += shared[i] for `bytes` / 4 floats (16-byte aligned).
-__device__ __forceinline__ void bulk_reduce_add_f32(float* gdst, uint32_t smem_src, uint32_t bytes) {
-  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;"
-               ::"l"(gdst), "r"(smem_src), "r"(bytes) : "memory");
-}
 // Tiled TMA reduction shared -> global (fp32 add) of the box of `m` at coordinates (x, h, t, b).
 __device__ __forceinline__ void tma_reduce_add_4d(const CUtensorMap* m, uint32_t smem_src, int x, int h, int t, int b) {
   asm volatile("cp.reduce.async.bulk.tensor.4d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
