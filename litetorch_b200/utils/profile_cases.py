@@ -1,6 +1,6 @@
 """Small, self-terminating workloads for `ncu` captures of one kernel each.
 
-    python -m litetorch_b200.utils.profile_cases gemm|gemm_vs_cublas|gemm_wgrad|gemm_fp8|gemm_e4m3|gemm_rs|ag_gemm|rs_adamw|flash_fwd|flash_bwd|flash_fwd_d128|flash_bwd_d128|paged_decode|shard_gather|
+    python -m litetorch_b200.utils.profile_cases gemm|gemm_vs_cublas|gemm_wgrad|gemm_fp8|gemm_e4m3|gemm_rs|ag_gemm|rs_adamw|flash_fwd|flash_bwd|flash_fwd_d128|flash_bwd_d128|paged_decode|paged_decode_f8|weight_stream|shard_gather|
                                                  rmsnorm|rmsnorm_bwd|swiglu|adamw|ce [reps]
 
 Every case touches more than the 126 MB L2 but only a few hundred MB of device memory, launches the kernel a
@@ -96,6 +96,17 @@ def main():
         bt = torch.arange(nb, device=dev, dtype=torch.int32).view(S, ctx // bs)
         cl = torch.full((S,), ctx, device=dev, dtype=torch.int32)
         fn = lambda: K.paged_decode(q, kc, vc, bt, cl, bs, 8, D ** -0.5)
+    elif case == "paged_decode_f8":  # 8-bit cache, batch 16, 8 k context, 32 q / 8 kv heads of 128: 0.27 GB of K / V per launch
+        S, H, Hkv, D, bs, ctx = 16, 32, 8, 128, 16, 8192
+        nb = S * ctx // bs
+        kc, vc = (torch.randn(nb, Hkv, bs, D, device=dev).bfloat16().to(torch.float8_e4m3fn) for _ in range(2))
+        q = torch.randn(S, H, D, device=dev).bfloat16()
+        bt = torch.arange(nb, device=dev, dtype=torch.int32).view(S, ctx // bs)
+        cl = torch.full((S,), ctx, device=dev, dtype=torch.int32)
+        fn = lambda: K.paged_decode(q, kc, vc, bt, cl, bs, 5, D ** -0.5)
+    elif case == "weight_stream":    # 8 rows times the gate and up matrix of an 8B layer: 0.23 GB of weights per launch
+        x, w = torch.randn(8, 4096, device=dev).bfloat16(), torch.randn(28672, 4096, device=dev).bfloat16()
+        fn = lambda: K.gemm(x, w)
     elif case == "shard_gather":     # 512 MB pulled from four "ranks" (local buffers stand in for peers)
         n = 1 << 26
         shards = [torch.randn(n, device=dev).bfloat16() for _ in range(4)]

@@ -43,7 +43,7 @@ def test_e4m3_decode_against_64_bits(D, H, G, bs, window, contexts, splits):
     kc, vc = (torch.randn(n_blocks, G, bs, D, device="cuda").mul_(20).to(torch.float8_e4m3fn) for _ in range(2))
     tables = torch.randperm(n_blocks, device="cuda").int().view(S, width).contiguous()
     q = torch.randn(S, H, D, device="cuda").to(torch.bfloat16)
-    q[0, 0] *= 1e-6                                       # a head far below fp16's range as it stands, and one above it
+    q[0, 0] *= 1e-6                                       # a head far below fp16's range as it stands, and one above it (see test_queries_of_any_size)
     q[0, -1] *= 1e6
     ctx = torch.tensor(contexts, dtype=torch.int32, device="cuda")
     # what lies past a sequence's end, or before its window, must not matter
@@ -111,3 +111,23 @@ def test_partial_sums_in_32_bits(D, n, splits):
     # a warp adds up to n / 128 chunks, each addition rounded to 2^-24 of a sum that is at most some times the result's size (values of
     # both signs), in either direction: (n / 128) ** 0.5 of them; scores of some units in 32 bits move weights by as much again
     assert float((out - ref).norm() / ref.norm()) <= 2 * 2.0 ** -24 * (n / 128) ** 0.5 / 3 ** 0.5 + 3e-7
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("up", [-80, -30, -14, 14, 30, 80])
+def test_queries_of_any_size(D, up):
+    """Queries far outside fp16's range, with the scale that brings the scores back: powers of two change nothing, bit for bit.  Heads of
+    very different sizes side by side."""
+    from litetorch_b200.ops import kernels as K
+    torch.manual_seed(D)
+    kc, vc = (torch.randn(40, 2, 16, D, device="cuda").to(torch.float8_e4m3fn) for _ in range(2))
+    tables = torch.randperm(40, device="cuda").int().view(2, 20).contiguous()
+    ctx = torch.tensor([317, 40], dtype=torch.int32, device="cuda")
+    q = torch.randn(2, 8, D, device="cuda").bfloat16()
+    q[:, 1] *= 2.0 ** -5
+    q[:, 2] *= 4
+    plain = K.paged_decode(q, kc, vc, tables, ctx, 16, 2, D ** -0.5)
+    ref = reference(q, kc, vc, tables, ctx, 16, D ** -0.5, 1.0, 1.0, 0)
+    assert ((plain.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * ref.abs().max()).all()      # rounded to bf16; 32-bit sums of values of both signs
+    assert torch.equal(K.paged_decode(q * 2.0 ** up, kc, vc, tables, ctx, 16, 2, D ** -0.5 * 2.0 ** -up), plain)
+    assert K.status_fetch() == 0
