@@ -168,3 +168,16 @@ def test_more_rows_that_overlap(M):
     want = torch.nn.functional.silu(a) * u
     assert ((KK.glu_rows(x, w, "silu").double() - want).abs() <= 2.0 ** -7 * want.abs() + 1e-3).all()
     assert KK.status_fetch() == 0
+
+
+@pytest.mark.parametrize("act", ["gelu", "silu"])
+@pytest.mark.parametrize("M,F,K", [(129, 1000, 2048), (1025, 1000, 4096), (1337, 14336, 4096), (2050, 2824, 1024)])
+def test_gated_prompts(M, F, K, act):
+    from litetorch_b200.ops import kernels as KK
+    torch.manual_seed(M + F)
+    x, gu = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(2 * F, K, device="cuda") * K ** -0.5).bfloat16()
+    g, u = (x.double() @ gu.double().t()).chunk(2, -1)
+    want = (torch.nn.functional.silu(g) if act == "silu" else torch.nn.functional.gelu(g, approximate="tanh")) * u
+    # rounded to bf16; sums of K products of size 1 / sqrt(K) in 32 bits, cut off
+    assert ((KK.glu_rows(x, gu, act).double() - want).abs() <= 2.0 ** -8 * want.abs() + K * 2.0 ** -23 * 2 * (1 + u.abs() + g.abs())).all()
+    assert KK.status_fetch() == 0
