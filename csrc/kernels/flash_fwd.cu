@@ -20,7 +20,7 @@
 // goes through shared memory, scale, sum and conversion work on pairs, and the body for blocks that every row sees whole
 // holds no tests: with a test per score, most of the time went into branches and instruction fetches.
 // Measured against the kernel before it (four softmax warps to either parity of key blocks, P through shared memory, one CTA an SM), causal,
-// 32 heads, L2 flushed: D 64, 4 x 2048 tokens 363 -> 136 us; D 64, 4096 tokens 299 -> 122; D 128, 8192 tokens 1177 -> 474 (1160 TFLOP/s);
+// 32 heads, L2 flushed: D 64, 4 x 2048 tokens 363 -> 136 us; D 64, 4096 tokens 299 -> 122; D 128, 8192 tokens 1177 -> 474 to 478 (1150 TFLOP/s);
 // D 128, 1337 queries on 5437 keys 301 -> 155.  (That kernel had itself been 210 us and 673 us in the first and the third of these before its
 // bodies got a lower limit beside the upper one, for windows, and with it tests per score.)  With 128-key blocks a thread holds 128 scores: 168
 // registers, 64 bytes spilled.  Left: 1.3 to 1.5 times the exponentials' time in the loop, and 3 to 5 us a CTA of

@@ -11,12 +11,13 @@
 //
 // Where the caller vouches for the weights (a step of serving), the kernel is launched to start under the one before it and fills its rings
 // with weights meanwhile: decode steps of six 8B layers 1343 -> 1312 us (32 sequences) and 963 -> 935 (8 on an 8-bit cache), of the 1.1B
-// model 1020 -> 1004.
+// model 1020 -> 1004 (1030 to 1042 on other cards).
 //
 // Measured (graph replay over different weights, us; before: CUDA-core dot products for up to 8 rows, register-fed mma.sync beyond; bytes of W at
 // the copy rate in brackets): 28672 x 4096 [35.8]: 1 row 40.5 -> 37.9, 8 rows 121 -> 39, 16 rows 81 -> 42, 32 rows 100 -> 53, 64 rows
 // 163 -> 87; 4096 x 14336 [17.9]: 24 -> 21, 74 -> 21, 41 -> 21, 47 -> 24, 71 -> 36; 2048 x 2048 [1.3]: 4.7 -> 4.3, 8.2 -> 4.3, 8.0 -> 4.4,
-// 10.0 -> 5.2, 16.4 -> 8.5.  With 32 rows and more it is bound by x, which every tile reads again from L2; small matrices by the start.
+// 10.0 -> 5.2, 16.4 -> 8.5.  Additions with rounding, up to 16 rows (see the loop), were added since: 38.7 -> 38.8, 39.6 -> 39.9, 42.2 -> 42.6 and
+// 4.79 -> 4.88 (2048 x 2048, 8 rows).  With 32 rows and more it is bound by x, which every tile reads again from L2; small matrices by the start.
 #include "lt_cuda.h"
 #include "common/host.h"
 #include "common/ptx.cuh"
