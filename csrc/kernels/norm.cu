@@ -47,6 +47,19 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
   *reinterpret_cast<uint4*>(p) = u;
 }
 
+// Sum of v over the W warps of a group, given to all of them.  `sums` alternates between two arrays from call to call: what is read here is
+// overwritten only after the next call's barrier.
+__device__ __forceinline__ float row_sum(float v, float* sums, int W, int group, int warp, int lane) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (W == 1) return v;
+  if (lane == 0) sums[warp] = v;
+  asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(W * 32) : "memory");
+  v = 0.f;
+  for (int k = 0; k < W; ++k) v += sums[group * W + k];
+  return v;
+}
+
 // y = norm(x (+ res)) * w (+ b).  RMS: mean unused.  If sum_out != nullptr the pre-norm sum is stored.
 template <bool kLayerNorm>
 __global__ void __launch_bounds__(kNormThreads)
@@ -107,6 +120,63 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
         for (int j = 0; j < 8; ++j) f[j] += bv[j];
       }
       store8(y + (long long)row * D + c, f);
+    }
+  }
+}
+
+// RMSNorm forward of many rows (D = 256 * IT * W): W warps of a CTA share a row, a lane owns 8 * IT of its columns, whose values and
+// gains stay in registers: x and the gains are read once, all of a row's loads are in flight together, and the row's sum crosses the W
+// warps through shared memory with one barrier of these warps alone.  The next row is fetched meanwhile: without that a group alternates between
+// loads and stores.  Bound by HBM.  Measured, launches included (before: a CTA a row, read twice, two barriers): 8192 x 2048 22.8 -> 16.6 us, 8192 x 4096
+// 34.0 -> 29.0, 4096 x 2048 12.5 -> 10.5, 1337 x 4096 9.4 -> 8.4 (bytes at the copy rate: 10.2, 20.5, 5.1, 3.3).
+template <int IT>
+__global__ void __launch_bounds__(kNormThreads)
+rmsnorm_fwd_wide_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
+                        float* __restrict__ rstd_out, int M, int W, float eps) {
+  __shared__ float sums[2][8];
+  const int D = 256 * IT * W;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, group = warp / W, sub = warp - group * W;
+  const int groups = (blockDim.x >> 5) / W;
+  const int c0 = (sub * IT * 32 + lane) * 8;    // column of piece i: c0 + 256 i
+  pdl_launch_dependents();
+  uint4 wq[IT];
+#pragma unroll
+  for (int i = 0; i < IT; ++i) wq[i] = *reinterpret_cast<const uint4*>(w + c0 + i * 256);
+  const int step = gridDim.x * groups;
+  int parity = 0, row = blockIdx.x * groups + group;
+  uint4 nq[IT];                                 // the next row of this group, on its way while this one is worked on
+  if (row < M) {
+#pragma unroll
+    for (int i = 0; i < IT; ++i) nq[i] = *reinterpret_cast<const uint4*>(x + (long long)row * D + c0 + i * 256);
+  }
+  for (; row < M; row += step, parity ^= 1) {
+    const long long off = (long long)row * D + c0;
+    uint4 xq[IT];
+#pragma unroll
+    for (int i = 0; i < IT; ++i) xq[i] = nq[i];
+    if (row + step < M) {
+#pragma unroll
+      for (int i = 0; i < IT; ++i) nq[i] = *reinterpret_cast<const uint4*>(x + off + (long long)step * D + i * 256);
+    }
+    float sq = 0.f;
+#pragma unroll
+    for (int i = 0; i < IT; ++i) {
+      float f[8];
+      unpack8(xq[i], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sq += f[j] * f[j];
+    }
+    sq = row_sum(sq, sums[parity], W, group, warp, lane);
+    const float rstd = rsqrtf(sq / D + eps);
+    if (sub == 0 && lane == 0 && rstd_out) rstd_out[row] = rstd;
+#pragma unroll
+    for (int i = 0; i < IT; ++i) {
+      float f[8], wv[8];
+      unpack8(xq[i], f);
+      unpack8(wq[i], wv);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = f[j] * rstd * wv[j];
+      store8(y + off + i * 256, f);
     }
   }
 }
@@ -191,7 +261,104 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
   }
 }
 
-// RMSNorm backward with ONE WARP PER ROW (D = 256 * ITERS, ITERS in {1, 2, 4, 8}): dy and x of the row stay in
+// RMSNorm backward of many rows (D = 256 * IT * W), split as the forward kernel: dy, x and the gradient that joins are loaded together and
+// stay in registers between the reduction and the dx pass; rows of a CTA and CTAs of an SM run past one another.  Bound by HBM.
+// Measured with the fold behind it (before: a warp a row up to 2048 columns, beyond that a CTA a row with both operands read twice): 8192 x 2048
+// 37.9 -> 29.4 us, 8192 x 4096 107.9 -> 50.1, 4096 x 3072 56.3 -> 26.9, 4096 x 8192 107.3 -> 66.1 (IT = 4, one CTA an SM), 300 x 4096 18.2 -> 10.5 (bytes at
+// the copy rate: 20.5, 41.0, 15.4, 41.0, 1.5).
+template <int IT>
+__global__ void __launch_bounds__(kNormThreads, IT == 2 ? 2 : 1)
+rmsnorm_bwd_wide_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                        const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
+                        float* __restrict__ dw_part, int M, int W) {
+  __shared__ float sums[2][8];
+  extern __shared__ float fold[];          // [groups][D]
+  const int D = 256 * IT * W;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, group = warp / W, sub = warp - group * W;
+  const int groups = (blockDim.x >> 5) / W;
+  const int c0 = (sub * IT * 32 + lane) * 8;    // column of piece i: c0 + 256 i
+  uint4 wq[IT];
+  float dw_acc[IT][8];
+#pragma unroll
+  for (int i = 0; i < IT; ++i) {
+    wq[i] = *reinterpret_cast<const uint4*>(w + c0 + i * 256);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) dw_acc[i][j] = 0.f;
+  }
+  const int step = gridDim.x * groups;
+  int parity = 0, row = blockIdx.x * groups + group;
+  uint4 ng[IT], nx[IT], rq[IT];                 // dy and x of the next row of this group, on their way while this one is worked on
+#pragma unroll
+  for (int i = 0; i < IT; ++i) rq[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (row < M) {
+#pragma unroll
+    for (int i = 0; i < IT; ++i) {
+      ng[i] = *reinterpret_cast<const uint4*>(dy + (long long)row * D + c0 + i * 256);
+      nx[i] = *reinterpret_cast<const uint4*>(x + (long long)row * D + c0 + i * 256);
+    }
+  }
+  for (; row < M; row += step, parity ^= 1) {
+    const long long off = (long long)row * D + c0;
+    uint4 gq[IT], xq[IT];
+#pragma unroll
+    for (int i = 0; i < IT; ++i) {
+      gq[i] = ng[i];
+      xq[i] = nx[i];
+    }
+    if (dres) {
+#pragma unroll
+      for (int i = 0; i < IT; ++i) rq[i] = *reinterpret_cast<const uint4*>(dres + off + i * 256);
+    }
+    if (row + step < M) {
+#pragma unroll
+      for (int i = 0; i < IT; ++i) {
+        ng[i] = *reinterpret_cast<const uint4*>(dy + off + (long long)step * D + i * 256);
+        nx[i] = *reinterpret_cast<const uint4*>(x + off + (long long)step * D + i * 256);
+      }
+    }
+    const float rstd = rstd_in[row];
+    float s_gx = 0.f;
+#pragma unroll
+    for (int i = 0; i < IT; ++i) {
+      float g[8], xv[8], wv[8];
+      unpack8(gq[i], g);
+      unpack8(xq[i], xv);
+      unpack8(wq[i], wv);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float xh = xv[j] * rstd;
+        dw_acc[i][j] += g[j] * xh;
+        s_gx += g[j] * wv[j] * xh;
+      }
+    }
+    s_gx = row_sum(s_gx, sums[parity], W, group, warp, lane);
+    const float m_gx = s_gx / D;
+#pragma unroll
+    for (int i = 0; i < IT; ++i) {
+      float g[8], xv[8], wv[8], r[8], o[8];
+      unpack8(gq[i], g);
+      unpack8(xq[i], xv);
+      unpack8(wq[i], wv);
+      unpack8(rq[i], r);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = rstd * (g[j] * wv[j] - xv[j] * rstd * m_gx) + r[j];
+      store8(dx + off + i * 256, o);
+    }
+  }
+  // one partial dgamma row per CTA
+#pragma unroll
+  for (int i = 0; i < IT; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) fold[group * D + c0 + i * 256 + j] = dw_acc[i][j];
+  __syncthreads();
+  for (int c = threadIdx.x; c < D; c += blockDim.x) {
+    float sum = 0.f;
+    for (int k = 0; k < groups; ++k) sum += fold[k * D + c];
+    dw_part[(long long)blockIdx.x * D + c] = sum;
+  }
+}
+
+// RMSNorm backward with ONE WARP PER ROW (D = 256 * ITERS, ITERS in {1, 2}): dy and x of the row stay in
 // registers between the reduction and the dx pass, the row sums are warp shuffles (no block barrier per row), and a
 // lane has 16 * ITERS bytes x 2 of loads in flight, so a CTA of 8 warps keeps 8 rows moving instead of one.
 // dgamma is accumulated per lane over all rows of the warp and folded to one partial row per CTA at the end.
@@ -271,26 +438,30 @@ rmsnorm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat1
   }
 }
 
-// out[c] (+)= sum_p part[p, c]; out is bf16 or fp32.  A block owns 32 columns; its 8 warps split the partial rows.
-__global__ void fold_partials_kernel(const float* __restrict__ part, void* __restrict__ out, int P, int D,
+// out[c] (+)= sum_p part[p, c]; out is bf16 or fp32.  A block owns 32 columns; its 32 warps split the partial rows.
+__global__ void __launch_bounds__(1024) fold_partials_kernel(const float* __restrict__ part, void* __restrict__ out, int P, int D,
                                      int out_fp32, int accumulate) {
-  __shared__ float red[8][32];
+  __shared__ float red[32][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
   float s = 0.f;
-  if (c < D)
-    for (int p = w; p < P; p += 8) s += part[(long long)p * D + c];
+  if (c < D) {
+#pragma unroll 4
+    for (int p = w; p < P; p += 32) s += part[(long long)p * D + c];
+  }
   red[w][lane] = s;
   __syncthreads();
-  if (w != 0 || c >= D) return;
+  s = red[lane][w];                        // column w of the block
 #pragma unroll
-  for (int i = 1; i < 8; ++i) s += red[i][lane];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  const int col = blockIdx.x * 32 + w;
+  if (lane != 0 || col >= D) return;
   if (out_fp32) {
     float* o = static_cast<float*>(out);
-    o[c] = accumulate ? o[c] + s : s;
+    o[col] = accumulate ? o[col] + s : s;
   } else {
     __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
-    o[c] = __float2bfloat16(accumulate ? __bfloat162float(o[c]) + s : s);
+    o[col] = __float2bfloat16(accumulate ? __bfloat162float(o[col]) + s : s);
   }
 }
 
@@ -317,6 +488,17 @@ int lt_norm_fwd(int layer_norm, const void* x, const void* res, const void* w, c
   auto B = static_cast<const __nv_bfloat16*>(b);
   auto Y = static_cast<__nv_bfloat16*>(y);
   auto S = static_cast<__nv_bfloat16*>(sum_out);
+  // Two rows an SM and more (below that a CTA a row has more loads in flight: decode steps).
+  if (!layer_norm && !res && !b && M >= 2 * sm_count() && (D == 256 || (D % 512 == 0 && D <= 4096) || (D % 1024 == 0 && D <= 8192)) &&
+      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15) == 0) {
+    const int it = D == 256 ? 1 : D % 1024 == 0 ? 4 : 2, wide = D / (256 * it), groups = 8 / wide, threads = wide * groups * 32;
+    const int need = (M + groups - 1) / groups, full = sm_count() * (it == 4 ? 2 : 4), g2 = need < full ? need : full;
+    if (it == 1) rmsnorm_fwd_wide_kernel<1><<<g2, threads, 0, st>>>(X, W, Y, rstd_out, M, wide, eps);
+    else if (it == 2) rmsnorm_fwd_wide_kernel<2><<<g2, threads, 0, st>>>(X, W, Y, rstd_out, M, wide, eps);
+    else rmsnorm_fwd_wide_kernel<4><<<g2, threads, 0, st>>>(X, W, Y, rstd_out, M, wide, eps);
+    LT_LAUNCH_CHECK();
+    return 0;
+  }
   if (layer_norm) norm_fwd_kernel<true><<<grid, kNormThreads, 0, st>>>(X, R, W, B, Y, S, mean_out, rstd_out, M, D, eps);
   else            norm_fwd_kernel<false><<<grid, kNormThreads, 0, st>>>(X, R, W, nullptr, Y, S, nullptr, rstd_out, M, D, eps);
   LT_LAUNCH_CHECK();
@@ -338,19 +520,24 @@ int lt_norm_bwd(int layer_norm, const void* dy, const void* x, const void* w, co
   auto W = static_cast<const __nv_bfloat16*>(w);
   auto DR = static_cast<const __nv_bfloat16*>(dres);
   auto DX = static_cast<__nv_bfloat16*>(dx);
-  if (!layer_norm && (D == 256 || D == 512 || D == 1024 || D == 2048) && M >= 8 * grid / 2) {
+  if (!layer_norm && D == 256 && M >= 8 * grid / 2) {
     // warp-per-row kernel; grid CTAs of 8 warps, one partial dgamma row per CTA
     int g2 = (M + 7) / 8;
     if (g2 > grid) g2 = grid;
     if (g2 > sm_count()) g2 = sm_count();
-    switch (D) {
-      case 256: rmsnorm_bwd_warp_kernel<1><<<g2, kNormThreads, 0, st>>>(DY, X, W, rstd, DR, DX, dw_part, M); break;
-      case 512: rmsnorm_bwd_warp_kernel<2><<<g2, kNormThreads, 0, st>>>(DY, X, W, rstd, DR, DX, dw_part, M); break;
-      case 1024: rmsnorm_bwd_warp_kernel<4><<<g2, kNormThreads, 0, st>>>(DY, X, W, rstd, DR, DX, dw_part, M); break;
-      default: rmsnorm_bwd_warp_kernel<8><<<g2, kNormThreads, 0, st>>>(DY, X, W, rstd, DR, DX, dw_part, M); break;
-    }
+    rmsnorm_bwd_warp_kernel<1><<<g2, kNormThreads, 0, st>>>(DY, X, W, rstd, DR, DX, dw_part, M);
     LT_LAUNCH_CHECK();
-    fold_partials_kernel<<<(D + 31) / 32, 256, 0, st>>>(dw_part, dw, g2, D, grads_fp32, accumulate);
+    fold_partials_kernel<<<(D + 31) / 32, 1024, 0, st>>>(dw_part, dw, g2, D, grads_fp32, accumulate);
+    LT_LAUNCH_CHECK();
+    return 0;
+  }
+  if (!layer_norm && ((D % 512 == 0 && D <= 4096) || (D % 1024 == 0 && D <= 8192)) && M >= 2 * sm_count()) {
+    const int it = D <= 4096 ? 2 : 4, wide = D / (256 * it), groups = 8 / wide, threads = wide * groups * 32, bytes = groups * D * 4;
+    const int need = (M + groups - 1) / groups, g2 = need < grid ? need : grid;
+    if (it == 2) rmsnorm_bwd_wide_kernel<2><<<g2, threads, bytes, st>>>(DY, X, W, rstd, DR, DX, dw_part, M, wide);
+    else rmsnorm_bwd_wide_kernel<4><<<g2, threads, bytes, st>>>(DY, X, W, rstd, DR, DX, dw_part, M, wide);
+    LT_LAUNCH_CHECK();
+    fold_partials_kernel<<<(D + 31) / 32, 1024, 0, st>>>(dw_part, dw, g2, D, grads_fp32, accumulate);
     LT_LAUNCH_CHECK();
     return 0;
   }
@@ -366,8 +553,8 @@ int lt_norm_bwd(int layer_norm, const void* dy, const void* x, const void* w, co
 #undef LT_NORM_BWD
   LT_LAUNCH_CHECK();
   const int fb = (D + 31) / 32;
-  fold_partials_kernel<<<fb, 256, 0, st>>>(dw_part, dw, grid, D, grads_fp32, accumulate);
-  if (layer_norm && db && db_part) fold_partials_kernel<<<fb, 256, 0, st>>>(db_part, db, grid, D, grads_fp32, accumulate);
+  fold_partials_kernel<<<fb, 1024, 0, st>>>(dw_part, dw, grid, D, grads_fp32, accumulate);
+  if (layer_norm && db && db_part) fold_partials_kernel<<<fb, 1024, 0, st>>>(db_part, db, grid, D, grads_fp32, accumulate);
   LT_LAUNCH_CHECK();
   return 0;
 }
@@ -441,8 +628,8 @@ extern "C" int lt_norm_bwd_noalloc(int layer_norm, const void* dy, const void* x
 #undef LT_NORM_BWD_NA
   LT_LAUNCH_CHECK();
   const int fb = (D + 31) / 32;
-  fold_partials_kernel<<<fb, 256, 0, st>>>(dw_part, dw, grid, D, grads_fp32, accumulate);
-  if (layer_norm && db) fold_partials_kernel<<<fb, 256, 0, st>>>(db_part, db, grid, D, grads_fp32, accumulate);
+  fold_partials_kernel<<<fb, 1024, 0, st>>>(dw_part, dw, grid, D, grads_fp32, accumulate);
+  if (layer_norm && db) fold_partials_kernel<<<fb, 1024, 0, st>>>(db_part, db, grid, D, grads_fp32, accumulate);
   LT_LAUNCH_CHECK();
   return 0;
 }
