@@ -49,6 +49,26 @@ class OncePerDevice {
   std::atomic<uint64_t> done_{0};
 };
 
+// Launch of a kernel that calls pdl_wait() ahead of its first access to global memory: it may take its place on the SMs and set up its shared and
+// tensor memory while the kernel ahead of it in the stream ends (from that one's pdl_launch_dependents() on; a kernel with tensor memory calls that
+// after its own allocation, so that a successor cannot take the columns that it still needs).  Between kernels of a stream 2.2 us pass otherwise, 0.4 in
+// a recorded graph, and set-up comes on top.  Training step of 1.1B layers over 2 x 2000 tokens (506 kernels) 18.4 -> 17.7 ms, four 8B layers over 8192
+// tokens 82.9 -> 80.5 (1 % of it the norms), prompt of 4096 tokens 11.7 -> 11.4, decode step of the 1.1B model 1038 -> 956 us, latent decode step 510 -> 470.
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 inline int cuda_ok(cudaError_t e) { return e == cudaSuccess ? 0 : int(e); }
 
 }  // namespace lt

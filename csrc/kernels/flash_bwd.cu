@@ -97,6 +97,8 @@ struct FaBwdCfg {
 __global__ void flash_bwd_delta_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __restrict__ dO,
                                        float* __restrict__ delta, int B, int Tq, int Hq, int D, long long so_b,
                                        long long so_t, long long sdo_b, long long sdo_t) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int tpr = D / 8;  // 8 or 16 threads per row
   const long long gid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long row = gid / tpr;
@@ -123,6 +125,8 @@ __global__ void flash_bwd_delta_kernel(const __nv_bfloat16* __restrict__ O, cons
 
 __global__ void flash_bwd_convert_dq_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, int B, int Tq,
                                             int HD, long long sdq_b, long long sdq_t) {
+  pdl_launch_dependents();
+  pdl_wait();
   const long long n4 = (long long)B * Tq * HD / 4;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
     const long long e = i * 4;
@@ -281,6 +285,8 @@ flash_bwd_kernel(const __grid_constant__ QMaps qm, const __grid_constant__ CUten
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  pdl_launch_dependents();
+  pdl_wait();
 
   if (warp == 0) {
     // ---------------------------------------------------------------- producer
@@ -647,7 +653,7 @@ static int launch_flash_bwd(const QMaps& qm, const CUtensorMap& tk, const CUtens
     configured.finish();
   }
   dim3 grid(p.Hkv, p.B, (p.Tk + kFbBlock - 1) / kFbBlock);
-  kern<<<grid, kFbThreads, Cfg::kSmemBytes, st>>>(qm, tk, tv, tdq, p);
+  LT_RETURN_IF_CUDA(launch_chained(kern, grid, kFbThreads, Cfg::kSmemBytes, st, qm, tk, tv, tdq, p));
   LT_LAUNCH_CHECK();
   return 0;
 }
@@ -657,9 +663,9 @@ static int bwd_delta(const void* o, const void* d_o, float* delta, int B, int Tq
   const long long rows = (long long)B * Tq * Hq;
   const int threads = 256;
   const long long blocks = (rows * (D / 8) + threads - 1) / threads;
-  flash_bwd_delta_kernel<<<(unsigned)blocks, threads, 0, st>>>(static_cast<const __nv_bfloat16*>(o),
+  LT_RETURN_IF_CUDA(launch_chained(flash_bwd_delta_kernel, (unsigned)blocks, threads, 0, st, static_cast<const __nv_bfloat16*>(o),
                                                                static_cast<const __nv_bfloat16*>(d_o), delta, B, Tq, Hq, D, so_b,
-                                                               so_t, sdo_b, sdo_t);
+                                                               so_t, sdo_b, sdo_t));
   LT_LAUNCH_CHECK();
   return 0;
 }
@@ -670,7 +676,7 @@ static int bwd_convert(const float* dq_acc, void* dq, int B, int Tq, int Hq, int
   long long blocks = (n4 + 255) / 256;
   const long long cap = (long long)sm_count() * 16;
   if (blocks > cap) blocks = cap;
-  flash_bwd_convert_dq_kernel<<<(unsigned)blocks, 256, 0, st>>>(dq_acc, static_cast<__nv_bfloat16*>(dq), B, Tq, Hq * D, sdq_b, sdq_t);
+  LT_RETURN_IF_CUDA(launch_chained(flash_bwd_convert_dq_kernel, (unsigned)blocks, 256, 0, st, dq_acc, static_cast<__nv_bfloat16*>(dq), B, Tq, Hq * D, sdq_b, sdq_t));
   LT_LAUNCH_CHECK();
   return 0;
 }

@@ -205,6 +205,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  pdl_launch_dependents();
+  pdl_wait();
   const int n_blocks = *n_blocks_s;
   // block j of the schedule -> (owner rank, first local key row, global position of its first key)
   auto locate = [&](int j, int& owner, int& kv0, int& kbase) {
@@ -499,7 +501,7 @@ static int launch_flash_fwd(const CUtensorMap& tq, const KvMaps& maps, const Fla
     configured.finish();
   }
   dim3 grid(p.Hq, p.B, (p.Tq + kFaBlockQ - 1) / kFaBlockQ);
-  kern<<<grid, kFaThreads, Cfg::kSmemBytes, st>>>(tq, maps, p);
+  LT_RETURN_IF_CUDA(launch_chained(kern, grid, kFaThreads, Cfg::kSmemBytes, st, tq, maps, p));
   LT_LAUNCH_CHECK();
   return 0;
 }

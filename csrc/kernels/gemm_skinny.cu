@@ -72,6 +72,8 @@ enum { kSkPlain = 0, kSkBatch = 1, kSkGrouped = 2 };
 template <int MT, int MODE, bool GLU>
 __global__ void __launch_bounds__(kSkWarps * 32, (MODE != kSkPlain || GLU) && MT == 1 ? 2 : 1)
 gemm_skinny_kernel(const SkinnyParams p) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float red[];   // [4 slots][MT * 16 registers][32 lanes]
   constexpr int R = MT * 16;
   constexpr int U = MT <= 2 ? 4 : 2;   // chunks whose weight loads are in flight together
@@ -320,8 +322,7 @@ static int launch_skinny(SkinnyParams p, int z, cudaStream_t st) {
   p.chunks_per_cta = per;
   p.ws = wsp.ws;
   p.counters = wsp.counters;
-  kern<<<dim3(groups, splits, z), kSkWarps * 32, smem, st>>>(p);
-  LT_LAUNCH_CHECK();
+  LT_RETURN_IF_CUDA(launch_chained(kern, dim3(groups, splits, z), kSkWarps * 32, smem, st, p));
   return 0;
 }
 

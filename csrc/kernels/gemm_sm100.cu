@@ -28,7 +28,7 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const Gem
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
     configured.finish();
   }
-  kern<<<grid, kGemmThreads, Cfg::kSmemBytes, st>>>(tmA, tmB, p);
+  LT_RETURN_IF_CUDA(launch_chained(kern, grid, kGemmThreads, Cfg::kSmemBytes, st, tmA, tmB, p));
   LT_LAUNCH_CHECK();
   return 0;
 }
@@ -47,7 +47,7 @@ static int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, cons
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes));
     configured.finish();
   }
-  kern<<<grid, kGemmThreads, kPairSmemBytes, st>>>(tmA, tmB, p);
+  LT_RETURN_IF_CUDA(launch_chained(kern, grid, kGemmThreads, kPairSmemBytes, st, tmA, tmB, p));
   LT_LAUNCH_CHECK();
   return 0;
 }
@@ -68,7 +68,7 @@ static int launch_staged(const CUtensorMap& tmA, const CUtensorMap& tmB, const C
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<BLOCK_N>::kStagedSmemBytes));
     configured.finish();
   }
-  kern<<<grid, kGemmThreads, GemmCfg<BLOCK_N>::kStagedSmemBytes, st>>>(tmA, tmB, tmC, p);
+  LT_RETURN_IF_CUDA(launch_chained(kern, grid, kGemmThreads, GemmCfg<BLOCK_N>::kStagedSmemBytes, st, tmA, tmB, tmC, p));
   LT_LAUNCH_CHECK();
   return 0;
 }
@@ -88,7 +88,7 @@ static int launch_block_diag(const CUtensorMap& tmA, const CUtensorMap& tmB, con
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
     configured.finish();
   }
-  kern<<<grid, kGemmThreads, Cfg::kSmemBytes, st>>>(tmA, tmB, p);
+  LT_RETURN_IF_CUDA(launch_chained(kern, grid, kGemmThreads, Cfg::kSmemBytes, st, tmA, tmB, p));
   LT_LAUNCH_CHECK();
   return 0;
 }

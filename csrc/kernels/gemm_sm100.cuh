@@ -386,6 +386,8 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* tmA, const CUtensor
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  pdl_launch_dependents();
+  pdl_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer

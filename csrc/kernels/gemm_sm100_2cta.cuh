@@ -116,6 +116,8 @@ __device__ __forceinline__ void gemm_body_pair(const CUtensorMap* tmA, const CUt
   cluster_sync_all();   // both CTAs' barriers are initialised before either signals the other's
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  pdl_launch_dependents();
+  pdl_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)

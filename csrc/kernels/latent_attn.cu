@@ -42,6 +42,8 @@ __device__ __forceinline__ void stf2(__nv_bfloat16* p, float2 v) { *reinterpret_
 
 template <typename T>
 __global__ void __launch_bounds__(kRopeThreads) latent_rope_kernel(const RopeParams p) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float2 cs[];         // [rot / 2] (cos, sin) of this token
   __shared__ float red[64];
   const int n = blockIdx.x;
@@ -182,6 +184,8 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap tmap, const LatentDecod
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sp = blockIdx.x, h0 = blockIdx.y * MH, s = blockIdx.z;
   const int heads = min(MH, p.H - h0);
+  pdl_launch_dependents();
+  pdl_wait();
   const int ctx = p.ctx[s];
   const int lo = p.window > 0 ? max(0, ctx - p.window) : 0;
   const int base = lo & ~(kLdKeys - 1);          // tiles start on multiples of 32 keys, and so on a page or its half, quarter, ..
@@ -461,6 +465,8 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap tmap, const LatentDecod
 // out[row, :] from the splits of one (sequence, head): a thread per four columns, eight splits in flight.
 __global__ void __launch_bounds__(128) latent_merge_kernel(const float* __restrict__ part, const float* __restrict__ stat,
                                                            __nv_bfloat16* __restrict__ out, int splits, int c) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float share[kLdMaxSplits];
   const long long row = blockIdx.x;
   const float2* st = reinterpret_cast<const float2*>(stat) + row * splits;
@@ -508,7 +514,7 @@ static int launch_latent_decode(const CUtensorMap& tmap, LatentDecodeParams& p, 
   if (smem > 227 * 1024) return -4;
   auto kern = latent_decode_kernel<MT, FULL>;
   LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  kern<<<dim3(p.splits, (p.H + MH - 1) / MH, S), kLdThreads, smem, st>>>(tmap, p);
+  LT_RETURN_IF_CUDA(launch_chained(kern, dim3(p.splits, (p.H + MH - 1) / MH, S), kLdThreads, smem, st, tmap, p));
   LT_LAUNCH_CHECK();
   return 0;
 }
@@ -530,8 +536,8 @@ int lt_latent_rope(int fp32, void* proj, long long ld, int n, int H, int d, int 
     return -4;
   RopeParams p{proj, ld, H, d, r, rot, c_off, rank, c, c_norm, eps, positions, slots, freq, gain, q_out, q_ld, q_col, cache, lin};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (fp32) latent_rope_kernel<float><<<n, kRopeThreads, rot * 4, st>>>(p);
-  else latent_rope_kernel<__nv_bfloat16><<<n, kRopeThreads, rot * 4, st>>>(p);
+  if (fp32) LT_RETURN_IF_CUDA(launch_chained(latent_rope_kernel<float>, n, kRopeThreads, rot * 4, st, p));
+  else LT_RETURN_IF_CUDA(launch_chained(latent_rope_kernel<__nv_bfloat16>, n, kRopeThreads, rot * 4, st, p));
   LT_LAUNCH_CHECK();
   return 0;
 }
@@ -558,7 +564,7 @@ int lt_latent_decode(const void* q, const void* cache, const int* tables, const 
   const int rc = H <= 16 ? (full ? launch_latent_decode<1, true>(tmap, p, S, st) : launch_latent_decode<1, false>(tmap, p, S, st))
                          : (full ? launch_latent_decode<2, true>(tmap, p, S, st) : launch_latent_decode<2, false>(tmap, p, S, st));
   if (rc != 0 || splits == 1) return rc;
-  latent_merge_kernel<<<S * H, 128, 0, st>>>(part, stat, static_cast<__nv_bfloat16*>(out), splits, c);
+  LT_RETURN_IF_CUDA(launch_chained(latent_merge_kernel, S * H, 128, 0, st, part, stat, static_cast<__nv_bfloat16*>(out), splits, c));
   LT_LAUNCH_CHECK();
   return 0;
 }

@@ -29,6 +29,8 @@ __device__ __forceinline__ void ce_ld8(const __nv_bfloat16* p, float (&f)[8]) {
 __global__ void __launch_bounds__(kCeThreads)
 ce_stats_kernel(const __nv_bfloat16* __restrict__ logits, long long ldl, const long long* __restrict__ targets,
                 int vocab_start, int N, int V, float* __restrict__ stats, int vec_ok) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float sm[32], ss[32];
   for (int row = blockIdx.x; row < N; row += gridDim.x) {
     const __nv_bfloat16* lr = logits + (long long)row * ldl;
@@ -93,6 +95,8 @@ __global__ void __launch_bounds__(kCeThreads)
 ce_finish_kernel(__nv_bfloat16* __restrict__ logits, long long ldl, const long long* __restrict__ targets,
                  int vocab_start, int N, int V, const float* __restrict__ gstats, float* __restrict__ loss,
                  float grad_scale, long long ignore_index, int write_grad, int vec_ok) {
+  pdl_launch_dependents();
+  pdl_wait();
   for (int row = blockIdx.x; row < N; row += gridDim.x) {
     __nv_bfloat16* lr = logits + (long long)row * ldl;
     const long long tgt = targets[row];
@@ -435,8 +439,7 @@ int lt_ce_stats(const void* logits, long long ldl, const long long* targets, int
   if (N == 0) return 0;
   const int vec_ok = (ldl % 8 == 0) && ((reinterpret_cast<uintptr_t>(logits) & 15) == 0);
   const int grid = N < sm_count() * 8 ? N : sm_count() * 8;
-  ce_stats_kernel<<<grid, kCeThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(logits), ldl, targets, vocab_start, N, V, stats, vec_ok);
+  LT_RETURN_IF_CUDA(launch_chained(ce_stats_kernel, grid, kCeThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(logits), ldl, targets, vocab_start, N, V, stats, vec_ok));
   LT_LAUNCH_CHECK();
   return 0;
 }
@@ -447,8 +450,7 @@ int lt_ce_finish(void* logits, long long ldl, const long long* targets, int voca
   if (N == 0) return 0;
   const int vec_ok = (ldl % 8 == 0) && ((reinterpret_cast<uintptr_t>(logits) & 15) == 0);
   const int grid = N < sm_count() * 8 ? N : sm_count() * 8;
-  ce_finish_kernel<<<grid, kCeThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<__nv_bfloat16*>(logits), ldl, targets, vocab_start, N, V, gstats, loss, grad_scale, ignore_index, write_grad, vec_ok);
+  LT_RETURN_IF_CUDA(launch_chained(ce_finish_kernel, grid, kCeThreads, 0, static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(logits), ldl, targets, vocab_start, N, V, gstats, loss, grad_scale, ignore_index, write_grad, vec_ok));
   LT_LAUNCH_CHECK();
   return 0;
 }

@@ -67,8 +67,9 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
                 const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
                 __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ sum_out, float* __restrict__ mean_out,
                 float* __restrict__ rstd_out, int M, int D, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[32];
-  pdl_launch_dependents();   // a product behind this one may fetch its weights
   for (int row = blockIdx.x; row < M; row += gridDim.x) {
     const __nv_bfloat16* xr = x + (long long)row * D;
     const __nv_bfloat16* rr = res ? res + (long long)row * D : nullptr;
@@ -139,6 +140,7 @@ rmsnorm_fwd_wide_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
   const int groups = (blockDim.x >> 5) / W;
   const int c0 = (sub * IT * 32 + lane) * 8;    // column of piece i: c0 + 256 i
   pdl_launch_dependents();
+  pdl_wait();
   uint4 wq[IT];
 #pragma unroll
   for (int i = 0; i < IT; ++i) wq[i] = *reinterpret_cast<const uint4*>(w + c0 + i * 256);
@@ -188,6 +190,8 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
                 const __nv_bfloat16* __restrict__ w, const float* __restrict__ mean_in,
                 const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
                 __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_part, float* __restrict__ db_part, int M, int D) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[32];
   float dw_acc[ITERS][8], db_acc[ITERS][8];
 #pragma unroll
@@ -271,6 +275,8 @@ __global__ void __launch_bounds__(kNormThreads, IT == 2 ? 2 : 1)
 rmsnorm_bwd_wide_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                         const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                         float* __restrict__ dw_part, int M, int W) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float sums[2][8];
   extern __shared__ float fold[];          // [groups][D]
   const int D = 256 * IT * W;
@@ -368,6 +374,8 @@ rmsnorm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat1
                         const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in,
                         const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                         float* __restrict__ dw_part, int M) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int D = 256 * ITERS;
   constexpr int kWarps = kNormThreads / 32;
   __shared__ float fold[kWarps][256];
@@ -441,6 +449,8 @@ rmsnorm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat1
 // out[c] (+)= sum_p part[p, c]; out is bf16 or fp32.  A block owns 32 columns; its 32 warps split the partial rows.
 __global__ void __launch_bounds__(1024) fold_partials_kernel(const float* __restrict__ part, void* __restrict__ out, int P, int D,
                                      int out_fp32, int accumulate) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[32][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
@@ -493,14 +503,14 @@ int lt_norm_fwd(int layer_norm, const void* x, const void* res, const void* w, c
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15) == 0) {
     const int it = D == 256 ? 1 : D % 1024 == 0 ? 4 : 2, wide = D / (256 * it), groups = 8 / wide, threads = wide * groups * 32;
     const int need = (M + groups - 1) / groups, full = sm_count() * (it == 4 ? 2 : 4), g2 = need < full ? need : full;
-    if (it == 1) rmsnorm_fwd_wide_kernel<1><<<g2, threads, 0, st>>>(X, W, Y, rstd_out, M, wide, eps);
-    else if (it == 2) rmsnorm_fwd_wide_kernel<2><<<g2, threads, 0, st>>>(X, W, Y, rstd_out, M, wide, eps);
-    else rmsnorm_fwd_wide_kernel<4><<<g2, threads, 0, st>>>(X, W, Y, rstd_out, M, wide, eps);
+    if (it == 1) LT_RETURN_IF_CUDA(launch_chained(rmsnorm_fwd_wide_kernel<1>, g2, threads, 0, st, X, W, Y, rstd_out, M, wide, eps));
+    else if (it == 2) LT_RETURN_IF_CUDA(launch_chained(rmsnorm_fwd_wide_kernel<2>, g2, threads, 0, st, X, W, Y, rstd_out, M, wide, eps));
+    else LT_RETURN_IF_CUDA(launch_chained(rmsnorm_fwd_wide_kernel<4>, g2, threads, 0, st, X, W, Y, rstd_out, M, wide, eps));
     LT_LAUNCH_CHECK();
     return 0;
   }
-  if (layer_norm) norm_fwd_kernel<true><<<grid, kNormThreads, 0, st>>>(X, R, W, B, Y, S, mean_out, rstd_out, M, D, eps);
-  else            norm_fwd_kernel<false><<<grid, kNormThreads, 0, st>>>(X, R, W, nullptr, Y, S, nullptr, rstd_out, M, D, eps);
+  if (layer_norm) LT_RETURN_IF_CUDA(launch_chained(norm_fwd_kernel<true>, grid, kNormThreads, 0, st, X, R, W, B, Y, S, mean_out, rstd_out, M, D, eps));
+  else            LT_RETURN_IF_CUDA(launch_chained(norm_fwd_kernel<false>, grid, kNormThreads, 0, st, X, R, W, nullptr, Y, S, nullptr, rstd_out, M, D, eps));
   LT_LAUNCH_CHECK();
   return 0;
 }
@@ -525,24 +535,24 @@ int lt_norm_bwd(int layer_norm, const void* dy, const void* x, const void* w, co
     int g2 = (M + 7) / 8;
     if (g2 > grid) g2 = grid;
     if (g2 > sm_count()) g2 = sm_count();
-    rmsnorm_bwd_warp_kernel<1><<<g2, kNormThreads, 0, st>>>(DY, X, W, rstd, DR, DX, dw_part, M);
+    LT_RETURN_IF_CUDA(launch_chained(rmsnorm_bwd_warp_kernel<1>, g2, kNormThreads, 0, st, DY, X, W, rstd, DR, DX, dw_part, M));
     LT_LAUNCH_CHECK();
-    fold_partials_kernel<<<(D + 31) / 32, 1024, 0, st>>>(dw_part, dw, g2, D, grads_fp32, accumulate);
+    LT_RETURN_IF_CUDA(launch_chained(fold_partials_kernel, (D + 31) / 32, 1024, 0, st, dw_part, dw, g2, D, grads_fp32, accumulate));
     LT_LAUNCH_CHECK();
     return 0;
   }
   if (!layer_norm && ((D % 512 == 0 && D <= 4096) || (D % 1024 == 0 && D <= 8192)) && M >= 2 * sm_count()) {
     const int it = D <= 4096 ? 2 : 4, wide = D / (256 * it), groups = 8 / wide, threads = wide * groups * 32, bytes = groups * D * 4;
     const int need = (M + groups - 1) / groups, g2 = need < grid ? need : grid;
-    if (it == 2) rmsnorm_bwd_wide_kernel<2><<<g2, threads, bytes, st>>>(DY, X, W, rstd, DR, DX, dw_part, M, wide);
-    else rmsnorm_bwd_wide_kernel<4><<<g2, threads, bytes, st>>>(DY, X, W, rstd, DR, DX, dw_part, M, wide);
+    if (it == 2) LT_RETURN_IF_CUDA(launch_chained(rmsnorm_bwd_wide_kernel<2>, g2, threads, bytes, st, DY, X, W, rstd, DR, DX, dw_part, M, wide));
+    else LT_RETURN_IF_CUDA(launch_chained(rmsnorm_bwd_wide_kernel<4>, g2, threads, bytes, st, DY, X, W, rstd, DR, DX, dw_part, M, wide));
     LT_LAUNCH_CHECK();
-    fold_partials_kernel<<<(D + 31) / 32, 1024, 0, st>>>(dw_part, dw, g2, D, grads_fp32, accumulate);
+    LT_RETURN_IF_CUDA(launch_chained(fold_partials_kernel, (D + 31) / 32, 1024, 0, st, dw_part, dw, g2, D, grads_fp32, accumulate));
     LT_LAUNCH_CHECK();
     return 0;
   }
 #define LT_NORM_BWD(LN, IT) \
-  norm_bwd_kernel<LN, IT><<<grid, kNormThreads, 0, st>>>(DY, X, W, mean, rstd, DR, DX, dw_part, db_part, M, D)
+  LT_RETURN_IF_CUDA(launch_chained(norm_bwd_kernel<LN, IT>, grid, kNormThreads, 0, st, DY, X, W, mean, rstd, DR, DX, dw_part, db_part, M, D))
   if (layer_norm) {
     if (iters <= 1) LT_NORM_BWD(true, 1); else if (iters <= 2) LT_NORM_BWD(true, 2);
     else if (iters <= 4) LT_NORM_BWD(true, 4); else LT_NORM_BWD(true, 8);
@@ -553,8 +563,8 @@ int lt_norm_bwd(int layer_norm, const void* dy, const void* x, const void* w, co
 #undef LT_NORM_BWD
   LT_LAUNCH_CHECK();
   const int fb = (D + 31) / 32;
-  fold_partials_kernel<<<fb, 1024, 0, st>>>(dw_part, dw, grid, D, grads_fp32, accumulate);
-  if (layer_norm && db && db_part) fold_partials_kernel<<<fb, 1024, 0, st>>>(db_part, db, grid, D, grads_fp32, accumulate);
+  LT_RETURN_IF_CUDA(launch_chained(fold_partials_kernel, fb, 1024, 0, st, dw_part, dw, grid, D, grads_fp32, accumulate));
+  if (layer_norm && db && db_part) LT_RETURN_IF_CUDA(launch_chained(fold_partials_kernel, fb, 1024, 0, st, db_part, db, grid, D, grads_fp32, accumulate));
   LT_LAUNCH_CHECK();
   return 0;
 }

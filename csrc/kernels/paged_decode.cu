@@ -424,6 +424,8 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     fence_barrier_init();
     fence_proxy_async();
   }
+  pdl_launch_dependents();
+  pdl_wait();
   // A fragments of the query block: rows = heads of the group (g and g + 8), zero past G
   uint32_t qa[KS][4];
   {
@@ -671,6 +673,8 @@ paged_decode_f8_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     fence_barrier_init();
     fence_proxy_async();
   }
+  pdl_launch_dependents();
+  pdl_wait();
   // offset of 16-byte unit u of row r inside a tile
   auto unit = [](int r, int u) { return D == 128 ? r * 128 + ((u ^ (r & 7)) << 4) : r * 64 + (u << 4); };
   // A fragments of the query block, columns permuted: step kk = 4 h + r takes columns 64 h + 16 qd + 4 r + {0 .. 3}.  Rows = heads of the
@@ -869,9 +873,10 @@ paged_decode_f8_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
 template <int D>
 __global__ void paged_decode_merge_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ o, int rows, int splits,
                                           const __nv_bfloat16* __restrict__ gate, long long ldg, int Hq, int vdim) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int row = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  pdl_launch_dependents();   // a product behind this one may fetch its weights
   if (row >= rows) return;
   constexpr int E = D / 32;
   // A lane reads maximum and sum of one split, so that their loads are under way together, as are then those of the outputs (one split
@@ -988,10 +993,10 @@ int lt_paged_decode_window(const void* q, const void* k_cache, const void* v_cac
       LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdMmaCfg<128>::kSmemBytes));
       configured_mma.finish();
     }
-    if (kv_fp8 && D == 64) paged_decode_f8_kernel<64><<<ctas, kPdWarps * 32, PdF8Cfg<64>::kSmemBytes, st>>>(tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale * k_scale, v_scale, window, status);
-    else if (kv_fp8) paged_decode_f8_kernel<128><<<ctas, kPdWarps * 32, PdF8Cfg<128>::kSmemBytes, st>>>(tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale * k_scale, v_scale, window, status);
-    else if (D == 64) paged_decode_mma_kernel<64><<<ctas, kPdWarps * 32, PdMmaCfg<64>::kSmemBytes, st>>>(tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale, window, status);
-    else paged_decode_mma_kernel<128><<<ctas, kPdWarps * 32, PdMmaCfg<128>::kSmemBytes, st>>>(tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale, window, status);
+    if (kv_fp8 && D == 64) LT_RETURN_IF_CUDA(launch_chained(paged_decode_f8_kernel<64>, ctas, kPdWarps * 32, PdF8Cfg<64>::kSmemBytes, st, tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale * k_scale, v_scale, window, status));
+    else if (kv_fp8) LT_RETURN_IF_CUDA(launch_chained(paged_decode_f8_kernel<128>, ctas, kPdWarps * 32, PdF8Cfg<128>::kSmemBytes, st, tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale * k_scale, v_scale, window, status));
+    else if (D == 64) LT_RETURN_IF_CUDA(launch_chained(paged_decode_mma_kernel<64>, ctas, kPdWarps * 32, PdMmaCfg<64>::kSmemBytes, st, tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale, window, status));
+    else LT_RETURN_IF_CUDA(launch_chained(paged_decode_mma_kernel<128>, ctas, kPdWarps * 32, PdMmaCfg<128>::kSmemBytes, st, tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale, window, status));
   } else if (!kv_fp8 && window == 0 && G <= kPdMaxG && bs_ok && (reinterpret_cast<uintptr_t>(k_cache) & 15) == 0 && (reinterpret_cast<uintptr_t>(v_cache) & 15) == 0) {
     // bf16 caches: every K / V byte is read once for the whole group of query heads, through a shared-memory pipeline
     const int ctas = S * Hkv * splits;
@@ -1014,8 +1019,8 @@ int lt_paged_decode_window(const void* q, const void* k_cache, const void* v_cac
   const int mb = (rows + 3) / 4;
   auto O = static_cast<__nv_bfloat16*>(o);
   auto GT = static_cast<const __nv_bfloat16*>(gate);
-  if (D == 64) paged_decode_merge_kernel<64><<<mb, 128, 0, st>>>(part, O, rows, splits, GT, ldg, Hq, vdim);
-  else paged_decode_merge_kernel<128><<<mb, 128, 0, st>>>(part, O, rows, splits, GT, ldg, Hq, vdim);
+  if (D == 64) LT_RETURN_IF_CUDA(launch_chained(paged_decode_merge_kernel<64>, mb, 128, 0, st, part, O, rows, splits, GT, ldg, Hq, vdim));
+  else LT_RETURN_IF_CUDA(launch_chained(paged_decode_merge_kernel<128>, mb, 128, 0, st, part, O, rows, splits, GT, ldg, Hq, vdim));
   LT_LAUNCH_CHECK();
   return 0;
 }

@@ -35,6 +35,8 @@ __device__ __forceinline__ void st8(__nv_bfloat16* p, const float (&f)[8]) {
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ cos_t,
                             const float* __restrict__ sin_t, const int* __restrict__ pos, long long rows, int T,
                             int heads, int hd, long long row_stride, float sign) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int vec_per_head = hd / 8;
   const long long total = rows * heads * vec_per_head;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -67,6 +69,8 @@ __global__ void rope_append_kernel(__nv_bfloat16* __restrict__ qkv, long long ld
                                    const int* __restrict__ pos, const int* __restrict__ slots, __nv_bfloat16* __restrict__ q_out,
                                    void* __restrict__ k_cache, void* __restrict__ v_cache, long long rows, int Hq, int Hkv, int hd, int block_size,
                                    float k_inv, float v_inv) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int vph = hd / 8, heads = Hq + 2 * Hkv;
   const long long total = rows * heads * vph;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -111,6 +115,8 @@ __global__ void rope_append_kernel(__nv_bfloat16* __restrict__ qkv, long long ld
 // ---------------------------------------------------------------------------------------------- SwiGLU
 // gu: [M, 2F] with gate in columns [0,F) and up in [F,2F).  h = silu(gate) * up.
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h, long long M, int F) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int vpr = F / 8;
   const long long total = M * vpr;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -192,6 +198,8 @@ __global__ void act_glu_kernel(const T* __restrict__ gu, T* __restrict__ h, long
 template <typename T>
 __global__ void token_gate_kernel(const T* __restrict__ g, const int* __restrict__ tokens, const T* __restrict__ table, long long ldt,
                                   int off, int dim, int ld, T* __restrict__ out, long long total) {
+  pdl_launch_dependents();
+  pdl_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long n = i / ld;
     const int c = int(i - n * ld);
@@ -201,6 +209,8 @@ __global__ void token_gate_kernel(const T* __restrict__ g, const int* __restrict
 
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* gu, const __nv_bfloat16* __restrict__ dh, __nv_bfloat16* dgu,
                                   long long M, int F) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int vpr = F / 8;
   const long long total = M * vpr;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -270,6 +280,8 @@ __global__ void axpby_kernel(const __nv_bfloat16* a, const __nv_bfloat16* b, __n
 // ---------------------------------------------------------------------------------------------- embedding
 __global__ void embedding_fwd_kernel(const long long* __restrict__ idx, const __nv_bfloat16* __restrict__ table,
                                      __nv_bfloat16* __restrict__ out, long long n_tok, int D, int V) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int vpr = D / 8;
   const long long total = n_tok * vpr;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -283,6 +295,8 @@ __global__ void embedding_fwd_kernel(const long long* __restrict__ idx, const __
 // dtable[idx[r]] += dout[r]   (bf16x2 atomics; dtable must be zeroed or hold the running gradient)
 __global__ void embedding_bwd_kernel(const long long* __restrict__ idx, const __nv_bfloat16* __restrict__ dout,
                                      __nv_bfloat16* __restrict__ dtable, long long n_tok, int D, int V) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int ppr = D / 2;
   const long long total = n_tok * ppr;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -339,8 +353,7 @@ int lt_rope(void* x, const float* cos_t, const float* sin_t, const int* pos, lon
   if (hd % 8 != 0 || row_stride % 8 != 0) return -int(kStatusBadArgument);
   const long long work = rows * heads * (hd / 8);
   if (work == 0) return 0;
-  rope_kernel<<<grid_for(work, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<__nv_bfloat16*>(x), cos_t, sin_t, pos, rows, T, heads, hd, row_stride, backward ? -1.f : 1.f);
+  LT_RETURN_IF_CUDA(launch_chained(rope_kernel, grid_for(work, 256), 256, 0, static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(x), cos_t, sin_t, pos, rows, T, heads, hd, row_stride, backward ? -1.f : 1.f));
   LT_LAUNCH_CHECK();
   return 0;
 }
@@ -359,9 +372,9 @@ int lt_rope_append(void* qkv, long long ld, const float* cos_t, const float* sin
   auto X = static_cast<__nv_bfloat16*>(qkv);
   auto Q = static_cast<__nv_bfloat16*>(q_out);
   if (kv_fp8)
-    rope_append_kernel<true><<<grid_for(work, 256), 256, 0, st>>>(X, ld, cos_t, sin_t, pos, slots, Q, k_cache, v_cache, rows, Hq, Hkv, hd, block_size, 1.f / k_scale, 1.f / v_scale);
+    LT_RETURN_IF_CUDA(launch_chained(rope_append_kernel<true>, grid_for(work, 256), 256, 0, st, X, ld, cos_t, sin_t, pos, slots, Q, k_cache, v_cache, rows, Hq, Hkv, hd, block_size, 1.f / k_scale, 1.f / v_scale));
   else
-    rope_append_kernel<false><<<grid_for(work, 256), 256, 0, st>>>(X, ld, cos_t, sin_t, pos, slots, Q, k_cache, v_cache, rows, Hq, Hkv, hd, block_size, 1.f, 1.f);
+    LT_RETURN_IF_CUDA(launch_chained(rope_append_kernel<false>, grid_for(work, 256), 256, 0, st, X, ld, cos_t, sin_t, pos, slots, Q, k_cache, v_cache, rows, Hq, Hkv, hd, block_size, 1.f, 1.f));
   LT_LAUNCH_CHECK();
   return 0;
 }
@@ -370,8 +383,7 @@ int lt_swiglu_fwd(const void* gu, void* h, long long M, int F, void* stream) {
   using namespace lt;
   if (F % 8 != 0) return -int(kStatusBadArgument);
   if (M == 0) return 0;
-  swiglu_fwd_kernel<<<grid_for(M * (F / 8), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(h), M, F);
+  LT_RETURN_IF_CUDA(launch_chained(swiglu_fwd_kernel, grid_for(M * (F / 8), 256), 256, 0, static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(h), M, F));
   LT_LAUNCH_CHECK();
   return 0;
 }
@@ -409,8 +421,8 @@ int lt_token_gate(int fp32, const void* g, const int* tokens, const void* table,
   if (total == 0) return 0;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   using bf = __nv_bfloat16;
-  if (fp32) token_gate_kernel<float><<<grid_for(total, 256), 256, 0, st>>>(static_cast<const float*>(g), tokens, static_cast<const float*>(table), ldt, off, dim, ld, static_cast<float*>(out), total);
-  else token_gate_kernel<bf><<<grid_for(total, 256), 256, 0, st>>>(static_cast<const bf*>(g), tokens, static_cast<const bf*>(table), ldt, off, dim, ld, static_cast<bf*>(out), total);
+  if (fp32) LT_RETURN_IF_CUDA(launch_chained(token_gate_kernel<float>, grid_for(total, 256), 256, 0, st, static_cast<const float*>(g), tokens, static_cast<const float*>(table), ldt, off, dim, ld, static_cast<float*>(out), total));
+  else LT_RETURN_IF_CUDA(launch_chained(token_gate_kernel<bf>, grid_for(total, 256), 256, 0, st, static_cast<const bf*>(g), tokens, static_cast<const bf*>(table), ldt, off, dim, ld, static_cast<bf*>(out), total));
   LT_LAUNCH_CHECK();
   return 0;
 }
@@ -418,8 +430,7 @@ int lt_swiglu_bwd(const void* gu, const void* dh, void* dgu, long long M, int F,
   using namespace lt;
   if (F % 8 != 0) return -int(kStatusBadArgument);
   if (M == 0) return 0;
-  swiglu_bwd_kernel<<<grid_for(M * (F / 8), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(gu), static_cast<const __nv_bfloat16*>(dh), static_cast<__nv_bfloat16*>(dgu), M, F);
+  LT_RETURN_IF_CUDA(launch_chained(swiglu_bwd_kernel, grid_for(M * (F / 8), 256), 256, 0, static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(gu), static_cast<const __nv_bfloat16*>(dh), static_cast<__nv_bfloat16*>(dgu), M, F));
   LT_LAUNCH_CHECK();
   return 0;
 }
@@ -454,8 +465,7 @@ int lt_embedding_fwd(const long long* idx, const void* table, void* out, long lo
   using namespace lt;
   if (D % 8 != 0) return -int(kStatusBadArgument);
   if (n_tok == 0) return 0;
-  embedding_fwd_kernel<<<grid_for(n_tok * (D / 8), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      idx, static_cast<const __nv_bfloat16*>(table), static_cast<__nv_bfloat16*>(out), n_tok, D, V);
+  LT_RETURN_IF_CUDA(launch_chained(embedding_fwd_kernel, grid_for(n_tok * (D / 8), 256), 256, 0, static_cast<cudaStream_t>(stream), idx, static_cast<const __nv_bfloat16*>(table), static_cast<__nv_bfloat16*>(out), n_tok, D, V));
   LT_LAUNCH_CHECK();
   return 0;
 }
@@ -463,8 +473,7 @@ int lt_embedding_bwd(const long long* idx, const void* dout, void* dtable, long 
   using namespace lt;
   if (D % 2 != 0) return -int(kStatusBadArgument);
   if (n_tok == 0) return 0;
-  embedding_bwd_kernel<<<grid_for(n_tok * (D / 2), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      idx, static_cast<const __nv_bfloat16*>(dout), static_cast<__nv_bfloat16*>(dtable), n_tok, D, V);
+  LT_RETURN_IF_CUDA(launch_chained(embedding_bwd_kernel, grid_for(n_tok * (D / 2), 256), 256, 0, static_cast<cudaStream_t>(stream), idx, static_cast<const __nv_bfloat16*>(dout), static_cast<__nv_bfloat16*>(dtable), n_tok, D, V));
   LT_LAUNCH_CHECK();
   return 0;
 }

@@ -8,6 +8,7 @@
 // embedding row; the last one takes the wanted rows only and keeps nothing.
 #include "lt_cuda.h"
 #include "common/host.h"
+#include "common/ptx.cuh"
 #include "common/scalar.cuh"
 
 namespace lt {
@@ -35,6 +36,8 @@ struct ResidualParams {
 constexpr int max_threads(int V) { return V == 4 ? 512 : 1024; }
 template <typename T, int V, int NC>
 __global__ void __launch_bounds__(max_threads(V)) residual_norm_kernel(const ResidualParams p) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[64];
   const int W = p.width, nt = blockDim.x;
   const long long row = p.rows ? p.rows[blockIdx.x] : blockIdx.x;
@@ -175,10 +178,10 @@ static int launch_residual(const ResidualParams& p, int rows, cudaStream_t st) {
   if (pieces > max_threads(V) * nc) return -4;
   const int threads = ((pieces + nc - 1) / nc + 31) / 32 * 32;
   switch (nc) {
-    case 1: residual_norm_kernel<T, V, 1><<<rows, threads, 0, st>>>(p); break;
-    case 2: residual_norm_kernel<T, V, 2><<<rows, threads, 0, st>>>(p); break;
-    case 4: residual_norm_kernel<T, V, 4><<<rows, threads, 0, st>>>(p); break;
-    default: residual_norm_kernel<T, V, 8><<<rows, threads, 0, st>>>(p); break;
+    case 1: LT_RETURN_IF_CUDA(launch_chained(residual_norm_kernel<T, V, 1>, rows, threads, 0, st, p)); break;
+    case 2: LT_RETURN_IF_CUDA(launch_chained(residual_norm_kernel<T, V, 2>, rows, threads, 0, st, p)); break;
+    case 4: LT_RETURN_IF_CUDA(launch_chained(residual_norm_kernel<T, V, 4>, rows, threads, 0, st, p)); break;
+    default: LT_RETURN_IF_CUDA(launch_chained(residual_norm_kernel<T, V, 8>, rows, threads, 0, st, p)); break;
   }
   LT_LAUNCH_CHECK();
   return 0;

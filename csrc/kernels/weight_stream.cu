@@ -101,9 +101,10 @@ weight_stream_kernel(const __grid_constant__ CUtensorMap tw, const __grid_consta
     }
   };
   pdl_launch_dependents();
+  if (!p.early) pdl_wait();
 #pragma unroll
   for (int s = 0; s < S; ++s) load(true, false);
-  pdl_wait();
+  if (p.early) pdl_wait();
   at_tile = blockIdx.x; at = 0; at_slot = 0;
 #pragma unroll
   for (int s = 0; s < S; ++s) load(false, true);
@@ -226,17 +227,7 @@ static int launch_ws(const StreamProduct& p, cudaStream_t st) {
   r = encode_tmap_2d(&tx, p.x, 2, p.K, p.M, (uint64_t)p.ldx * 2, 64, XR, 1);
   if (r) return 2000 + r;
   const int tiles = (p.N + cols - 1) / cols;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(tiles < room ? tiles : room);
-  cfg.blockDim = dim3(Cfg::kWarps * 32);
-  cfg.dynamicSmemBytes = Cfg::kSmem;
-  cfg.stream = st;
-  cfg.attrs = &attr;
-  cfg.numAttrs = p.early ? 1 : 0;
-  LT_RETURN_IF_CUDA(cudaLaunchKernelEx(&cfg, kern, tw, tx, p, tiles, cols, device_status_word()));
+  LT_RETURN_IF_CUDA(launch_chained(kern, dim3(tiles < room ? tiles : room), dim3(Cfg::kWarps * 32), Cfg::kSmem, st, tw, tx, p, tiles, cols, device_status_word()));
   return 0;
 }
 
