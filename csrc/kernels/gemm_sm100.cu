@@ -6,6 +6,7 @@
 #include "gemm_sm100_2cta.cuh"
 
 #include <atomic>
+#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -52,24 +53,42 @@ static int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, cons
   return 0;
 }
 
-template <int BLOCK_N, int EPI>
-__global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_staged_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
-                   const GemmParams p) {
-  gemm_body<BLOCK_N, 0, 0, 0, false, EPI>(&tmA, &tmB, p, NoGate(), NoDone(), 0, &tmC);
+template <int A_MAJOR, int B_MAJOR, int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kStagedThreads, 1)
+gemm_pair_staged_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ PairOutMaps outs,
+                        const GemmParams p) {
+  gemm_body_pair<A_MAJOR, B_MAJOR, 0, EPI>(&tmA, &tmB, p, NoGate(), NoDone(), 0, nullptr, &outs);
 }
 
-template <int BLOCK_N, int EPI>
+template <int A_MAJOR, int B_MAJOR, int EPI>
+static int launch_pair_staged(const CUtensorMap& tmA, const CUtensorMap& tmB, const PairOutMaps& outs, const GemmParams& p, int grid, cudaStream_t st) {
+  static OncePerDevice configured;
+  auto kern = gemm_pair_staged_kernel<A_MAJOR, B_MAJOR, EPI>;
+  if (configured.pending()) {
+    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairStagedSmemBytes));
+    configured.finish();
+  }
+  LT_RETURN_IF_CUDA(launch_chained(kern, grid, kStagedThreads, kPairStagedSmemBytes, st, tmA, tmB, outs, p));
+  return 0;
+}
+
+template <int BLOCK_N, int A_MAJOR, int B_MAJOR>
+__global__ void __launch_bounds__(kStagedThreads, 1)
+gemm_staged_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
+                   const GemmParams p) {
+  gemm_body<BLOCK_N, A_MAJOR, B_MAJOR, 0, false, kEpiStaged>(&tmA, &tmB, p, NoGate(), NoDone(), 0, &tmC);
+}
+
+template <int BLOCK_N, int A_MAJOR = 0, int B_MAJOR = 0>
 static int launch_staged(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const GemmParams& p, int grid,
                          cudaStream_t st) {
   static OncePerDevice configured;
-  auto kern = gemm_staged_kernel<BLOCK_N, EPI>;
+  auto kern = gemm_staged_kernel<BLOCK_N, A_MAJOR, B_MAJOR>;
   if (configured.pending()) {
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<BLOCK_N>::kStagedSmemBytes));
     configured.finish();
   }
-  LT_RETURN_IF_CUDA(launch_chained(kern, grid, kGemmThreads, GemmCfg<BLOCK_N>::kStagedSmemBytes, st, tmA, tmB, tmC, p));
-  LT_LAUNCH_CHECK();
+  LT_RETURN_IF_CUDA(launch_chained(kern, grid, kStagedThreads, GemmCfg<BLOCK_N>::kStagedSmemBytes, st, tmA, tmB, tmC, p));
   return 0;
 }
 
@@ -207,8 +226,34 @@ int lt_gemm_e4m3(const void* A, const void* B, void* C, int M, int N, int K, lon
                      a_scale, b_scale);
 }
 
-// C [M, N] bf16 = alpha * A [M, K] @ B [N, K]^T with the staged epilogue; block_n 0: choose, 128 or 256.  With act (1 GELU, 2 SiLU): B is
-// [2 N, K], gate rows, then up rows, and C = act(gate) * up.  Pitches in elements, multiples of 8; N a multiple of 8.
+// A @ B^T with gates on CTA pairs; GU: where gate and up go too, [M, 2 N] of pitch ldg, or nullptr.
+static int glu_on_pairs(const void* A, const void* B, void* C, void* GU, int M, int N, int K, long long lda, long long ldb, long long ldc, long long ldg,
+                        int act, float alpha, cudaStream_t st) {
+  using namespace lt;
+  GemmParams p{};
+  p.M = M; p.N = N; p.K = K;
+  p.C = C; p.ldc = ldc; p.alpha = alpha;
+  p.glu_act = act;
+  p.status = device_status_word();
+  fill_tiles(p, kPairBlockN);
+  fill_pair_tiles(p);
+  p.n_blocks = (N + kPairBlockN / 2 - 1) / (kPairBlockN / 2);
+  p.num_tiles = p.dp_tiles = p.m_blocks * p.n_blocks;
+  CUtensorMap tmA, tmB;
+  PairOutMaps outs{};
+  int r = make_operand_maps(&tmA, &tmB, A, B, M, 2 * N, K, lda, ldb, 0, 0, kPairBlockN / 2);
+  if (r) return r;
+  r = make_staged_map(&outs.c, C, M, N, ldc);
+  if (!r && GU) r = make_staged_map(&outs.gate, GU, M, N, ldg);
+  if (!r && GU) r = make_staged_map(&outs.up, static_cast<const __nv_bfloat16*>(GU) + N, M, N, ldg);
+  if (r) return 3000 + r;
+  const int pairs = sm_count() / 2, grid = 2 * (pairs < p.num_tiles ? pairs : p.num_tiles);
+  return GU ? launch_pair_staged<0, 0, kEpiGluKeep>(tmA, tmB, outs, p, grid, st) : launch_pair_staged<0, 0, kEpiGlu>(tmA, tmB, outs, p, grid, st);
+}
+
+// C [M, N] bf16 = alpha * A [M, K] @ B [N, K]^T with the staged epilogue; block_n 0: choose, 128 or 256: width of a CTA's tile.  With act (1 GELU, 2 SiLU): B
+// is [2 N, K], gate rows, then up rows, and C = act(gate) * up, on CTA pairs (us, a CTA a tile / pairs: 8192 x 5632 x 2048 280 / 264, 1337 x 14336 x 4096 265 / 254,
+// 512 x 14336 x 4096 120 / 102, 129 x 5632 x 2048 27.7 / 20.7).  Pitches in elements, multiples of 8; N a multiple of 8.
 int lt_gemm_staged(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc, int act,
                    float alpha, int block_n, void* stream) {
   using namespace lt;
@@ -216,24 +261,34 @@ int lt_gemm_staged(const void* A, const void* B, void* C, int M, int N, int K, l
   if ((lda & 7) || (ldb & 7) || (ldc & 7) || (N & 7) || act < 0 || act > 2 || (reinterpret_cast<uintptr_t>(A) & 15) ||
       (reinterpret_cast<uintptr_t>(B) & 15) || (reinterpret_cast<uintptr_t>(C) & 15))
     return -int(kStatusBadArgument);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (act) return glu_on_pairs(A, B, C, nullptr, M, N, K, lda, ldb, ldc, 0, act, alpha, st);
   const int sms = sm_count();
-  if (act) block_n = 256;
-  else if (block_n != 128 && block_n != 256) block_n = pick_block_n(M, N, sms);
+  if (block_n != 128 && block_n != 256) block_n = pick_block_n(M, N, sms);
   GemmParams p{};
   p.M = M; p.N = N; p.K = K;
   p.C = C; p.ldc = ldc; p.alpha = alpha;
-  p.glu_act = act;
   p.status = device_status_word();
-  fill_tiles(p, act ? 128 : block_n);
+  fill_tiles(p, block_n);
   CUtensorMap tmA, tmB, tmC;
-  int r = make_operand_maps(&tmA, &tmB, A, B, M, act ? 2 * N : N, K, lda, ldb, 0, 0, act ? 128 : block_n);
+  int r = make_operand_maps(&tmA, &tmB, A, B, M, N, K, lda, ldb, 0, 0, block_n);
   if (r) return r;
   r = make_staged_map(&tmC, C, M, N, ldc);
   if (r) return 3000 + r;
   const int grid = p.num_tiles < sms ? p.num_tiles : sms;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (act) return launch_staged<256, kEpiGlu>(tmA, tmB, tmC, p, grid, st);
-  return block_n == 256 ? launch_staged<256, kEpiStaged>(tmA, tmB, tmC, p, grid, st) : launch_staged<128, kEpiStaged>(tmA, tmB, tmC, p, grid, st);
+  return block_n == 256 ? launch_staged<256>(tmA, tmB, tmC, p, grid, st) : launch_staged<128>(tmA, tmB, tmC, p, grid, st);
+}
+
+// GU [M, 2 N] = A @ B^T for B [2 N, K] = gate rows, then up rows, and C [M, N] = act(gate) * up of the 32-bit sums, in one pass (a training step keeps
+// GU for the way back).  Pitches in elements, multiples of 8; N a multiple of 8; bases 16-byte aligned.
+int lt_gemm_glu_keep(const void* A, const void* B, void* C, void* GU, int M, int N, int K, long long lda, long long ldb, long long ldc, long long ldg,
+                     int act, void* stream) {
+  using namespace lt;
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  for (const void* q : {A, B, static_cast<const void*>(C), static_cast<const void*>(GU)})
+    if (!q || (reinterpret_cast<uintptr_t>(q) & 15)) return -int(kStatusBadArgument);
+  if ((lda & 7) || (ldb & 7) || (ldc & 7) || (ldg & 7) || (N & 7) || act < 1 || act > 2) return -int(kStatusBadArgument);
+  return glu_on_pairs(A, B, C, GU, M, N, K, lda, ldb, ldc, ldg, act, 1.f, static_cast<cudaStream_t>(stream));
 }
 
 // C[M, blocks * nb] (fp32) = A[M, blocks * K] @ blockdiag(B_0 .. )^T with B [blocks, nb, K]: columns z * nb .. of C are the
@@ -275,8 +330,11 @@ static int gemm_launch(int kind, const void* A, const void* B, void* C, int M, i
   // int8: integer accumulators are converted in the one-CTA kernel's epilogue; no K split (its workspace holds floats)
   const bool split_on = kind != 3 && g_split_enabled.load() != 0;
   const int pair_mode = kind == 3 ? 0 : g_pair_mode.load();
+  // bf16 results with nothing but a residual (or C itself) added leave through shared memory and TMA
+  const bool stage = kind == 0 && !out_fp32 && !bias && !act && !(accumulate && residual) && !(ldc & 7) && !(N & 7) &&
+                     !(residual && (ldr & 7)) && ((reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(residual)) & 15) == 0;
   if (pair_mode > 0 && block_n != 128 && (max_ctas <= 0 || max_ctas >= sms)) {
-    const double c256 = wave_cost(M, N, K, sms, 256), c128 = wave_cost(M, N, K, sms, 128);
+    const double c256 = wave_cost(M, N, K, sms, 256, split_on && !stage), c128 = wave_cost(M, N, K, sms, 128, split_on && !stage);
     const double single = c256 < c128 ? c256 : c128;
     if (pair_mode == 2 || pair_cost(M, N, K, sms, split_on) < single) {
       GemmParams q{};
@@ -297,11 +355,12 @@ static int gemm_launch(int kind, const void* A, const void* B, void* C, int M, i
       if (pairs > q.num_tiles) pairs = q.num_tiles;
       cudaStream_t st = static_cast<cudaStream_t>(stream);
       if (split_on) {
-        const int split = pair_tail_split(q.num_tiles, q.k_blocks, pairs);
+        const int split = tail_split(q.num_tiles, q.k_blocks, sms / 2);
         SplitWs w;
         if (split > 1 && get_split_ws(st, &w)) {
-          q.dp_tiles = (q.num_tiles / pairs) * pairs;
+          q.dp_tiles = q.num_tiles / (sms / 2) * (sms / 2);
           q.sk_tiles = q.num_tiles - q.dp_tiles;
+          if (q.dp_tiles == 0) pairs = q.sk_tiles * split;
           q.sk_split = split;
           q.sk_ws = w.ws;
           q.sk_flags = w.flags;
@@ -310,6 +369,18 @@ static int gemm_launch(int kind, const void* A, const void* B, void* C, int M, i
       if (kind == 2) return launch_gemm_pair<0, 0, 2>(tmA, tmB, q, 2 * pairs, st);   // tf32: both operands K-major
       if (kind == 4) return launch_gemm_pair<0, 0, 4>(tmA, tmB, q, 2 * pairs, st);   // e4m3: both operands K-major
       const int key2 = (a_major ? 2 : 0) | (b_major ? 1 : 0);
+      if (stage) {
+        if (accumulate) { q.residual = static_cast<const __nv_bfloat16*>(C); q.ldr = ldc; }
+        PairOutMaps outs{};
+        r = make_staged_map(&outs.c, C, M, N, ldc);
+        if (r) return 3000 + r;
+        switch (key2) {
+          case 0: return launch_pair_staged<0, 0, kEpiStaged>(tmA, tmB, outs, q, 2 * pairs, st);
+          case 1: return launch_pair_staged<0, 1, kEpiStaged>(tmA, tmB, outs, q, 2 * pairs, st);
+          case 2: return launch_pair_staged<1, 0, kEpiStaged>(tmA, tmB, outs, q, 2 * pairs, st);
+          default: return launch_pair_staged<1, 1, kEpiStaged>(tmA, tmB, outs, q, 2 * pairs, st);
+        }
+      }
       switch (key2) {
         case 0: return launch_gemm_pair<0, 0>(tmA, tmB, q, 2 * pairs, st);
         case 1: return launch_gemm_pair<0, 1>(tmA, tmB, q, 2 * pairs, st);
@@ -318,7 +389,7 @@ static int gemm_launch(int kind, const void* A, const void* B, void* C, int M, i
       }
     }
   }
-  if (block_n != 128 && block_n != 256) block_n = split_on ? pick_block_n_split(M, N, K, sms) : pick_block_n(M, N, sms);
+  if (block_n != 128 && block_n != 256) block_n = split_on && !stage ? pick_block_n_split(M, N, K, sms) : pick_block_n(M, N, sms);
   GemmParams p{};
   p.kind = kind;
   p.M = M; p.N = N; p.K = K;
@@ -334,14 +405,32 @@ static int gemm_launch(int kind, const void* A, const void* B, void* C, int M, i
   if (r) return r;
   int grid = sms;
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
+  const int slots = grid;
   if (grid > p.num_tiles) grid = p.num_tiles;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (stage) {
+    if (accumulate) { p.residual = static_cast<const __nv_bfloat16*>(C); p.ldr = ldc; }
+    CUtensorMap tmC;
+    r = make_staged_map(&tmC, C, M, N, ldc);
+    if (r) return 3000 + r;
+    switch ((block_n == 256 ? 4 : 0) | (a_major ? 2 : 0) | (b_major ? 1 : 0)) {
+      case 0: return launch_staged<128, 0, 0>(tmA, tmB, tmC, p, grid, st);
+      case 1: return launch_staged<128, 0, 1>(tmA, tmB, tmC, p, grid, st);
+      case 2: return launch_staged<128, 1, 0>(tmA, tmB, tmC, p, grid, st);
+      case 3: return launch_staged<128, 1, 1>(tmA, tmB, tmC, p, grid, st);
+      case 4: return launch_staged<256, 0, 0>(tmA, tmB, tmC, p, grid, st);
+      case 5: return launch_staged<256, 0, 1>(tmA, tmB, tmC, p, grid, st);
+      case 6: return launch_staged<256, 1, 0>(tmA, tmB, tmC, p, grid, st);
+      default: return launch_staged<256, 1, 1>(tmA, tmB, tmC, p, grid, st);
+    }
+  }
   if (split_on) {
-    const int split = tail_split(p.num_tiles, p.k_blocks, grid);
+    const int split = tail_split(p.num_tiles, p.k_blocks, slots);
     SplitWs w;
     if (split > 1 && get_split_ws(st, &w)) {
-      p.dp_tiles = (p.num_tiles / grid) * grid;
+      p.dp_tiles = p.num_tiles / slots * slots;
       p.sk_tiles = p.num_tiles - p.dp_tiles;
+      if (p.dp_tiles == 0) grid = p.sk_tiles * split;
       p.sk_split = split;
       p.sk_ws = w.ws;
       p.sk_flags = w.flags;

@@ -27,6 +27,7 @@ constexpr int kBlockM = 128;
 constexpr int kBlockK = 64;
 constexpr int kUmmaK = 16;
 constexpr int kGemmThreads = 192;
+constexpr int kStagedThreads = 64 + 8 * 32;   // kernels with a staged epilogue: eight epilogue warps
 
 struct GemmParams {
   // Operand element kind: 0 = bf16, 1 = fp16 (both kind::f16), 2 = fp32 used as tf32 (kind::tf32), 3 = signed int8
@@ -119,14 +120,14 @@ struct GemmCfg {
   static constexpr int kTmemCols = 2 * BLOCK_N;
   static constexpr int kBarrierBytes = 512;
   static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + kBarrierBytes;
-  // With a staged epilogue: two 32 x 64 bf16 pieces for each of the four epilogue warps behind the barriers.
+  // With a staged epilogue: a 32 x 64 bf16 piece for each of the eight epilogue warps behind the barriers.
   static constexpr int kOffStaging = kStages * kStageBytes + 1024;
-  static constexpr int kStagedSmemBytes = kOffStaging + 4 * 2 * 4096 + 1024;
+  static constexpr int kStagedSmemBytes = kOffStaging + 8 * 4096 + 1024;
 };
 
-// Epilogues of the one-CTA kernel: everything in registers and stored from there; bf16 results staged in shared memory and
-// written by TMA (alpha alone is applied); the same with act(gate) * up of a tile's two column halves.
-enum { kEpiDirect = 0, kEpiStaged = 1, kEpiGlu = 2 };
+// Epilogues: everything in registers and stored from there; bf16 results staged in shared memory and written by TMA, by eight warps (alpha is applied and a
+// residual added, nothing else); act(gate) * up of a tile's two column halves, staged; the same with gate and up written as well (CTA pairs).
+enum { kEpiDirect = 0, kEpiStaged = 1, kEpiGlu = 2, kEpiGluKeep = 3 };
 
 struct NoGate {
   __device__ __forceinline__ bool operator()(int, int, int, int*) const { return true; }
@@ -340,7 +341,8 @@ __device__ __forceinline__ void store_f32_lines(const GemmParams& p, int row, in
 template <int BLOCK_N, int A_MAJOR, int B_MAJOR, int MMA_KIND = 0, bool DIAG = false, int EPI = kEpiDirect, class TileGate, class TileDone>
 __device__ __forceinline__ void gemm_body(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p,
                                           TileGate gate, TileDone done, int cta_first = 0, const CUtensorMap* tmC = nullptr) {
-  static_assert(EPI == kEpiDirect || (B_MAJOR == 0 && !DIAG), "staged epilogues go with K-major weights");
+  static_assert(EPI != kEpiGluKeep && !(EPI == kEpiGlu && B_MAJOR) && !(EPI != kEpiDirect && DIAG), "no such epilogue");
+  constexpr int EW = EPI == kEpiDirect ? 4 : 8;   // epilogue warps
   // CTAs [0, cta_first) of the grid belong to another role of a fused kernel; the GEMM uses the rest.
   const int cta_id = int(blockIdx.x) - cta_first;
   const int cta_count = int(gridDim.x) - cta_first;
@@ -370,7 +372,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* tmA, const CUtensor
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(tfull_bar(b), 1);
-      mbar_init(tempty_bar(b), 4);
+      mbar_init(tempty_bar(b), EW);
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -471,25 +473,35 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* tmA, const CUtensor
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (4 warps)
+    // ------------------------------------------------------------------ epilogue
     const int quarter = warp & 3;  // TMEM lane quarter this warp may read
     WorkItem w;
-    [[maybe_unused]] int staged = 0;   // pieces this warp has handed to TMA
+    [[maybe_unused]] const int half = EW == 8 ? (warp - 2) >> 2 : 0;   // which 64-column pieces of a tile this warp takes
     for (int it = 0; get_item(p, cta_id, cta_count, it, w); ++it) {
       int m_blk, n_blk;
       tile_coords(p, w.tile, m_blk, n_blk);
       const int buf = it & 1;
       const uint32_t aphase = (it >> 1) & 1;
+      const int row = m_blk * kBlockM + quarter * 32 + lane;
+      // kEpiStaged: the residual's next 64 columns of this row are on their way while the tile is made, then while the columns before them leave
+      [[maybe_unused]] uint4 ahead[8];
+      [[maybe_unused]] auto fetch = [&](int c) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int col = n_blk * BLOCK_N + c * 64 + u * 8;
+          ahead[u] = make_uint4(0u, 0u, 0u, 0u);
+          if (p.residual && row < p.M && col < p.N) ahead[u] = *reinterpret_cast<const uint4*>(p.residual + (long long)row * p.ldr + col);
+        }
+      };
+      if constexpr (EPI == kEpiStaged) fetch(half);
       const bool got = mbar_wait(tfull_bar(buf), aphase, abort_flag, p.status, kStatusTimeoutTmemFull);
       if (!__all_sync(0xffffffffu, got)) break;
       tc_fence_after();
-      const int row = m_blk * kBlockM + quarter * 32 + lane;
       const uint32_t t_addr = tmem_base + (uint32_t(quarter * 32) << 16) + buf * BLOCK_N;
       if constexpr (EPI != kEpiDirect) {
         constexpr int OUT_N = EPI == kEpiGlu ? BLOCK_N / 2 : BLOCK_N;
 #pragma unroll 1
-        for (int c = 0; c < OUT_N / 64; ++c) {
-          if (n_blk * OUT_N + c * 64 >= p.N) break;
+        for (int c = half; c < OUT_N / 64; c += 2) {
           uint32_t w[32];                          // 64 results of this lane's row as bf16 pairs
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
@@ -507,13 +519,21 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* tmA, const CUtensor
             } else {
               tmem_ld_wait();
 #pragma unroll
-              for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * p.alpha);
+              for (int j = 0; j < 16; ++j) {
+                const uint4& q = ahead[hh * 4 + j / 4];
+                const float2 f = unpack_bf16x2(j % 4 == 0 ? q.x : j % 4 == 1 ? q.y : j % 4 == 2 ? q.z : q.w);
+                r[2 * j] = __float_as_uint(__uint_as_float(r[2 * j]) * p.alpha + f.x);
+                r[2 * j + 1] = __float_as_uint(__uint_as_float(r[2 * j + 1]) * p.alpha + f.y);
+              }
             }
 #pragma unroll
             for (int j = 0; j < 16; ++j) w[hh * 16 + j] = pack_bf16x2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
           }
-          uint8_t* piece = smem + Cfg::kOffStaging + ((warp - 2) * 2 + (staged & 1)) * 4096;
-          if (lane == 0) tma_store_wait_read<1>();   // the store that last used this piece has read it
+          if constexpr (EPI == kEpiStaged) {
+            if (c + 2 < OUT_N / 64) fetch(c + 2);
+          }
+          uint8_t* piece = smem + Cfg::kOffStaging + (warp - 2) * 4096;
+          if (lane == 0) tma_store_wait_read<0>();   // the store before has read the piece
           __syncwarp();
 #pragma unroll
           for (int u = 0; u < 8; ++u)
@@ -521,11 +541,10 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* tmA, const CUtensor
           fence_proxy_async();
           __syncwarp();
           if (lane == 0) {
-            if (m_blk * kBlockM + quarter * 32 < p.M)
+            if (m_blk * kBlockM + quarter * 32 < p.M && n_blk * OUT_N + c * 64 < p.N)
               tma_store_2d(tmC, smem_u32(piece), n_blk * OUT_N + c * 64, m_blk * kBlockM + quarter * 32);
             tma_store_commit();
           }
-          ++staged;
         }
         tc_fence_before();
         __syncwarp();
@@ -663,29 +682,27 @@ inline void fill_tiles(GemmParams& p, int block_n) {
   p.sk_ws = nullptr; p.sk_flags = nullptr;
 }
 
-// How many ways the tiles of the last, partly filled wave are cut along K (1 = not cut) on `grid` CTAs.
-inline int tail_split(int num_tiles, int k_blocks, int grid) {
-  if (grid <= 0 || num_tiles <= grid) return 1;        // a single wave: nothing to balance against
-  const int rem = num_tiles % grid;
-  if (rem == 0) return 1;
-  // Measured on B200: the cut pays off only when a tile's K loop is long (the tail wave of a short-K GEMM is bound
-  // by L2 bandwidth, not by the tensor core, and already runs faster with fewer CTAs) and with few parts per tile.
-  if (k_blocks < 64) return 1;
-  int s = grid / rem;
-  if (s > 4) s = 4;
-  return s < 1 ? 1 : s;
+// How many ways the tiles of the last, partly filled wave of `slots` tiles (the only one, perhaps) are cut along K (1 = not cut).  Only long K
+// loops: the parts' sums go through L2, which costs as much as five K blocks and a start.  Measured on CTA pairs (us, not cut / cut in 4 from 64 K blocks
+// on / from 32 on): 300 x 2048 x 11264 57 / 31 / 31, 512 x 4096 x 14336 82 / 55 / 55, 1337 x 4096 x 4096 67 / 50 / 50, 2000 x 2560 x 2048 29 / 29 / 33,
+// 2000 x 5632 x 2048 42 / 42 / 45; in 8: 140 x 2048 x 5632 34 / 23 / 31.
+inline int tail_split(int num_tiles, int k_blocks, int slots) {
+  const int rem = slots > 0 ? num_tiles % slots : 0;
+  if (rem == 0 || k_blocks < 64) return 1;
+  int s = slots / rem;
+  return s < 1 ? 1 : s > 4 ? 4 : s;
+}
+// Time of `num_tiles` tiles in waves of `slots`; parts of a cut tile cost about five K blocks more (their sums go through L2).
+inline double waves(int num_tiles, int k_blocks, int slots, bool split_on) {
+  const int s = split_on ? tail_split(num_tiles, k_blocks, slots) : 1;
+  const int rem = num_tiles % slots;
+  return double(num_tiles / slots) + (rem == 0 ? 0.0 : s > 1 ? 1.0 / s + 5.0 / k_blocks : 1.0);
 }
 
 // Time of a GEMM in units of one full 128 x 256 tile wave, used to pick the tile width.
-inline double wave_cost(int M, int N, int K, int sms, int bn) {
+inline double wave_cost(int M, int N, int K, int sms, int bn, bool split_on = true) {
   const int tiles = ((M + kBlockM - 1) / kBlockM) * ((N + bn - 1) / bn);
-  const int grid = tiles < sms ? tiles : sms;
-  const int kb = (K + kBlockK - 1) / kBlockK;
-  const int s = tail_split(tiles, kb, grid);
-  double waves;
-  if (s > 1) waves = double(tiles / grid) + 1.0 / s + 0.06;   // + the workspace round trip of the cut tiles
-  else       waves = double((tiles + grid - 1) / grid);
-  return waves * (bn == 256 ? 1.0 : 0.5 / 0.84);   // measured: the 128-wide tile runs at ~0.84 of the 256-wide one
+  return waves(tiles, (K + kBlockK - 1) / kBlockK, sms, split_on) * (bn == 256 ? 1.0 : 0.5 / 0.84);   // measured: the 128-wide tile runs at ~0.84 of the 256-wide one
 }
 
 inline int pick_block_n_split(int M, int N, int K, int sms) {

@@ -9,6 +9,10 @@
 // Roles per CTA (192 threads): warp 0 TMA producer (both CTAs; the bytes of both are counted on the even CTA's
 // full barrier), warp 1 TMEM allocation in both CTAs and MMA issue in the even CTA only, warps 2-5 epilogue of the
 // CTA's own 128 rows (they release the accumulator buffer on the even CTA's barrier).
+// With a staged epilogue (bf16 results with at most a residual added, or gates) there are eight epilogue warps (warps 2-9): pieces of 32 rows x 64
+// columns go through shared memory and leave by TMA.  Row-wise stores of a lane cost 4 to 6 us at the end of a kernel, where no main loop hides them.
+// Measured (us, stores by lanes / staged): 4096 x 2560 x 2048 49 / 44, 4096 x 2048 x 2048 with residual 45 / 34, 8192 x 2048 x 2048 69 / 58, 2000 x 2048 x 2048
+// 27 / 22, 1337 x 6144 x 4096 69 / 62, 11264 x 2048 x 2000 (into a gradient) 105 / 78.
 // The reference reaches its GEMMs through cuBLAS (src/backend/gpu_native/math/gemm.cu:3-189).
 #pragma once
 #include "gemm_sm100.cuh"
@@ -23,6 +27,15 @@ constexpr int kPairSmemBytes = kPairStages * kPairStageBytes + 1024 + 512;
 // Scatter epilogue (GEMM -> reduce-scatter): 8 KB of staging per epilogue warp behind the pipeline stages.
 constexpr int kPairScatterStage = 32 * 128 * 2;          // 32 rows x 128 bf16 columns = two 128-byte-swizzled boxes
 constexpr int kPairScatterSmemBytes = kPairStages * kPairStageBytes + 1024 + 4 * kPairScatterStage + 1024;   // stages, barriers, staging, alignment slack
+
+// Staged epilogues: eight epilogue warps, a piece of 32 rows x 64 bf16 columns for each behind the barriers.
+constexpr int kPairOffStaging = kPairStages * kPairStageBytes + 1024;
+constexpr int kPairStagedSmemBytes = kPairOffStaging + 8 * 4096 + 1024;
+// Where a staged epilogue's results go: C (box 64 columns x 32 rows, 128-byte swizzle), and gate and up of kEpiGluKeep, each a map that ends with
+// its own columns.
+struct PairOutMaps {
+  CUtensorMap c, gate, up;
+};
 
 // One tensor map per destination rank over its staging buffer [world * rows_per_rank, N] bf16, box 64 columns x 32
 // rows, 128-byte swizzle: tiles travel to the owner as TMA stores (whole 128-byte lines over NVLink) instead of
@@ -42,36 +55,26 @@ inline void fill_pair_tiles(GemmParams& p) {
   p.group_m = 8;
 }
 
-// Parts per tile of the last, partly filled wave of pair tiles (1 = not cut).
-inline int pair_tail_split(int num_tiles, int k_blocks, int pairs) {
-  if (pairs <= 0 || num_tiles <= pairs) return 1;
-  const int rem = num_tiles % pairs;
-  if (rem == 0) return 1;
-  // Measured: handing partial sums over through L2 costs about as much as a 32-block K loop, so only long-K GEMMs
-  // (weight gradients, the down projection and its input gradient) come out ahead.
-  if (k_blocks < 64) return 1;
-  int s = pairs / rem;
-  if (s > 4) s = 4;
-  return s < 1 ? 1 : s;
-}
-
 // Time of the GEMM on CTA pairs in the unit of wave_cost (one wave of 128 x 256 tiles on every SM).
 inline double pair_cost(int M, int N, int K, int sms, bool split_on) {
   const int tiles = ((M + kPairBlockM - 1) / kPairBlockM) * ((N + kPairBlockN - 1) / kPairBlockN);
-  const int pairs = sms / 2 < tiles ? sms / 2 : tiles;
-  const int s = split_on ? pair_tail_split(tiles, (K + kBlockK - 1) / kBlockK, pairs) : 1;
-  const double waves = s > 1 ? double(tiles / pairs) + 1.0 / s + 0.06 : double((tiles + pairs - 1) / pairs);
-  return waves * 0.88;   // a pair wave does the work of one single-CTA wave, measured 10-14 % faster (operand sharing)
+  const int kb = (K + kBlockK - 1) / kBlockK;
+  // a pair wave does the work of one single-CTA wave, measured 10-14 % faster (operand sharing); start and end of a pair cost about five K blocks more
+  return waves(tiles, kb, sms / 2, split_on) * 0.88 + 5.0 / kb;
 }
 
 // p.m_blocks / p.n_blocks / p.num_tiles count 256 x 256 tiles; everything else as in gemm_body.
 // `gate(m_chunk, n_blk, kb, status)` and `done(m_chunk, n_blk)` are the hooks of gemm_body; m_chunk counts 128-row
 // blocks (the rows one CTA of the pair loads and writes), n_blk counts 256-column blocks.  CTAs [0, cta_first) of
 // the grid (an even number) belong to another role of a fused kernel.
-template <int A_MAJOR, int B_MAJOR, int MMA_KIND = 0, class TileGate, class TileDone>   // MMA_KIND: see gemm_body
+// EPI: with kEpiGlu and kEpiGluKeep a tile is 128 result columns; the even CTA stages their gate rows of B, the odd CTA their up rows.
+template <int A_MAJOR, int B_MAJOR, int MMA_KIND = 0, int EPI = kEpiDirect, class TileGate, class TileDone>   // MMA_KIND: see gemm_body
 __device__ __forceinline__ void gemm_body_pair(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p,
                                                TileGate gate, TileDone done, int cta_first = 0,
-                                               const ScatterMaps* scatter = nullptr) {
+                                               const ScatterMaps* scatter = nullptr, const PairOutMaps* outs = nullptr) {
+  constexpr bool GLU = EPI == kEpiGlu || EPI == kEpiGluKeep;
+  constexpr int EW = EPI == kEpiDirect ? 4 : 8;   // epilogue warps per CTA
+  static_assert(!GLU || B_MAJOR == 0, "gates go with K-major weights");
   constexpr int S = kPairStages;
   constexpr int kABytes = kBlockM * kBlockK * 2;
   extern __shared__ uint8_t smem_raw[];
@@ -100,7 +103,7 @@ __device__ __forceinline__ void gemm_body_pair(const CUtensorMap* tmA, const CUt
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(tfull_bar(b), 1);
-      mbar_init(tempty_bar(b), 8);
+      mbar_init(tempty_bar(b), 2 * EW);
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -130,7 +133,7 @@ __device__ __forceinline__ void gemm_body_pair(const CUtensorMap* tmA, const CUt
         int m_blk, n_blk;
         tile_coords(p, w.tile, m_blk, n_blk);
         const int m0 = m_blk * kPairBlockM + int(cta_rank) * kBlockM;
-        const int n0 = n_blk * kPairBlockN + int(cta_rank) * (kPairBlockN / 2);
+        const int n0 = GLU ? n_blk * (kPairBlockN / 2) + int(cta_rank) * p.N : n_blk * kPairBlockN + int(cta_rank) * (kPairBlockN / 2);
         for (int kl = w.kb0; kl < w.kb1; ++kl) {
           int kb = kl + p.k_rot;
           if (kb >= p.k_blocks) kb -= p.k_blocks;
@@ -198,6 +201,9 @@ __device__ __forceinline__ void gemm_body_pair(const CUtensorMap* tmA, const CUt
   } else {
     // ------------------------------------------------------------------ epilogue (4 warps per CTA, own 128 rows)
     const int quarter = warp & 3;
+    // columns of a tile this warp takes, in chunks of 32
+    constexpr int kChunks = kPairBlockN / 32;
+    const int half = EW == 8 ? (warp - 2) >> 2 : 0, c_first = half * (kChunks / 2), c_last = EW == 8 ? c_first + kChunks / 2 : kChunks;
     int pend_m = -1, pend_n = 0;   // scatter epilogue: tile whose completion signal is still owed
     WorkItem w;
     for (int it = 0; get_item(p, pair_id, pair_count, it, w); ++it) {
@@ -205,10 +211,21 @@ __device__ __forceinline__ void gemm_body_pair(const CUtensorMap* tmA, const CUt
       tile_coords(p, w.tile, m_blk, n_blk);
       const int buf = it & 1;
       const uint32_t aphase = (it >> 1) & 1;
+      const int row = m_blk * kPairBlockM + int(cta_rank) * kBlockM + quarter * 32 + lane;
+      // kEpiStaged: the residual's next 64 columns of this row are on their way while the tile is made, then while the columns before them leave
+      [[maybe_unused]] uint4 ahead[8];
+      [[maybe_unused]] auto fetch = [&](int c) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int col = n_blk * kPairBlockN + c * 32 + u * 8;
+          ahead[u] = make_uint4(0u, 0u, 0u, 0u);
+          if (p.residual && row < p.M && col < p.N) ahead[u] = *reinterpret_cast<const uint4*>(p.residual + (long long)row * p.ldr + col);
+        }
+      };
+      if constexpr (EPI == kEpiStaged) fetch(c_first);
       const bool got = mbar_wait(tfull_bar(buf), aphase, abort_flag, p.status, kStatusTimeoutTmemFull);
       if (!__all_sync(0xffffffffu, got)) break;
       tc_fence_after();
-      const int row = m_blk * kPairBlockM + int(cta_rank) * kBlockM + quarter * 32 + lane;
       const uint32_t t_addr = tmem_base + (uint32_t(quarter * 32) << 16) + buf * kPairBlockN;
       if (scatter != nullptr) {
         // GEMM -> reduce-scatter: this warp's 32 rows x 256 columns go to the rank that owns the rows as four TMA
@@ -274,17 +291,16 @@ __device__ __forceinline__ void gemm_body_pair(const CUtensorMap* tmA, const CUt
         continue;
       }
       // Split tail (see GemmParams): per split tile the workspace holds, for each other part, the two CTAs'
-      // 128 x 256 fp32 accumulators as [chunk of 32 columns][group of 4 columns][row][4]; one flag per (tile, CTA, lane quarter).
-      constexpr int kChunks = kPairBlockN / 32;
+      // 128 x 256 fp32 accumulators as [chunk of 32 columns][group of 4 columns][row][4]; one flag per (tile, CTA, epilogue warp).
       auto part_base = [&](int part) {
         return p.sk_ws + ((long long)((w.slot * (p.sk_split - 1) + part) * 2 + int(cta_rank)) * kChunks) * (kBlockM * 32) +
                (quarter * 32 + lane) * 4;
       };
-      unsigned* flag = p.sk_flags + (w.slot * 2 + int(cta_rank)) * 4 + quarter;
+      unsigned* flag = p.sk_flags + (w.slot * 2 + int(cta_rank)) * EW + (EW == 8 ? warp - 2 : quarter);
       if (w.split > 0) {
         float* ws = part_base(w.split - 1);
 #pragma unroll 1
-        for (int c = 0; c < kChunks; ++c) {
+        for (int c = c_first; c < c_last; ++c) {
           uint32_t r[32];
           tmem_ld_32x32(t_addr + c * 32, r);
           tmem_ld_wait();
@@ -326,7 +342,7 @@ __device__ __forceinline__ void gemm_body_pair(const CUtensorMap* tmA, const CUt
           }
         }
       };
-      if (w.split == 0) load_parts(0);
+      if (w.split == 0) load_parts(c_first);
       auto add_parts = [&](uint32_t (&r)[32]) {
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
@@ -336,6 +352,82 @@ __device__ __forceinline__ void gemm_body_pair(const CUtensorMap* tmA, const CUt
           r[q * 4 + 3] = __float_as_uint(__uint_as_float(r[q * 4 + 3]) + pre[q].w);
         }
       };
+      if constexpr (EPI != kEpiDirect) {
+        // 64 columns of this lane's row at a time, as bf16 pairs
+        const int row0 = m_blk * kPairBlockM + int(cta_rank) * kBlockM + quarter * 32;
+        auto emit = [&](const CUtensorMap* tm, const uint32_t (&v)[32], int col) {
+          uint8_t* piece = smem + kPairOffStaging + (warp - 2) * 4096;
+          if (lane == 0) tma_store_wait_read<0>();   // the store before has read the piece
+          __syncwarp();
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            *reinterpret_cast<uint4*>(piece + lane * 128 + ((u ^ (lane & 7)) << 4)) = make_uint4(v[u * 4], v[u * 4 + 1], v[u * 4 + 2], v[u * 4 + 3]);
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) {
+            if (row0 < p.M && col < p.N) tma_store_2d(tm, smem_u32(piece), col, row0);
+            tma_store_commit();
+          }
+        };
+        if constexpr (GLU) {
+#pragma unroll 1
+          for (int c = half; c < kPairBlockN / 128; c += EW / 4) {
+            uint32_t h[32], wg[32], wu[32];
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+              uint32_t r[32], u[32];
+              tmem_ld_32x32(t_addr + c * 64 + hh * 32, r);
+              tmem_ld_32x32(t_addr + kPairBlockN / 2 + c * 64 + hh * 32, u);
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const float g0 = __uint_as_float(r[2 * j]) * p.alpha, g1 = __uint_as_float(r[2 * j + 1]) * p.alpha;
+                const float u0 = __uint_as_float(u[2 * j]) * p.alpha, u1 = __uint_as_float(u[2 * j + 1]) * p.alpha;
+                if constexpr (EPI == kEpiGluKeep) {
+                  wg[hh * 16 + j] = pack_bf16x2(g0, g1);
+                  wu[hh * 16 + j] = pack_bf16x2(u0, u1);
+                }
+                h[hh * 16 + j] = p.glu_act == 1 ? pack_bf16x2(gelu_tanh_f(g0) * u0, gelu_tanh_f(g1) * u1)
+                                                : pack_bf16x2(silu_quick_f(g0) * u0, silu_quick_f(g1) * u1);
+              }
+            }
+            const int col = n_blk * (kPairBlockN / 2) + c * 64;
+            if constexpr (EPI == kEpiGluKeep) {
+              emit(&outs->gate, wg, col);
+              emit(&outs->up, wu, col);
+            }
+            emit(&outs->c, h, col);
+          }
+        } else {
+#pragma unroll 1
+          for (int c = c_first; c < c_last; c += 2) {
+            const int col = n_blk * kPairBlockN + c * 32;
+            uint32_t out[32];
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+              uint32_t r[32];
+              tmem_ld_32x32(t_addr + (c + hh) * 32, r);
+              tmem_ld_wait();
+              if (w.split == 0) {
+                add_parts(r);
+                if (c + hh + 1 < c_last) load_parts(c + hh + 1);
+              }
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const uint4& q = ahead[hh * 4 + j / 4];
+                const float2 f = unpack_bf16x2(j % 4 == 0 ? q.x : j % 4 == 1 ? q.y : j % 4 == 2 ? q.z : q.w);
+                out[hh * 16 + j] = pack_bf16x2(__uint_as_float(r[2 * j]) * p.alpha + f.x, __uint_as_float(r[2 * j + 1]) * p.alpha + f.y);
+              }
+            }
+            if (c + 2 < c_last) fetch(c + 2);
+            emit(&outs->c, out, col);
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(tempty_bar(buf), 0);
+        continue;
+      }
       // two 32-column chunks per step: both tensor-memory loads are in flight before the first is consumed
 #pragma unroll 1
       for (int c = 0; c < kChunks; c += 2) {
@@ -360,6 +452,9 @@ __device__ __forceinline__ void gemm_body_pair(const CUtensorMap* tmA, const CUt
         mbar_arrive_cluster(tempty_bar(buf), 0);
         done(m_blk * (kPairBlockM / kBlockM) + int(cta_rank), n_blk);
       }
+    }
+    if constexpr (EPI != kEpiDirect) {
+      if (lane == 0) tma_store_wait<0>();
     }
     if (scatter != nullptr && lane == 0 && pend_m >= 0) {
       tma_store_wait<0>();

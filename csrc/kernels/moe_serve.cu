@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256) moe_place_kernel(const int2* __restrict__
 
 // C[slots, N] = A[slots, K] @ W[expert of the slot's 128-row block]^T, gated or not; only the blocks in use are computed.
 template <int BLOCK_N, int EPI>
-__global__ void __launch_bounds__(kGemmThreads, 1)
+__global__ void __launch_bounds__(kStagedThreads, 1)
 moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                         const __grid_constant__ CUtensorMap tmC, const GemmParams p, const int* __restrict__ live) {
   __shared__ GemmParams q;
@@ -206,7 +206,7 @@ static int launch_grouped(const CUtensorMap& tmA, const CUtensorMap& tmB, const 
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<BLOCK_N>::kStagedSmemBytes));
     configured.finish();
   }
-  kern<<<grid, kGemmThreads, GemmCfg<BLOCK_N>::kStagedSmemBytes, st>>>(tmA, tmB, tmC, p, live);
+  kern<<<grid, kStagedThreads, GemmCfg<BLOCK_N>::kStagedSmemBytes, st>>>(tmA, tmB, tmC, p, live);
   LT_LAUNCH_CHECK();
   return 0;
 }

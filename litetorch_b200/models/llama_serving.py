@@ -62,10 +62,7 @@ class LlamaKVModel(ServingModel):
             o = attend(i, q, k, v)
             x1 = K.product_of_constants(o.reshape(n, Hq * hd), w.p(p + "wo"), residual=x)
             h2, _, _, _ = K.norm_fwd(x1, w.p(p + "mlp_norm"), eps=cfg.rms_eps)
-            # Gates in the product's epilogue, except in prompts of up to 1024 rows, whose tiles are too few to hide it (us, epilogue / separate
-            # pass; widths x feed-forwards of 1024 x 2816 to 5120 x 13824 alike): 2048 x 5632 33.8 / 31.6 with 129 rows, 45.9 / 45.8 with 512, 58 /
-            # 60 with 1024, 70 / 75 with 1337, 143 / 167 with 4096; 4096 x 14336 102 / 97, 163 / 165, 249 / 271, 312 / 369, 660 / 753
-            hm = K.product_of_constants(h2, w.p(p + "w_gu"), act="silu") if n <= 128 or n > 1024 else K.swiglu_fwd(K.gemm(h2, w.p(p + "w_gu")))
+            hm = K.product_of_constants(h2, w.p(p + "w_gu"), act="silu")
             x = K.product_of_constants(hm, w.p(p + "w_down"), residual=x1)
         return x
 

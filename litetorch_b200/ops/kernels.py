@@ -863,9 +863,6 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype=None, alpha: float = 1.0)
     if M == 0:
         return torch.empty((0, N), dtype=out_dtype, device=x.device)
     if x.dtype == torch.bfloat16 and Kd % 8 == 0 and (M == 1 or x.stride(0) % 8 == 0) and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0:
-        if M > 128 and Kd <= 2048 and N >= 512 and N % 8 == 0 and out_dtype == torch.bfloat16:
-            # a short K loop is bound by how its results leave; a narrow tile where wide ones would not fill the GPU
-            return gemm_staged(x, w, alpha=alpha, block_n=256 if (M + 127) // 128 * ((N + 255) // 256) >= 100 else 128)
         return gemm(x, w, out_dtype=out_dtype, alpha=alpha)
     y = torch.empty((M, N), dtype=out_dtype, device=x.device)
     rc = _fn("lt_gemm_simt")(_f32(x), _f32(y), x.data_ptr(), w.data_ptr(), y.data_ptr(), M, N, Kd, x.stride(0), Kd, N, 1, 0, 0, 0,
