@@ -51,6 +51,9 @@ struct FlashBwdParams {
   // Optional phase timing (nullptr: off): the CTA of key block 0 / head 0 / batch 0 adds the SM cycles its compute
   // warp 2 and its MMA thread spend in each phase to trace[0..15] and counts iterations in trace[15].
   long long* trace;
+  // Tables of cosines and sines [., D / 2] by position: dK is turned back by the angles of its rows (nullptr: it is not).
+  const float* cos_t;
+  const float* sin_t;
 };
 
 struct QMaps {
@@ -93,9 +96,22 @@ struct FaBwdCfg {
   static constexpr bool kDqOverDp = (D != 64);
 };
 
-// delta[b,h,t] = sum_d O * dO ; D/8 threads per (b,t,h) row, 16 bytes each.
+// Four pairs (x, y) of neighbouring columns turned by the negative angles: (x c + y s, y c - x s).
+__device__ __forceinline__ void turn_back(float (&v)[8], const float* cos_row, const float* sin_row) {
+  const float4 c = *reinterpret_cast<const float4*>(cos_row), s = *reinterpret_cast<const float4*>(sin_row);
+  const float cc[4] = {c.x, c.y, c.z, c.w}, ss[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float x = v[2 * j], y = v[2 * j + 1];
+    v[2 * j] = x * cc[j] + y * ss[j];
+    v[2 * j + 1] = y * cc[j] - x * ss[j];
+  }
+}
+
+// delta[b,h,t] = sum_d O * dO ; D/8 threads per (b,t,h) row, 16 bytes each.  They also zero their columns of the dQ accumulator [B, Tq, Hq, D] (nullptr: the
+// caller has).
 __global__ void flash_bwd_delta_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __restrict__ dO,
-                                       float* __restrict__ delta, int B, int Tq, int Hq, int D, long long so_b,
+                                       float* __restrict__ delta, float* __restrict__ dq_acc, int B, int Tq, int Hq, int D, long long so_b,
                                        long long so_t, long long sdo_b, long long sdo_t) {
   pdl_launch_dependents();
   pdl_wait();
@@ -107,9 +123,14 @@ __global__ void flash_bwd_delta_kernel(const __nv_bfloat16* __restrict__ O, cons
   float s = 0.f;
   int h = 0, t = 0, b = 0;
   if (row < total) {
-    h = int(row % Hq);
-    t = int((row / Hq) % Tq);
-    b = int(row / ((long long)Hq * Tq));
+    const long long bt = row / Hq;
+    h = int(row - bt * Hq);
+    b = int(bt / Tq);
+    t = int(bt - (long long)b * Tq);
+    if (dq_acc) {
+      float4* z = reinterpret_cast<float4*>(dq_acc + row * D + sub * 8);
+      z[0] = z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     const uint4 a = *reinterpret_cast<const uint4*>(O + b * so_b + t * so_t + (long long)h * D + sub * 8);
     const uint4 g = *reinterpret_cast<const uint4*>(dO + b * sdo_b + t * sdo_t + (long long)h * D + sub * 8);
     const uint32_t av[4] = {a.x, a.y, a.z, a.w}, gv[4] = {g.x, g.y, g.z, g.w};
@@ -123,22 +144,33 @@ __global__ void flash_bwd_delta_kernel(const __nv_bfloat16* __restrict__ O, cons
   if (row < total && sub == 0) delta[((long long)b * Hq + h) * Tq + t] = s;
 }
 
-__global__ void flash_bwd_convert_dq_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, int B, int Tq,
-                                            int HD, long long sdq_b, long long sdq_t) {
+// dQ leaves its accumulator as bf16, eight columns a thread; with tables [., D / 2] of cosines and sines (nullptr: as it is) turned back by the angles of
+// its row's position t, pairs of neighbouring columns together.
+__global__ void __launch_bounds__(256) flash_bwd_convert_dq_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, long long rows, int Tq,
+                                                                   int HD, int D, long long sdq_b, long long sdq_t, const float* __restrict__ cos_t,
+                                                                   const float* __restrict__ sin_t) {
   pdl_launch_dependents();
   pdl_wait();
-  const long long n4 = (long long)B * Tq * HD / 4;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
-    const long long e = i * 4;
-    const int c = int(e % HD);
-    const long long bt = e / HD;
-    const int t = int(bt % Tq);
-    const int b = int(bt / Tq);
-    const float4 v = *reinterpret_cast<const float4*>(acc + e);
-    uint2 o;
-    o.x = pack_bf16x2(v.x, v.y);
-    o.y = pack_bf16x2(v.z, v.w);
-    *reinterpret_cast<uint2*>(dq + b * sdq_b + t * sdq_t + c) = o;
+  const int per_row = HD / 8;                          // threads of a block go through whole rows
+  const int rows_at_once = max(1, 256 / per_row);
+  const int r_in = threadIdx.x / per_row;
+  if (r_in >= rows_at_once) return;
+  for (long long r = (long long)blockIdx.x * rows_at_once + r_in; r < rows; r += (long long)gridDim.x * rows_at_once) {
+    const long long b = r / Tq;
+    const int t = int(r - b * Tq);
+    for (int c = (threadIdx.x - r_in * per_row) * 8; c < HD; c += rows_at_once > 1 ? HD : 256 * 8) {
+      const float4 lo = *reinterpret_cast<const float4*>(acc + r * HD + c), hi = *reinterpret_cast<const float4*>(acc + r * HD + c + 4);
+      float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+      if (cos_t) turn_back(v, cos_t + (long long)t * (D / 2) + (c % D) / 2, sin_t + (long long)t * (D / 2) + (c % D) / 2);
+      const uint4 o = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+      __nv_bfloat16* to = dq + b * sdq_b + t * sdq_t + c;
+      if (reinterpret_cast<uintptr_t>(to) & 15) {      // rows of dQ need 8-byte alignment only
+        reinterpret_cast<uint2*>(to)[0] = make_uint2(o.x, o.y);
+        reinterpret_cast<uint2*>(to)[1] = make_uint2(o.z, o.w);
+      } else {
+        *reinterpret_cast<uint4*>(to) = o;
+      }
+    }
   }
 }
 
@@ -614,10 +646,17 @@ flash_bwd_kernel(const __grid_constant__ QMaps qm, const __grid_constant__ CUten
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             uint4 w, z;
-            w.x = pack_bf16x2(__uint_as_float(a[u * 8 + 0]), __uint_as_float(a[u * 8 + 1]));
-            w.y = pack_bf16x2(__uint_as_float(a[u * 8 + 2]), __uint_as_float(a[u * 8 + 3]));
-            w.z = pack_bf16x2(__uint_as_float(a[u * 8 + 4]), __uint_as_float(a[u * 8 + 5]));
-            w.w = pack_bf16x2(__uint_as_float(a[u * 8 + 6]), __uint_as_float(a[u * 8 + 7]));
+            float k8[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) k8[i] = __uint_as_float(a[u * 8 + i]);
+            if (p.cos_t) {
+              const long long at = (long long)kv_idx * (D / 2) + (c * 32 + u * 8) / 2;
+              turn_back(k8, p.cos_t + at, p.sin_t + at);
+            }
+            w.x = pack_bf16x2(k8[0], k8[1]);
+            w.y = pack_bf16x2(k8[2], k8[3]);
+            w.z = pack_bf16x2(k8[4], k8[5]);
+            w.w = pack_bf16x2(k8[6], k8[7]);
             z.x = pack_bf16x2(__uint_as_float(g[u * 8 + 0]), __uint_as_float(g[u * 8 + 1]));
             z.y = pack_bf16x2(__uint_as_float(g[u * 8 + 2]), __uint_as_float(g[u * 8 + 3]));
             z.z = pack_bf16x2(__uint_as_float(g[u * 8 + 4]), __uint_as_float(g[u * 8 + 5]));
@@ -658,26 +697,26 @@ static int launch_flash_bwd(const QMaps& qm, const CUtensorMap& tk, const CUtens
   return 0;
 }
 
-static int bwd_delta(const void* o, const void* d_o, float* delta, int B, int Tq, int Hq, int D, long long so_b, long long so_t,
+static int bwd_delta(const void* o, const void* d_o, float* delta, float* dq_acc, int B, int Tq, int Hq, int D, long long so_b, long long so_t,
                      long long sdo_b, long long sdo_t, cudaStream_t st) {
   const long long rows = (long long)B * Tq * Hq;
   const int threads = 256;
   const long long blocks = (rows * (D / 8) + threads - 1) / threads;
   LT_RETURN_IF_CUDA(launch_chained(flash_bwd_delta_kernel, (unsigned)blocks, threads, 0, st, static_cast<const __nv_bfloat16*>(o),
-                                                               static_cast<const __nv_bfloat16*>(d_o), delta, B, Tq, Hq, D, so_b,
+                                                               static_cast<const __nv_bfloat16*>(d_o), delta, dq_acc, B, Tq, Hq, D, so_b,
                                                                so_t, sdo_b, sdo_t));
   LT_LAUNCH_CHECK();
   return 0;
 }
 
 static int bwd_convert(const float* dq_acc, void* dq, int B, int Tq, int Hq, int D, long long sdq_b, long long sdq_t,
-                       cudaStream_t st) {
-  const long long n4 = (long long)B * Tq * Hq * D / 4;
-  long long blocks = (n4 + 255) / 256;
+                       cudaStream_t st, const float* cos_t = nullptr, const float* sin_t = nullptr) {
+  const long long rows = (long long)B * Tq, at_once = 256 / (Hq * D / 8) > 1 ? 256 / (Hq * D / 8) : 1;
+  long long blocks = (rows + at_once - 1) / at_once;
   const long long cap = (long long)sm_count() * 16;
   if (blocks > cap) blocks = cap;
-  LT_RETURN_IF_CUDA(launch_chained(flash_bwd_convert_dq_kernel, (unsigned)blocks, 256, 0, st, dq_acc, static_cast<__nv_bfloat16*>(dq), B, Tq, Hq * D, sdq_b, sdq_t));
-  LT_LAUNCH_CHECK();
+  LT_RETURN_IF_CUDA(launch_chained(flash_bwd_convert_dq_kernel, (unsigned)blocks, 256, 0, st, dq_acc, static_cast<__nv_bfloat16*>(dq), rows, Tq, Hq * D, D, sdq_b,
+                                   sdq_t, cos_t, sin_t));
   return 0;
 }
 
@@ -688,7 +727,8 @@ static int bwd_main(const void* const* q_ptrs, const void* k, const void* v, con
                     const float* const* lse_ptrs, const float* const* delta_ptrs, float* const* dq_acc_ptrs, void* dk, void* dv,
                     int B, int Tq, int Tk, int Hq, int Hkv, int D, long long sq_b, long long sq_t, long long sk_b, long long sk_t,
                     long long sv_b, long long sv_t, long long sdo_b, long long sdo_t, long long sdk_b, long long sdk_t,
-                    float scale, int causal, int cp_world, int cp_rank, int zigzag, cudaStream_t st) {
+                    float scale, int causal, int cp_world, int cp_rank, int zigzag, cudaStream_t st, const float* cos_t = nullptr,
+                    const float* sin_t = nullptr) {
   if (cp_world < 1 || cp_world > kFbMaxRanks) return -int(kStatusBadArgument);
   if (cp_world > 1 && zigzag && ((Tq / 2) % kFbBlock != 0 || (Tk / 2) % kFbBlock != 0)) return -int(kStatusBadArgument);
   if (cp_world > 1 && !zigzag && (Tq % kFbBlock != 0 || Tk % kFbBlock != 0)) return -int(kStatusBadArgument);
@@ -723,6 +763,7 @@ static int bwd_main(const void* const* q_ptrs, const void* k, const void* v, con
   p.causal = causal;
   p.status = device_status_word();
   p.trace = g_bwd_trace;
+  p.cos_t = cos_t; p.sin_t = sin_t;
   // fp32 dQ accumulator of this rank, [B, Tq, Hq, D]: boxes of 32 rows x 32 columns (128 bytes, swizzled)
   CUtensorMap tdq;
   r = encode_tmap_4d(&tdq, dq_acc_ptrs[cp_rank], 4, D, Hq, Tq, B, (uint64_t)D * 4, (uint64_t)Hq * D * 4,
@@ -735,22 +776,25 @@ static int bwd_main(const void* const* q_ptrs, const void* k, const void* v, con
 
 extern "C" {
 
-// Shapes as lt_flash_fwd.  delta: scratch [B, Hq, Tq] fp32.  dq_acc: scratch [B, Tq, Hq, D] fp32, must be zero.
-// dk and dv share the strides sdk_b / sdk_t.
 // Debug aid: a device buffer of 16 int64 that the next backward launches fill with per-phase SM cycle counts of one
 // CTA (see FlashBwdParams::trace); nullptr switches it off.
 void lt_flash_bwd_set_trace(void* buf) { lt::g_bwd_trace = static_cast<long long*>(buf); }
 
-int lt_flash_bwd(const void* q, const void* k, const void* v, const void* o, const float* lse, const void* d_o, void* dq,
-                 void* dk, void* dv, float* delta, float* dq_acc, int B, int Tq, int Tk, int Hq, int Hkv, int D,
-                 long long sq_b, long long sq_t, long long sk_b, long long sk_t, long long sv_b, long long sv_t,
-                 long long so_b, long long so_t, long long sdo_b, long long sdo_t, long long sdq_b, long long sdq_t,
-                 long long sdk_b, long long sdk_t, float scale, int causal, void* stream) {
+// Shapes as lt_flash_fwd.  delta: scratch [B, Hq, Tq] fp32.  dq_acc: scratch [B, Tq, Hq, D] fp32.
+// dk and dv share the strides sdk_b / sdk_t.  cos_t, sin_t (fp32 [>= Tq, D / 2], 16-byte aligned, Tq = Tk; or both nullptr): q and k are pairs of neighbouring
+// columns turned by the angles of their rows 0, 1, ..; dq and dk are turned back by these.
+int lt_flash_bwd_rope(const void* q, const void* k, const void* v, const void* o, const float* lse, const void* d_o, void* dq,
+                      void* dk, void* dv, float* delta, float* dq_acc, int B, int Tq, int Tk, int Hq, int Hkv, int D,
+                      long long sq_b, long long sq_t, long long sk_b, long long sk_t, long long sv_b, long long sv_t,
+                      long long so_b, long long so_t, long long sdo_b, long long sdo_t, long long sdq_b, long long sdq_t,
+                      long long sdk_b, long long sdk_t, float scale, int causal, const float* cos_t, const float* sin_t, void* stream) {
   using namespace lt;
-  if ((D != 64 && D != 128) || Hq % Hkv != 0) return -int(kStatusBadArgument);
+  if ((D != 64 && D != 128) || Hq % Hkv != 0 || !cos_t != !sin_t || (cos_t && Tq != Tk) ||
+      ((reinterpret_cast<uintptr_t>(cos_t) | reinterpret_cast<uintptr_t>(sin_t)) & 15))
+    return -int(kStatusBadArgument);
   if (B == 0 || Tq == 0 || Tk == 0) return 0;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  int rc = bwd_delta(o, d_o, delta, B, Tq, Hq, D, so_b, so_t, sdo_b, sdo_t, st);
+  int rc = bwd_delta(o, d_o, delta, dq_acc, B, Tq, Hq, D, so_b, so_t, sdo_b, sdo_t, st);
   if (rc) return rc;
   const void* qs[1] = {q};
   const void* dos[1] = {d_o};
@@ -758,9 +802,19 @@ int lt_flash_bwd(const void* q, const void* k, const void* v, const void* o, con
   const float* deltas[1] = {delta};
   float* accs[1] = {dq_acc};
   rc = bwd_main(qs, k, v, dos, lses, deltas, accs, dk, dv, B, Tq, Tk, Hq, Hkv, D, sq_b, sq_t, sk_b, sk_t, sv_b, sv_t, sdo_b, sdo_t,
-                sdk_b, sdk_t, scale, causal, 1, 0, 0, st);
+                sdk_b, sdk_t, scale, causal, 1, 0, 0, st, cos_t, sin_t);
   if (rc) return rc;
-  return bwd_convert(dq_acc, dq, B, Tq, Hq, D, sdq_b, sdq_t, st);
+  return bwd_convert(dq_acc, dq, B, Tq, Hq, D, sdq_b, sdq_t, st, cos_t, sin_t);
+}
+
+// The same without angles.
+int lt_flash_bwd(const void* q, const void* k, const void* v, const void* o, const float* lse, const void* d_o, void* dq,
+                 void* dk, void* dv, float* delta, float* dq_acc, int B, int Tq, int Tk, int Hq, int Hkv, int D,
+                 long long sq_b, long long sq_t, long long sk_b, long long sk_t, long long sv_b, long long sv_t,
+                 long long so_b, long long so_t, long long sdo_b, long long sdo_t, long long sdq_b, long long sdq_t,
+                 long long sdk_b, long long sdk_t, float scale, int causal, void* stream) {
+  return lt_flash_bwd_rope(q, k, v, o, lse, d_o, dq, dk, dv, delta, dq_acc, B, Tq, Tk, Hq, Hkv, D, sq_b, sq_t, sk_b, sk_t, sv_b, sv_t, so_b, so_t, sdo_b,
+                           sdo_t, sdq_b, sdq_t, sdk_b, sdk_t, scale, causal, nullptr, nullptr, stream);
 }
 
 // Context-parallel backward in three stream-ordered phases; the caller crosses a rank barrier between them.
@@ -778,7 +832,7 @@ int lt_flash_bwd_cp(int phase, const void* const* q_ptrs, const void* k, const v
   if ((D != 64 && D != 128) || Hq % Hkv != 0 || cp_rank < 0 || cp_rank >= cp_world) return -int(kStatusBadArgument);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (phase == 0)
-    return bwd_delta(o, do_ptrs[cp_rank], const_cast<float*>(delta_ptrs[cp_rank]), B, Tq, Hq, D, so_b, so_t, sdo_b, sdo_t, st);
+    return bwd_delta(o, do_ptrs[cp_rank], const_cast<float*>(delta_ptrs[cp_rank]), nullptr, B, Tq, Hq, D, so_b, so_t, sdo_b, sdo_t, st);
   if (phase == 1)
     return bwd_main(q_ptrs, k, v, do_ptrs, lse_ptrs, delta_ptrs, dq_acc_ptrs, dk, dv, B, Tq, Tk, Hq, Hkv, D, sq_b, sq_t, sk_b, sk_t,
                     sv_b, sv_t, sdo_b, sdo_t, sdk_b, sdk_t, scale, causal, cp_world, cp_rank, zigzag, st);

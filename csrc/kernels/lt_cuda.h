@@ -29,6 +29,11 @@ int lt_flash_bwd(const void* q, const void* k, const void* v, const void* o, con
                  int D, long long sq_b, long long sq_t, long long sk_b, long long sk_t, long long sv_b, long long sv_t,
                  long long so_b, long long so_t, long long sdo_b, long long sdo_t, long long sdq_b, long long sdq_t,
                  long long sdk_b, long long sdk_t, float scale, int causal, void* stream);
+int lt_flash_bwd_rope(const void* q, const void* k, const void* v, const void* o, const float* lse, const void* d_o,
+                 void* dq, void* dk, void* dv, float* delta, float* dq_acc, int B, int Tq, int Tk, int Hq, int Hkv,
+                 int D, long long sq_b, long long sq_t, long long sk_b, long long sk_t, long long sv_b, long long sv_t,
+                 long long so_b, long long so_t, long long sdo_b, long long sdo_t, long long sdq_b, long long sdq_t,
+                 long long sdk_b, long long sdk_t, float scale, int causal, const float* cos_t, const float* sin_t, void* stream);
 int lt_flash_bwd_cp(int phase, const void* const* q_ptrs, const void* k, const void* v, const void* o,
                     const void* const* do_ptrs, const float* const* lse_ptrs, const float* const* delta_ptrs,
                     float* const* dq_acc_ptrs, void* dq, void* dk, void* dv, int B, int Tq, int Tk, int Hq, int Hkv,
@@ -109,6 +114,8 @@ int lt_gemm_e4m3(const void* A, const void* B, void* C, int M, int N, int K, lon
                  const void* residual, long long ldr, int act, float alpha, void* stream);
 int lt_gemm_staged(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc, int act,
                    float alpha, int block_n, void* stream);
+int lt_gemm_glu_keep(const void* A, const void* B, void* C, void* GU, int M, int N, int K, long long lda, long long ldb, long long ldc, long long ldg,
+                     int act, void* stream);
 int lt_gemm_block_diag(const void* A, const void* B, float* C, int M, int blocks, int nb, int K, long long lda,
                        long long ldc, void* stream);
 

@@ -32,30 +32,30 @@ __device__ __forceinline__ void st8(__nv_bfloat16* p, const float (&f)[8]) {
 // Row r belongs to position (r % T) + pos_offset... positions are given explicitly when pos != nullptr.
 // Pair convention: (x[2i], x[2i+1]) rotated by angle pos * theta^(-2i/hd)  (interleaved, as the reference).
 // cos/sin tables are [max_pos, hd/2] fp32. sign = +1 forward, -1 backward (inverse rotation).
+// IDX: 32 bits where the count of 8-element pieces fits (64-bit divisions cost more than the bytes: 8192 rows of 32 heads of 64, 20 us).
+template <typename IDX>
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ cos_t,
-                            const float* __restrict__ sin_t, const int* __restrict__ pos, long long rows, int T,
-                            int heads, int hd, long long row_stride, float sign) {
+                            const float* __restrict__ sin_t, const int* __restrict__ pos, IDX rows, IDX T,
+                            IDX heads, IDX hd, long long row_stride, float sign) {
   pdl_launch_dependents();
   pdl_wait();
-  const int vec_per_head = hd / 8;
-  const long long total = rows * heads * vec_per_head;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int v = int(i % vec_per_head);
-    const int h = int((i / vec_per_head) % heads);
-    const long long r = i / ((long long)vec_per_head * heads);
+  const IDX vec_per_head = hd / 8, per_row = heads * vec_per_head;
+  const IDX total = rows * per_row;
+  for (IDX i = IDX(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += IDX(gridDim.x) * blockDim.x) {
+    const IDX r = i / per_row, c = i - r * per_row, v = c % vec_per_head;
     const int t = pos ? pos[r] : int(r % T);
-    __nv_bfloat16* p = x + r * row_stride + (long long)h * hd + v * 8;
+    __nv_bfloat16* p = x + r * row_stride + (long long)c * 8;
     float f[8];
     ld8(p, f);
     const float4 c4 = *reinterpret_cast<const float4*>(cos_t + (long long)t * (hd / 2) + v * 4);
     const float4 s4 = *reinterpret_cast<const float4*>(sin_t + (long long)t * (hd / 2) + v * 4);
-    const float c[4] = {c4.x, c4.y, c4.z, c4.w};
+    const float cs[4] = {c4.x, c4.y, c4.z, c4.w};
     const float s[4] = {s4.x * sign, s4.y * sign, s4.z * sign, s4.w * sign};
     float o[8];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      o[2 * j] = f[2 * j] * c[j] - f[2 * j + 1] * s[j];
-      o[2 * j + 1] = f[2 * j] * s[j] + f[2 * j + 1] * c[j];
+      o[2 * j] = f[2 * j] * cs[j] - f[2 * j + 1] * s[j];
+      o[2 * j + 1] = f[2 * j] * s[j] + f[2 * j + 1] * cs[j];
     }
     st8(p, o);
   }
@@ -353,7 +353,14 @@ int lt_rope(void* x, const float* cos_t, const float* sin_t, const int* pos, lon
   if (hd % 8 != 0 || row_stride % 8 != 0) return -int(kStatusBadArgument);
   const long long work = rows * heads * (hd / 8);
   if (work == 0) return 0;
-  LT_RETURN_IF_CUDA(launch_chained(rope_kernel, grid_for(work, 256), 256, 0, static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(x), cos_t, sin_t, pos, rows, T, heads, hd, row_stride, backward ? -1.f : 1.f));
+  auto X = static_cast<__nv_bfloat16*>(x);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const float sign = backward ? -1.f : 1.f;
+  const int grid = grid_for(work, 256);
+  if (work + (long long)grid * 256 < (1ll << 32))
+    LT_RETURN_IF_CUDA(launch_chained(rope_kernel<unsigned>, grid, 256, 0, st, X, cos_t, sin_t, pos, rows, T, heads, hd, row_stride, sign));
+  else
+    LT_RETURN_IF_CUDA(launch_chained(rope_kernel<long long>, grid, 256, 0, st, X, cos_t, sin_t, pos, rows, T, heads, hd, row_stride, sign));
   LT_LAUNCH_CHECK();
   return 0;
 }

@@ -38,6 +38,11 @@ class SingleTPMixin:
     def col_linear(self, x, name):
         return self.linear(x, name), x
 
+    def col_swiglu(self, x, name):
+        """(gate and up, silu(gate) * up, gathered x) of the column-parallel linear whose rows are gates, then ups."""
+        gu, xf = self.col_linear(x, name)
+        return gu, kernels_for(gu.device).swiglu_fwd(gu), xf
+
     def row_linear(self, x, name, residual=None):
         return self.linear(x, name, residual=residual)
 
@@ -196,6 +201,10 @@ class LocalWeights(SingleTPMixin):
     def linear(self, x, name, **kw):
         return self.K.gemm(x, self.p(name), **kw)
 
+    def col_swiglu(self, x, name):
+        gu, h = self.K.gemm_swiglu(x, self.p(name))
+        return gu, h, x
+
     def dgrad(self, dy, name, **kw):
         return self.K.gemm(dy, self.p(name), b_major=1, **kw)
 
@@ -336,17 +345,15 @@ class LlamaEngine:
         Hq, Hkv, hd = self.Hq, self.Hkv, cfg.head_dim
         h1, _, _, rstd1 = K.norm_fwd(x, w.p(p + "attn_norm"), eps=cfg.rms_eps, out=w.gather_slot(*x.shape))
         qkv, h1f = w.col_linear(h1, p + "wqkv")
-        K.rope_(qkv, self.cos, self.sin, T, Hq, hd, col_offset=0)
-        K.rope_(qkv, self.cos, self.sin, T, Hkv, hd, col_offset=Hq * hd)
+        K.rope_(qkv, self.cos, self.sin, T, Hq + Hkv, hd)
         q, k, v = self._split_qkv(qkv, B, T)
         o, lse = K.flash_fwd(q, k, v, causal=True)
         o2 = o.view(B * T, Hq * hd)
         x1 = w.row_linear(o2, p + "wo", residual=x)
         h2, _, _, rstd2 = K.norm_fwd(x1, w.p(p + "mlp_norm"), eps=cfg.rms_eps, out=w.gather_slot(*x1.shape))
-        gu, h2f = w.col_linear(h2, p + "w_gu")
-        hm = K.swiglu_fwd(gu)
+        gu, hm, h2f = w.col_swiglu(h2, p + "w_gu")
         x2 = w.row_linear(hm, p + "w_down", residual=x1)
-        self.kernel_launches += 11
+        self.kernel_launches += 10
         return x2, (x, h1f, rstd1, qkv, o, lse, x1, h2f, rstd2, gu, hm)
 
     def _split_qkv(self, qkv, B, T):
@@ -377,9 +384,7 @@ class LlamaEngine:
         dqkv = torch.empty_like(qkv)
         q, k, v = self._split_qkv(qkv, B, T)
         dq, dk, dv = self._split_qkv(dqkv, B, T)
-        K.flash_bwd(q, k, v, o, lse, do.view(B, T, Hq, hd), causal=True, dq=dq, dk=dk, dv=dv)
-        K.rope_(dqkv, self.cos, self.sin, T, Hq, hd, col_offset=0, backward=True)
-        K.rope_(dqkv, self.cos, self.sin, T, Hkv, hd, col_offset=Hq * hd, backward=True)
+        K.flash_bwd(q, k, v, o, lse, do.view(B, T, Hq, hd), causal=True, dq=dq, dk=dk, dv=dv, rope=(self.cos, self.sin))
         dh1 = w.col_dgrad(dqkv, p + "wqkv")
         w.wgrad(dqkv, h1f, p + "wqkv", accumulate)
         # The gradient that leaves this layer is the input of the next gathered GEMM - unless that layer recomputes its
@@ -387,7 +392,7 @@ class LlamaEngine:
         direct = i > 0 and (i - 1) >= self.ckpt_layers
         dx, _, _ = K.norm_bwd(dh1, x, w.p(p + "attn_norm"), None, rstd1, dres=dx1, dw=w.vector_grad(p + "attn_norm"),
                               accumulate=accumulate, out=w.gather_slot(*x.shape) if direct else None)
-        self.kernel_launches += 22
+        self.kernel_launches += 20
         return dx
 
     # ------------------------------------------------------------------------------------------ model

@@ -23,6 +23,7 @@ _SIGS = {
     "lt_moe_plan": [_vp] * 12 + [_i] * 5 + [_vp],
     "lt_moe_grouped_gemm": [_vp] * 5 + [_i] * 5 + [_vp],
     "lt_gemm_staged": [_vp, _vp, _vp, _i, _i, _i, _ll, _ll, _ll, _i, _f, _i, _vp],
+    "lt_gemm_glu_keep": [_vp] * 4 + [_i] * 3 + [_ll] * 4 + [_i, _vp],
     "lt_gemm_skinny_glu": [_vp, _ll, _vp, _vp, _i, _i, _i, _i, _vp],
     "lt_gemm_skinny_batch": [_vp, _ll, _ll, _vp, _vp, _ll, _ll, _i, _i, _i, _i, _vp],
     "lt_gemm_skinny_grouped": [_vp, _ll] + [_vp] * 6 + [_i] * 5 + [_vp],
@@ -119,12 +120,14 @@ _SIGS = {
                         _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _f, _i, _i, _i, _i, _vp],
     "lt_flash_bwd": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i,
                      _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _f, _i, _vp],
+    "lt_flash_bwd_rope": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i,
+                     _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _f, _i, _vp, _vp, _vp],
 }
 
 _bound = {}
 
 # Kernels launched per native call; `launch_count()` is what bench.py reports as "gpu_launches".
-_LAUNCHES_PER_CALL = {"lt_gemm_num_tiles": 0, "lt_gemm_skinny_set_target": 0, "lt_adam_q8": 3, "lt_set_wait_budget_cycles": 0, "lt_norm_bwd": 2, "lt_paged_decode": 2, "lt_paged_decode_window": 2, "lt_mlstm_prefill": 4, "lt_rglru_scan": 3, "lt_rglru_step": 2, "lt_flash_bwd": 3, "lt_status_fetch": 0, "lt_sm_count": 0, "lt_gemm_set_tail_split": 0, "lt_reduce_parts": 0, "lt_reduce_all": 2, "lt_gemm_set_pair_mode": 0, "lt_flash_bwd_set_trace": 0, "lt_flash_fwd_set_trace": 0, "lt_norm_bwd_ctas": 0,
+_LAUNCHES_PER_CALL = {"lt_gemm_num_tiles": 0, "lt_gemm_skinny_set_target": 0, "lt_adam_q8": 3, "lt_set_wait_budget_cycles": 0, "lt_norm_bwd": 2, "lt_paged_decode": 2, "lt_paged_decode_window": 2, "lt_mlstm_prefill": 4, "lt_rglru_scan": 3, "lt_rglru_step": 2, "lt_flash_bwd": 3, "lt_flash_bwd_rope": 3, "lt_status_fetch": 0, "lt_sm_count": 0, "lt_gemm_set_tail_split": 0, "lt_reduce_parts": 0, "lt_reduce_all": 2, "lt_gemm_set_pair_mode": 0, "lt_flash_bwd_set_trace": 0, "lt_flash_fwd_set_trace": 0, "lt_norm_bwd_ctas": 0,
                       "lt_adam_chunk_elems": 0}
 _launches = [0]
 
@@ -517,6 +520,23 @@ def swiglu_fwd(gu: torch.Tensor) -> torch.Tensor:
     return h
 
 
+def gemm_swiglu(x, w):
+    """(gate and up of x @ w^T, [M, 2 F]; silu(gate) * up, [M, F]) for w = gate rows, then up rows.  With more rows than the kernels for few
+    take, both leave the product's epilogue, and the second is made of the 32-bit sums."""
+    M, Kd = x.shape
+    F = w.shape[0] // 2
+    assert w.shape == (2 * F, Kd)
+    if M > 128 and x.dtype == w.dtype == torch.bfloat16 and F % 8 == 0 and x.stride(1) == 1 and w.stride(1) == 1 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 \
+            and _aligned(x, w):
+        gu = torch.empty((M, 2 * F), dtype=x.dtype, device=x.device)
+        h = torch.empty((M, F), dtype=x.dtype, device=x.device)
+        rc = _fn("lt_gemm_glu_keep")(x.data_ptr(), w.data_ptr(), h.data_ptr(), gu.data_ptr(), M, F, Kd, x.stride(0), w.stride(0), F, 2 * F, _ACT["silu"], _stream())
+        _check(rc, "lt_gemm_glu_keep")
+        return gu, h
+    gu = gemm(x, w)
+    return gu, swiglu_fwd(gu)
+
+
 def clamped_glu(gu: torch.Tensor, limit: float, slope: float = 1.702) -> torch.Tensor:
     """g sigmoid(slope g) (u + 1) with g = min(gate, limit), u = clamp(up, -limit, limit); gu is [M, gate | up]."""
     M, F2 = gu.shape
@@ -653,8 +673,9 @@ def flash_fwd(q, k, v, *, causal=True, scale=None, window=0):
     return o, lse
 
 
-def flash_bwd(q, k, v, o, lse, do, *, causal=True, scale=None, dq=None, dk=None, dv=None):
-    """Returns (dq, dk, dv) with the shapes/strides of the given outputs (allocated contiguous when None)."""
+def flash_bwd(q, k, v, o, lse, do, *, causal=True, scale=None, dq=None, dk=None, dv=None, rope=None):
+    """Returns (dq, dk, dv) with the shapes/strides of the given outputs (allocated contiguous when None).  rope (cos, sin): q and k are
+    `rope_`d by the positions 0, 1, .. of their rows, and dq and dk are turned back."""
     B, Tq, Hq, D = q.shape
     _, Tk, Hkv, _ = k.shape
     scale = (D ** -0.5) if scale is None else scale
@@ -662,14 +683,17 @@ def flash_bwd(q, k, v, o, lse, do, *, causal=True, scale=None, dq=None, dk=None,
     dk = torch.empty((B, Tk, Hkv, D), dtype=q.dtype, device=q.device) if dk is None else dk
     dv = torch.empty((B, Tk, Hkv, D), dtype=q.dtype, device=q.device) if dv is None else dv
     delta = torch.empty((B, Hq, Tq), dtype=torch.float32, device=q.device)
-    dq_acc = torch.zeros((B, Tq, Hq, D), dtype=torch.float32, device=q.device)
-    rc = _fn("lt_flash_bwd")(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), do.data_ptr(),
-                             dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(),
+    dq_acc = torch.empty((B, Tq, Hq, D), dtype=torch.float32, device=q.device)
+    cos, sin = rope or (None, None)
+    if rope:
+        assert Tq == Tk and all(t.dtype == torch.float32 and t.is_contiguous() and t.shape[1] == D // 2 and t.shape[0] >= Tq for t in rope)
+    rc = _fn("lt_flash_bwd_rope")(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), do.data_ptr(),
+                                  dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(),
                              B, Tq, Tk, Hq, Hkv, D,
                              q.stride(0), q.stride(1), k.stride(0), k.stride(1), v.stride(0), v.stride(1),
                              o.stride(0), o.stride(1), do.stride(0), do.stride(1),
                              dq.stride(0), dq.stride(1), dk.stride(0), dk.stride(1),
-                             float(scale), 1 if causal else 0, _stream())
+                             float(scale), 1 if causal else 0, _p(cos), _p(sin), _stream())
     _check(rc, "lt_flash_bwd")
     return dq, dk, dv
 

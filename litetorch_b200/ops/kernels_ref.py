@@ -144,6 +144,11 @@ def swiglu_fwd(gu):
     return (torch.nn.functional.silu(g) * u).to(gu.dtype)
 
 
+def gemm_swiglu(x, w):
+    gu = gemm(x, w)
+    return gu, swiglu_fwd(gu)
+
+
 def swiglu_bwd(gu, dh, inplace=True):
     F = gu.shape[1] // 2
     g, u, d = gu[:, :F].float(), gu[:, F:].float(), dh.float()
@@ -219,7 +224,7 @@ def flash_fwd(q, k, v, *, causal=True, scale=None, window=0):
     return o.permute(0, 2, 1, 3).contiguous().to(q.dtype), lse.contiguous()
 
 
-def flash_bwd(q, k, v, o, lse, do, *, causal=True, scale=None, dq=None, dk=None, dv=None):
+def flash_bwd(q, k, v, o, lse, do, *, causal=True, scale=None, dq=None, dk=None, dv=None, rope=None):
     B, Tq, Hq, D = q.shape
     _, Tk, Hkv, _ = k.shape
     scale = (D ** -0.5) if scale is None else scale
@@ -243,8 +248,12 @@ def flash_bwd(q, k, v, o, lse, do, *, causal=True, scale=None, dq=None, dk=None,
     dkf = dkf.reshape(B, Hkv, g, Tk, D).sum(2)
     dvf = dvf.reshape(B, Hkv, g, Tk, D).sum(2)
     res = []
-    for buf, val in ((dq, dqf), (dk, dkf), (dv, dvf)):
+    for i, (buf, val) in enumerate(((dq, dqf), (dk, dkf), (dv, dvf))):
         val = val.permute(0, 2, 1, 3)
+        if rope and i < 2:
+            c, s = (t[:Tq, None] for t in rope)
+            x, y = val[..., 0::2], val[..., 1::2]
+            val = torch.stack([x * c + y * s, y * c - x * s], -1).flatten(-2)
         if buf is None:
             res.append(val.contiguous().to(q.dtype))
         else:

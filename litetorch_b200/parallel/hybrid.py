@@ -377,6 +377,10 @@ class HybridWeights:
         xf = self._all_gather_rows(x)
         return self.K.gemm(xf, W), xf
 
+    def col_swiglu(self, x, name):
+        gu, xf = self.col_linear(x, name)
+        return gu, self.K.swiglu_fwd(gu), xf
+
     def row_linear(self, x, name, residual=None):
         """reduce_scatter(x @ W^T) + residual: x holds this rank's input columns for all rows, W the matching columns."""
         W = self.weight(name)
