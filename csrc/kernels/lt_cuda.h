@@ -22,6 +22,11 @@ typedef struct LtNextGather {
 extern "C" {
 #endif
 
+// ---- cuda_runtime/llama_layer.cu: a decoder layer of a training step, forward or backward, as one call
+struct LtLlamaLayer;
+int lt_llama_layer_fwd(const struct LtLlamaLayer* layer, void* stream);
+int lt_llama_layer_bwd(const struct LtLlamaLayer* layer, void* stream);
+
 // ---- flash_bwd.cu: FlashAttention backward: dQ, dK, dV from dO, O, LSE
 void lt_flash_bwd_set_trace(void* buf);
 int lt_flash_bwd(const void* q, const void* k, const void* v, const void* o, const float* lse, const void* d_o,

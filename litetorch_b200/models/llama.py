@@ -267,9 +267,8 @@ class LocalWeights(SingleTPMixin):
             return
         a, b = self._bucket_range(bucket)
         self._side.wait_stream(torch.cuda.current_stream())
-        with torch.cuda.stream(self._side):
-            self.K.adam_flat(self.master[a:b], self.flat_g[a:b], self.m[a:b], self.v[a:b], self.flat_p[a:b], lr=h["lr"],
-                        beta1=h["beta1"], beta2=h["beta2"], eps=h["eps"], wd=h["weight_decay"], step=h["step"], adamw=True)
+        self.K.adam_flat(self.master, self.flat_g, self.m, self.v, self.flat_p, lr=h["lr"], beta1=h["beta1"], beta2=h["beta2"], eps=h["eps"],
+                         wd=h["weight_decay"], step=h["step"], adamw=True, span=(a, b), stream=self._side)
         self._updated += b - a
 
     def finish_step(self):
@@ -339,7 +338,64 @@ class LlamaEngine:
         self.qkv_local = (self.Hq + 2 * self.Hkv) * cfg.head_dim
 
     # ------------------------------------------------------------------------------------------ layer
+    def _native_layer(self, i: int, B: int, T: int, saved: Optional[torch.Tensor] = None):
+        """(arguments, buffer of what the layer keeps) of the native layer calls, or None where they do not apply: whole bf16 weights on a GPU and
+        more rows than the kernels for few rows take.  Weights, gradients and what is kept are filled in."""
+        cfg, w = self.cfg, self.w
+        M = B * T
+        if type(w) is not LocalWeights or not w.flat_p.is_cuda or w.flat_p.dtype != torch.bfloat16 or M <= 128 or cfg.d_model % 8 or cfg.ffn % 8 \
+                or cfg.head_dim not in (64, 128) or T > self.cos.shape[0]:
+            return None
+        a = K.LlamaLayer(B, T, cfg.d_model, cfg.n_heads, cfg.n_kv_heads, cfg.head_dim, cfg.ffn, 0, cfg.rms_eps, self.cos.data_ptr(), self.sin.data_ptr())
+        pp, gp = w.flat_p.data_ptr(), w.flat_g.data_ptr()
+        for n in ("attn_norm", "wqkv", "wo", "mlp_norm", "w_gu", "w_down"):
+            at = 2 * w._base(w.by_name["layers.%d.%s" % (i, n)])
+            setattr(a, n, pp + at)
+            setattr(a, "g_" + n, gp + at)
+        sizes = (("h1", 2 * M * cfg.d_model), ("qkv", 2 * M * self.qkv_local), ("o", 2 * M * cfg.n_heads * cfg.head_dim), ("x1", 2 * M * cfg.d_model),
+                 ("h2", 2 * M * cfg.d_model), ("gu", 4 * M * cfg.ffn), ("hm", 2 * M * cfg.ffn), ("rstd1", 4 * M), ("rstd2", 4 * M), ("lse", 4 * M * cfg.n_heads))
+        return a, self._carve(a, sizes, saved)
+
+    def _carve(self, a, sizes, buf=None):
+        """One buffer for several fields of the arguments, each at a multiple of 256 bytes."""
+        if buf is None:
+            buf = torch.empty(sum((n + 255) // 256 * 256 for _, n in sizes), dtype=torch.uint8, device=self.device)
+        at = buf.data_ptr()
+        for name, n in sizes:
+            setattr(a, name, at)
+            at += (n + 255) // 256 * 256
+        return buf
+
     def _layer_fwd(self, i: int, x: torch.Tensor, B: int, T: int):
+        native = self._native_layer(i, B, T)
+        if native is not None:
+            a, kept = native
+            x2 = torch.empty_like(x)
+            a.x, a.x2 = x.data_ptr(), x2.data_ptr()
+            K.llama_layer("lt_llama_layer_fwd", a)
+            self.kernel_launches += 8
+            return x2, (x, kept)
+        return self._layer_fwd_steps(i, x, B, T)
+
+    def _layer_bwd(self, i: int, dx2: torch.Tensor, ctx, B: int, T: int, accumulate: bool):
+        if len(ctx) > 2:
+            return self._layer_bwd_steps(i, dx2, ctx, B, T, accumulate)
+        cfg = self.cfg
+        x, kept = ctx
+        M, q = B * T, 2 * B * T * cfg.n_heads * cfg.head_dim
+        a, _ = self._native_layer(i, B, T, kept)
+        dx = torch.empty_like(x)
+        a.x, a.dx2, a.dx, a.accumulate = x.data_ptr(), dx2.data_ptr(), dx.data_ptr(), int(accumulate)
+        scratch = self._carve(a, (("dhm", 2 * M * cfg.ffn), ("dh", 2 * M * cfg.d_model), ("dx1", 2 * M * cfg.d_model), ("d_o", q),
+                                  ("dqkv", 2 * M * self.qkv_local), ("delta", 4 * M * cfg.n_heads), ("dq_acc", 2 * q),
+                                  ("part", 4 * K.norm_bwd_ctas(M) * cfg.d_model)))
+        K.llama_layer("lt_llama_layer_bwd", a)
+        del scratch
+        self.kernel_launches += 16
+        return dx
+
+    # The schedule step by step: tensor-parallel and sharded weights, the CPU, few rows.
+    def _layer_fwd_steps(self, i: int, x: torch.Tensor, B: int, T: int):
         cfg, w, K = self.cfg, self.w, self.K
         p = "layers.%d." % i
         Hq, Hkv, hd = self.Hq, self.Hkv, cfg.head_dim
@@ -364,7 +420,7 @@ class LlamaEngine:
         v = q3[:, :, (Hq + Hkv) * hd:].view(B, T, Hkv, hd)
         return q, k, v
 
-    def _layer_bwd(self, i: int, dx2: torch.Tensor, ctx, B: int, T: int, accumulate: bool):
+    def _layer_bwd_steps(self, i: int, dx2: torch.Tensor, ctx, B: int, T: int, accumulate: bool):
         cfg, w, K = self.cfg, self.w, self.K
         p = "layers.%d." % i
         Hq, Hkv, hd = self.Hq, self.Hkv, cfg.head_dim

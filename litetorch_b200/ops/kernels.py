@@ -20,6 +20,8 @@ _SIGS = {
     "lt_latent_rope": [_i, _vp, _ll] + [_i] * 8 + [_vp, _f, _vp, _vp, _vp, _f, _vp, _i, _i, _vp, _vp, _vp],
     "lt_latent_decode": [_vp] * 7 + [_i] * 9 + [_f, _vp],
     "lt_flash_fwd_shared": [_vp] * 6 + [_i] * 5 + [_ll] * 4 + [_f, _i, _vp],
+    "lt_llama_layer_fwd": [_vp, _vp],
+    "lt_llama_layer_bwd": [_vp, _vp],
     "lt_moe_plan": [_vp] * 12 + [_i] * 5 + [_vp],
     "lt_moe_grouped_gemm": [_vp] * 5 + [_i] * 5 + [_vp],
     "lt_gemm_staged": [_vp, _vp, _vp, _i, _i, _i, _ll, _ll, _ll, _i, _f, _i, _vp],
@@ -124,10 +126,18 @@ _SIGS = {
                      _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _f, _i, _vp, _vp, _vp],
 }
 
+class LlamaLayer(ctypes.Structure):
+    """Arguments of `lt_llama_layer_fwd` / `_bwd` (csrc/cuda_runtime/llama_layer.cu)."""
+    _fields_ = ([(n, _i) for n in ("B", "T", "width", "heads", "kv_heads", "head_dim", "ffn", "accumulate")] + [("eps", _f)] +
+                [(n, _vp) for n in ("cos", "sin", "attn_norm", "wqkv", "wo", "mlp_norm", "w_gu", "w_down", "g_attn_norm", "g_wqkv", "g_wo", "g_mlp_norm",
+                                    "g_w_gu", "g_w_down", "x", "h1", "qkv", "o", "x1", "h2", "gu", "hm", "x2", "rstd1", "rstd2", "lse", "dx2", "dx", "dhm",
+                                    "dh", "dx1", "d_o", "dqkv", "delta", "dq_acc", "part")])
+
+
 _bound = {}
 
 # Kernels launched per native call; `launch_count()` is what bench.py reports as "gpu_launches".
-_LAUNCHES_PER_CALL = {"lt_gemm_num_tiles": 0, "lt_gemm_skinny_set_target": 0, "lt_adam_q8": 3, "lt_set_wait_budget_cycles": 0, "lt_norm_bwd": 2, "lt_paged_decode": 2, "lt_paged_decode_window": 2, "lt_mlstm_prefill": 4, "lt_rglru_scan": 3, "lt_rglru_step": 2, "lt_flash_bwd": 3, "lt_flash_bwd_rope": 3, "lt_status_fetch": 0, "lt_sm_count": 0, "lt_gemm_set_tail_split": 0, "lt_reduce_parts": 0, "lt_reduce_all": 2, "lt_gemm_set_pair_mode": 0, "lt_flash_bwd_set_trace": 0, "lt_flash_fwd_set_trace": 0, "lt_norm_bwd_ctas": 0,
+_LAUNCHES_PER_CALL = {"lt_gemm_num_tiles": 0, "lt_gemm_skinny_set_target": 0, "lt_adam_q8": 3, "lt_set_wait_budget_cycles": 0, "lt_norm_bwd": 2, "lt_paged_decode": 2, "lt_paged_decode_window": 2, "lt_mlstm_prefill": 4, "lt_rglru_scan": 3, "lt_rglru_step": 2, "lt_flash_bwd": 3, "lt_flash_bwd_rope": 3, "lt_llama_layer_fwd": 8, "lt_llama_layer_bwd": 16, "lt_status_fetch": 0, "lt_sm_count": 0, "lt_gemm_set_tail_split": 0, "lt_reduce_parts": 0, "lt_reduce_all": 2, "lt_gemm_set_pair_mode": 0, "lt_flash_bwd_set_trace": 0, "lt_flash_fwd_set_trace": 0, "lt_norm_bwd_ctas": 0,
                       "lt_adam_chunk_elems": 0}
 _launches = [0]
 
@@ -178,7 +188,8 @@ def _check(rc, name):
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    # (torch.cuda.current_stream() makes an object for it: 3 us a launch)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _p(t):
@@ -443,6 +454,11 @@ def norm_fwd(x, weight, bias=None, residual=None, *, layer_norm=False, eps=1e-5,
     return y, s, mean, rstd
 
 
+def norm_bwd_ctas(M: int) -> int:
+    """Rows of fp32 partial sums that `lt_norm_bwd` of M rows needs."""
+    return _fn("lt_norm_bwd_ctas")(M)
+
+
 def norm_bwd(dy, x, weight, mean, rstd, *, layer_norm=False, dres=None, dw=None, db=None, accumulate=False, out=None):
     """Returns (dx, dw, db).  `x` is the tensor that was normalised (the residual sum when one was fused).
     `out`: optional contiguous [M, D] buffer for dx."""
@@ -615,12 +631,20 @@ def ce_finish(logits, targets, gstats, *, vocab_start=0, grad_scale=1.0, ignore_
 
 
 # ------------------------------------------------------------------------------------------------ optimizers
-def adam_flat(master, grad, m, v, param_bf16, *, lr, beta1, beta2, eps, wd, step, adamw=True, dyn=None):
+def adam_flat(master, grad, m, v, param_bf16, *, lr, beta1, beta2, eps, wd, step, adamw=True, dyn=None, span=None, stream=None):
+    """One Adam(W) step of flat tensors, or of their elements `span` = (first, end).  `stream`: the torch stream to launch on (default: the current one)."""
     bc1 = 1.0 - beta1 ** step
     bc2 = 1.0 - beta2 ** step
-    _check(_fn("lt_adam_flat")(master.data_ptr(), grad.data_ptr(), 1 if grad.dtype == torch.bfloat16 else 0, m.data_ptr(),
-                               v.data_ptr(), _p(param_bf16), master.numel(), lr, beta1, beta2, eps, wd, bc1, bc2,
-                               1 if adamw else 0, _p(dyn), _stream()), "lt_adam_flat")
+    a, b = span or (0, master.numel())
+    g16 = grad.dtype == torch.bfloat16
+    _check(_fn("lt_adam_flat")(master.data_ptr() + 4 * a, grad.data_ptr() + (2 if g16 else 4) * a, 1 if g16 else 0, m.data_ptr() + 4 * a,
+                               v.data_ptr() + 4 * a, None if param_bf16 is None else param_bf16.data_ptr() + 2 * a, b - a, lr, beta1, beta2, eps, wd, bc1, bc2,
+                               1 if adamw else 0, _p(dyn), _stream() if stream is None else stream.cuda_stream), "lt_adam_flat")
+
+
+def llama_layer(name: str, layer: "LlamaLayer"):
+    """`lt_llama_layer_fwd` or `_bwd` on the current stream."""
+    _check(_fn(name)(ctypes.addressof(layer), _stream()), name)
 
 
 def sgd_flat(p, g, vel, *, lr, momentum, wd):

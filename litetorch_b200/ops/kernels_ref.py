@@ -262,7 +262,9 @@ def flash_bwd(q, k, v, o, lse, do, *, causal=True, scale=None, dq=None, dk=None,
     return tuple(res)
 
 
-def adam_flat(master, grad, m, v, param_bf16, *, lr, beta1, beta2, eps, wd, step, adamw=True, dyn=None):
+def adam_flat(master, grad, m, v, param_bf16, *, lr, beta1, beta2, eps, wd, step, adamw=True, dyn=None, span=None, stream=None):
+    if span is not None:
+        master, grad, m, v, param_bf16 = (None if t is None else t[span[0]:span[1]] for t in (master, grad, m, v, param_bf16))
     g = grad.float()
     if dyn is not None:
         if float(dyn[1]) != 0.0:
