@@ -128,6 +128,9 @@ int lt_gemm_block_diag(const void* A, const void* B, float* C, int M, int blocks
 int lt_weight_stream(const void* x, long long ldx, const void* w, long long ldw, void* y, long long ldy, const void* residual, long long ldr, int M,
                      int N, int K, int act, int early, void* stream);
 
+int lt_weight_stream_norm(const void* x, long long ldx, const void* gain, float eps, const void* w, long long ldw, void* y, long long ldy, int fp32,
+                          const void* residual, long long ldr, int M, int N, int K, int act, int early, void* stream);
+
 // ---- gemv.cu: GEMV for 1-8 rows
 int lt_gemv_bf16(const void* x, long long ldx, const void* w, long long ldw, void* y, long long ldy,
                  const void* residual, long long ldr, int M, int N, int K, void* stream);

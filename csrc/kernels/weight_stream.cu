@@ -18,6 +18,13 @@
 // 163 -> 87; 4096 x 14336 [17.9]: 24 -> 21, 74 -> 21, 41 -> 21, 47 -> 24, 71 -> 36; 2048 x 2048 [1.3]: 4.7 -> 4.3, 8.2 -> 4.3, 8.0 -> 4.4,
 // 10.0 -> 5.2, 16.4 -> 8.5.  Additions with rounding, up to 16 rows (see the loop), were added since: 38.7 -> 38.8, 39.6 -> 39.9, 42.2 -> 42.6 and
 // 4.79 -> 4.88 (2048 x 2048, 8 rows).  With 32 rows and more it is bound by x, which every tile reads again from L2; small matrices by the start.
+//
+// With up to 16 rows the kernel can normalise x on the way: the fragments are multiplied by the gains and rounded, as normalised rows would be, the
+// squares are summed beside them, and 1 / rms multiplies the results.  A kernel in front of the product takes 2 to 3 us of a step's chain: decode
+// steps of the 1.1B model 956 -> 880 us (one sequence), six 8B layers 943 -> 930 (8 sequences on an 8-bit cache).
+//
+// Rings of half the size, so that the next product lies beside this one and has all of its first weights early, are slower (1.1B step 880 -> 1037 us, tiles of
+// 16 rows with 8 rows of x as well 1069): its copies queue ahead of this kernel's own.  Deeper rings with 8 rows of x: 880 -> 911.
 #include "lt_cuda.h"
 #include "common/host.h"
 #include "common/ptx.cuh"
@@ -39,6 +46,17 @@ __device__ __forceinline__ void ws_mma_0(float (&d)[4], uint32_t a0, uint32_t a1
       : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
+// Eight bf16 values of x times eight gains, rounded to bf16; their squares join `sq`.
+__device__ __forceinline__ void ws_times(uint4& x, const uint4& gain, float& sq) {
+  uint32_t* xw = &x.x;
+  const uint32_t* gw = &gain.x;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 a = unpack_bf16x2(xw[j]), b = unpack_bf16x2(gw[j]);
+    sq = fmaf(a.x, a.x, fmaf(a.y, a.y, sq));
+    xw[j] = pack_bf16x2(a.x * b.x, a.y * b.y);
+  }
+}
 __device__ __forceinline__ uint4 lds_16(uint32_t src) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(src) : "memory");
@@ -51,14 +69,15 @@ struct WsCfg {
   static constexpr int kWarps = 8;
   static constexpr int kStage = (R + XR) * 128;
   static constexpr int kCtas = XR == 8 && R == 32 ? 2 : 1;                              // a SM
-  static constexpr int kStages = ((kCtas == 2 ? 96 : 192) * 1024 / (kWarps * kStage) < 6 ? (kCtas == 2 ? 96 : 192) * 1024 / (kWarps * kStage) : 6);
+  static constexpr int kRing = (kCtas == 2 ? 96 : 192) * 1024;
+  static constexpr int kStages = kRing / (kWarps * kStage) < 6 ? kRing / (kWarps * kStage) : 6;
   static constexpr int kOffPart = kWarps * kStages * kStage;                            // [warp][16 rows of x][R] partial sums
   static constexpr int kOffBar = kOffPart + kWarps * R * 64;
   static constexpr int kSmem = kOffBar + kWarps * kStages * 8 + 16 + 1024;
   static_assert(kStages >= 2 && kSmem * kCtas <= 227 * 1024 - (kCtas - 1) * 1024, "does not fit");
 };
 
-template <int XR, int R, bool GLU>
+template <int XR, int R, bool GLU, bool NORM>
 __global__ void __launch_bounds__(WsCfg<XR, R>::kWarps * 32, WsCfg<XR, R>::kCtas)
 weight_stream_kernel(const __grid_constant__ CUtensorMap tw, const __grid_constant__ CUtensorMap tx, const StreamProduct p, const int tiles, const int cols, int* status) {
   using Cfg = WsCfg<XR, R>;
@@ -71,6 +90,9 @@ weight_stream_kernel(const __grid_constant__ CUtensorMap tw, const __grid_consta
   const uint32_t bars = smem_u32(smem) + Cfg::kOffBar + warp * (S * 8);
   float* part = reinterpret_cast<float*>(smem + Cfg::kOffPart);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + Cfg::kOffBar + W * S * 8);
+  // with NORM: [warp][16 rows] sums of squares, then the gains, zero past K
+  float* squares = reinterpret_cast<float*>(smem + Cfg::kOffBar + W * S * 8 + 16);
+  const uint32_t gains = smem_u32(smem) + Cfg::kOffBar + W * S * 8 + 16 + W * 64;
   if (threadIdx.x == 0) *abort_flag = 0;
   if (lane == 0) {
     for (int s = 0; s < S; ++s) mbar_init(bars + s * 8, 1);
@@ -102,6 +124,13 @@ weight_stream_kernel(const __grid_constant__ CUtensorMap tw, const __grid_consta
   };
   pdl_launch_dependents();
   if (!p.early) pdl_wait();
+  if constexpr (NORM) {   // (a weight like w)
+    for (int k = threadIdx.x * 8; k < chunks * 64; k += W * 32 * 8) {
+      const uint4 v = k < p.K ? *reinterpret_cast<const uint4*>(p.gain + k) : make_uint4(0u, 0u, 0u, 0u);
+      asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(gains + k * 2), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+    }
+    __syncthreads();
+  }
 #pragma unroll
   for (int s = 0; s < S; ++s) load(true, false);
   if (p.early) pdl_wait();
@@ -114,6 +143,7 @@ weight_stream_kernel(const __grid_constant__ CUtensorMap tw, const __grid_consta
   int slot = 0;
   uint32_t phase = 0;
   bool ok = true;
+  [[maybe_unused]] float sq_lo = 0.f, sq_hi = 0.f;   // this lane's share of the sums of squares of rows g and g + 8
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     float acc[MT][R / 8][4];
 #pragma unroll
@@ -137,6 +167,12 @@ weight_stream_kernel(const __grid_constant__ CUtensorMap tw, const __grid_consta
         for (int m = 0; m < MT; ++m) {
           xv[m][0] = lds_16(from + R * 128 + m * 2048);
           xv[m][1] = XR == 8 ? make_uint4(0u, 0u, 0u, 0u) : lds_16(from + R * 128 + m * 2048 + 1024);
+        }
+        if constexpr (NORM) {
+          // the rows times the gains, rounded to 16 bits as normalised rows would be; their common factor 1 / rms waits for the sums
+          const uint4 gn = lds_16(gains + ((warp + i * W) * 64 + (2 * q + c) * 8) * 2);
+          ws_times(xv[0][0], gn, sq_lo);
+          if constexpr (XR != 8) ws_times(xv[0][1], gn, sq_hi);
         }
 #pragma unroll
         for (int f = 0; f < R / 8; ++f) {
@@ -165,6 +201,13 @@ weight_stream_kernel(const __grid_constant__ CUtensorMap tw, const __grid_consta
       if (++slot == S) { slot = 0; phase ^= 1u; }
     }
 
+    if constexpr (NORM) {
+      if (tile == blockIdx.x) {   // the first tile has met every column; its sums serve all of them
+        sq_lo += __shfl_xor_sync(0xffffffffu, sq_lo, 1); sq_lo += __shfl_xor_sync(0xffffffffu, sq_lo, 2);
+        sq_hi += __shfl_xor_sync(0xffffffffu, sq_hi, 1); sq_hi += __shfl_xor_sync(0xffffffffu, sq_hi, 2);
+        if (q == 0) { squares[warp * 16 + g] = sq_lo; squares[warp * 16 + g + 8] = sq_hi; }
+      }
+    }
     constexpr int F = R / 8 / (GLU ? 2 : 1);   // fragments of results
 #pragma unroll
     for (int m = 0; m < MT; ++m) {
@@ -179,6 +222,13 @@ weight_stream_kernel(const __grid_constant__ CUtensorMap tw, const __grid_consta
         const int row = m * 16 + h * 8 + (l >> 2), at_col = f * 8 + (l & 3) * 2, col = tile * cols + at_col;
         if (row >= M || at_col >= cols) continue;   // cols is even
         float v[2];
+        float factor = 1.f;
+        if constexpr (NORM) {
+          float sq = 0.f;
+#pragma unroll
+          for (int w = 0; w < W; ++w) sq += squares[w * 16 + row];
+          factor = rsqrtf(sq / p.K + p.eps);
+        }
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
           const int from = (f * 4 + h * 2 + b) * 32 + l;
@@ -188,9 +238,15 @@ weight_stream_kernel(const __grid_constant__ CUtensorMap tw, const __grid_consta
             s += part[w * (R * 16) + from];
             if constexpr (GLU) up += part[w * (R * 16) + from + F * 128];
           }
+          if constexpr (NORM) { s *= factor; up *= factor; }
           if constexpr (GLU) s = (p.act == 1 ? gelu_tanh_f(s) : silu_quick_f(s)) * up;
           else if (p.residual && col + b < N) s += __bfloat162float(p.residual[(long long)row * p.ldr + col + b]);
           v[b] = s;
+        }
+        if (p.y32) {
+          if (col < N) p.y32[(long long)row * p.ldy + col] = v[0];
+          if (col + 1 < N) p.y32[(long long)row * p.ldy + col + 1] = v[1];
+          continue;
         }
         __nv_bfloat16* to = p.y + (long long)row * p.ldy + col;
         if (col + 1 < N && !(reinterpret_cast<uintptr_t>(to) & 3)) {
@@ -206,13 +262,17 @@ weight_stream_kernel(const __grid_constant__ CUtensorMap tw, const __grid_consta
     for (int spin = 0; spin < 2000; ++spin) __nanosleep(100);  // bounded grace period for copies in flight
 }
 
-template <int XR, int R, bool GLU>
+template <int XR, int R, bool GLU, bool NORM = false>
 static int launch_ws(const StreamProduct& p, cudaStream_t st) {
   using Cfg = WsCfg<XR, R>;
+  if constexpr (!NORM && XR <= 16) {
+    if (p.gain) return launch_ws<XR, R, GLU, true>(p, st);
+  }
   static OncePerDevice configured;
-  auto kern = weight_stream_kernel<XR, R, GLU>;
+  auto kern = weight_stream_kernel<XR, R, GLU, NORM>;
+  const int smem = Cfg::kSmem + (NORM ? Cfg::kWarps * 64 + (p.K + 63) / 64 * 128 : 0);
   if (configured.pending()) {
-    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
+    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem + (NORM ? Cfg::kWarps * 64 + kStreamNormK * 2 : 0)));
     configured.finish();
   }
   // As many tiles as CTAs, or a multiple of that, so that none ends in a round of a few tiles: tiles get as wide as that takes, and
@@ -227,7 +287,7 @@ static int launch_ws(const StreamProduct& p, cudaStream_t st) {
   r = encode_tmap_2d(&tx, p.x, 2, p.K, p.M, (uint64_t)p.ldx * 2, 64, XR, 1);
   if (r) return 2000 + r;
   const int tiles = (p.N + cols - 1) / cols;
-  LT_RETURN_IF_CUDA(launch_chained(kern, dim3(tiles < room ? tiles : room), dim3(Cfg::kWarps * 32), Cfg::kSmem, st, tw, tx, p, tiles, cols, device_status_word()));
+  LT_RETURN_IF_CUDA(launch_chained(kern, dim3(tiles < room ? tiles : room), dim3(Cfg::kWarps * 32), smem, st, tw, tx, p, tiles, cols, device_status_word()));
   return 0;
 }
 
@@ -250,6 +310,7 @@ static int stream_by_size(const StreamProduct& p, cudaStream_t st) {
 }
 
 bool stream_takes(const StreamProduct& p) {
+  if (p.gain && (p.M > kStreamNormRows || p.K > kStreamNormK || (p.K & 7) || (reinterpret_cast<uintptr_t>(p.gain) & 15))) return false;
   return p.M >= 1 && p.M <= kStreamMaxRows && p.ldw >= p.K && (p.M == 1 || p.ldx >= p.K);
 }
 
@@ -262,17 +323,25 @@ int launch_stream(StreamProduct p, cudaStream_t st) {
 
 extern "C" {
 
-// The product of weight_stream.h by itself.  early: the kernel may start before the one ahead of it in the stream has ended and reads w
-// then, so that one must not write w; x, residual and y are touched only after it.
-int lt_weight_stream(const void* x, long long ldx, const void* w, long long ldw, void* y, long long ldy, const void* residual, long long ldr, int M,
-                     int N, int K, int act, int early, void* stream) {
+// The product of weight_stream.h by itself.  early: the kernel may start before the one ahead of it in the stream has ended and reads w (and gain)
+// then, so that one must not write them; x, residual and y are touched only after it.  gain (or nullptr), eps: x is normalised.  fp32: y holds 32-bit results.
+int lt_weight_stream_norm(const void* x, long long ldx, const void* gain, float eps, const void* w, long long ldw, void* y, long long ldy, int fp32,
+                          const void* residual, long long ldr, int M, int N, int K, int act, int early, void* stream) {
   using namespace lt;
-  const StreamProduct p{static_cast<const __nv_bfloat16*>(x), ldx, static_cast<const __nv_bfloat16*>(w), ldw, static_cast<__nv_bfloat16*>(y), ldy,
-                        static_cast<const __nv_bfloat16*>(residual), ldr, M, N, K, act, early};
+  StreamProduct p{static_cast<const __nv_bfloat16*>(x), ldx, static_cast<const __nv_bfloat16*>(w), ldw, static_cast<__nv_bfloat16*>(y), ldy,
+                  static_cast<const __nv_bfloat16*>(residual), ldr, M, N, K, act};
+  p.gain = static_cast<const __nv_bfloat16*>(gain);
+  p.eps = eps;
+  p.early = early;
+  if (fp32) p.y32 = static_cast<float*>(y);
   if (N <= 0 || K <= 0 || (K & 7) || (ldx & 7) || (ldw & 7) || act < 0 || act > 2 || (act && residual) || !stream_takes(p) ||
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15))
     return -int(kStatusBadArgument);
   return launch_stream(p, static_cast<cudaStream_t>(stream));
+}
+int lt_weight_stream(const void* x, long long ldx, const void* w, long long ldw, void* y, long long ldy, const void* residual, long long ldr, int M,
+                     int N, int K, int act, int early, void* stream) {
+  return lt_weight_stream_norm(x, ldx, nullptr, 0.f, w, ldw, y, ldy, 0, residual, ldr, M, N, K, act, early, stream);
 }
 
 }  // extern "C"

@@ -53,23 +53,20 @@ class LlamaKVModel(ServingModel):
         n = x.shape[0]
         for i in range(cfg.n_layers):
             p = "layers.%d." % i
-            h, _, _, _ = K.norm_fwd(x, w.p(p + "attn_norm"), eps=cfg.rms_eps)
-            qkv = K.product_of_constants(h, w.p(p + "wqkv"))
+            qkv = K.product_of_constants(x, w.p(p + "wqkv"), norm=(w.p(p + "attn_norm"), cfg.rms_eps))
             q = K.rope_append(qkv, e.cos, e.sin, positions, slots, Hq, Hkv, hd, self.cache.k[i], self.cache.v[i], self.block_size, self.cache.fp8,
                               self.cache.k_scale, self.cache.v_scale, in_place=in_place)
             k = qkv[:, Hq * hd:(Hq + Hkv) * hd].view(n, Hkv, hd)
             v = qkv[:, (Hq + Hkv) * hd:].view(n, Hkv, hd)
             o = attend(i, q, k, v)
             x1 = K.product_of_constants(o.reshape(n, Hq * hd), w.p(p + "wo"), residual=x)
-            h2, _, _, _ = K.norm_fwd(x1, w.p(p + "mlp_norm"), eps=cfg.rms_eps)
-            hm = K.product_of_constants(h2, w.p(p + "w_gu"), act="silu")
+            hm = K.product_of_constants(x1, w.p(p + "w_gu"), act="silu", norm=(w.p(p + "mlp_norm"), cfg.rms_eps))
             x = K.product_of_constants(hm, w.p(p + "w_down"), residual=x1)
         return x
 
     def _logits(self, hidden, rows=None):
         e, K = self.e, self.e.K
-        hf, _, _, _ = K.norm_fwd(hidden if rows is None else hidden[rows], e.w.p("final_norm"), eps=e.cfg.rms_eps)
-        return K.product_of_constants(hf, e.w.p("lm_head"))
+        return K.product_of_constants(hidden if rows is None else hidden[rows], e.w.p("lm_head"), norm=(e.w.p("final_norm"), e.cfg.rms_eps))
 
     # ------------------------------------------------------------------ prompt chunks
     @torch.no_grad()

@@ -55,6 +55,7 @@ _SIGS = {
     "lt_gemm_bf16": [_vp, _vp, _vp, _i, _i, _i, _ll, _ll, _ll, _i, _i, _i, _vp, _vp, _ll, _i, _i, _f, _i, _i, _vp],
     "lt_gemm_typed": [_i, _vp, _vp, _vp, _i, _i, _i, _ll, _ll, _ll, _i, _i, _i, _vp, _vp, _ll, _i, _i, _f, _vp],
     "lt_weight_stream": [_vp, _ll] * 4 + [_i] * 5 + [_vp],
+    "lt_weight_stream_norm": [_vp, _ll, _vp, _f, _vp, _ll, _vp, _ll, _i, _vp, _ll] + [_i] * 5 + [_vp],
     "lt_rope_append": [_vp, _ll] + [_vp] * 7 + [_ll, _i, _i, _i, _i, _i, _f, _f, _vp],
     "lt_gemv_bf16": [_vp, _ll, _vp, _ll, _vp, _ll, _vp, _ll, _i, _i, _i, _vp],
     "lt_gemm_skinny_bf16": [_vp, _ll, _vp, _ll, _vp, _ll, _vp, _ll, _i, _i, _i, _vp],
@@ -492,20 +493,26 @@ def rope_(x2d: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, T: int, heads
     return x2d
 
 
-def product_of_constants(x, w, residual=None, act: str = ""):
+def product_of_constants(x, w, residual=None, act: str = "", norm=None):
     """x @ w^T (+ residual), or with `act` glu_rows(x, w), for weights that no kernel of the pass writes: with up to 64 rows the kernel starts
-    under the one before it and fetches weights meanwhile."""
+    under the one before it and fetches weights meanwhile.  norm (gains, eps): x is RMS-normalised first, with up to 16 rows in the same kernel."""
     M, Kd = x.shape
     N = w.shape[0] // 2 if act else w.shape[0]
     assert x.dtype == w.dtype and w.dim() == 2 and w.shape[1] == Kd, "operands do not match: %s and %s" % (tuple(x.shape), tuple(w.shape))
     assert x.stride(1) == 1 and w.stride(1) == 1 and (not act or (residual is None and w.shape[0] % 2 == 0))
     if residual is not None:
         assert residual.dtype == x.dtype and residual.shape == (M, N) and residual.stride(1) == 1
-    if x.dtype == torch.bfloat16 and 0 < M <= 64 and Kd % 8 == 0 and w.is_contiguous() and x.stride(0) % 8 == 0 and x.stride(0) >= Kd and _aligned(x, w):
+    few = x.dtype == torch.bfloat16 and 0 < M <= 64 and Kd % 8 == 0 and w.is_contiguous() and x.stride(0) % 8 == 0 and x.stride(0) >= Kd and _aligned(x, w)
+    gain, eps = norm or (None, 0.0)
+    if gain is not None:
+        assert gain.dtype == x.dtype and gain.shape == (Kd,) and gain.is_contiguous()
+        if not (few and M <= 16 and Kd <= 8192 and _aligned(gain)):
+            return product_of_constants(norm_fwd(x, gain, eps=eps)[0], w, residual, act)
+    if few:
         y = torch.empty((M, N), dtype=x.dtype, device=x.device)
-        rc = _fn("lt_weight_stream")(x.data_ptr(), x.stride(0), w.data_ptr(), Kd, y.data_ptr(), N, _p(residual),
-                                     residual.stride(0) if residual is not None else 0, M, N, Kd, _ACT[act] if act else 0, 1, _stream())
-        _check(rc, "lt_weight_stream")
+        rc = _fn("lt_weight_stream_norm")(x.data_ptr(), x.stride(0), _p(gain), float(eps), w.data_ptr(), Kd, y.data_ptr(), N, 0, _p(residual),
+                                          residual.stride(0) if residual is not None else 0, M, N, Kd, _ACT[act] if act else 0, 1, _stream())
+        _check(rc, "lt_weight_stream_norm")
         return y
     return glu_rows(x, w, act) if act else gemm(x, w, residual=residual)
 
@@ -911,6 +918,13 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype=None, alpha: float = 1.0)
     if M == 0:
         return torch.empty((0, N), dtype=out_dtype, device=x.device)
     if x.dtype == torch.bfloat16 and Kd % 8 == 0 and (M == 1 or x.stride(0) % 8 == 0) and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0:
+        if M <= 16 and out_dtype == torch.float32 and alpha == 1.0 and (M == 1 or x.stride(0) >= Kd):
+            # few rows with 32-bit results (a head): the matrix is read once (16 x 32000 x 2048: 33 us on tiles of 128 rows, 21 here)
+            y = torch.empty((M, N), dtype=out_dtype, device=x.device)
+            rc = _fn("lt_weight_stream_norm")(x.data_ptr(), x.stride(0) if M > 1 else Kd, None, 0.0, w.data_ptr(), Kd, y.data_ptr(), N, 1, None, 0, M, N, Kd, 0, 0,
+                                              _stream())
+            _check(rc, "lt_weight_stream_norm")
+            return y
         return gemm(x, w, out_dtype=out_dtype, alpha=alpha)
     y = torch.empty((M, N), dtype=out_dtype, device=x.device)
     rc = _fn("lt_gemm_simt")(_f32(x), _f32(y), x.data_ptr(), w.data_ptr(), y.data_ptr(), M, N, Kd, x.stride(0), Kd, N, 1, 0, 0, 0,

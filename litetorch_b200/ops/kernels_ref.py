@@ -121,7 +121,9 @@ def rope_(x2d, cos, sin, T, heads, head_dim, *, col_offset=0, positions=None, ba
     return x2d
 
 
-def product_of_constants(x, w, residual=None, act=""):
+def product_of_constants(x, w, residual=None, act="", norm=None):
+    if norm is not None:
+        x = norm_fwd(x, norm[0], eps=norm[1])[0]
     return glu_rows(x, w, act) if act else gemm(x, w, residual=residual)
 
 

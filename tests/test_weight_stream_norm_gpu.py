@@ -1,0 +1,55 @@
+"""Products of a few rows that are normalised on the way, and those with 32-bit results, against 64 bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M", [1, 2, 7, 8, 9, 16])
+@pytest.mark.parametrize("N,Kd", [(2, 8), (100, 72), (2048, 2048), (2560, 2048), (18, 4096), (9472, 264), (33, 8192)])
+@pytest.mark.parametrize("act", ["", "silu"])
+def test_normalised_products(M, N, Kd, act):
+    from litetorch_b200.ops import kernels as K
+    g = torch.Generator(device="cuda").manual_seed(M + N + Kd)
+    x = (torch.randn(M, Kd + 8, device="cuda", generator=g) * torch.logspace(-3, 3, M, device="cuda")[:, None]).bfloat16()[:, :Kd]
+    gain = (1 + 0.1 * torch.randn(Kd, device="cuda", generator=g)).bfloat16()
+    w = (torch.randn((2 if act else 1) * N, Kd, device="cuda", generator=g) * Kd ** -0.5).bfloat16()
+    res = None if act else torch.randn(M, N, device="cuda", generator=g).bfloat16()
+    y = K.product_of_constants(x, w, res, act, norm=(gain, 1e-5))
+    x64 = x.double()
+    xh = x64 * torch.rsqrt((x64 ** 2).mean(-1, keepdim=True) + 1e-5) * gain.double()
+    z, size = xh @ w.double().t(), xh.abs() @ w.double().abs().t()      # a factor is rounded to bf16 (2^-9), as is the result; sums are of 32 bits
+    if act:
+        # |d silu(a) b| <= 1.1 |b| da + |silu(a)| db
+        a, b, da, db = z[:, :N], z[:, N:], size[:, :N] * 2.0 ** -8, size[:, N:] * 2.0 ** -8
+        want, bound = torch.nn.functional.silu(a) * b, 1.1 * b.abs() * da + a.abs() * db + da * db
+    else:
+        want, bound = z + res.double(), size * 2.0 ** -8
+    assert ((y.double() - want).abs() <= want.abs() * 2.0 ** -8 + bound + 1e-5).all()
+    assert float((y.double() - want).norm() / want.norm()) < 6e-3
+    # what it stands in for, whose normalised rows are rounded alike
+    h = K.norm_fwd(x.contiguous(), gain, eps=1e-5)[0]
+    z = K.product_of_constants(h, w, res, act)
+    assert float((y.double() - z.double()).norm() / want.norm()) < 6e-3
+    assert K.status_fetch() == 0
+
+
+def test_more_rows_or_columns_are_normalised_first():
+    from litetorch_b200.ops import kernels as K
+    for M, Kd in ((17, 256), (200, 256), (2, 8200)):
+        x = torch.randn(M, Kd, device="cuda").bfloat16()
+        gain, w = (1 + 0.1 * torch.randn(Kd, device="cuda")).bfloat16(), (torch.randn(64, Kd, device="cuda") * Kd ** -0.5).bfloat16()
+        assert torch.equal(K.product_of_constants(x, w, norm=(gain, 1e-6)), K.product_of_constants(K.norm_fwd(x, gain, eps=1e-6)[0], w))
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("N,Kd", [(3, 8), (32000, 2048), (1001, 264)])
+def test_32_bit_results(M, N, Kd):
+    from litetorch_b200.ops import kernels as K
+    g = torch.Generator(device="cuda").manual_seed(M + N + Kd)
+    x = torch.randn(M, Kd, device="cuda", generator=g).bfloat16()
+    w = torch.randn(N, Kd, device="cuda", generator=g).bfloat16()
+    y = K.linear(x, w, out_dtype=torch.float32)
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    assert y.dtype == torch.float32 and ((y.double() - want).abs() <= size * 2.0 ** -20).all()
+    assert K.status_fetch() == 0
