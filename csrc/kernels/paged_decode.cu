@@ -10,6 +10,7 @@
 // Cache layout: [num_blocks, Hkv, block_size, D] as in the reference.
 #include "lt_cuda.h"
 #include <cuda_fp8.h>
+#include <initializer_list>
 
 #include "common/host.h"
 #include "common/ptx.cuh"
@@ -389,20 +390,104 @@ __device__ __forceinline__ void pd_write_partial(uint8_t* smem, float* part, int
       lsum += red_l[w * kPdMmaMaxG + gg] * a;
       o += red_o[(w * kPdMmaMaxG + gg) * D + d] * a;
     }
-    float* out = part + ((long long)gg * splits + sp) * (D + 2);
+    float* out = part + ((long long)gg * splits + sp) * (D + 2);   // (in shared memory: splits 1, sp 0)
     out[d] = lsum > 0.f ? o / lsum * out_scale : 0.f;
     if (d == 0) { out[D] = gm; out[D + 1] = lsum; }
   }
 }
 
+// A decode step's attention in one launch (STEP): the kernel reads the rows [q | k | v] of the product in front of it as they lie, turns queries and
+// the newest key by the angles of their positions, writes the newest key and value to their cache slots and puts them into its own tile, and the
+// splits of a (sequence, KV head), a cluster, merge their results through each other's shared memory.  Rotation and cache write, and the merge,
+// were launches of their own: 2.6 and 3 to 5 us of a chain in which every kernel waits for the one before it.
+struct PdStep {
+  const __nv_bfloat16* qkv;      // [S, ld], 16-byte aligned rows
+  long long ld;
+  const float *cos_t, *sin_t;    // [positions, D / 2]
+  const int *pos, *slots;        // [S]; a sequence's newest token is the last of its context; slot < 0: not written
+  void *k_cache, *v_cache;
+  float k_inv, v_inv;            // what 8-bit keys and values are multiplied by
+  __nv_bfloat16* out;            // [S, Hq, D]
+  int early;                     // block tables, lengths and all cached rows but the newest were complete before the kernels that may still run
+};
+constexpr int kPdMaxCluster = 16;
+
+// Lane `lane` < D / 4 holds eight columns of the newest key (lane < D / 8) or value of (s, hkv), turned and rounded to bf16.
+template <int D>
+__device__ __forceinline__ uint4 pd_newest(const PdStep& f, int s, int hkv, int Hq, int Hkv, int lane) {
+  if (lane >= D / 4) return make_uint4(0u, 0u, 0u, 0u);
+  const bool is_k = lane < D / 8;
+  const int u = is_k ? lane : lane - D / 8;
+  uint4 w = *reinterpret_cast<const uint4*>(f.qkv + s * f.ld + (long long)(Hq + (is_k ? 0 : Hkv) + hkv) * D + u * 8);
+  if (is_k) {
+    const long long at = (long long)f.pos[s] * (D / 2) + u * 4;
+    const float4 c = *reinterpret_cast<const float4*>(f.cos_t + at), n = *reinterpret_cast<const float4*>(f.sin_t + at);
+    const float cc[4] = {c.x, c.y, c.z, c.w}, nn[4] = {n.x, n.y, n.z, n.w};
+    uint32_t* p = &w.x;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 a = unpack_bf16x2(p[j]);
+      p[j] = pack_bf16x2(a.x * cc[j] - a.y * nn[j], a.x * nn[j] + a.y * cc[j]);
+    }
+  }
+  return w;
+}
+// Element offset of this lane's eight columns in its cache; negative: not cached.
+template <int D>
+__device__ __forceinline__ long long pd_newest_at(const PdStep& f, int s, int hkv, int Hkv, int block_size, int lane) {
+  const int slot = f.slots[s];
+  if (slot < 0 || lane >= D / 4) return -1;
+  return (((long long)(slot / block_size) * Hkv + hkv) * block_size + slot % block_size) * D + (lane % (D / 8)) * 8;
+}
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr, int cta) {
+  float v;
+  asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.f32 %0, [ra];\n\t}" : "=f"(v) : "r"(addr), "r"(cta) : "memory");
+  return v;
+}
+// The cluster's splits (their rows [G][D + 2] at `mine` in each one's shared memory) merged and written, every CTA a share of the G * D results.
+template <int D>
+__device__ __forceinline__ void pd_merge_cluster(const float* mine, __nv_bfloat16* out, int G, int splits, int sp) {
+  cluster_sync_all();
+  const uint32_t base = smem_u32(mine);
+  for (int e = sp * blockDim.x + threadIdx.x; e < G * D; e += splits * blockDim.x) {
+    const int gg = e / D, d = e % D;
+    float gm = -INFINITY, sum = 0.f, acc = 0.f;
+    // eight splits at a time, their loads under way together
+    for (int i0 = 0; i0 < splits; i0 += 8) {
+      float m[8], l[8], o[8], top = gm;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        m[i] = -INFINITY; l[i] = 0.f; o[i] = 0.f;
+        if (i0 + i < splits) {
+          m[i] = ld_cluster_f32(base + (gg * (D + 2) + D) * 4, i0 + i);
+          l[i] = ld_cluster_f32(base + (gg * (D + 2) + D + 1) * 4, i0 + i);
+          o[i] = ld_cluster_f32(base + (gg * (D + 2) + d) * 4, i0 + i);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) top = fmaxf(top, m[i]);
+      const float before = gm == -INFINITY ? 0.f : __expf(gm - top);
+      sum *= before; acc *= before; gm = top;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float w = !(l[i] <= 0.f) ? l[i] * __expf(m[i] - gm) : 0.f;     // a split without keys has outputs of zero
+        sum += w;
+        acc += w * o[i];
+      }
+    }
+    out[e] = __float2bfloat16(sum > 0.f ? acc / sum : 0.f);
+  }
+  cluster_sync_all();   // nobody leaves while its rows are read
+}
+
 // tmK / tmV: the caches seen as [num_blocks * Hkv * block_size rows, D] bf16, box 64 columns x min(block_size, 32) rows,
 // 128-byte swizzle.  block_size is a multiple of 8 and divides 32 or is a multiple of it.
-template <int D>
+template <int D, bool STEP>
 __global__ void __launch_bounds__(kPdWarps * 32)
 paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                         const __nv_bfloat16* __restrict__ q, const int* __restrict__ block_tables,
                         const int* __restrict__ context_lens, float* __restrict__ part, int S, int Hq, int Hkv, int block_size,
-                        int max_blocks, int splits, float scale, int window, int* status) {
+                        int max_blocks, int splits, float scale, int window, int* status, const __grid_constant__ PdStep step) {
   using Cfg = PdMmaCfg<D>;
   constexpr int ST = Cfg::kStages;
   constexpr int KS = D / 16;     // k-steps of the score product
@@ -425,22 +510,9 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     fence_proxy_async();
   }
   pdl_launch_dependents();
-  pdl_wait();
-  // A fragments of the query block: rows = heads of the group (g and g + 8), zero past G
-  uint32_t qa[KS][4];
-  {
-    const bool lo = g < G, hi = g + 8 < G;
-    const __nv_bfloat16* qlo = q + ((long long)s * Hq + hkv * G + (lo ? g : 0)) * D + qd * 2;
-    const __nv_bfloat16* qhi = q + ((long long)s * Hq + hkv * G + (hi ? g + 8 : 0)) * D + qd * 2;
-#pragma unroll
-    for (int kk = 0; kk < KS; ++kk) {
-      qa[kk][0] = lo ? *reinterpret_cast<const uint32_t*>(qlo + kk * 16) : 0u;
-      qa[kk][1] = hi ? *reinterpret_cast<const uint32_t*>(qhi + kk * 16) : 0u;
-      qa[kk][2] = lo ? *reinterpret_cast<const uint32_t*>(qlo + kk * 16 + 8) : 0u;
-      qa[kk][3] = hi ? *reinterpret_cast<const uint32_t*>(qhi + kk * 16 + 8) : 0u;
-    }
-  }
-  __syncthreads();
+  const bool early = STEP && step.early;
+  if (!early) pdl_wait();
+  __syncthreads();   // (each warp waits on barriers of its own; the flags are shared)
   volatile int* abort_flag = &abort_s;
   const int ctx = context_lens[s];
   const int lo = window > 0 ? max(0, ctx - window) : 0;              // first visible key
@@ -480,6 +552,46 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
 
   if (lane == 0)
     for (int i = 0; i < ST - 1 && i < my_n; ++i) request(i);
+  if (early) pdl_wait();
+  // A fragments of the query block: rows = heads of the group (g and g + 8), zero past G
+  uint32_t qa[KS][4];
+  {
+    const bool lo = g < G, hi = g + 8 < G;
+    const __nv_bfloat16* rows = STEP ? step.qkv + s * step.ld + (long long)hkv * G * D : q + ((long long)s * Hq + hkv * G) * D;
+    const __nv_bfloat16* qlo = rows + (lo ? g : 0) * D + qd * 2;
+    const __nv_bfloat16* qhi = rows + (hi ? g + 8 : 0) * D + qd * 2;
+#pragma unroll
+    for (int kk = 0; kk < KS; ++kk) {
+      qa[kk][0] = lo ? *reinterpret_cast<const uint32_t*>(qlo + kk * 16) : 0u;
+      qa[kk][1] = hi ? *reinterpret_cast<const uint32_t*>(qhi + kk * 16) : 0u;
+      qa[kk][2] = lo ? *reinterpret_cast<const uint32_t*>(qlo + kk * 16 + 8) : 0u;
+      qa[kk][3] = hi ? *reinterpret_cast<const uint32_t*>(qhi + kk * 16 + 8) : 0u;
+    }
+    if constexpr (STEP) {
+      const long long at = (long long)step.pos[s] * (D / 2) + qd;
+#pragma unroll
+      for (int kk = 0; kk < KS; ++kk)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {     // columns kk * 16 + 8 half + 2 qd and the next
+          const float c = step.cos_t[at + kk * 8 + half * 4], n = step.sin_t[at + kk * 8 + half * 4];
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const float2 a = unpack_bf16x2(qa[kk][half * 2 + r]);
+            qa[kk][half * 2 + r] = pack_bf16x2(a.x * c - a.y * n, a.x * n + a.y * c);
+          }
+        }
+    }
+  }
+  // the newest token's row, for the warp whose last chunk it ends
+  const int newest = STEP && t1 == ctx && my_n > 0 && (n_chunks - 1) % kPdWarps == warp ? my_n - 1 : -1;
+  [[maybe_unused]] uint4 fresh;
+  [[maybe_unused]] long long fresh_at = -1;
+  if constexpr (STEP) {
+    if (newest >= 0) {
+      fresh = pd_newest<D>(step, s, hkv, Hq, Hkv, lane);
+      fresh_at = pd_newest_at<D>(step, s, hkv, Hkv, block_size, lane);
+    }
+  }
   bool ok = true;
   const int lj = lane >> 3, lr = lane & 7;   // ldmatrix: this lane addresses row lr of matrix lj
   for (int i = 0; i < my_n; ++i) {
@@ -497,6 +609,16 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     uint8_t* vt = kt + Cfg::kTileBytes;
     const uint32_t kt_addr = smem_u32(kt), vt_addr = smem_u32(vt);
     const int nk = min(32, t1 - c0);
+    if constexpr (STEP) {
+      if (i == newest) {
+        if (lane < D / 4) {
+          const int r = nk - 1, u = lane % (D / 8);
+          *reinterpret_cast<uint4*>((lane < D / 8 ? kt : vt) + (u >> 3) * 4096 + r * 128 + (((u & 7) ^ (r & 7)) << 4)) = fresh;
+          if (fresh_at >= 0) *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(lane < D / 8 ? step.k_cache : step.v_cache) + fresh_at) = fresh;
+        }
+        __syncwarp();
+      }
+    }
     if (nk < 32) {
       // rows past the context (the tail of the last block, or never copied) may hold anything: zero them in V so that
       // their zero probabilities do not meet a NaN
@@ -590,7 +712,13 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     *reinterpret_cast<float2*>(lo) = make_float2(oacc[nt][0], oacc[nt][1]);
     *reinterpret_cast<float2*>(hi) = make_float2(oacc[nt][2], oacc[nt][3]);
   }
-  pd_write_partial<D>(pd_smem, part + ((long long)s * Hq + hkv * G) * splits * (D + 2), G, splits, sp, 1.f);
+  if (STEP && !part) {
+    float* mine = red_o + kPdWarps * kPdMmaMaxG * D;
+    pd_write_partial<D>(pd_smem, mine, G, 1, 0, 1.f);
+    pd_merge_cluster<D>(mine, step.out + ((long long)s * Hq + hkv * G) * D, G, splits, sp);
+  } else {
+    pd_write_partial<D>(pd_smem, part + ((long long)s * Hq + hkv * G) * splits * (D + 2), G, splits, sp, 1.f);
+  }
 }
 
 // The same split of the work for e4m3 caches.  What was a warp per query head that walked the keys one at a time (968 us for 8
@@ -610,7 +738,7 @@ struct PdF8Cfg {
   static constexpr int kWarpBytes = kStages * 2 * kTileBytes;
   static constexpr int kOffBar = kPdWarps * kWarpBytes;
   static constexpr int kSmemBytes = kOffBar + kPdWarps * kStages * 8 + 16 + 1024;   // + slack to align the tiles to 1024 bytes
-  static_assert(kOffBar >= kPdWarps * kPdMmaMaxG * (D + 2) * 4, "the reduction at the end reuses the tile area");
+  static_assert(kOffBar >= (kPdWarps + 1) * kPdMmaMaxG * (D + 2) * 4, "the reduction at the end reuses the tile area");
 };
 constexpr float kPdWeightScale = 16384.f;   // weights are at most 1: the largest fp16 part is 2^14, the smallest 2^-24 stands for 2^-38
 
@@ -646,12 +774,12 @@ __device__ __forceinline__ void split_f16x2(float x0, float x1, uint32_t& hi, ui
 
 // tmK / tmV: the caches seen as [num_blocks * Hkv * block_size rows, D] bytes, box D columns x min(block_size, 32) rows; rows of 128
 // bytes arrive with the 128-byte swizzle, rows of 64 as they are.
-template <int D>
+template <int D, bool STEP>
 __global__ void __launch_bounds__(kPdWarps * 32)
 paged_decode_f8_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                        const __nv_bfloat16* __restrict__ q, const int* __restrict__ block_tables,
                        const int* __restrict__ context_lens, float* __restrict__ part, int S, int Hq, int Hkv, int block_size,
-                       int max_blocks, int splits, float scale, float v_scale, int window, int* status) {
+                       int max_blocks, int splits, float scale, float v_scale, int window, int* status, const __grid_constant__ PdStep step) {
   using Cfg = PdF8Cfg<D>;
   constexpr int ST = Cfg::kStages;
   constexpr int KS = D / 16;     // k-steps of the score product
@@ -674,41 +802,11 @@ paged_decode_f8_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     fence_proxy_async();
   }
   pdl_launch_dependents();
-  pdl_wait();
+  const bool early = STEP && step.early;
+  if (!early) pdl_wait();
   // offset of 16-byte unit u of row r inside a tile
   auto unit = [](int r, int u) { return D == 128 ? r * 128 + ((u ^ (r & 7)) << 4) : r * 64 + (u << 4); };
-  // A fragments of the query block, columns permuted: step kk = 4 h + r takes columns 64 h + 16 qd + 4 r + {0 .. 3}.  Rows = heads of the
-  // group (g and g + 8), zero past G, scaled by a power of two to a largest value in [2^14, 2^15).
-  uint32_t qa[KS][4];
-  float scale_lo, scale_hi;
-  {
-    uint2 raw[2][KS];
-    float top[2] = {0.f, 0.f};
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const bool there = g + 8 * half < G;
-      const __nv_bfloat16* row = q + ((long long)s * Hq + hkv * G + (there ? g + 8 * half : 0)) * D + qd * 16;
-#pragma unroll
-      for (int kk = 0; kk < KS; ++kk) {
-        raw[half][kk] = there ? *reinterpret_cast<const uint2*>(row + (kk >> 2) * 64 + (kk & 3) * 4) : make_uint2(0u, 0u);
-        const float2 a = unpack_bf16x2(raw[half][kk].x), b = unpack_bf16x2(raw[half][kk].y);
-        top[half] = fmaxf(top[half], fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y))));
-      }
-      top[half] = fmaxf(top[half], __shfl_xor_sync(0xffffffffu, top[half], 1));
-      top[half] = fmaxf(top[half], __shfl_xor_sync(0xffffffffu, top[half], 2));
-      // (a row of zeros or with an infinity stays as it is)
-      const int e = top[half] > 0.f && top[half] <= 3.4e38f ? max(-120, min(100, 14 - ilogbf(top[half]))) : 0;
-      const float up = ldexpf(1.f, e);
-      (half ? scale_hi : scale_lo) = scale * ldexpf(1.f, -e);
-#pragma unroll
-      for (int kk = 0; kk < KS; ++kk) {
-        const float2 a = unpack_bf16x2(raw[half][kk].x), b = unpack_bf16x2(raw[half][kk].y);
-        qa[kk][half] = pack_f16x2(a.x * up, a.y * up);
-        qa[kk][2 + half] = pack_f16x2(b.x * up, b.y * up);
-      }
-    }
-  }
-  __syncthreads();
+  __syncthreads();   // (each warp waits on barriers of its own; the flags are shared)
   volatile int* abort_flag = &abort_s;
   const int ctx = context_lens[s];
   const int lo = window > 0 ? max(0, ctx - window) : 0;              // first visible key
@@ -743,6 +841,55 @@ paged_decode_f8_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
 
   if (lane == 0)
     for (int i = 0; i < ST - 1 && i < my_n; ++i) request(i);
+  if (early) pdl_wait();
+  // A fragments of the query block, columns permuted: step kk = 4 h + r takes columns 64 h + 16 qd + 4 r + {0 .. 3}.  Rows = heads of the
+  // group (g and g + 8), zero past G, scaled by a power of two to a largest value in [2^14, 2^15).
+  uint32_t qa[KS][4];
+  float scale_lo, scale_hi;
+  {
+    uint2 raw[2][KS];
+    float top[2] = {0.f, 0.f};
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const bool there = g + 8 * half < G;
+      const __nv_bfloat16* rows = STEP ? step.qkv + s * step.ld + (long long)hkv * G * D : q + ((long long)s * Hq + hkv * G) * D;
+      const __nv_bfloat16* row = rows + (there ? g + 8 * half : 0) * D + qd * 16;
+#pragma unroll
+      for (int kk = 0; kk < KS; ++kk) {
+        raw[half][kk] = there ? *reinterpret_cast<const uint2*>(row + (kk >> 2) * 64 + (kk & 3) * 4) : make_uint2(0u, 0u);
+        if constexpr (STEP) {
+          const long long at = (long long)step.pos[s] * (D / 2) + (kk >> 2) * 32 + qd * 8 + (kk & 3) * 2;
+          const float2 c = *reinterpret_cast<const float2*>(step.cos_t + at), n = *reinterpret_cast<const float2*>(step.sin_t + at);
+          const float2 x = unpack_bf16x2(raw[half][kk].x), y = unpack_bf16x2(raw[half][kk].y);
+          raw[half][kk] = make_uint2(pack_bf16x2(x.x * c.x - x.y * n.x, x.x * n.x + x.y * c.x), pack_bf16x2(y.x * c.y - y.y * n.y, y.x * n.y + y.y * c.y));
+        }
+        const float2 a = unpack_bf16x2(raw[half][kk].x), b = unpack_bf16x2(raw[half][kk].y);
+        top[half] = fmaxf(top[half], fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y))));
+      }
+      top[half] = fmaxf(top[half], __shfl_xor_sync(0xffffffffu, top[half], 1));
+      top[half] = fmaxf(top[half], __shfl_xor_sync(0xffffffffu, top[half], 2));
+      // (a row of zeros or with an infinity stays as it is)
+      const int e = top[half] > 0.f && top[half] <= 3.4e38f ? max(-120, min(100, 14 - ilogbf(top[half]))) : 0;
+      const float up = ldexpf(1.f, e);
+      (half ? scale_hi : scale_lo) = scale * ldexpf(1.f, -e);
+#pragma unroll
+      for (int kk = 0; kk < KS; ++kk) {
+        const float2 a = unpack_bf16x2(raw[half][kk].x), b = unpack_bf16x2(raw[half][kk].y);
+        qa[kk][half] = pack_f16x2(a.x * up, a.y * up);
+        qa[kk][2 + half] = pack_f16x2(b.x * up, b.y * up);
+      }
+    }
+  }
+  // the newest token's row, for the warp whose last chunk it ends
+  const int newest = STEP && t1 == ctx && my_n > 0 && (n_chunks - 1) % kPdWarps == warp ? my_n - 1 : -1;
+  [[maybe_unused]] uint4 fresh;
+  [[maybe_unused]] long long fresh_at = -1;
+  if constexpr (STEP) {
+    if (newest >= 0) {
+      fresh = pd_newest<D>(step, s, hkv, Hq, Hkv, lane);
+      fresh_at = pd_newest_at<D>(step, s, hkv, Hkv, block_size, lane);
+    }
+  }
   bool ok = true;
   const int lj = lane >> 3, lr = lane & 7;   // ldmatrix: this lane addresses row lr of matrix lj
   for (int i = 0; i < my_n; ++i) {
@@ -760,6 +907,26 @@ paged_decode_f8_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     uint8_t* vt = kt + Cfg::kTileBytes;
     const uint32_t vt_addr = smem_u32(vt);
     const int nk = min(32, t1 - c0);
+    if constexpr (STEP) {
+      if (i == newest) {
+        if (lane < D / 4) {
+          const int r = nk - 1, u = lane % (D / 8);
+          const float inv = lane < D / 8 ? step.k_inv : step.v_inv;
+          alignas(8) uint8_t eight[8];
+          const uint32_t* p = &fresh.x;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 a = unpack_bf16x2(p[j]);
+            eight[2 * j] = __nv_fp8_e4m3(a.x * inv).__x;
+            eight[2 * j + 1] = __nv_fp8_e4m3(a.y * inv).__x;
+          }
+          const uint2 two = *reinterpret_cast<const uint2*>(eight);
+          *reinterpret_cast<uint2*>((lane < D / 8 ? kt : vt) + unit(r, u >> 1) + (u & 1) * 8) = two;
+          if (fresh_at >= 0) *reinterpret_cast<uint2*>(static_cast<uint8_t*>(lane < D / 8 ? step.k_cache : step.v_cache) + fresh_at) = two;
+        }
+        __syncwarp();
+      }
+    }
     if (nk < 32 || c0 < lo) {
       // rows past the context or before the window may hold anything: zero them in V so that their zero weights do not meet a NaN
       // (a window starts in a warp's first chunk, whose stage a later copy fills again: that copy has to come after these stores)
@@ -867,7 +1034,13 @@ paged_decode_f8_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     *reinterpret_cast<float4*>(at) = make_float4(oacc[u][0][0], oacc[u][1][0], oacc[u][0][1], oacc[u][1][1]);
     *reinterpret_cast<float4*>(at + 8 * D) = make_float4(oacc[u][0][2], oacc[u][1][2], oacc[u][0][3], oacc[u][1][3]);
   }
-  pd_write_partial<D>(pd_smem, part + ((long long)s * Hq + hkv * G) * splits * (D + 2), G, splits, sp, v_scale / kPdWeightScale);
+  if (STEP && !part) {
+    float* mine = red_o + kPdWarps * kPdMmaMaxG * D;
+    pd_write_partial<D>(pd_smem, mine, G, 1, 0, v_scale / kPdWeightScale);
+    pd_merge_cluster<D>(mine, step.out + ((long long)s * Hq + hkv * G) * D, G, splits, sp);
+  } else {
+    pd_write_partial<D>(pd_smem, part + ((long long)s * Hq + hkv * G) * splits * (D + 2), G, splits, sp, v_scale / kPdWeightScale);
+  }
 }
 
 template <int D>
@@ -936,6 +1109,14 @@ __global__ void kv_append_kernel(const __nv_bfloat16* __restrict__ k_new, const 
   }
 }
 
+static int merge_splits(const float* part, __nv_bfloat16* o, int rows, int splits, int D, const __nv_bfloat16* gate, long long ldg, int Hq, int vdim,
+                        cudaStream_t st) {
+  const int mb = (rows + 3) / 4;
+  if (D == 64) LT_RETURN_IF_CUDA(launch_chained(paged_decode_merge_kernel<64>, mb, 128, 0, st, part, o, rows, splits, gate, ldg, Hq, vdim));
+  else LT_RETURN_IF_CUDA(launch_chained(paged_decode_merge_kernel<128>, mb, 128, 0, st, part, o, rows, splits, gate, ldg, Hq, vdim));
+  return 0;
+}
+
 }  // namespace lt
 
 extern "C" {
@@ -987,16 +1168,16 @@ int lt_paged_decode_window(const void* q, const void* k_cache, const void* v_cac
     int* status = device_status_word();
     static OncePerDevice configured_mma;
     if (configured_mma.pending()) {
-      LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_f8_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdF8Cfg<64>::kSmemBytes));
-      LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_f8_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdF8Cfg<128>::kSmemBytes));
-      LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdMmaCfg<64>::kSmemBytes));
-      LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdMmaCfg<128>::kSmemBytes));
+      LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_f8_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdF8Cfg<64>::kSmemBytes));
+      LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_f8_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdF8Cfg<128>::kSmemBytes));
+      LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_mma_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdMmaCfg<64>::kSmemBytes));
+      LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_mma_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdMmaCfg<128>::kSmemBytes));
       configured_mma.finish();
     }
-    if (kv_fp8 && D == 64) LT_RETURN_IF_CUDA(launch_chained(paged_decode_f8_kernel<64>, ctas, kPdWarps * 32, PdF8Cfg<64>::kSmemBytes, st, tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale * k_scale, v_scale, window, status));
-    else if (kv_fp8) LT_RETURN_IF_CUDA(launch_chained(paged_decode_f8_kernel<128>, ctas, kPdWarps * 32, PdF8Cfg<128>::kSmemBytes, st, tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale * k_scale, v_scale, window, status));
-    else if (D == 64) LT_RETURN_IF_CUDA(launch_chained(paged_decode_mma_kernel<64>, ctas, kPdWarps * 32, PdMmaCfg<64>::kSmemBytes, st, tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale, window, status));
-    else LT_RETURN_IF_CUDA(launch_chained(paged_decode_mma_kernel<128>, ctas, kPdWarps * 32, PdMmaCfg<128>::kSmemBytes, st, tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale, window, status));
+    if (kv_fp8 && D == 64) LT_RETURN_IF_CUDA(launch_chained(paged_decode_f8_kernel<64, false>, ctas, kPdWarps * 32, PdF8Cfg<64>::kSmemBytes, st, tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale * k_scale, v_scale, window, status, PdStep{}));
+    else if (kv_fp8) LT_RETURN_IF_CUDA(launch_chained(paged_decode_f8_kernel<128, false>, ctas, kPdWarps * 32, PdF8Cfg<128>::kSmemBytes, st, tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale * k_scale, v_scale, window, status, PdStep{}));
+    else if (D == 64) LT_RETURN_IF_CUDA(launch_chained(paged_decode_mma_kernel<64, false>, ctas, kPdWarps * 32, PdMmaCfg<64>::kSmemBytes, st, tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale, window, status, PdStep{}));
+    else LT_RETURN_IF_CUDA(launch_chained(paged_decode_mma_kernel<128, false>, ctas, kPdWarps * 32, PdMmaCfg<128>::kSmemBytes, st, tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale, window, status, PdStep{}));
   } else if (!kv_fp8 && window == 0 && G <= kPdMaxG && bs_ok && (reinterpret_cast<uintptr_t>(k_cache) & 15) == 0 && (reinterpret_cast<uintptr_t>(v_cache) & 15) == 0) {
     // bf16 caches: every K / V byte is read once for the whole group of query heads, through a shared-memory pipeline
     const int ctas = S * Hkv * splits;
@@ -1015,14 +1196,73 @@ int lt_paged_decode_window(const void* q, const void* k_cache, const void* v_cac
   else { if (kv_fp8) LT_PD(128, true); else LT_PD(128, false); }
 #undef LT_PD
   LT_LAUNCH_CHECK();
-  const int rows = S * Hq;
-  const int mb = (rows + 3) / 4;
-  auto O = static_cast<__nv_bfloat16*>(o);
-  auto GT = static_cast<const __nv_bfloat16*>(gate);
-  if (D == 64) LT_RETURN_IF_CUDA(launch_chained(paged_decode_merge_kernel<64>, mb, 128, 0, st, part, O, rows, splits, GT, ldg, Hq, vdim));
-  else LT_RETURN_IF_CUDA(launch_chained(paged_decode_merge_kernel<128>, mb, 128, 0, st, part, O, rows, splits, GT, ldg, Hq, vdim));
-  LT_LAUNCH_CHECK();
-  return 0;
+  return merge_splits(part, static_cast<__nv_bfloat16*>(o), S * Hq, splits, D, static_cast<const __nv_bfloat16*>(gate), ldg, Hq, vdim, st);
+}
+
+// One decode step's attention (see PdStep): qkv [S, ld] bf16 rows [q | k | v], the newest token of every sequence, which is the last of its context;
+// o [S, Hq, D].  part: scratch [S, Hq, splits, D + 2] fp32, or nullptr: the splits, at most 16, are a cluster.  early: block tables, lengths and every cached row but the newest were complete before the kernels in
+// front of this one that may still run.  Caches as in lt_paged_decode, in blocks of 8, 16 or a multiple of 32 keys.
+int lt_paged_decode_step(const void* qkv, long long ld, const float* cos_t, const float* sin_t, const int* pos, const int* slots, void* k_cache, void* v_cache,
+                         const int* block_tables, const int* context_lens, float* part, void* o, int S, int Hq, int Hkv, int D, int block_size,
+                         int max_blocks, int num_blocks, int splits, float scale, int kv_fp8, float k_scale, float v_scale, int early, void* stream) {
+  using namespace lt;
+  if ((D != 64 && D != 128) || Hkv < 1 || Hq % Hkv != 0 || Hq / Hkv > kPdMmaMaxG || splits < 1 || (!part && splits > kPdMaxCluster) || (ld & 7) || num_blocks < 1 ||
+      block_size < 8 || !(32 % block_size == 0 || block_size % 32 == 0) || (long long)num_blocks * Hkv * block_size >= (1ll << 31))
+    return -int(kStatusBadArgument);
+  for (const void* p : {qkv, static_cast<const void*>(cos_t), static_cast<const void*>(sin_t), static_cast<const void*>(k_cache), static_cast<const void*>(v_cache)})
+    if (!p || (reinterpret_cast<uintptr_t>(p) & 15)) return -int(kStatusBadArgument);
+  if (S == 0) return 0;
+  const uint64_t rows = uint64_t(num_blocks) * Hkv * block_size;
+  const uint32_t run = block_size < 32 ? block_size : 32;
+  const int bytes = kv_fp8 ? 1 : 2;
+  CUtensorMap tmK, tmV;
+  int r = encode_tmap_2d(&tmK, k_cache, bytes, D, rows, uint64_t(D) * bytes, kv_fp8 ? D : 64, run, !kv_fp8 || D == 128);
+  if (r == 0) r = encode_tmap_2d(&tmV, v_cache, bytes, D, rows, uint64_t(D) * bytes, kv_fp8 ? D : 64, run, !kv_fp8 || D == 128);
+  if (r) return r > 0 ? 1000 + r : r;
+  static OncePerDevice configured;
+  if (configured.pending()) {
+    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_f8_kernel<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdF8Cfg<64>::kSmemBytes));
+    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_f8_kernel<64, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_f8_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdF8Cfg<128>::kSmemBytes));
+    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_f8_kernel<128, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_mma_kernel<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdMmaCfg<64>::kSmemBytes));
+    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_mma_kernel<64, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_mma_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdMmaCfg<128>::kSmemBytes));
+    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_mma_kernel<128, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    configured.finish();
+  }
+  const PdStep step{static_cast<const __nv_bfloat16*>(qkv), ld, cos_t, sin_t, pos, slots, k_cache, v_cache, kv_fp8 ? 1.f / k_scale : 1.f, kv_fp8 ? 1.f / v_scale : 1.f,
+                    static_cast<__nv_bfloat16*>(o), early};
+  const __nv_bfloat16* none = nullptr;
+  int* status = device_status_word();
+  cudaLaunchAttribute attr[2]{};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = part ? 1 : splits;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(S * Hkv * splits);
+  cfg.blockDim = dim3(kPdWarps * 32);
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cfg.attrs = attr;
+  cfg.numAttrs = part ? 1 : 2;
+#define LT_PD_F8(DD)                                                                                                                            \
+  cfg.dynamicSmemBytes = PdF8Cfg<DD>::kSmemBytes;                                                                                              \
+  LT_RETURN_IF_CUDA(cudaLaunchKernelEx(&cfg, paged_decode_f8_kernel<DD, true>, tmK, tmV, none, block_tables, context_lens, part, S, Hq, Hkv, block_size, \
+                                       max_blocks, splits, scale * k_scale, v_scale, 0, status, step))
+#define LT_PD_MMA(DD)                                                                                                                           \
+  cfg.dynamicSmemBytes = PdMmaCfg<DD>::kSmemBytes;                                                                                             \
+  LT_RETURN_IF_CUDA(cudaLaunchKernelEx(&cfg, paged_decode_mma_kernel<DD, true>, tmK, tmV, none, block_tables, context_lens, part, S, Hq, Hkv, block_size, \
+                                       max_blocks, splits, scale, 0, status, step))
+  if (kv_fp8) {
+    if (D == 64) { LT_PD_F8(64); } else { LT_PD_F8(128); }
+  } else {
+    if (D == 64) { LT_PD_MMA(64); } else { LT_PD_MMA(128); }
+  }
+#undef LT_PD_F8
+#undef LT_PD_MMA
+  return part ? merge_splits(part, static_cast<__nv_bfloat16*>(o), S * Hq, splits, D, nullptr, 0, Hq, D, cfg.stream) : 0;
 }
 
 int lt_kv_append(const void* k_new, const void* v_new, void* k_cache, void* v_cache, const int* slots, long long n_tok, int Hkv,

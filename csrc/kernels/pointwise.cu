@@ -472,7 +472,8 @@ int lt_embedding_fwd(const long long* idx, const void* table, void* out, long lo
   using namespace lt;
   if (D % 8 != 0) return -int(kStatusBadArgument);
   if (n_tok == 0) return 0;
-  LT_RETURN_IF_CUDA(launch_chained(embedding_fwd_kernel, grid_for(n_tok * (D / 8), 256), 256, 0, static_cast<cudaStream_t>(stream), idx, static_cast<const __nv_bfloat16*>(table), static_cast<__nv_bfloat16*>(out), n_tok, D, V));
+  // (a full stop: what was launched before it is complete, and the kernels of a step behind it count on that for its tables)
+  embedding_fwd_kernel<<<grid_for(n_tok * (D / 8), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(idx, static_cast<const __nv_bfloat16*>(table), static_cast<__nv_bfloat16*>(out), n_tok, D, V);
   LT_LAUNCH_CHECK();
   return 0;
 }

@@ -45,21 +45,15 @@ class LlamaKVModel(ServingModel):
             self._index = PrefixCache()
 
     # ------------------------------------------------------------------ shared layer body
-    def _layers(self, x, positions, slots, attend, in_place: bool):
-        """attend(i, q, k, v) of rotated queries; k and v are those of the rows, rotated only if `in_place`: a pass that reads the cache
-        alone has its queries packed instead."""
+    def _layers(self, x, attend):
+        """attend(i, qkv) of a layer's unrotated rows [q | k | v] writes their keys and values to the cache; its result joins x."""
         e, cfg, w, K = self.e, self.e.cfg, self.e.w, self.e.K
-        Hq, Hkv, hd = cfg.n_heads, cfg.n_kv_heads, cfg.head_dim
         n = x.shape[0]
         for i in range(cfg.n_layers):
             p = "layers.%d." % i
             qkv = K.product_of_constants(x, w.p(p + "wqkv"), norm=(w.p(p + "attn_norm"), cfg.rms_eps))
-            q = K.rope_append(qkv, e.cos, e.sin, positions, slots, Hq, Hkv, hd, self.cache.k[i], self.cache.v[i], self.block_size, self.cache.fp8,
-                              self.cache.k_scale, self.cache.v_scale, in_place=in_place)
-            k = qkv[:, Hq * hd:(Hq + Hkv) * hd].view(n, Hkv, hd)
-            v = qkv[:, (Hq + Hkv) * hd:].view(n, Hkv, hd)
-            o = attend(i, q, k, v)
-            x1 = K.product_of_constants(o.reshape(n, Hq * hd), w.p(p + "wo"), residual=x)
+            o = attend(i, qkv)
+            x1 = K.product_of_constants(o.reshape(n, -1), w.p(p + "wo"), residual=x)
             hm = K.product_of_constants(x1, w.p(p + "w_gu"), act="silu", norm=(w.p(p + "mlp_norm"), cfg.rms_eps))
             x = K.product_of_constants(hm, w.p(p + "w_down"), residual=x1)
         return x
@@ -154,12 +148,18 @@ class LlamaKVModel(ServingModel):
         nb = (start + n + bs - 1) // bs
         blocks = torch.tensor(list(block_ids[:nb]), dtype=torch.int64, device=dev) if start > 0 else None
 
-        def attend(i, q, k, v):
+        Hq, Hkv, hd = e.cfg.n_heads, e.cfg.n_kv_heads, e.cfg.head_dim
+
+        def attend(i, qkv):
+            # a first portion attends to its own rows, rotated in place; a later one to the cache, for which its queries are packed
+            q = K.rope_append(qkv, e.cos, e.sin, pos, slots, Hq, Hkv, hd, self.cache.k[i], self.cache.v[i], bs, self.cache.fp8, self.cache.k_scale,
+                              self.cache.v_scale, in_place=start == 0)
+            k = qkv[:, Hq * hd:(Hq + Hkv) * hd].view(n, Hkv, hd)
+            v = qkv[:, (Hq + Hkv) * hd:(Hq + 2 * Hkv) * hd].view(n, Hkv, hd)
             if start == 0:
                 o, _ = K.flash_fwd(q.unsqueeze(0), k.unsqueeze(0), v.unsqueeze(0), causal=True)
                 return o[0]
             # later chunk: keys and values of the whole context so far, read back from the sequence's blocks
-            Hkv, hd = k.shape[1], k.shape[2]
             kc = self.cache.k[i][blocks].permute(0, 2, 1, 3).reshape(nb * bs, Hkv, hd)[:start + n]
             vc = self.cache.v[i][blocks].permute(0, 2, 1, 3).reshape(nb * bs, Hkv, hd)[:start + n]
             if self.cache.fp8:
@@ -169,20 +169,17 @@ class LlamaKVModel(ServingModel):
             o, _ = K.flash_fwd(q.unsqueeze(0), kc.contiguous().unsqueeze(0), vc.contiguous().unsqueeze(0), causal=True)
             return o[0]
 
-        return self._layers(K.embedding_fwd(tok, e.w.p("embed")), pos, slots, attend, start == 0)
+        return self._layers(K.embedding_fwd(tok, e.w.p("embed")), attend)
 
     # ------------------------------------------------------------------ one token for every running sequence
     def _decode_hidden(self, d: torch.Tensor, S: int, width: int) -> torch.Tensor:
-        from ..serving import paged_attention
         e, K = self.e, self.e.K
-        bs = self.block_size
+        cfg, c, bs = e.cfg, self.cache, self.block_size
         tok = d[0]
         pos, slots, ctx = d[1].to(torch.int32), d[2].to(torch.int32), d[3].to(torch.int32)
         bt = d[5:].t().contiguous().to(torch.int32)
-        splits = self.num_splits or self._splits_for(S * e.cfg.n_kv_heads, width * bs)
 
-        def attend(i, q, k, v):
-            return paged_attention(q, self.cache.k[i], self.cache.v[i], bt, ctx, bs, num_splits=splits,
-                                   k_scale=self.cache.k_scale, v_scale=self.cache.v_scale)
+        def attend(i, qkv):
+            return K.decode_step(qkv, e.cos, e.sin, pos, slots, cfg.n_heads, cfg.n_kv_heads, cfg.head_dim, c.k[i], c.v[i], bt, ctx, bs, self.num_splits, c.k_scale, c.v_scale)
 
-        return self._layers(K.embedding_fwd(tok, e.w.p("embed")), pos, slots, attend, False)
+        return self._layers(K.embedding_fwd(tok, e.w.p("embed")), attend)

@@ -113,6 +113,7 @@ _SIGS = {
     "lt_gather_shards": [_vp, _i, _vp, _vp, _i, _i, _vp],
     "lt_gemm_num_tiles": [_i, _i, _i],
     "lt_paged_decode": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _f, _f, _vp],
+    "lt_paged_decode_step": [_vp, _ll] + [_vp] * 10 + [_i] * 8 + [_f, _i, _f, _f, _i, _vp],
     "lt_kv_append": [_vp, _vp, _vp, _vp, _vp, _ll, _i, _i, _i, _i, _f, _f, _vp],
     "lt_gemm_rs_bf16": [_vp, _vp, _i, _i, _i, _ll, _ll, _i, _vp, _vp, ctypes.c_uint, _i, _i, _i, _vp, _ll, _vp, _vp, _ll, _vp],
     "lt_flash_fwd": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _f, _i, _vp],
@@ -841,6 +842,59 @@ def paged_decode(q, k_cache, v_cache, block_tables, context_lens, block_size: in
                                        int(window), _p(gate), gate.stride(0) if gate is not None else 0, vdim, _stream())
     _check(rc, "lt_paged_decode_window")
     return o
+
+
+def _decode_splits(pairs: int, keys: int, head_dim: int, fp8: bool):
+    """(how the splits of a (sequence, KV head) meet, how many there are) for a decode step's attention over contexts of up to `keys`:
+
+    cluster  they merge in a cluster, as many as fill the SMs once (a cluster wants its places together: nine tenths of them); a second round
+             is weighed against shorter splits.  Four layers of a model (us; separate launches / their splits in one launch with a merge
+             kernel / clusters of 2, 4, 8): 1.1b 16 x 2000 234 / 225 / 229, 209, 245; 8b 8 x 9000 on 8 bits 642 / 645 / 808, 606, 630; 8b 3 x 3000
+             454 / 452 / 473, 433, 452 (of 5: 425); 8b 16 x 2000 568 / 572 / 535, 584, 709 (of 1: 522).
+    part     a few long sequences: more splits than a cluster holds, and a merge kernel: 1.1b 1 x 16384 229 / 216 / 542, 368, 276; of 16 (which only
+             heads of 64 find places for) 230, but with 4096 keys 193 against 196.
+    parts    more pairs than places: queries rotated once a launch are cheaper than in every CTA: 8b 32 x 4096 859 / 869 / 873, 994."""
+    a_sm = (3 if head_dim == 64 else 2) if fp8 else (2 if head_dim == 64 else 1)      # CTAs, by shared memory
+    places = sm_count() * a_sm * 9 // 10
+    many = max(1, min(32, keys // 256, (sm_count() * 4 + pairs - 1) // pairs))
+    if pairs <= 8 and many > 8:
+        return ("cluster", 16) if head_dim == 64 and keys <= 8192 else ("part", many)
+    if pairs > places:
+        return "parts", many
+    return "cluster", min(range(1, max(1, min(8, keys // 128)) + 1), key=lambda n: (-(-pairs * n // places) / n, n))
+
+
+def decode_step(qkv, cos, sin, positions, slots, heads: int, kv_heads: int, head_dim: int, k_cache, v_cache, block_tables, context_lens, block_size: int,
+                splits: int = 0, k_scale: float = 1.0, v_scale: float = 1.0):
+    """Attention of a decode step from the rows [q | k | v] of its product: queries and keys are rotated, the newest keys and values cached, and every
+    sequence attends to its context, whose last token is the row's.  Returns [S, heads, head_dim].  Block tables, lengths and the cached rows
+    before were complete when the step's embedding was launched.  positions, slots, context_lens [S], block_tables [S, width]: int32.
+
+    splits: how many the keys of a (sequence, KV head) are cut into (0: by size).  One launch, or two; caches that it does not take and large
+    batches go through rope_append and paged_decode."""
+    S, D = qkv.shape[0], head_dim
+    fp8 = k_cache.dtype == torch.float8_e4m3fn
+    how = "part"
+    if splits <= 0:
+        how, splits = _decode_splits(max(1, S * kv_heads), block_tables.shape[1] * block_size, D, fp8)
+    if (how != "parts" and qkv.dtype == torch.bfloat16 and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0 and D in (64, 128) and heads % kv_heads == 0 and heads // kv_heads <= 16
+            and block_size % 8 == 0 and (32 % block_size == 0 or block_size % 32 == 0) and k_cache.is_contiguous() and v_cache.is_contiguous()
+            and _aligned(qkv, cos, sin, k_cache, v_cache)):
+        assert qkv.dim() == 2 and qkv.shape[1] >= (heads + 2 * kv_heads) * D and k_cache.dtype == v_cache.dtype and (fp8 or k_cache.dtype == torch.bfloat16)
+        assert all(t.dtype == torch.int32 and t.is_contiguous() for t in (positions, slots, context_lens, block_tables))
+        assert positions.numel() == slots.numel() == context_lens.numel() == block_tables.shape[0] == S
+        assert all(t.dtype == torch.float32 and t.is_contiguous() and t.shape[-1] == D // 2 for t in (cos, sin))
+        assert all(t.shape[1:] == (kv_heads, block_size, D) for t in (k_cache, v_cache)) and k_cache.shape[0] == v_cache.shape[0]
+        part = torch.empty((S, heads, splits, D + 2), dtype=torch.float32, device=qkv.device) if how == "part" and splits > 1 else None
+        o = torch.empty((S, heads, D), dtype=qkv.dtype, device=qkv.device)
+        rc = _fn("lt_paged_decode_step")(qkv.data_ptr(), qkv.stride(0), cos.data_ptr(), sin.data_ptr(), positions.data_ptr(), slots.data_ptr(),
+                                         k_cache.data_ptr(), v_cache.data_ptr(), block_tables.data_ptr(), context_lens.data_ptr(), _p(part), o.data_ptr(), S, heads,
+                                         kv_heads, D, block_size, block_tables.shape[1], k_cache.shape[0], splits, float(D ** -0.5),
+                                         1 if fp8 else 0, float(k_scale), float(v_scale), 1, _stream())
+        _check(rc, "lt_paged_decode_step")
+        return o
+    q = rope_append(qkv, cos, sin, positions, slots, heads, kv_heads, D, k_cache, v_cache, block_size, fp8, k_scale, v_scale)
+    return paged_decode(q, k_cache, v_cache, block_tables, context_lens, block_size, splits, D ** -0.5, k_scale, v_scale)
 
 
 def kv_append(k_new, v_new, k_cache, v_cache, slots, block_size: int, fp8: bool, k_scale: float = 1.0, v_scale: float = 1.0):

@@ -140,6 +140,14 @@ def rope_append(qkv, cos, sin, positions, slots, heads, kv_heads, head_dim, k_ca
     return x[:, :heads * D].unflatten(1, (heads, D))
 
 
+def decode_step(qkv, cos, sin, positions, slots, heads, kv_heads, head_dim, k_cache, v_cache, block_tables, context_lens, block_size, splits=0, k_scale=1.0,
+                v_scale=1.0):
+    from ..serving import paged_attention
+    q = rope_append(qkv, cos, sin, positions, slots, heads, kv_heads, head_dim, k_cache, v_cache, block_size, k_cache.dtype == torch.float8_e4m3fn, k_scale,
+                    v_scale)
+    return paged_attention(q, k_cache, v_cache, block_tables, context_lens, block_size, num_splits=splits, k_scale=k_scale, v_scale=v_scale)
+
+
 def swiglu_fwd(gu):
     F = gu.shape[1] // 2
     g, u = gu[:, :F].float(), gu[:, F:].float()

@@ -1,0 +1,98 @@
+"""Attention of a decode step in one launch (rotation, cache write, splits merged in a cluster) against the launches it stands in for and against 64 bits."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(S, G, Hkv, D, bs, longest, fp8, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    H = G * Hkv
+    ctx = [longest] + [1 + (longest - 1) * (37 * s % 101) // 101 for s in range(1, S)]
+    width = (longest + bs - 1) // bs + 1
+    order = torch.randperm(S * width + 3, generator=torch.Generator().manual_seed(seed)).tolist()
+    bt = torch.tensor(order[:S * width], dtype=torch.int32).view(S, width)
+    dt = torch.float8_e4m3fn if fp8 else torch.bfloat16
+    kc, vc = (torch.randn(S * width + 3, Hkv, bs, D, device="cuda", generator=g).bfloat16().to(dt) for _ in range(2))
+    pos = torch.tensor([c - 1 for c in ctx], dtype=torch.int32)
+    slots = torch.tensor([int(bt[s, (c - 1) // bs]) * bs + (c - 1) % bs for s, c in enumerate(ctx)], dtype=torch.int32)
+    qkv = torch.randn(S, (H + 2 * Hkv) * D + 8, device="cuda", generator=g).bfloat16()[:, :(H + 2 * Hkv) * D]
+    ang = torch.arange(longest + 1, device="cuda", dtype=torch.float64)[:, None] * 1e4 ** (-torch.arange(0, D, 2, device="cuda", dtype=torch.float64) / D)[None]
+    return qkv, ang.cos().float().contiguous(), ang.sin().float().contiguous(), pos.cuda(), slots.cuda(), kc, vc, bt.cuda(), torch.tensor(ctx, dtype=torch.int32).cuda(), ctx
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("S,G,Hkv,D,bs", [(1, 8, 4, 64, 16), (3, 4, 2, 128, 16), (5, 1, 3, 64, 8), (2, 16, 1, 128, 32), (4, 9, 2, 64, 64)])
+@pytest.mark.parametrize("longest,splits", [(1, 1), (2, 8), (31, 1), (32, 2), (33, 3), (128, 1), (129, 4), (700, 8), (1500, 5), (3000, 32), (300, 0), (3000, 0), (4500, 0)])
+def test_step_against_its_parts(S, G, Hkv, D, bs, longest, splits, fp8):
+    from litetorch_b200.ops import kernels as K
+    H = G * Hkv
+    qkv, cos, sin, pos, slots, kc, vc, bt, ctx, lens = _case(S, G, Hkv, D, bs, longest, fp8, longest + S)
+    ks, vs = (0.5, 2.0) if fp8 else (1.0, 1.0)
+    k1, v1, k2, v2 = kc.clone(), vc.clone(), kc.clone(), vc.clone()
+    keep = qkv.clone()
+    o = K.decode_step(qkv, cos, sin, pos, slots, H, Hkv, D, k1, v1, bt, ctx, bs, splits, ks, vs)
+    assert torch.equal(qkv, keep)
+    q = K.rope_append(qkv, cos, sin, pos, slots, H, Hkv, D, k2, v2, bs, fp8, ks, vs)
+    want = K.paged_decode(q, k2, v2, bt, ctx, bs, max(1, splits), D ** -0.5, ks, vs)
+    bits = torch.uint8 if fp8 else torch.int16
+    assert torch.equal(k1.view(bits), k2.view(bits)) and torch.equal(v1.view(bits), v2.view(bits))
+    assert ((o.float() - want.float()).abs() <= want.float().abs() * 2.0 ** -7 + 2e-3).all()
+    # 64 bits, from the rotated queries and the caches
+    for s, n in enumerate(lens):
+        at = bt[s].long()[torch.arange(n, device="cuda") // bs], torch.arange(n, device="cuda") % bs
+        kk, vv = (t[at[0], :, at[1]].double() * f for t, f in ((k1, ks), (v1, vs)))                    # [n, Hkv, D]
+        p = torch.softmax(torch.einsum("hgd,nhd->hgn", q[s].double().view(Hkv, G, D), kk) * D ** -0.5, -1)
+        ref = torch.einsum("hgn,nhd->hgd", p, vv).reshape(H, D)
+        # a rounding of the result; of the 16-bit kernel's weights too, each within 2^-9 of itself
+        size = torch.einsum("hgn,nhd->hgd", p, vv.abs()).reshape(H, D)
+        assert ((o[s].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + size * 2.0 ** -8 + 1e-4).all()
+    assert K.status_fetch() == 0
+
+
+def test_splits_by_size():
+    from litetorch_b200.ops import kernels as K
+    sms = K.sm_count()
+    seen = set()
+    for pairs in (1, 4, 8, 9, 24, 64, 96, 128, 256, 512):
+        for keys in (16, 300, 1000, 4096, 16384):
+            for D in (64, 128):
+                for fp8 in (False, True):
+                    how, n = K._decode_splits(pairs, keys, D, fp8)
+                    seen.add(how)
+                    assert n >= 1 and (how != "cluster" or n <= 16) and (n == 1 or keys // n >= 100)
+                    assert how != "cluster" or n == 1 or n <= 8 or (D == 64 and pairs * n <= sms)
+    assert seen == {"cluster", "part", "parts"}
+
+
+def test_tokens_without_a_slot_and_caches_it_does_not_take():
+    from litetorch_b200.ops import kernels as K
+    qkv, cos, sin, pos, slots, kc, vc, bt, ctx, lens = _case(4, 4, 2, 64, 16, 200, False, 1)
+    none = slots.clone()
+    none[1:] = -1
+    k1, v1, k2, v2 = kc.clone(), vc.clone(), kc.clone(), vc.clone()
+    a = K.decode_step(qkv, cos, sin, pos, slots, 8, 2, 64, k1, v1, bt, ctx, 16, 4)
+    b = K.decode_step(qkv, cos, sin, pos, none, 8, 2, 64, k2, v2, bt, ctx, 16, 4)
+    assert torch.equal(a, b)                        # the newest row comes from the product, not from the cache
+    assert torch.equal(k2[[i for i in range(k2.shape[0]) if i != int(slots[0]) // 16]], kc[[i for i in range(k2.shape[0]) if i != int(slots[0]) // 16]])
+    # blocks of four keys go through the parts
+    qkv, cos, sin, pos, slots, kc, vc, bt, ctx, lens = _case(4, 4, 2, 64, 4, 200, False, 1)
+    k1, v1, k2, v2 = kc.clone(), vc.clone(), kc.clone(), vc.clone()
+    a = K.decode_step(qkv, cos, sin, pos, slots, 8, 2, 64, k1, v1, bt, ctx, 4, 3)
+    b = K.paged_decode(K.rope_append(qkv, cos, sin, pos, slots, 8, 2, 64, k2, v2, 4, False), k2, v2, bt, ctx, 4, 3, 64 ** -0.5)
+    assert torch.equal(a, b) and torch.equal(k1.view(torch.int16), k2.view(torch.int16))
+    assert K.status_fetch() == 0
+
+
+def test_not_a_number_past_the_context():
+    """What lies in a block past the newest row, and in the newest row's place, is not seen."""
+    from litetorch_b200.ops import kernels as K
+    qkv, cos, sin, pos, slots, kc, vc, bt, ctx, lens = _case(3, 4, 2, 128, 16, 45, False, 7)
+    a = K.decode_step(qkv, cos, sin, pos, slots, 8, 2, 128, kc.clone(), vc.clone(), bt, ctx, 16, 2)
+    for s, n in enumerate(lens):
+        for t in (kc, vc):
+            t[int(bt[s, (n - 1) // 16]), :, (n - 1) % 16:] = math.nan
+    b = K.decode_step(qkv, cos, sin, pos, slots, 8, 2, 128, kc, vc, bt, ctx, 16, 2)
+    assert torch.equal(a, b) and bool(torch.isfinite(b.float()).all())
