@@ -289,6 +289,8 @@ int lt_gelu_fwd(const void* x, void* y, long long n, void* stream);
 int lt_gelu_bwd(const void* x, const void* dy, void* dx, long long n, void* stream);
 int lt_axpby(const void* a, const void* b, void* out, float alpha, float beta, long long n, void* stream);
 int lt_embedding_fwd(const long long* idx, const void* table, void* out, long long n_tok, int D, int V, void* stream);
+int lt_embedding_fwd_idx(const void* idx, int idx32, const void* table, void* out, long long n_tok, int D, int V, void* stream);
+int lt_argmax_rows(const void* x, int fp32, long long* out, int rows, int V, long long ld, void* stream);
 int lt_embedding_bwd(const long long* idx, const void* dout, void* dtable, long long n_tok, int D, int V, void* stream);
 int lt_cast_f32_to_bf16(const float* in, void* out, long long n, void* stream);
 int lt_cast_bf16_to_f32(const void* in, float* out, long long n, void* stream);

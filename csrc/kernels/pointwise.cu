@@ -277,8 +277,93 @@ __global__ void axpby_kernel(const __nv_bfloat16* a, const __nv_bfloat16* b, __n
   }
 }
 
+// ---------------------------------------------------------------------------------------------- cached rows
+// Rows [pos0, pos0 + n) of one sequence out of its blocks into [n, G, D] arrays.
+__global__ void kv_gather_kernel(const uint4* __restrict__ k_cache, const uint4* __restrict__ v_cache, uint4* __restrict__ k_lin,
+                                 uint4* __restrict__ v_lin, const int* __restrict__ table, int pos0, int G, int ku, int vu,
+                                 int block_size) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int pos = pos0 + blockIdx.x;
+  const long long blk = table[pos / block_size];
+  const int off = pos % block_size;
+  for (int i = threadIdx.x; i < G * (ku + vu); i += blockDim.x) {
+    const bool is_k = i < G * ku;
+    const int j = is_k ? i : i - G * ku, w = is_k ? ku : vu;
+    const int g = j / w, u = j % w;
+    const long long src = ((blk * G + g) * block_size + off) * w + u, dst = ((long long)blockIdx.x * G + g) * w + u;
+    if (is_k) k_lin[dst] = k_cache[src];
+    else v_lin[dst] = v_cache[src];
+  }
+}
+
+// ---------------------------------------------------------------------------------------------- greedy tokens
+// Whether a at index i goes before b at j as the largest of a row: a NaN is the largest, of equals the first.
+template <typename T>
+__device__ __forceinline__ bool goes_before(T a, int i, T b, int j) {
+  const bool na = a != a, nb = b != b;
+  if (na || nb) return na && (!nb || i < j);
+  return a > b || (a == b && i < j);
+}
+// Index of the largest element of every row, a CTA a row.  (A conversion to fp32 and a library reduction took 13 us of a decode step; 16 rows of
+// 32000 here 4.)
+template <bool F32>
+__global__ void __launch_bounds__(1024) argmax_rows_kernel(const void* __restrict__ x, long long* __restrict__ out, int V, long long ld) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ float bv[32];
+  __shared__ int bi[32];
+  const long long row = blockIdx.x;
+  float best = -INFINITY;
+  int at = V;
+  auto take = [&](float v, int i) { if (goes_before(v, i, best, at)) { best = v; at = i; } };
+  if (F32) {
+    const float* r = static_cast<const float*>(x) + row * ld;
+    if ((reinterpret_cast<uintptr_t>(r) & 15) == 0) {
+      for (int c = threadIdx.x * 4; c + 3 < V; c += 4096) {
+        const float4 f = *reinterpret_cast<const float4*>(r + c);
+        take(f.x, c); take(f.y, c + 1); take(f.z, c + 2); take(f.w, c + 3);
+      }
+      for (int c = V / 4 * 4 + threadIdx.x; c < V; c += 1024) take(r[c], c);
+    } else {
+      for (int c = threadIdx.x; c < V; c += 1024) take(r[c], c);
+    }
+  } else {
+    const __nv_bfloat16* r = static_cast<const __nv_bfloat16*>(x) + row * ld;
+    if ((reinterpret_cast<uintptr_t>(r) & 15) == 0) {
+      for (int c = threadIdx.x * 8; c + 7 < V; c += 8192) {
+        float f[8];
+        ld8(r + c, f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) take(f[j], c + j);
+      }
+      for (int c = V / 8 * 8 + threadIdx.x; c < V; c += 1024) take(__bfloat162float(r[c]), c);
+    } else {
+      for (int c = threadIdx.x; c < V; c += 1024) take(__bfloat162float(r[c]), c);
+    }
+  }
+  auto reduce = [&]() {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float v = __shfl_xor_sync(0xffffffffu, best, o);
+      const int i = __shfl_xor_sync(0xffffffffu, at, o);
+      take(v, i);
+    }
+  };
+  reduce();
+  if ((threadIdx.x & 31) == 0) { bv[threadIdx.x >> 5] = best; bi[threadIdx.x >> 5] = at; }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    best = bv[threadIdx.x];
+    at = bi[threadIdx.x];
+    reduce();
+    if (threadIdx.x == 0) out[row] = at < V ? at : 0;
+  }
+}
+
 // ---------------------------------------------------------------------------------------------- embedding
-__global__ void embedding_fwd_kernel(const long long* __restrict__ idx, const __nv_bfloat16* __restrict__ table,
+template <typename IDX>
+__global__ void embedding_fwd_kernel(const IDX* __restrict__ idx, const __nv_bfloat16* __restrict__ table,
                                      __nv_bfloat16* __restrict__ out, long long n_tok, int D, int V) {
   pdl_launch_dependents();
   pdl_wait();
@@ -469,12 +554,43 @@ int lt_axpby(const void* a, const void* b, void* out, float alpha, float beta, l
   return 0;
 }
 int lt_embedding_fwd(const long long* idx, const void* table, void* out, long long n_tok, int D, int V, void* stream) {
+  return lt_embedding_fwd_idx(idx, 0, table, out, n_tok, D, V, stream);
+}
+// idx32: the tokens are 32-bit.
+int lt_embedding_fwd_idx(const void* idx, int idx32, const void* table, void* out, long long n_tok, int D, int V, void* stream) {
   using namespace lt;
   if (D % 8 != 0) return -int(kStatusBadArgument);
   if (n_tok == 0) return 0;
   // (a full stop: what was launched before it is complete, and the kernels of a step behind it count on that for its tables)
-  embedding_fwd_kernel<<<grid_for(n_tok * (D / 8), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(idx, static_cast<const __nv_bfloat16*>(table), static_cast<__nv_bfloat16*>(out), n_tok, D, V);
+  auto tb = static_cast<const __nv_bfloat16*>(table);
+  auto to = static_cast<__nv_bfloat16*>(out);
+  const int grid = grid_for(n_tok * (D / 8), 256);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (idx32) embedding_fwd_kernel<int><<<grid, 256, 0, st>>>(static_cast<const int*>(idx), tb, to, n_tok, D, V);
+  else embedding_fwd_kernel<long long><<<grid, 256, 0, st>>>(static_cast<const long long*>(idx), tb, to, n_tok, D, V);
   LT_LAUNCH_CHECK();
+  return 0;
+}
+// Head sizes here are bytes of one (token, head) row; multiples of 16.
+int lt_kv_gather(const void* k_cache, const void* v_cache, void* k_lin, void* v_lin, const int* table, int pos0, int n, int G,
+                 int k_bytes, int v_bytes, int block_size, void* stream) {
+  using namespace lt;
+  if (n <= 0) return 0;
+  if ((k_bytes & 15) || (v_bytes & 15)) return -4;
+  LT_RETURN_IF_CUDA(launch_chained(kv_gather_kernel, n, 128, 0, static_cast<cudaStream_t>(stream), static_cast<const uint4*>(k_cache),
+                                   static_cast<const uint4*>(v_cache), static_cast<uint4*>(k_lin), static_cast<uint4*>(v_lin), table, pos0, G, k_bytes / 16,
+                                   v_bytes / 16, block_size));
+  return 0;
+}
+
+// out[r] (64-bit) = index of the largest of the V elements of row r (bf16, or fp32) at pitch ld; a NaN is the largest, of equals the first.
+int lt_argmax_rows(const void* x, int fp32, long long* out, int rows, int V, long long ld, void* stream) {
+  using namespace lt;
+  if (rows == 0) return 0;
+  if (V < 1) return -int(kStatusBadArgument);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (fp32) LT_RETURN_IF_CUDA(launch_chained(argmax_rows_kernel<true>, rows, 1024, 0, st, x, out, V, ld));
+  else LT_RETURN_IF_CUDA(launch_chained(argmax_rows_kernel<false>, rows, 1024, 0, st, x, out, V, ld));
   return 0;
 }
 int lt_embedding_bwd(const long long* idx, const void* dout, void* dtable, long long n_tok, int D, int V, void* stream) {

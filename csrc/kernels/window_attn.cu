@@ -113,23 +113,6 @@ __global__ void __launch_bounds__(kQkvThreads) qkv_rope_kernel(const QkvParams p
   }
 }
 
-// Rows [pos0, pos0 + n) of one sequence out of its blocks into [n, G, D] arrays.
-__global__ void kv_gather_kernel(const uint4* __restrict__ k_cache, const uint4* __restrict__ v_cache, uint4* __restrict__ k_lin,
-                                 uint4* __restrict__ v_lin, const int* __restrict__ table, int pos0, int G, int ku, int vu,
-                                 int block_size) {
-  const int pos = pos0 + blockIdx.x;
-  const long long blk = table[pos / block_size];
-  const int off = pos % block_size;
-  for (int i = threadIdx.x; i < G * (ku + vu); i += blockDim.x) {
-    const bool is_k = i < G * ku;
-    const int j = is_k ? i : i - G * ku, w = is_k ? ku : vu;
-    const int g = j / w, u = j % w;
-    const long long src = ((blk * G + g) * block_size + off) * w + u, dst = ((long long)blockIdx.x * G + g) * w + u;
-    if (is_k) k_lin[dst] = k_cache[src];
-    else v_lin[dst] = v_cache[src];
-  }
-}
-
 // One warp per (row, query head): scores of 32 keys at a time (a lane per key), online softmax, value columns over the lanes.
 // Rows are tokens of one sequence (table_stride 0) or one token of every sequence.
 constexpr int kWaWarps = 4;
@@ -244,19 +227,6 @@ int lt_qkv_rope(int fp32, const void* proj, long long ld, int n, int q_off, int 
   auto kern = fp32 ? qkv_rope_kernel<float, 1> : v8 ? qkv_rope_kernel<__nv_bfloat16, 8> : qkv_rope_kernel<__nv_bfloat16, 1>;
   if (smem > 48 * 1024) LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   kern<<<n, kQkvThreads, smem, st>>>(p);
-  LT_LAUNCH_CHECK();
-  return 0;
-}
-
-// Head sizes here are bytes of one (token, head) row; multiples of 16.
-int lt_kv_gather(const void* k_cache, const void* v_cache, void* k_lin, void* v_lin, const int* table, int pos0, int n, int G,
-                 int k_bytes, int v_bytes, int block_size, void* stream) {
-  using namespace lt;
-  if (n <= 0) return 0;
-  if ((k_bytes & 15) || (v_bytes & 15)) return -4;
-  kv_gather_kernel<<<n, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint4*>(k_cache), static_cast<const uint4*>(v_cache), static_cast<uint4*>(k_lin), static_cast<uint4*>(v_lin),
-      table, pos0, G, k_bytes / 16, v_bytes / 16, block_size);
   LT_LAUNCH_CHECK();
   return 0;
 }

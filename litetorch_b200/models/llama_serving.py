@@ -146,7 +146,7 @@ class LlamaKVModel(ServingModel):
         tok, pos, slots = d[0], d[1].to(torch.int32), d[2].to(torch.int32)
         bs = self.block_size
         nb = (start + n + bs - 1) // bs
-        blocks = torch.tensor(list(block_ids[:nb]), dtype=torch.int64, device=dev) if start > 0 else None
+        blocks = torch.tensor(list(block_ids[:nb]), dtype=torch.int32, device=dev) if start > 0 else None
 
         Hq, Hkv, hd = e.cfg.n_heads, e.cfg.n_kv_heads, e.cfg.head_dim
 
@@ -160,13 +160,12 @@ class LlamaKVModel(ServingModel):
                 o, _ = K.flash_fwd(q.unsqueeze(0), k.unsqueeze(0), v.unsqueeze(0), causal=True)
                 return o[0]
             # later chunk: keys and values of the whole context so far, read back from the sequence's blocks
-            kc = self.cache.k[i][blocks].permute(0, 2, 1, 3).reshape(nb * bs, Hkv, hd)[:start + n]
-            vc = self.cache.v[i][blocks].permute(0, 2, 1, 3).reshape(nb * bs, Hkv, hd)[:start + n]
+            kc, vc = torch.empty(2, start + n, Hkv, hd, dtype=self.cache.k[i].dtype, device=dev)
+            K.kv_gather(self.cache.k[i], self.cache.v[i], blocks, 0, start + n, kc, vc)
             if self.cache.fp8:
                 kc = (kc.float() * self.cache.k_scale).to(q.dtype)
                 vc = (vc.float() * self.cache.v_scale).to(q.dtype)
-            # (a single block is not copied by the reshape: its heads lie a block apart, and attention takes them side by side)
-            o, _ = K.flash_fwd(q.unsqueeze(0), kc.contiguous().unsqueeze(0), vc.contiguous().unsqueeze(0), causal=True)
+            o, _ = K.flash_fwd(q.unsqueeze(0), kc.unsqueeze(0), vc.unsqueeze(0), causal=True)
             return o[0]
 
         return self._layers(K.embedding_fwd(tok, e.w.p("embed")), attend)

@@ -52,7 +52,7 @@ class ServingModel:
         self.last_logits = logits
         if self.sampler is not None:
             return self.sampler(logits.float())
-        return logits.float().argmax(-1)
+        return self.e.K.argmax_rows(logits)
 
     # ------------------------------------------------------------------ prompt chunks
     @torch.no_grad()

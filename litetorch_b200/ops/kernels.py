@@ -92,6 +92,8 @@ _SIGS = {
     "lt_gelu_bwd": [_vp, _vp, _vp, _ll, _vp],
     "lt_axpby": [_vp, _vp, _vp, _f, _f, _ll, _vp],
     "lt_embedding_fwd": [_vp, _vp, _vp, _ll, _i, _i, _vp],
+    "lt_embedding_fwd_idx": [_vp, _i, _vp, _vp, _ll, _i, _i, _vp],
+    "lt_argmax_rows": [_vp, _i, _vp, _i, _i, _ll, _vp],
     "lt_embedding_bwd": [_vp, _vp, _vp, _ll, _i, _i, _vp],
     "lt_cast_f32_to_bf16": [_vp, _vp, _ll, _vp],
     "lt_cast_bf16_to_f32": [_vp, _vp, _ll, _vp],
@@ -595,10 +597,22 @@ def axpby(a, b=None, alpha=1.0, beta=1.0, out=None):
 
 
 def embedding_fwd(idx: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
-    idx = idx.reshape(-1).to(torch.int64)
+    idx = idx.reshape(-1)
+    if idx.dtype != torch.int32:
+        idx = idx.to(torch.int64)
     V, D = table.shape
     out = torch.empty((idx.numel(), D), dtype=table.dtype, device=table.device)
-    _check(_fn("lt_embedding_fwd")(idx.data_ptr(), table.data_ptr(), out.data_ptr(), idx.numel(), D, V, _stream()), "lt_embedding_fwd")
+    _check(_fn("lt_embedding_fwd_idx")(idx.data_ptr(), 1 if idx.dtype == torch.int32 else 0, table.data_ptr(), out.data_ptr(), idx.numel(), D, V, _stream()),
+           "lt_embedding_fwd_idx")
+    return out
+
+
+def argmax_rows(x: torch.Tensor) -> torch.Tensor:
+    """x.argmax(-1) of [rows, V] bf16 or fp32."""
+    if x.dim() != 2 or x.dtype not in (torch.bfloat16, torch.float32) or x.stride(1) != 1 or x.shape[1] == 0:
+        return x.float().argmax(-1)
+    out = torch.empty(x.shape[0], dtype=torch.int64, device=x.device)
+    _check(_fn("lt_argmax_rows")(x.data_ptr(), _f32(x), out.data_ptr(), x.shape[0], x.shape[1], x.stride(0), _stream()), "lt_argmax_rows")
     return out
 
 
