@@ -60,7 +60,10 @@ class LlamaKVModel(ServingModel):
 
     def _logits(self, hidden, rows=None):
         e, K = self.e, self.e.K
-        return K.product_of_constants(hidden if rows is None else hidden[rows], e.w.p("lm_head"), norm=(e.w.p("final_norm"), e.cfg.rms_eps))
+        if rows is not None:
+            run = self._run_of(rows)
+            hidden = hidden[rows if run is None else run]
+        return K.product_of_constants(hidden, e.w.p("lm_head"), norm=(e.w.p("final_norm"), e.cfg.rms_eps))
 
     # ------------------------------------------------------------------ prompt chunks
     @torch.no_grad()
@@ -138,16 +141,8 @@ class LlamaKVModel(ServingModel):
         e, K = self.e, self.e.K
         dev = e.device
         n = len(tokens)
-        host = torch.empty(3, n, dtype=torch.int64)
-        host[0] = torch.tensor(tokens, dtype=torch.int64)
-        host[1] = torch.arange(start, start + n)
-        host[2] = self._slots(block_ids, start, n)
-        d = host.to(dev, non_blocking=True)
-        tok, pos, slots = d[0], d[1].to(torch.int32), d[2].to(torch.int32)
+        tok, pos, slots, blocks = self._prompt_inputs(tokens, start, block_ids)
         bs = self.block_size
-        nb = (start + n + bs - 1) // bs
-        blocks = torch.tensor(list(block_ids[:nb]), dtype=torch.int32, device=dev) if start > 0 else None
-
         Hq, Hkv, hd = e.cfg.n_heads, e.cfg.n_kv_heads, e.cfg.head_dim
 
         def attend(i, qkv):
@@ -174,9 +169,8 @@ class LlamaKVModel(ServingModel):
     def _decode_hidden(self, d: torch.Tensor, S: int, width: int) -> torch.Tensor:
         e, K = self.e, self.e.K
         cfg, c, bs = e.cfg, self.cache, self.block_size
-        tok = d[0]
-        pos, slots, ctx = d[1].to(torch.int32), d[2].to(torch.int32), d[3].to(torch.int32)
-        bt = d[5:].t().contiguous().to(torch.int32)
+        tok, pos, slots, ctx = d[0], d[1], d[2], d[3]
+        bt = d[5:].t().contiguous()
 
         def attend(i, qkv):
             return K.decode_step(qkv, e.cos, e.sin, pos, slots, cfg.n_heads, cfg.n_kv_heads, cfg.head_dim, c.k[i], c.v[i], bt, ctx, bs, self.num_splits, c.k_scale, c.v_scale)

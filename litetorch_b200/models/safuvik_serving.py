@@ -69,7 +69,9 @@ class SafuvikModel(ServingModel):
         e, K = self.e, self.e.K
         x, pending = hidden
         if rows is not None:
-            rows = torch.tensor(rows, dtype=torch.int32, device=e.device)
+            run = self._run_of(rows)
+            rows = (torch.tensor(rows, dtype=torch.int32, device=e.device) if run is None else      # (a copy that is waited for)
+                    torch.arange(run.start, run.stop, dtype=torch.int32, device=e.device))
         h = K.hyper_norm(x, e.final_norm, e.cfg.eps, dtype=e.dtype, rows=rows, write=False, **pending)
         return K.linear(h, e.head, out_dtype=torch.float32, alpha=e.cfg.logit_scale)
 
@@ -97,15 +99,8 @@ class SafuvikModel(ServingModel):
     # ------------------------------------------------------------------ prompt portions
     def _prompt_hidden(self, tokens: Sequence[int], start: int, block_ids: Sequence[int], slot: int):
         e, K = self.e, self.e.K
-        n, bs = len(tokens), self.block_size
-        nb = (start + n + bs - 1) // bs
-        host = torch.empty(3 * n + nb, dtype=torch.int32)
-        host[:n] = torch.tensor(list(tokens), dtype=torch.int32)
-        host[n:2 * n] = torch.arange(start, start + n, dtype=torch.int32)
-        host[2 * n:3 * n] = self._slots(block_ids, start, n)
-        host[3 * n:] = torch.tensor(list(block_ids[:nb]), dtype=torch.int32)
-        d = host.to(e.device, non_blocking=True)
-        tok, pos, slots, table = d[:n], d[n:2 * n], d[2 * n:3 * n], d[3 * n:]
+        n = len(tokens)
+        tok, pos, slots, table = self._prompt_inputs(tokens, start, block_ids)
 
         def attention(i, lay, proj, gate):
             a = lay.cfg.mixer.left
@@ -147,7 +142,6 @@ class SafuvikModel(ServingModel):
 
     def _decode_hidden(self, d: torch.Tensor, S: int, width: int):
         e, K = self.e, self.e.K
-        d = d.to(torch.int32)
         tok, pos, slots, ctx, rows = d[0], d[1], d[2], d[3], d[4]
         tables = d[5:].t().contiguous()
 

@@ -9,13 +9,19 @@ A model supplies four pieces of device work and inherits the rest:
     _logits(hidden, rows)                           logits of the given rows (None: all)
     new_serving(...)                                on the engine: how to make the serving model (see `models.registry`)
 
-The packed int64 input block of a decode step is [5 + width, S]: token, position, cache slot, context length, state slot
+The packed int32 input block of a decode step is [5 + width, S]: token, position, cache slot, context length, state slot
 of every sequence, then its block table (transposed).
+
+Inputs reach the device through pinned memory (the host allocator hands a block out again only when the copies out of it are
+done), so that the host prepares a pass while the one before it runs: a copy from pageable memory, or a copy that is waited
+for, ends when everything before it has run.
 """
 from __future__ import annotations
 
+from itertools import chain
 from typing import List, Optional, Sequence
 
+import numpy as np
 import torch
 
 
@@ -88,17 +94,18 @@ class ServingModel:
         use_graph = self.graphs and dev.type == "cuda"
         if use_graph:
             width = (width + 15) // 16 * 16                     # fewer distinct graphs: table widths in steps of 16 blocks
-        host = torch.zeros(5 + width, S, dtype=torch.int64)
-        host[0] = torch.tensor(list(last_tokens), dtype=torch.int64)
-        host[1] = torch.tensor(list(positions), dtype=torch.int64)
-        for s in range(S):
-            p = positions[s]
-            host[2, s] = block_tables[s][p // bs] * bs + p % bs
-            row = block_tables[s][:width]
-            host[5:5 + len(row), s] = torch.tensor(list(row), dtype=torch.int64)
-        host[3] = host[1] + 1
-        if slots is not None:
-            host[4] = torch.tensor(list(slots), dtype=torch.int64)
+        host = self._host(5 + width, S)
+        h = host.numpy()
+        h[0] = last_tokens
+        h[1] = positions
+        h[2] = [block_tables[s][p // bs] * bs + p % bs for s, p in enumerate(positions)]
+        h[3] = h[1] + 1
+        h[4] = 0 if slots is None else list(slots)
+        n = [min(len(t), width) for t in block_tables]
+        flat = np.fromiter(chain.from_iterable(t if len(t) <= width else t[:width] for t in block_tables), np.int32, sum(n))
+        table = np.zeros((S, width), np.int32)
+        table[np.arange(width) < np.array(n)[:, None]] = flat
+        h[5:] = table.T
         if not use_graph:
             return self._decode_body(host.to(dev, non_blocking=True), S, width)
         entry = self._graphs.get((S, width))
@@ -111,8 +118,13 @@ class ServingModel:
             torch.cuda.current_stream().wait_stream(side)
             torch.cuda.synchronize()
             g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g, stream=side):
-                static_out = self._decode_body(static_in, S, width)
+            # (not `torch.cuda.graph`: it gives all cached memory back first, which takes a tenth of a second and more after large states)
+            with torch.cuda.stream(side):
+                g.capture_begin()
+                try:
+                    static_out = self._decode_body(static_in, S, width)
+                finally:
+                    g.capture_end()
             entry = self._graphs[S, width] = (g, static_in, static_out)
             # the eager pass wrote this step's cache cells already; the replay below rewrites the same ones
         g, static_in, static_out = entry
@@ -132,13 +144,34 @@ class ServingModel:
     def decode_logits(self, last_tokens: Sequence[int], positions: Sequence[int], block_tables: List[Sequence[int]],
                       slots: Optional[Sequence[int]] = None) -> torch.Tensor:
         """The same step; returns its fp32 logits [S, vocab]."""
-        return self._run_decode(last_tokens, positions, block_tables, slots)[0].float().clone()
+        out = self._run_decode(last_tokens, positions, block_tables, slots)[0]
+        return out.clone() if out.dtype == torch.float32 else out.float()
 
     # ------------------------------------------------------------------ helpers
-    def _slots(self, block_ids: Sequence[int], start: int, n: int) -> torch.Tensor:
-        bs = self.block_size
-        p = torch.arange(start, start + n)
-        return (torch.tensor(list(block_ids), dtype=torch.int64)[p // bs] * bs + p % bs).to(torch.int32)
+    def _host(self, *shape: int) -> torch.Tensor:
+        """Host memory for 32-bit inputs, pinned where there is a GPU."""
+        return torch.empty(shape, dtype=torch.int32, pin_memory=self.e.device.type == "cuda")
+
+    def _prompt_inputs(self, tokens: Sequence[int], start: int, block_ids: Sequence[int]):
+        """(tokens, positions, cache slots, block table) of a portion on the device, int32, through one copy."""
+        n, bs = len(tokens), self.block_size
+        nb = (start + n + bs - 1) // bs
+        host = self._host(3 * n + nb)
+        h = host.numpy()
+        p = np.arange(start, start + n, dtype=np.int32)
+        table = np.fromiter(block_ids[:nb], np.int32, nb)
+        h[:n] = np.fromiter(tokens, np.int32, n)
+        h[n:2 * n] = p
+        h[2 * n:3 * n] = table[p // bs] * bs + p % bs
+        h[3 * n:] = table
+        d = host.to(self.e.device, non_blocking=True)
+        return d[:n], d[n:2 * n], d[2 * n:3 * n], d[3 * n:]
+
+    @staticmethod
+    def _run_of(rows: Sequence[int]) -> Optional[slice]:
+        """The rows as a slice, if they are one after another."""
+        r = list(rows)
+        return slice(r[0], r[-1] + 1) if r and r[0] >= 0 and r == list(range(r[0], r[-1] + 1)) else None
 
     @staticmethod
     def _splits_for(ctas: int, keys: int) -> int:

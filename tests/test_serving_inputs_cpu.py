@@ -1,0 +1,39 @@
+"""Inputs of prompt portions and decode steps as they are packed on the host."""
+import torch
+
+
+def _model():
+    from litetorch_b200.models.llama import LlamaConfig, LlamaEngine
+    from litetorch_b200.models.registry import new_serving
+    cfg = LlamaConfig(vocab_size=64, n_layers=1, d_model=64, n_heads=2, n_kv_heads=1, head_dim=32, ffn=64, max_seq=256)
+    return new_serving(LlamaEngine(cfg, "cpu", seed=1), num_blocks=40, block_size=4, max_num_seqs=4)
+
+
+def test_prompt_inputs():
+    m = _model()
+    for start, n in ((0, 1), (0, 9), (3, 5), (8, 4)):
+        blocks = [7, 3, 30, 11, 2][:(start + n + 3) // 4 + 1]
+        tok, pos, slots, table = m._prompt_inputs(list(range(10, 10 + n)), start, blocks)
+        assert tok.tolist() == list(range(10, 10 + n)) and pos.tolist() == list(range(start, start + n))
+        assert slots.tolist() == [blocks[p // 4] * 4 + p % 4 for p in range(start, start + n)] and table.tolist() == blocks[:(start + n + 3) // 4]
+        assert all(t.dtype == torch.int32 for t in (tok, pos, slots, table))
+
+
+def test_decode_inputs():
+    m = _model()
+    seen = []
+    m._decode_body = lambda d, S, width: seen.append((d, S, width)) or (torch.zeros(S, 64), torch.zeros(S))
+    tables = [[5], [9, 1, 8, 12, 13], (4, 6, 20)]         # the second is longer than its sequence
+    m._run_decode([3, 1, 2], [2, 11, 8], tables, [7, 0, 5])
+    d, S, width = seen[0]
+    assert (S, width) == (3, 3) and d.shape == (8, 3) and d.dtype == torch.int32
+    assert d[:5].tolist() == [[3, 1, 2], [2, 11, 8], [22, 35, 80], [3, 12, 9], [7, 0, 5]]
+    assert d[5:].t().tolist() == [[5, 0, 0], [9, 1, 8], [4, 6, 20]]
+
+
+def test_runs_of_rows():
+    m = _model()
+    assert m._run_of([5]) == slice(5, 6) and m._run_of(range(2, 6)) == slice(2, 6)
+    assert m._run_of([]) is None and m._run_of([1, 3]) is None and m._run_of([2, 1]) is None and m._run_of([-1]) is None
+    x = torch.randn(8, 64)
+    assert torch.equal(m._logits(x, [3, 4]), m._logits(x)[3:5]) and torch.equal(m._logits(x, [4, 1]), m._logits(x)[[4, 1]])
