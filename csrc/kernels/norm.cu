@@ -530,7 +530,7 @@ int lt_norm_bwd(int layer_norm, const void* dy, const void* x, const void* w, co
   auto W = static_cast<const __nv_bfloat16*>(w);
   auto DR = static_cast<const __nv_bfloat16*>(dres);
   auto DX = static_cast<__nv_bfloat16*>(dx);
-  if (!layer_norm && D == 256 && M >= 8 * grid / 2) {
+  if (!layer_norm && D == 256 && M >= 2 * sm_count()) {
     // warp-per-row kernel; grid CTAs of 8 warps, one partial dgamma row per CTA
     int g2 = (M + 7) / 8;
     if (g2 > grid) g2 = grid;

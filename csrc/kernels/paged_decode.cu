@@ -320,18 +320,20 @@ paged_decode_gqa_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
 //
 // Same split of the work as paged_decode_gqa_kernel (one CTA of four warps per sequence, KV head and context split;
 // a warp streams chunks of 32 keys through its own shared-memory stages), but the tiles arrive as TMA tensor copies in
-// the 128-byte-swizzled layout, so that ldmatrix reads them without bank conflicts, and a chunk costs 16 ldmatrix.x4 and
-// 32 mma.sync (m16n8k16: the group's query heads padded to 16 rows, 8 keys or 8 output columns per instruction) instead
-// of one shared-memory pass over the whole query block per key.  The scores stay in registers: their accumulator
-// fragments are, after the softmax, exactly the A fragments of the P V product.  tcgen05 is not the tool here: its
-// smallest tile is 64 rows and the kernel is bound by the K / V stream, not by arithmetic.
+// the 128-byte-swizzled layout, so that ldmatrix reads them without bank conflicts.  Both products are made transposed: keys (and then
+// value columns) are the 16 rows of mma.sync m16n8k16, the group's query heads its 8 columns, so that groups of up to 8 heads, which is
+// what models have, waste half or nothing instead of half to three quarters (heads as the 16 rows: twice the instructions, of the softmax too).
+// The scores stay in registers; an 8 x 8 transpose in registers turns their fragments into those of the second product.  tcgen05 is not the tool
+// here: its smallest tile is 64 rows and the kernel is bound by the K / V stream and by issue.  Six warps where heads have 128 columns (a CTA an SM),
+// block tables read a chunk ahead by the lanes that request its runs: 32 sequences of 2048 to 4096 tokens, 8 KV heads of 128, 97 -> 72 us (61 at the copy rate).
 template <int D>
 struct PdMmaCfg {
+  static constexpr int kWarps = (D == 64) ? 4 : 6;
   static constexpr int kStages = (D == 64) ? 3 : 2;
   static constexpr int kTileBytes = 32 * D * 2;                           // 32 keys of K (or V); D = 128: two 4 KB halves of 64 columns
   static constexpr int kWarpBytes = kStages * 2 * kTileBytes;
-  static constexpr int kOffBar = kPdWarps * kWarpBytes;
-  static constexpr int kSmemBytes = kOffBar + kPdWarps * kStages * 8 + 16 + 1024;   // + slack to align the tiles to 1024 bytes
+  static constexpr int kOffBar = kWarps * kWarpBytes;
+  static constexpr int kSmemBytes = kOffBar + kWarps * kStages * 8 + 16 + 1024;   // + slack to align the tiles to 1024 bytes
 };
 constexpr int kPdMmaMaxG = 16;
 
@@ -350,40 +352,87 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4],
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// 8 x 8 matrix of 16-bit values, a row in four lanes, transposed.
+__device__ __forceinline__ uint32_t movmatrix(uint32_t a) {
+  uint32_t d;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
+  return d;
+}
+
 // End of a CTA of the tensor-core decode kernels: shared memory (the tile area: every requested copy has been waited for) takes
-// the four warps' maxima, sums and outputs, [warps][16], [warps][16] and [warps][16][D] floats; the last one is returned.
-__device__ __forceinline__ float* pd_row_sums(uint8_t* smem, int warp, int lane, bool ok, float m_lo, float m_hi, float l_lo, float l_hi) {
-  const int g = lane >> 2;
-  l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
-  l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
-  l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);
-  l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
+// the four warps' maxima, sums and outputs, [warps][16], [warps][16] and [warps][16][D] floats; the last one is returned.  m, l: of heads
+// 8 n + 2 (lane % 4) + e, l this lane's share.
+template <int W, int NT>
+__device__ __forceinline__ float* pd_row_sums(uint8_t* smem, int warp, int lane, bool ok, const float (&m)[NT][2], float (&l)[NT][2]) {
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+      for (int o = 4; o <= 16; o <<= 1) l[n][e] += __shfl_xor_sync(0xffffffffu, l[n][e], o);
   __syncthreads();
   float* red_m = reinterpret_cast<float*>(smem);
-  float* red_l = red_m + kPdWarps * kPdMmaMaxG;
-  if ((lane & 3) == 0) {
-    red_m[warp * kPdMmaMaxG + g] = ok ? m_lo : -INFINITY;
-    red_l[warp * kPdMmaMaxG + g] = ok ? l_lo : 0.f;
-    red_m[warp * kPdMmaMaxG + g + 8] = ok ? m_hi : -INFINITY;
-    red_l[warp * kPdMmaMaxG + g + 8] = ok ? l_hi : 0.f;
+  float* red_l = red_m + W * kPdMmaMaxG;
+  if (lane < 4) {
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        red_m[warp * kPdMmaMaxG + n * 8 + lane * 2 + e] = ok ? m[n][e] : -INFINITY;
+        red_l[warp * kPdMmaMaxG + n * 8 + lane * 2 + e] = ok ? l[n][e] : 0.f;
+      }
   }
-  return red_l + kPdWarps * kPdMmaMaxG;
+  return red_l + W * kPdMmaMaxG;
+}
+// Scores of a chunk of 32 keys, [16-key block][fragment] for every 8 heads: rows are keys g and g + 8, columns heads 2 qd and 2 qd + 1.  They become
+// weights; maxima m and sums l go on, and `a` is what the outputs so far are multiplied by.  factor: of the scores of this lane's heads.
+template <int NT>
+__device__ __forceinline__ void pd_softmax(float (&s)[NT][2][4], const float (&factor)[NT][2], float (&m)[NT][2], float (&l)[NT][2], float (&a)[NT][2], int g,
+                                           int nk, int c0, int lo) {
+  bool live[4];   // keys g, g + 8, g + 16, g + 24
+#pragma unroll
+  for (int i = 0; i < 4; ++i) live[i] = i * 8 + g < nk && c0 + i * 8 + g >= lo;
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      float mx = -INFINITY;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float& x = s[n][i >> 1][(i & 1) * 2 + e];
+        x = live[i] ? x * factor[n][e] : -INFINITY;
+        mx = fmaxf(mx, x);
+      }
+#pragma unroll
+      for (int o = 4; o <= 16; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      const float nm = fmaxf(m[n][e], mx);   // finite: every chunk has a live key (the first one ends after `lo`)
+      a[n][e] = m[n][e] == -INFINITY ? 0.f : __expf(m[n][e] - nm);
+      m[n][e] = nm;
+      float sum = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float& x = s[n][i >> 1][(i & 1) * 2 + e];
+        x = __expf(x - nm);
+        sum += x;
+      }
+      l[n][e] = l[n][e] * a[n][e] + sum;
+    }
 }
 // part: the group's rows [G][splits][D + 2]; out_scale multiplies the outputs.
-template <int D>
+template <int D, int W>
 __device__ __forceinline__ void pd_write_partial(uint8_t* smem, float* part, int G, int splits, int sp, float out_scale) {
   const float* red_m = reinterpret_cast<const float*>(smem);
-  const float* red_l = red_m + kPdWarps * kPdMmaMaxG;
-  const float* red_o = red_l + kPdWarps * kPdMmaMaxG;
+  const float* red_l = red_m + W * kPdMmaMaxG;
+  const float* red_o = red_l + W * kPdMmaMaxG;
   __syncthreads();
   for (int i = threadIdx.x; i < G * D; i += blockDim.x) {
     const int gg = i / D, d = i % D;
     float gm = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < kPdWarps; ++w) gm = fmaxf(gm, red_m[w * kPdMmaMaxG + gg]);
+    for (int w = 0; w < W; ++w) gm = fmaxf(gm, red_m[w * kPdMmaMaxG + gg]);
     float lsum = 0.f, o = 0.f;
 #pragma unroll
-    for (int w = 0; w < kPdWarps; ++w) {
+    for (int w = 0; w < W; ++w) {
       const float mw = red_m[w * kPdMmaMaxG + gg];
       if (mw == -INFINITY) continue;
       const float a = __expf(mw - gm);
@@ -482,8 +531,9 @@ __device__ __forceinline__ void pd_merge_cluster(const float* mine, __nv_bfloat1
 
 // tmK / tmV: the caches seen as [num_blocks * Hkv * block_size rows, D] bf16, box 64 columns x min(block_size, 32) rows,
 // 128-byte swizzle.  block_size is a multiple of 8 and divides 32 or is a multiple of it.
-template <int D, bool STEP>
-__global__ void __launch_bounds__(kPdWarps * 32)
+// NT: blocks of 8 query heads.
+template <int D, int NT, bool STEP>
+__global__ void __launch_bounds__(PdMmaCfg<D>::kWarps * 32)
 paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                         const __nv_bfloat16* __restrict__ q, const int* __restrict__ block_tables,
                         const int* __restrict__ context_lens, float* __restrict__ part, int S, int Hq, int Hkv, int block_size,
@@ -491,7 +541,7 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
   using Cfg = PdMmaCfg<D>;
   constexpr int ST = Cfg::kStages;
   constexpr int KS = D / 16;     // k-steps of the score product
-  constexpr int NT = D / 8;      // 8-column blocks of the output
+  constexpr int NU = D / 16;     // blocks of 16 value columns
   extern __shared__ uint8_t pd_raw[];
   uint8_t* pd_smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(pd_raw) + 1023) & ~uintptr_t(1023));
   const int G = Hq / Hkv;
@@ -521,51 +571,60 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
   const int t0 = base + sp * per, t1 = min(ctx, t0 + per);
   const int* bt = block_tables + (long long)s * max_blocks;
   const int n_chunks = t1 > t0 ? (t1 - t0 + 31) / 32 : 0;
-  const int my_n = n_chunks > warp ? (n_chunks - warp + kPdWarps - 1) / kPdWarps : 0;   // chunks warp, warp + 4, ...
+  const int my_n = n_chunks > warp ? (n_chunks - warp + Cfg::kWarps - 1) / Cfg::kWarps : 0;   // chunks warp, warp + 4, ...
   const int run = block_size < 32 ? block_size : 32;                 // rows per tensor copy
 
+  // The copies of a chunk, a lane for every run of rows; its block, read from the table a chunk ahead, is in `next_blk`.
+  const int last_row = t1 > t0 ? ((t1 - 1) / block_size + 1) * block_size : 0;   // end of the last block holding a live key
+  int next_blk = 0;
+  auto look_up = [&](int i) {
+    const int r = t0 + (warp + i * Cfg::kWarps) * 32 + lane * run;
+    if (i < my_n && lane * run < 32 && r < last_row) next_blk = bt[r / block_size];
+  };
   auto request = [&](int i) {
-    const int c0 = t0 + (warp + i * kPdWarps) * 32;
+    const int c0 = t0 + (warp + i * Cfg::kWarps) * 32;
     const uint32_t bar = bar0 + 8u * (i % ST);
-    uint8_t* kt = my_tiles + (i % ST) * 2 * Cfg::kTileBytes;
-    uint8_t* vt = kt + Cfg::kTileBytes;
-    const int last_row = ((t1 - 1) / block_size + 1) * block_size;   // end of the last block holding a live key
-    const int r_end = min(c0 + 32, last_row);
-    mbar_expect_tx(bar, uint32_t(2 * (r_end - c0) * D * 2));
-    for (int r = c0; r < r_end; r += run) {
-      const int blk = bt[r / block_size];
-      const int row = (blk * Hkv + hkv) * block_size + r % block_size;
+    const int r_end = min(c0 + 32, last_row), r = c0 + lane * run;
+    if (lane == 0) mbar_expect_tx(bar, uint32_t(2 * (r_end - c0) * D * 2));
+    if (r < r_end) {
+      const int row = (next_blk * Hkv + hkv) * block_size + r % block_size;
+      uint8_t* kt = my_tiles + (i % ST) * 2 * Cfg::kTileBytes + (r - c0) * 128;
 #pragma unroll
       for (int h = 0; h < D / 64; ++h) {
-        tma_load_2d(smem_u32(kt + h * 4096 + (r - c0) * 128), &tmK, bar, h * 64, row);
-        tma_load_2d(smem_u32(vt + h * 4096 + (r - c0) * 128), &tmV, bar, h * 64, row);
+        tma_load_2d(smem_u32(kt + h * 4096), &tmK, bar, h * 64, row);
+        tma_load_2d(smem_u32(kt + Cfg::kTileBytes + h * 4096), &tmV, bar, h * 64, row);
       }
     }
+    look_up(i + 1);
   };
 
-  float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.f, l_hi = 0.f;   // l: this lane's share of the row sums
-  float oacc[NT][4];
+  float m[NT][2], l[NT][2], factor[NT][2];   // of heads 8 n + 2 qd + e; l: this lane's share of the sums
+  float oacc[NT][NU][4];                     // rows = value columns 16 u + g and + 8, columns = heads
 #pragma unroll
-  for (int nt = 0; nt < NT; ++nt)
+  for (int n = 0; n < NT; ++n) {
 #pragma unroll
-    for (int r = 0; r < 4; ++r) oacc[nt][r] = 0.f;
+    for (int e = 0; e < 2; ++e) { m[n][e] = -INFINITY; l[n][e] = 0.f; factor[n][e] = scale; }
+#pragma unroll
+    for (int u = 0; u < NU; ++u)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) oacc[n][u][r] = 0.f;
+  }
 
-  if (lane == 0)
-    for (int i = 0; i < ST - 1 && i < my_n; ++i) request(i);
+  look_up(0);
+  for (int i = 0; i < ST - 1 && i < my_n; ++i) request(i);
   if (early) pdl_wait();
-  // A fragments of the query block: rows = heads of the group (g and g + 8), zero past G
-  uint32_t qa[KS][4];
+  // B fragments of the query block, transposed: columns = heads of the group (8 n + g), zero past G
+  uint32_t qb[NT][KS][2];
   {
-    const bool lo = g < G, hi = g + 8 < G;
     const __nv_bfloat16* rows = STEP ? step.qkv + s * step.ld + (long long)hkv * G * D : q + ((long long)s * Hq + hkv * G) * D;
-    const __nv_bfloat16* qlo = rows + (lo ? g : 0) * D + qd * 2;
-    const __nv_bfloat16* qhi = rows + (hi ? g + 8 : 0) * D + qd * 2;
 #pragma unroll
-    for (int kk = 0; kk < KS; ++kk) {
-      qa[kk][0] = lo ? *reinterpret_cast<const uint32_t*>(qlo + kk * 16) : 0u;
-      qa[kk][1] = hi ? *reinterpret_cast<const uint32_t*>(qhi + kk * 16) : 0u;
-      qa[kk][2] = lo ? *reinterpret_cast<const uint32_t*>(qlo + kk * 16 + 8) : 0u;
-      qa[kk][3] = hi ? *reinterpret_cast<const uint32_t*>(qhi + kk * 16 + 8) : 0u;
+    for (int n = 0; n < NT; ++n) {
+      const bool there = n * 8 + g < G;
+      const __nv_bfloat16* row = rows + (there ? n * 8 + g : 0) * D + qd * 2;
+#pragma unroll
+      for (int kk = 0; kk < KS; ++kk)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) qb[n][kk][half] = there ? *reinterpret_cast<const uint32_t*>(row + kk * 16 + half * 8) : 0u;
     }
     if constexpr (STEP) {
       const long long at = (long long)step.pos[s] * (D / 2) + qd;
@@ -573,17 +632,17 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
       for (int kk = 0; kk < KS; ++kk)
 #pragma unroll
         for (int half = 0; half < 2; ++half) {     // columns kk * 16 + 8 half + 2 qd and the next
-          const float c = step.cos_t[at + kk * 8 + half * 4], n = step.sin_t[at + kk * 8 + half * 4];
+          const float c = step.cos_t[at + kk * 8 + half * 4], w = step.sin_t[at + kk * 8 + half * 4];
 #pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            const float2 a = unpack_bf16x2(qa[kk][half * 2 + r]);
-            qa[kk][half * 2 + r] = pack_bf16x2(a.x * c - a.y * n, a.x * n + a.y * c);
+          for (int n = 0; n < NT; ++n) {
+            const float2 a = unpack_bf16x2(qb[n][kk][half]);
+            qb[n][kk][half] = pack_bf16x2(a.x * c - a.y * w, a.x * w + a.y * c);
           }
         }
     }
   }
   // the newest token's row, for the warp whose last chunk it ends
-  const int newest = STEP && t1 == ctx && my_n > 0 && (n_chunks - 1) % kPdWarps == warp ? my_n - 1 : -1;
+  const int newest = STEP && t1 == ctx && my_n > 0 && (n_chunks - 1) % Cfg::kWarps == warp ? my_n - 1 : -1;
   [[maybe_unused]] uint4 fresh;
   [[maybe_unused]] long long fresh_at = -1;
   if constexpr (STEP) {
@@ -595,7 +654,7 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
   bool ok = true;
   const int lj = lane >> 3, lr = lane & 7;   // ldmatrix: this lane addresses row lr of matrix lj
   for (int i = 0; i < my_n; ++i) {
-    if (lane == 0 && i + ST - 1 < my_n) request(i + ST - 1);      // its stage was consumed in iteration i - 1
+    if (i + ST - 1 < my_n) request(i + ST - 1);      // its stage was consumed in iteration i - 1
     ok = __all_sync(0xffffffffu, mbar_wait(bar0 + 8u * (i % ST), uint32_t(i / ST) & 1u, abort_flag, status, kStatusTimeoutFull));
     if (!ok) {
       // a copy never arrived: give the other requested stages one more bounded wait each, so that no copy of this
@@ -604,7 +663,7 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         mbar_wait(bar0 + 8u * (r % ST), uint32_t(r / ST) & 1u, &drain_s, status, kStatusTimeoutFull);
       break;
     }
-    const int c0 = t0 + (warp + i * kPdWarps) * 32;
+    const int c0 = t0 + (warp + i * Cfg::kWarps) * 32;
     uint8_t* kt = my_tiles + (i % ST) * 2 * Cfg::kTileBytes;
     uint8_t* vt = kt + Cfg::kTileBytes;
     const uint32_t kt_addr = smem_u32(kt), vt_addr = smem_u32(vt);
@@ -632,92 +691,71 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
       }
       __syncwarp();
     }
-    // ---- S = Q K^T: four blocks of 8 keys
-    float sacc[4][4];
+    // ---- S^T = K Q^T: two blocks of 16 keys, which take turns (an instruction that adds to what the one before it makes waits for it)
+    float sacc[NT][2][4];
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
+    for (int n = 0; n < NT; ++n)
 #pragma unroll
-      for (int r = 0; r < 4; ++r) sacc[t][r] = 0.f;
-      const int key = t * 8 + lr;
+      for (int t = 0; t < 2; ++t)
 #pragma unroll
-      for (int kk2 = 0; kk2 < KS / 2; ++kk2) {
-        const int u = kk2 * 4 + lj;                                 // 16-byte unit of the row: columns 8 u .. 8 u + 7
-        uint32_t b00, b01, b10, b11;
-        ldsm_x4(kt_addr + (u >> 3) * 4096 + key * 128 + (((u & 7) ^ (key & 7)) << 4), b00, b01, b10, b11);
-        mma_16816(sacc[t], qa[2 * kk2], b00, b01);
-        mma_16816(sacc[t], qa[2 * kk2 + 1], b10, b11);
+        for (int r = 0; r < 4; ++r) sacc[n][t][r] = 0.f;
+#pragma unroll
+    for (int kk = 0; kk < KS; ++kk) {
+      const int u = kk * 2 + (lj >> 1);                             // 16-byte unit of the row: columns 8 u .. 8 u + 7
+      uint32_t ka[2][4];
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const int key = t * 16 + (lj & 1) * 8 + lr;
+        ldsm_x4(kt_addr + (u >> 3) * 4096 + key * 128 + (((u & 7) ^ (key & 7)) << 4), ka[t][0], ka[t][1], ka[t][2], ka[t][3]);
       }
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int t = 0; t < 2; ++t) mma_16816(sacc[n][t], ka[t], qb[n][kk][0], qb[n][kk][1]);
     }
-    // ---- online softmax: this lane holds columns t * 8 + qd * 2 + {0, 1} of rows g (registers 0, 1) and g + 8 (2, 3)
-    float mx_lo = -INFINITY, mx_hi = -INFINITY;
+    float a[NT][2];
+    pd_softmax<NT>(sacc, factor, m, l, a, g, nk, c0, lo);
+    uint32_t pb[NT][4];                                             // weights of 8 keys each, heads as columns
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
+    for (int n = 0; n < NT; ++n)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int col = t * 8 + qd * 2 + e;
-        const bool live = col < nk && c0 + col >= lo;
-        sacc[t][e] = live ? sacc[t][e] * scale : -INFINITY;
-        sacc[t][2 + e] = live ? sacc[t][2 + e] * scale : -INFINITY;
-        mx_lo = fmaxf(mx_lo, sacc[t][e]);
-        mx_hi = fmaxf(mx_hi, sacc[t][2 + e]);
+      for (int i = 0; i < 4; ++i) pb[n][i] = movmatrix(pack_bf16x2(sacc[n][i >> 1][(i & 1) * 2], sacc[n][i >> 1][(i & 1) * 2 + 1]));
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int u = 0; u < NU; ++u) {
+        oacc[n][u][0] *= a[n][0]; oacc[n][u][1] *= a[n][1];
+        oacc[n][u][2] *= a[n][0]; oacc[n][u][3] *= a[n][1];
       }
-    }
-    mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 1));
-    mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 2));
-    mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1));
-    mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
-    const float nm_lo = fmaxf(m_lo, mx_lo), nm_hi = fmaxf(m_hi, mx_hi);   // finite: every chunk has a live key (the first one ends after `lo`)
-    const float a_lo = (m_lo == -INFINITY) ? 0.f : __expf(m_lo - nm_lo);
-    const float a_hi = (m_hi == -INFINITY) ? 0.f : __expf(m_hi - nm_hi);
-    m_lo = nm_lo; m_hi = nm_hi;
-    float ps_lo = 0.f, ps_hi = 0.f;
-    uint32_t pa[2][4];
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const float p0 = __expf(sacc[t][0] - nm_lo), p1 = __expf(sacc[t][1] - nm_lo);
-      const float p2 = __expf(sacc[t][2] - nm_hi), p3 = __expf(sacc[t][3] - nm_hi);
-      ps_lo += p0 + p1;
-      ps_hi += p2 + p3;
-      pa[t >> 1][(t & 1) * 2] = pack_bf16x2(p0, p1);         // keys 16 ks + 8 (t & 1) + ..: registers 0 / 2 rows g, 1 / 3 rows g + 8
-      pa[t >> 1][(t & 1) * 2 + 1] = pack_bf16x2(p2, p3);
-    }
-    l_lo = l_lo * a_lo + ps_lo;
-    l_hi = l_hi * a_hi + ps_hi;
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      oacc[nt][0] *= a_lo; oacc[nt][1] *= a_lo;
-      oacc[nt][2] *= a_hi; oacc[nt][3] *= a_hi;
-    }
-    // ---- O += P V: two steps of 16 keys, transposed loads of V
+    // ---- O^T += V^T P^T: two steps of 16 keys, transposed loads of V
 #pragma unroll
     for (int ks = 0; ks < 2; ++ks) {
-      const int key = ks * 16 + (lj & 1) * 8 + lr;
+      const int key = ks * 16 + (lj >> 1) * 8 + lr;
 #pragma unroll
-      for (int nt2 = 0; nt2 < NT / 2; ++nt2) {
-        const int u = nt2 * 2 + (lj >> 1);
-        uint32_t b0a, b1a, b0b, b1b;
-        ldsm_x4_trans(vt_addr + (u >> 3) * 4096 + key * 128 + (((u & 7) ^ (key & 7)) << 4), b0a, b1a, b0b, b1b);
-        mma_16816(oacc[2 * nt2], pa[ks], b0a, b1a);
-        mma_16816(oacc[2 * nt2 + 1], pa[ks], b0b, b1b);
+      for (int u = 0; u < NU; ++u) {
+        const int w = u * 2 + (lj & 1);
+        uint32_t va[4];
+        ldsm_x4_trans(vt_addr + (w >> 3) * 4096 + key * 128 + (((w & 7) ^ (key & 7)) << 4), va[0], va[1], va[2], va[3]);
+#pragma unroll
+        for (int n = 0; n < NT; ++n) mma_16816(oacc[n][u], va, pb[n][2 * ks], pb[n][2 * ks + 1]);
       }
     }
     __syncwarp();            // every lane is done with this stage before lane 0 requests into it again
   }
   // ---- merge the four warps (the tile area is free now: every requested copy has been waited for), write the partial result
-  float* red_o = pd_row_sums(pd_smem, warp, lane, ok, m_lo, m_hi, l_lo, l_hi);
+  float* red_o = pd_row_sums<Cfg::kWarps, NT>(pd_smem, warp, lane, ok, m, l);
 #pragma unroll
-  for (int nt = 0; nt < NT; ++nt) {
-    float* lo = red_o + (warp * kPdMmaMaxG + g) * D + nt * 8 + qd * 2;
-    float* hi = red_o + (warp * kPdMmaMaxG + g + 8) * D + nt * 8 + qd * 2;
-    *reinterpret_cast<float2*>(lo) = make_float2(oacc[nt][0], oacc[nt][1]);
-    *reinterpret_cast<float2*>(hi) = make_float2(oacc[nt][2], oacc[nt][3]);
-  }
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int u = 0; u < NU; ++u)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) red_o[(warp * kPdMmaMaxG + n * 8 + qd * 2 + (r & 1)) * D + u * 16 + g + (r >> 1) * 8] = oacc[n][u][r];
   if (STEP && !part) {
-    float* mine = red_o + kPdWarps * kPdMmaMaxG * D;
-    pd_write_partial<D>(pd_smem, mine, G, 1, 0, 1.f);
+    float* mine = red_o + Cfg::kWarps * kPdMmaMaxG * D;
+    pd_write_partial<D, Cfg::kWarps>(pd_smem, mine, G, 1, 0, 1.f);
     pd_merge_cluster<D>(mine, step.out + ((long long)s * Hq + hkv * G) * D, G, splits, sp);
   } else {
-    pd_write_partial<D>(pd_smem, part + ((long long)s * Hq + hkv * G) * splits * (D + 2), G, splits, sp, 1.f);
+    pd_write_partial<D, Cfg::kWarps>(pd_smem, part + ((long long)s * Hq + hkv * G) * splits * (D + 2), G, splits, sp, 1.f);
   }
 }
 
@@ -727,18 +765,21 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
 //   scores   a lane takes 16 contiguous bytes of a key row, which are its fragments of four instructions when the columns of
 //            the query are permuted alike; the query's rows are scaled by a power of two so that fp16 holds all of their bits;
 //   P V      ldmatrix transposes pairs of bytes, so that a lane gets two neighbouring columns of two neighbouring keys; even and odd
-//            columns go to instructions of their own.  2^14 times a softmax weight is the sum of two fp16 parts (22 bits or more), each
+//            columns are the upper and the lower eight rows of an instruction.  2^14 times a softmax weight is the sum of two fp16 parts (22 bits or more), each
 //            with an instruction of its own.
+// 8 sequences of 4500 to 9000 tokens: 60 us with heads as the instruction's 16 rows, 37 with heads as its 8 columns (1270 against about 600
+// instructions a chunk of 8 KB; the table read a chunk ahead), bytes at the copy rate 17.
 // Against 64 bits the 32-bit results are 1.3e-7 to 4.2e-7 off (2-norm; 32 to 16384 keys, one split or as many as a step takes, queries of
 // size 0.1 to 4), those of the kernel before 1.5e-7 to 7.7e-6.
 template <int D>
 struct PdF8Cfg {
+  static constexpr int kWarps = 4;
   static constexpr int kStages = (D == 64) ? 4 : 3;
   static constexpr int kTileBytes = 32 * D;                               // 32 keys of K (or V)
   static constexpr int kWarpBytes = kStages * 2 * kTileBytes;
-  static constexpr int kOffBar = kPdWarps * kWarpBytes;
-  static constexpr int kSmemBytes = kOffBar + kPdWarps * kStages * 8 + 16 + 1024;   // + slack to align the tiles to 1024 bytes
-  static_assert(kOffBar >= (kPdWarps + 1) * kPdMmaMaxG * (D + 2) * 4, "the reduction at the end reuses the tile area");
+  static constexpr int kOffBar = kWarps * kWarpBytes;
+  static constexpr int kSmemBytes = kOffBar + kWarps * kStages * 8 + 16 + 1024;   // + slack to align the tiles to 1024 bytes
+  static_assert(kOffBar >= (kWarps + 1) * kPdMmaMaxG * (D + 2) * 4, "the reduction at the end reuses the tile area");
 };
 constexpr float kPdWeightScale = 16384.f;   // weights are at most 1: the largest fp16 part is 2^14, the smallest 2^-24 stands for 2^-38
 
@@ -755,10 +796,9 @@ __device__ __forceinline__ void mma_f16_16816_0(float (&d)[4], const uint32_t (&
       : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
 }
-// Two e4m3 values (low byte first) -> fp16 pair, exactly.
-__device__ __forceinline__ uint32_t e4m3x2_to_f16x2(uint32_t two) {
-  const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(__nv_fp8x2_storage_t(two), __NV_E4M3);
-  return uint32_t(h.x) | (uint32_t(h.y) << 16);
+// Four e4m3 values (low byte first) -> two fp16 pairs, exactly.
+__device__ __forceinline__ void e4m3x4_to_f16(uint32_t four, uint32_t& lo, uint32_t& hi) {
+  asm("{\n\t.reg .b16 a, b;\n\tmov.b32 {a, b}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, a;\n\tcvt.rn.f16x2.e4m3x2 %1, b;\n\t}" : "=r"(lo), "=r"(hi) : "r"(four));
 }
 __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
   const __half2 v = __floats2half2_rn(lo, hi);
@@ -774,8 +814,8 @@ __device__ __forceinline__ void split_f16x2(float x0, float x1, uint32_t& hi, ui
 
 // tmK / tmV: the caches seen as [num_blocks * Hkv * block_size rows, D] bytes, box D columns x min(block_size, 32) rows; rows of 128
 // bytes arrive with the 128-byte swizzle, rows of 64 as they are.
-template <int D, bool STEP>
-__global__ void __launch_bounds__(kPdWarps * 32)
+template <int D, int NT, bool STEP>
+__global__ void __launch_bounds__(PdF8Cfg<D>::kWarps * 32)
 paged_decode_f8_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                        const __nv_bfloat16* __restrict__ q, const int* __restrict__ block_tables,
                        const int* __restrict__ context_lens, float* __restrict__ part, int S, int Hq, int Hkv, int block_size,
@@ -815,73 +855,84 @@ paged_decode_f8_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
   const int t0 = base + sp * per, t1 = min(ctx, t0 + per);
   const int* bt = block_tables + (long long)s * max_blocks;
   const int n_chunks = t1 > t0 ? (t1 - t0 + 31) / 32 : 0;
-  const int my_n = n_chunks > warp ? (n_chunks - warp + kPdWarps - 1) / kPdWarps : 0;   // chunks warp, warp + 4, ...
+  const int my_n = n_chunks > warp ? (n_chunks - warp + Cfg::kWarps - 1) / Cfg::kWarps : 0;   // chunks warp, warp + 4, ...
   const int run = block_size < 32 ? block_size : 32;                 // rows per tensor copy
 
+  // The copies of a chunk, a lane for every run of rows; its block, read from the table a chunk ahead, is in `next_blk`.
+  const int last_row = t1 > t0 ? ((t1 - 1) / block_size + 1) * block_size : 0;   // end of the last block holding a live key
+  int next_blk = 0;
+  auto look_up = [&](int i) {
+    const int r = t0 + (warp + i * Cfg::kWarps) * 32 + lane * run;
+    if (i < my_n && lane * run < 32 && r < last_row) next_blk = bt[r / block_size];
+  };
   auto request = [&](int i) {
-    const int c0 = t0 + (warp + i * kPdWarps) * 32;
+    const int c0 = t0 + (warp + i * Cfg::kWarps) * 32;
     const uint32_t bar = bar0 + 8u * (i % ST);
-    const uint32_t kt = smem_u32(my_tiles + (i % ST) * 2 * Cfg::kTileBytes);
-    const int last_row = ((t1 - 1) / block_size + 1) * block_size;   // end of the last block holding a live key
-    const int r_end = min(c0 + 32, last_row);
-    mbar_expect_tx(bar, uint32_t(2 * (r_end - c0) * D));
-    for (int r = c0; r < r_end; r += run) {
-      const int row = (bt[r / block_size] * Hkv + hkv) * block_size + r % block_size;
-      tma_load_2d(kt + (r - c0) * D, &tmK, bar, 0, row);
-      tma_load_2d(kt + Cfg::kTileBytes + (r - c0) * D, &tmV, bar, 0, row);
+    const int r_end = min(c0 + 32, last_row), r = c0 + lane * run;
+    if (lane == 0) mbar_expect_tx(bar, uint32_t(2 * (r_end - c0) * D));
+    if (r < r_end) {
+      const int row = (next_blk * Hkv + hkv) * block_size + r % block_size;
+      const uint32_t kt = smem_u32(my_tiles + (i % ST) * 2 * Cfg::kTileBytes) + (r - c0) * D;
+      tma_load_2d(kt, &tmK, bar, 0, row);
+      tma_load_2d(kt + Cfg::kTileBytes, &tmV, bar, 0, row);
     }
+    look_up(i + 1);
   };
 
-  float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.f, l_hi = 0.f;   // l: this lane's share of the row sums
-  float oacc[NU][2][4];                                               // [unit][even / odd column][fragment]
+  float m[NT][2], l[NT][2], factor[NT][2];   // of heads 8 n + 2 qd + e; l: this lane's share of the sums
+  float oacc[NT][NU][4];                     // rows = value columns 16 u + 2 g and the next, columns = heads
 #pragma unroll
-  for (int u = 0; u < NU; ++u)
+  for (int n = 0; n < NT; ++n) {
 #pragma unroll
-    for (int r = 0; r < 8; ++r) oacc[u][r >> 2][r & 3] = 0.f;
+    for (int e = 0; e < 2; ++e) { m[n][e] = -INFINITY; l[n][e] = 0.f; }
+#pragma unroll
+    for (int u = 0; u < NU; ++u)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) oacc[n][u][r] = 0.f;
+  }
 
-  if (lane == 0)
-    for (int i = 0; i < ST - 1 && i < my_n; ++i) request(i);
+  look_up(0);
+  for (int i = 0; i < ST - 1 && i < my_n; ++i) request(i);
   if (early) pdl_wait();
-  // A fragments of the query block, columns permuted: step kk = 4 h + r takes columns 64 h + 16 qd + 4 r + {0 .. 3}.  Rows = heads of the
-  // group (g and g + 8), zero past G, scaled by a power of two to a largest value in [2^14, 2^15).
-  uint32_t qa[KS][4];
-  float scale_lo, scale_hi;
-  {
-    uint2 raw[2][KS];
-    float top[2] = {0.f, 0.f};
+  // B fragments of the query block, transposed, its columns permuted: step kk = 4 h + r takes columns 64 h + 16 qd + 4 r + {0 .. 3}.  Columns =
+  // heads of the group (8 n + g), zero past G, scaled by a power of two to a largest value in [2^14, 2^15).
+  uint32_t qb[NT][KS][2];
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const bool there = g + 8 * half < G;
-      const __nv_bfloat16* rows = STEP ? step.qkv + s * step.ld + (long long)hkv * G * D : q + ((long long)s * Hq + hkv * G) * D;
-      const __nv_bfloat16* row = rows + (there ? g + 8 * half : 0) * D + qd * 16;
+  for (int n = 0; n < NT; ++n) {
+    uint2 raw[KS];
+    float top = 0.f;
+    const bool there = n * 8 + g < G;
+    const __nv_bfloat16* rows = STEP ? step.qkv + s * step.ld + (long long)hkv * G * D : q + ((long long)s * Hq + hkv * G) * D;
+    const __nv_bfloat16* row = rows + (there ? n * 8 + g : 0) * D + qd * 16;
 #pragma unroll
-      for (int kk = 0; kk < KS; ++kk) {
-        raw[half][kk] = there ? *reinterpret_cast<const uint2*>(row + (kk >> 2) * 64 + (kk & 3) * 4) : make_uint2(0u, 0u);
-        if constexpr (STEP) {
-          const long long at = (long long)step.pos[s] * (D / 2) + (kk >> 2) * 32 + qd * 8 + (kk & 3) * 2;
-          const float2 c = *reinterpret_cast<const float2*>(step.cos_t + at), n = *reinterpret_cast<const float2*>(step.sin_t + at);
-          const float2 x = unpack_bf16x2(raw[half][kk].x), y = unpack_bf16x2(raw[half][kk].y);
-          raw[half][kk] = make_uint2(pack_bf16x2(x.x * c.x - x.y * n.x, x.x * n.x + x.y * c.x), pack_bf16x2(y.x * c.y - y.y * n.y, y.x * n.y + y.y * c.y));
-        }
-        const float2 a = unpack_bf16x2(raw[half][kk].x), b = unpack_bf16x2(raw[half][kk].y);
-        top[half] = fmaxf(top[half], fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y))));
+    for (int kk = 0; kk < KS; ++kk) {
+      raw[kk] = there ? *reinterpret_cast<const uint2*>(row + (kk >> 2) * 64 + (kk & 3) * 4) : make_uint2(0u, 0u);
+      if constexpr (STEP) {
+        const long long at = (long long)step.pos[s] * (D / 2) + (kk >> 2) * 32 + qd * 8 + (kk & 3) * 2;
+        const float2 c = *reinterpret_cast<const float2*>(step.cos_t + at), w = *reinterpret_cast<const float2*>(step.sin_t + at);
+        const float2 x = unpack_bf16x2(raw[kk].x), y = unpack_bf16x2(raw[kk].y);
+        raw[kk] = make_uint2(pack_bf16x2(x.x * c.x - x.y * w.x, x.x * w.x + x.y * c.x), pack_bf16x2(y.x * c.y - y.y * w.y, y.x * w.y + y.y * c.y));
       }
-      top[half] = fmaxf(top[half], __shfl_xor_sync(0xffffffffu, top[half], 1));
-      top[half] = fmaxf(top[half], __shfl_xor_sync(0xffffffffu, top[half], 2));
-      // (a row of zeros or with an infinity stays as it is)
-      const int e = top[half] > 0.f && top[half] <= 3.4e38f ? max(-120, min(100, 14 - ilogbf(top[half]))) : 0;
-      const float up = ldexpf(1.f, e);
-      (half ? scale_hi : scale_lo) = scale * ldexpf(1.f, -e);
-#pragma unroll
-      for (int kk = 0; kk < KS; ++kk) {
-        const float2 a = unpack_bf16x2(raw[half][kk].x), b = unpack_bf16x2(raw[half][kk].y);
-        qa[kk][half] = pack_f16x2(a.x * up, a.y * up);
-        qa[kk][2 + half] = pack_f16x2(b.x * up, b.y * up);
-      }
+      const float2 a = unpack_bf16x2(raw[kk].x), b = unpack_bf16x2(raw[kk].y);
+      top = fmaxf(top, fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y))));
     }
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+    // (a row of zeros or with an infinity stays as it is)
+    const int e = top > 0.f && top <= 3.4e38f ? max(-120, min(100, 14 - ilogbf(top))) : 0;
+    const float up = ldexpf(1.f, e), down = scale * ldexpf(1.f, -e);
+#pragma unroll
+    for (int kk = 0; kk < KS; ++kk) {
+      const float2 a = unpack_bf16x2(raw[kk].x), b = unpack_bf16x2(raw[kk].y);
+      qb[n][kk][0] = pack_f16x2(a.x * up, a.y * up);
+      qb[n][kk][1] = pack_f16x2(b.x * up, b.y * up);
+    }
+    // scores lie in other lanes than their query: those of heads 2 qd and 2 qd + 1 here
+    factor[n][0] = __shfl_sync(0xffffffffu, down, qd * 8);
+    factor[n][1] = __shfl_sync(0xffffffffu, down, qd * 8 + 4);
   }
   // the newest token's row, for the warp whose last chunk it ends
-  const int newest = STEP && t1 == ctx && my_n > 0 && (n_chunks - 1) % kPdWarps == warp ? my_n - 1 : -1;
+  const int newest = STEP && t1 == ctx && my_n > 0 && (n_chunks - 1) % Cfg::kWarps == warp ? my_n - 1 : -1;
   [[maybe_unused]] uint4 fresh;
   [[maybe_unused]] long long fresh_at = -1;
   if constexpr (STEP) {
@@ -893,7 +944,7 @@ paged_decode_f8_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
   bool ok = true;
   const int lj = lane >> 3, lr = lane & 7;   // ldmatrix: this lane addresses row lr of matrix lj
   for (int i = 0; i < my_n; ++i) {
-    if (lane == 0 && i + ST - 1 < my_n) request(i + ST - 1);      // its stage was consumed in iteration i - 1
+    if (i + ST - 1 < my_n) request(i + ST - 1);      // its stage was consumed in iteration i - 1
     ok = __all_sync(0xffffffffu, mbar_wait(bar0 + 8u * (i % ST), uint32_t(i / ST) & 1u, abort_flag, status, kStatusTimeoutFull));
     if (!ok) {
       // a copy never arrived: give the other requested stages one more bounded wait each, so that no copy of this
@@ -902,7 +953,7 @@ paged_decode_f8_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
         mbar_wait(bar0 + 8u * (r % ST), uint32_t(r / ST) & 1u, &drain_s, status, kStatusTimeoutFull);
       break;
     }
-    const int c0 = t0 + (warp + i * kPdWarps) * 32;
+    const int c0 = t0 + (warp + i * Cfg::kWarps) * 32;
     uint8_t* kt = my_tiles + (i % ST) * 2 * Cfg::kTileBytes;
     uint8_t* vt = kt + Cfg::kTileBytes;
     const uint32_t vt_addr = smem_u32(vt);
@@ -937,109 +988,99 @@ paged_decode_f8_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
       }
       __syncwarp();
     }
-    // ---- S = Q K^T: four blocks of 8 keys
-    float sacc[4][4];
+    // ---- S^T = K Q^T: two blocks of 16 keys, which take turns
+    float sacc[NT][2][4];
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
+    for (int n = 0; n < NT; ++n)
 #pragma unroll
-      for (int r = 0; r < 4; ++r) sacc[t][r] = 0.f;
+      for (int t = 0; t < 2; ++t)
 #pragma unroll
-      for (int h = 0; h < D / 64; ++h) {
-        const uint4 w = *reinterpret_cast<const uint4*>(kt + unit(t * 8 + g, h * 4 + qd));
-        const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+        for (int r = 0; r < 4; ++r) sacc[n][t][r] = 0.f;
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-          mma_f16_16816(sacc[t], qa[h * 4 + r], e4m3x2_to_f16x2(ww[r] & 0xffffu), e4m3x2_to_f16x2(ww[r] >> 16));
+    for (int h = 0; h < D / 64; ++h) {
+      uint4 w[2][2];                                         // [block][keys g / g + 8]
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) w[t][half] = *reinterpret_cast<const uint4*>(kt + unit(t * 16 + half * 8 + g, h * 4 + qd));
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          uint32_t ka[4];
+#pragma unroll
+          for (int half = 0; half < 2; ++half) e4m3x4_to_f16(r == 0 ? w[t][half].x : r == 1 ? w[t][half].y : r == 2 ? w[t][half].z : w[t][half].w, ka[half], ka[2 + half]);
+#pragma unroll
+          for (int n = 0; n < NT; ++n) mma_f16_16816(sacc[n][t], ka, qb[n][h * 4 + r][0], qb[n][h * 4 + r][1]);
+        }
+    }
+    float a[NT][2];
+    pd_softmax<NT>(sacc, factor, m, l, a, g, nk, c0, lo);
+    uint32_t ph[NT][4], pl[NT][4];                           // weights of 8 keys each, heads as columns
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        uint32_t hi, low;
+        split_f16x2(sacc[n][i >> 1][(i & 1) * 2] * kPdWeightScale, sacc[n][i >> 1][(i & 1) * 2 + 1] * kPdWeightScale, hi, low);
+        ph[n][i] = movmatrix(hi);
+        pl[n][i] = movmatrix(low);
       }
-    }
-    // ---- online softmax: this lane holds columns t * 8 + qd * 2 + {0, 1} of rows g (registers 0, 1) and g + 8 (2, 3)
-    float mx_lo = -INFINITY, mx_hi = -INFINITY;
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int col = t * 8 + qd * 2 + e;
-        const bool live = col < nk && c0 + col >= lo;
-        sacc[t][e] = live ? sacc[t][e] * scale_lo : -INFINITY;
-        sacc[t][2 + e] = live ? sacc[t][2 + e] * scale_hi : -INFINITY;
-        mx_lo = fmaxf(mx_lo, sacc[t][e]);
-        mx_hi = fmaxf(mx_hi, sacc[t][2 + e]);
-      }
-    }
-    mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 1));
-    mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 2));
-    mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1));
-    mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
-    const float nm_lo = fmaxf(m_lo, mx_lo), nm_hi = fmaxf(m_hi, mx_hi);
-    const float a_lo = (m_lo == -INFINITY) ? 0.f : __expf(m_lo - nm_lo);
-    const float a_hi = (m_hi == -INFINITY) ? 0.f : __expf(m_hi - nm_hi);
-    m_lo = nm_lo; m_hi = nm_hi;
-    float ps_lo = 0.f, ps_hi = 0.f;
-    uint32_t ph[2][4], pl[2][4];
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const float p0 = __expf(sacc[t][0] - nm_lo), p1 = __expf(sacc[t][1] - nm_lo);
-      const float p2 = __expf(sacc[t][2] - nm_hi), p3 = __expf(sacc[t][3] - nm_hi);
-      ps_lo += p0 + p1;
-      ps_hi += p2 + p3;
-      const int at = (t & 1) * 2;                            // keys 16 ks + 8 (t & 1) + ..: registers 0 / 2 rows g, 1 / 3 rows g + 8
-      split_f16x2(p0 * kPdWeightScale, p1 * kPdWeightScale, ph[t >> 1][at], pl[t >> 1][at]);
-      split_f16x2(p2 * kPdWeightScale, p3 * kPdWeightScale, ph[t >> 1][at + 1], pl[t >> 1][at + 1]);
-    }
-    l_lo = l_lo * a_lo + ps_lo;
-    l_hi = l_hi * a_hi + ps_hi;
-    // ---- O += P V: two steps of 16 keys.  A chunk's products start from zero and are added with rounding: the instruction cuts off what it adds
-    // to its accumulator, which over hundreds of chunks would add up.
+    // ---- O^T += V^T P^T: two steps of 16 keys.  A chunk's products start from zero and are added with rounding: the instruction cuts off what it
+    // adds to its accumulator, which over hundreds of chunks would add up.
 #pragma unroll
     for (int u2 = 0; u2 < NU / 2; ++u2) {
-      float pv[2][2][4];                                     // [unit][even / odd column][fragment]
+      float pv[NT][2][4];                                    // [unit][fragment]
 #pragma unroll
       for (int ks = 0; ks < 2; ++ks) {
         const int key = ks * 16 + (lj & 1) * 8 + lr;
         uint32_t b[2][2];                                    // [unit][keys 0 .. 7 / 8 .. 15 of the step]
         ldsm_x4_trans(vt_addr + unit(key, u2 * 2 + (lj >> 1)), b[0][0], b[0][1], b[1][0], b[1][1]);
+        uint32_t va[2][4];                                   // rows 2 g (registers 0, 2) and 2 g + 1 (1, 3) of the unit
 #pragma unroll
-        for (int uu = 0; uu < 2; ++uu) {
-          uint32_t ev[2], od[2];
+        for (int uu = 0; uu < 2; ++uu)
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            const uint32_t ka = e4m3x2_to_f16x2(b[uu][h] & 0xffffu), kb = e4m3x2_to_f16x2(b[uu][h] >> 16);
-            ev[h] = __byte_perm(ka, kb, 0x5410);
-            od[h] = __byte_perm(ka, kb, 0x7632);
+            uint32_t ka, kb;                                 // both columns of a key, and of the next
+            e4m3x4_to_f16(b[uu][h], ka, kb);
+            va[uu][2 * h] = __byte_perm(ka, kb, 0x5410);
+            va[uu][2 * h + 1] = __byte_perm(ka, kb, 0x7632);
           }
-          if (ks == 0) {
-            mma_f16_16816_0(pv[uu][0], ph[ks], ev[0], ev[1]);
-            mma_f16_16816_0(pv[uu][1], ph[ks], od[0], od[1]);
-          } else {
-            mma_f16_16816(pv[uu][0], ph[ks], ev[0], ev[1]);
-            mma_f16_16816(pv[uu][1], ph[ks], od[0], od[1]);
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+          for (int uu = 0; uu < 2; ++uu) {
+            if (ks == 0) mma_f16_16816_0(pv[n][uu], va[uu], ph[n][0], ph[n][1]);
+            else mma_f16_16816(pv[n][uu], va[uu], ph[n][2], ph[n][3]);
           }
-          mma_f16_16816(pv[uu][0], pl[ks], ev[0], ev[1]);
-          mma_f16_16816(pv[uu][1], pl[ks], od[0], od[1]);
-        }
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+          for (int uu = 0; uu < 2; ++uu) mma_f16_16816(pv[n][uu], va[uu], pl[n][2 * ks], pl[n][2 * ks + 1]);
       }
 #pragma unroll
-      for (int uu = 0; uu < 2; ++uu)
+      for (int n = 0; n < NT; ++n)
 #pragma unroll
-        for (int e = 0; e < 2; ++e)
+        for (int uu = 0; uu < 2; ++uu)
 #pragma unroll
-          for (int r = 0; r < 4; ++r) oacc[u2 * 2 + uu][e][r] = fmaf(oacc[u2 * 2 + uu][e][r], r < 2 ? a_lo : a_hi, pv[uu][e][r]);
+          for (int r = 0; r < 4; ++r) oacc[n][u2 * 2 + uu][r] = fmaf(oacc[n][u2 * 2 + uu][r], a[n][r & 1], pv[n][uu][r]);
     }
     __syncwarp();            // every lane is done with this stage before lane 0 requests into it again
   }
-  float* red_o = pd_row_sums(pd_smem, warp, lane, ok, m_lo, m_hi, l_lo, l_hi);
+  float* red_o = pd_row_sums<Cfg::kWarps, NT>(pd_smem, warp, lane, ok, m, l);
 #pragma unroll
-  for (int u = 0; u < NU; ++u) {
-    float* at = red_o + (warp * kPdMmaMaxG + g) * D + u * 16 + qd * 4;
-    *reinterpret_cast<float4*>(at) = make_float4(oacc[u][0][0], oacc[u][1][0], oacc[u][0][1], oacc[u][1][1]);
-    *reinterpret_cast<float4*>(at + 8 * D) = make_float4(oacc[u][0][2], oacc[u][1][2], oacc[u][0][3], oacc[u][1][3]);
-  }
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int u = 0; u < NU; ++u)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        *reinterpret_cast<float2*>(red_o + (warp * kPdMmaMaxG + n * 8 + qd * 2 + e) * D + u * 16 + g * 2) = make_float2(oacc[n][u][e], oacc[n][u][2 + e]);
   if (STEP && !part) {
-    float* mine = red_o + kPdWarps * kPdMmaMaxG * D;
-    pd_write_partial<D>(pd_smem, mine, G, 1, 0, v_scale / kPdWeightScale);
+    float* mine = red_o + Cfg::kWarps * kPdMmaMaxG * D;
+    pd_write_partial<D, Cfg::kWarps>(pd_smem, mine, G, 1, 0, v_scale / kPdWeightScale);
     pd_merge_cluster<D>(mine, step.out + ((long long)s * Hq + hkv * G) * D, G, splits, sp);
   } else {
-    pd_write_partial<D>(pd_smem, part + ((long long)s * Hq + hkv * G) * splits * (D + 2), G, splits, sp, v_scale / kPdWeightScale);
+    pd_write_partial<D, Cfg::kWarps>(pd_smem, part + ((long long)s * Hq + hkv * G) * splits * (D + 2), G, splits, sp, v_scale / kPdWeightScale);
   }
 }
 
@@ -1109,6 +1150,52 @@ __global__ void kv_append_kernel(const __nv_bfloat16* __restrict__ k_new, const 
   }
 }
 
+// One of the tensor-core decode kernels, by cache type, head size and heads of a group; cluster: CTAs of a cluster.
+template <class K, class... A>
+static int launch_clustered(K kernel, int warps, int smem, OncePerDevice& configured, int ctas, int cluster, cudaStream_t st, A... args) {
+  if (configured.pending()) {
+    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    configured.finish();
+  }
+  cudaLaunchAttribute attr[2]{};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(warps * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  LT_RETURN_IF_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+  return 0;
+}
+template <bool STEP, int D, int NT>
+static int launch_tensor_decode_by(const CUtensorMap& tmK, const CUtensorMap& tmV, const __nv_bfloat16* q, const int* bt, const int* ctx, float* part, int S,
+                                   int Hq, int Hkv, int block_size, int max_blocks, int splits, float scale, int kv_fp8, float v_scale, int window, int* status,
+                                   const PdStep& step, int ctas, int cluster, cudaStream_t st) {
+  static OncePerDevice done8, done16;
+  if (kv_fp8)
+    return launch_clustered(paged_decode_f8_kernel<D, NT, STEP>, PdF8Cfg<D>::kWarps, PdF8Cfg<D>::kSmemBytes, done8, ctas, cluster, st, tmK, tmV, q, bt, ctx, part, S, Hq, Hkv, block_size,
+                            max_blocks, splits, scale, v_scale, window, status, step);
+  return launch_clustered(paged_decode_mma_kernel<D, NT, STEP>, PdMmaCfg<D>::kWarps, PdMmaCfg<D>::kSmemBytes, done16, ctas, cluster, st, tmK, tmV, q, bt, ctx, part, S, Hq, Hkv, block_size,
+                          max_blocks, splits, scale, window, status, step);
+}
+template <bool STEP>
+static int launch_tensor_decode(const CUtensorMap& tmK, const CUtensorMap& tmV, const __nv_bfloat16* q, const int* bt, const int* ctx, float* part, int S, int Hq,
+                                int Hkv, int D, int block_size, int max_blocks, int splits, float scale, int kv_fp8, float v_scale, int window, int* status,
+                                const PdStep& step, int ctas, int cluster, cudaStream_t st) {
+#define LT_PD(DD, NT) \
+  launch_tensor_decode_by<STEP, DD, NT>(tmK, tmV, q, bt, ctx, part, S, Hq, Hkv, block_size, max_blocks, splits, scale, kv_fp8, v_scale, window, status, step, ctas, cluster, st)
+  if (Hq / Hkv <= 8) return D == 64 ? LT_PD(64, 1) : LT_PD(128, 1);
+  return D == 64 ? LT_PD(64, 2) : LT_PD(128, 2);
+#undef LT_PD
+}
+
 static int merge_splits(const float* part, __nv_bfloat16* o, int rows, int splits, int D, const __nv_bfloat16* gate, long long ldg, int Hq, int vdim,
                         cudaStream_t st) {
   const int mb = (rows + 3) / 4;
@@ -1166,18 +1253,9 @@ int lt_paged_decode_window(const void* q, const void* k_cache, const void* v_cac
     if (r == 0) r = encode_tmap_2d(&tmV, v_cache, bytes, D, rows, uint64_t(D) * bytes, kv_fp8 ? D : 64, run, !kv_fp8 || D == 128);
     if (r) return r > 0 ? 1000 + r : r;
     int* status = device_status_word();
-    static OncePerDevice configured_mma;
-    if (configured_mma.pending()) {
-      LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_f8_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdF8Cfg<64>::kSmemBytes));
-      LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_f8_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdF8Cfg<128>::kSmemBytes));
-      LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_mma_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdMmaCfg<64>::kSmemBytes));
-      LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_mma_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdMmaCfg<128>::kSmemBytes));
-      configured_mma.finish();
-    }
-    if (kv_fp8 && D == 64) LT_RETURN_IF_CUDA(launch_chained(paged_decode_f8_kernel<64, false>, ctas, kPdWarps * 32, PdF8Cfg<64>::kSmemBytes, st, tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale * k_scale, v_scale, window, status, PdStep{}));
-    else if (kv_fp8) LT_RETURN_IF_CUDA(launch_chained(paged_decode_f8_kernel<128, false>, ctas, kPdWarps * 32, PdF8Cfg<128>::kSmemBytes, st, tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale * k_scale, v_scale, window, status, PdStep{}));
-    else if (D == 64) LT_RETURN_IF_CUDA(launch_chained(paged_decode_mma_kernel<64, false>, ctas, kPdWarps * 32, PdMmaCfg<64>::kSmemBytes, st, tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale, window, status, PdStep{}));
-    else LT_RETURN_IF_CUDA(launch_chained(paged_decode_mma_kernel<128, false>, ctas, kPdWarps * 32, PdMmaCfg<128>::kSmemBytes, st, tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, block_size, max_blocks, splits, scale, window, status, PdStep{}));
+    const int rc = launch_tensor_decode<false>(tmK, tmV, Q, block_tables, context_lens, part, S, Hq, Hkv, D, block_size, max_blocks, splits,
+                                               kv_fp8 ? scale * k_scale : scale, kv_fp8, v_scale, window, status, PdStep{}, ctas, 1, st);
+    if (rc) return rc;
   } else if (!kv_fp8 && window == 0 && G <= kPdMaxG && bs_ok && (reinterpret_cast<uintptr_t>(k_cache) & 15) == 0 && (reinterpret_cast<uintptr_t>(v_cache) & 15) == 0) {
     // bf16 caches: every K / V byte is read once for the whole group of query heads, through a shared-memory pipeline
     const int ctas = S * Hkv * splits;
@@ -1219,50 +1297,13 @@ int lt_paged_decode_step(const void* qkv, long long ld, const float* cos_t, cons
   int r = encode_tmap_2d(&tmK, k_cache, bytes, D, rows, uint64_t(D) * bytes, kv_fp8 ? D : 64, run, !kv_fp8 || D == 128);
   if (r == 0) r = encode_tmap_2d(&tmV, v_cache, bytes, D, rows, uint64_t(D) * bytes, kv_fp8 ? D : 64, run, !kv_fp8 || D == 128);
   if (r) return r > 0 ? 1000 + r : r;
-  static OncePerDevice configured;
-  if (configured.pending()) {
-    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_f8_kernel<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdF8Cfg<64>::kSmemBytes));
-    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_f8_kernel<64, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_f8_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdF8Cfg<128>::kSmemBytes));
-    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_f8_kernel<128, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_mma_kernel<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdMmaCfg<64>::kSmemBytes));
-    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_mma_kernel<64, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_mma_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PdMmaCfg<128>::kSmemBytes));
-    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(paged_decode_mma_kernel<128, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    configured.finish();
-  }
   const PdStep step{static_cast<const __nv_bfloat16*>(qkv), ld, cos_t, sin_t, pos, slots, k_cache, v_cache, kv_fp8 ? 1.f / k_scale : 1.f, kv_fp8 ? 1.f / v_scale : 1.f,
                     static_cast<__nv_bfloat16*>(o), early};
-  const __nv_bfloat16* none = nullptr;
-  int* status = device_status_word();
-  cudaLaunchAttribute attr[2]{};
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = part ? 1 : splits;
-  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(S * Hkv * splits);
-  cfg.blockDim = dim3(kPdWarps * 32);
-  cfg.stream = static_cast<cudaStream_t>(stream);
-  cfg.attrs = attr;
-  cfg.numAttrs = part ? 1 : 2;
-#define LT_PD_F8(DD)                                                                                                                            \
-  cfg.dynamicSmemBytes = PdF8Cfg<DD>::kSmemBytes;                                                                                              \
-  LT_RETURN_IF_CUDA(cudaLaunchKernelEx(&cfg, paged_decode_f8_kernel<DD, true>, tmK, tmV, none, block_tables, context_lens, part, S, Hq, Hkv, block_size, \
-                                       max_blocks, splits, scale * k_scale, v_scale, 0, status, step))
-#define LT_PD_MMA(DD)                                                                                                                           \
-  cfg.dynamicSmemBytes = PdMmaCfg<DD>::kSmemBytes;                                                                                             \
-  LT_RETURN_IF_CUDA(cudaLaunchKernelEx(&cfg, paged_decode_mma_kernel<DD, true>, tmK, tmV, none, block_tables, context_lens, part, S, Hq, Hkv, block_size, \
-                                       max_blocks, splits, scale, 0, status, step))
-  if (kv_fp8) {
-    if (D == 64) { LT_PD_F8(64); } else { LT_PD_F8(128); }
-  } else {
-    if (D == 64) { LT_PD_MMA(64); } else { LT_PD_MMA(128); }
-  }
-#undef LT_PD_F8
-#undef LT_PD_MMA
-  return part ? merge_splits(part, static_cast<__nv_bfloat16*>(o), S * Hq, splits, D, nullptr, 0, Hq, D, cfg.stream) : 0;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int rc = launch_tensor_decode<true>(tmK, tmV, nullptr, block_tables, context_lens, part, S, Hq, Hkv, D, block_size, max_blocks, splits,
+                                            kv_fp8 ? scale * k_scale : scale, kv_fp8, v_scale, 0, device_status_word(), step, S * Hkv * splits, part ? 1 : splits, st);
+  if (rc) return rc;
+  return part ? merge_splits(part, static_cast<__nv_bfloat16*>(o), S * Hq, splits, D, nullptr, 0, Hq, D, st) : 0;
 }
 
 int lt_kv_append(const void* k_new, const void* v_new, void* k_cache, void* v_cache, const int* slots, long long n_tok, int Hkv,

@@ -861,21 +861,29 @@ def paged_decode(q, k_cache, v_cache, block_tables, context_lens, block_size: in
 def _decode_splits(pairs: int, keys: int, head_dim: int, fp8: bool):
     """(how the splits of a (sequence, KV head) meet, how many there are) for a decode step's attention over contexts of up to `keys`:
 
-    cluster  they merge in a cluster, as many as fill the SMs once (a cluster wants its places together: nine tenths of them); a second round
-             is weighed against shorter splits.  Four layers of a model (us; separate launches / their splits in one launch with a merge
-             kernel / clusters of 2, 4, 8): 1.1b 16 x 2000 234 / 225 / 229, 209, 245; 8b 8 x 9000 on 8 bits 642 / 645 / 808, 606, 630; 8b 3 x 3000
-             454 / 452 / 473, 433, 452 (of 5: 425); 8b 16 x 2000 568 / 572 / 535, 584, 709 (of 1: 522).
-    part     a few long sequences: more splits than a cluster holds, and a merge kernel: 1.1b 1 x 16384 229 / 216 / 542, 368, 276; of 16 (which only
-             heads of 64 find places for) 230, but with 4096 keys 193 against 196.
-    parts    more pairs than places: queries rotated once a launch are cheaper than in every CTA: 8b 32 x 4096 859 / 869 / 873, 994."""
+    cluster  they merge in a cluster, as many as fill the SMs in one or two rounds (a cluster wants its places together: nine tenths of them).
+             Four layers of a model (us, clusters of 1, 2, 4, 8 / as many splits as give every SM four CTAs, with a merge kernel): 1.1b 16 x 2000
+             247, 208, 192, 226 / 215; 8b 8 x 9000 on 8 bits 832, 614, 497, 528 / 542; 8b 3 x 3000 454, 416, 397, 420 / 419 (of 5: 398); 8b 16 x 2000
+             463, 483, 529, 634 / 524; 8b 32 x 4096 736, 752, 835, . / 751.  One sequence: 8b 1 x 4096 484, 428, 398, 388 / 397, of 16 412; 1.1b
+             1 x 4096 300, 238, 200, 181 / 180, of 16 (which heads of 64 find places for) 173.
+    part     more splits than a cluster holds, and a merge kernel: a few very long sequences (1.1b 1 x 16384 199, clusters of 16 202), and batches
+             that would leave the SMs with a last round of few."""
     a_sm = (3 if head_dim == 64 else 2) if fp8 else (2 if head_dim == 64 else 1)      # CTAs, by shared memory
-    places = sm_count() * a_sm * 9 // 10
+    slots = sm_count() * a_sm
+    places = slots * 9 // 10
     many = max(1, min(32, keys // 256, (sm_count() * 4 + pairs - 1) // pairs))
     if pairs <= 8 and many > 8:
-        return ("cluster", 16) if head_dim == 64 and keys <= 8192 else ("part", many)
-    if pairs > places:
-        return "parts", many
-    return "cluster", min(range(1, max(1, min(8, keys // 128)) + 1), key=lambda n: (-(-pairs * n // places) / n, n))
+        if keys <= (8192 if head_dim == 64 else 32768):
+            return "cluster", 16 if head_dim == 64 else 8
+        return "part", many
+
+    def rounds(n):
+        return -(-pairs * n // (places if n > 1 else slots))
+
+    n = min((n for n in range(1, max(1, min(8, keys // 128)) + 1) if n == 1 or rounds(n) <= 2), key=lambda n: (rounds(n) / n, n))
+    if many > 1 and 1.5 * -(-pairs * many // slots) / many < rounds(n) / n:           # (the merge costs a launch)
+        return "part", many
+    return "cluster", n
 
 
 def decode_step(qkv, cos, sin, positions, slots, heads: int, kv_heads: int, head_dim: int, k_cache, v_cache, block_tables, context_lens, block_size: int,
@@ -884,14 +892,14 @@ def decode_step(qkv, cos, sin, positions, slots, heads: int, kv_heads: int, head
     sequence attends to its context, whose last token is the row's.  Returns [S, heads, head_dim].  Block tables, lengths and the cached rows
     before were complete when the step's embedding was launched.  positions, slots, context_lens [S], block_tables [S, width]: int32.
 
-    splits: how many the keys of a (sequence, KV head) are cut into (0: by size).  One launch, or two; caches that it does not take and large
-    batches go through rope_append and paged_decode."""
+    splits: how many the keys of a (sequence, KV head) are cut into (0: by size).  One launch, or two; caches that it does not take go through
+    rope_append and paged_decode."""
     S, D = qkv.shape[0], head_dim
     fp8 = k_cache.dtype == torch.float8_e4m3fn
     how = "part"
     if splits <= 0:
         how, splits = _decode_splits(max(1, S * kv_heads), block_tables.shape[1] * block_size, D, fp8)
-    if (how != "parts" and qkv.dtype == torch.bfloat16 and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0 and D in (64, 128) and heads % kv_heads == 0 and heads // kv_heads <= 16
+    if (qkv.dtype == torch.bfloat16 and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0 and D in (64, 128) and heads % kv_heads == 0 and heads // kv_heads <= 16
             and block_size % 8 == 0 and (32 % block_size == 0 or block_size % 32 == 0) and k_cache.is_contiguous() and v_cache.is_contiguous()
             and _aligned(qkv, cos, sin, k_cache, v_cache)):
         assert qkv.dim() == 2 and qkv.shape[1] >= (heads + 2 * kv_heads) * D and k_cache.dtype == v_cache.dtype and (fp8 or k_cache.dtype == torch.bfloat16)

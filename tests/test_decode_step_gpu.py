@@ -56,15 +56,15 @@ def test_splits_by_size():
     from litetorch_b200.ops import kernels as K
     sms = K.sm_count()
     seen = set()
-    for pairs in (1, 4, 8, 9, 24, 64, 96, 128, 256, 512):
-        for keys in (16, 300, 1000, 4096, 16384):
+    for pairs in (1, 4, 8, 9, 24, 64, 96, 128, 160, 256, 512):
+        for keys in (16, 300, 1000, 4096, 16384, 70000):
             for D in (64, 128):
                 for fp8 in (False, True):
                     how, n = K._decode_splits(pairs, keys, D, fp8)
                     seen.add(how)
                     assert n >= 1 and (how != "cluster" or n <= 16) and (n == 1 or keys // n >= 100)
                     assert how != "cluster" or n == 1 or n <= 8 or (D == 64 and pairs * n <= sms)
-    assert seen == {"cluster", "part", "parts"}
+    assert seen == {"cluster", "part"}
 
 
 def test_tokens_without_a_slot_and_caches_it_does_not_take():
