@@ -63,20 +63,20 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restri
 
 // Rotation of queries and keys and the write of keys and values into a paged cache, in one pass over the rows [q | k | v] of a product.
 // Queries go to q_out, packed, or stay where they are (q_out nullptr: keys are then rotated in place too, for a prompt's own attention).
-// A launch for each of these (two rotations, two or three copies, the write) took 9 to 16 us a layer of a decode step, this one 2.
-template <bool FP8>
+// A launch for each of these (two rotations, two or three copies, the write) took 9 to 16 us a layer of a decode step, this one 2.  Items are counted
+// in 32 bits where they fit: three 64-bit divisions an item were most of a prompt's time here (12 us a layer of 4096 tokens, 8 without).
+template <bool FP8, typename IDX>
 __global__ void rope_append_kernel(__nv_bfloat16* __restrict__ qkv, long long ld, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                    const int* __restrict__ pos, const int* __restrict__ slots, __nv_bfloat16* __restrict__ q_out,
-                                   void* __restrict__ k_cache, void* __restrict__ v_cache, long long rows, int Hq, int Hkv, int hd, int block_size,
+                                   void* __restrict__ k_cache, void* __restrict__ v_cache, IDX rows, int Hq, int Hkv, int hd, int block_size,
                                    float k_inv, float v_inv) {
   pdl_launch_dependents();
   pdl_wait();
   const int vph = hd / 8, heads = Hq + 2 * Hkv;
-  const long long total = rows * heads * vph;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int v = int(i % vph);
-    const int h = int((i / vph) % heads);
-    const long long r = i / ((long long)vph * heads);
+  const IDX per_row = IDX(heads) * vph, total = rows * per_row;
+  for (IDX i = IDX(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += IDX(gridDim.x) * blockDim.x) {
+    const long long r = i / per_row;
+    const int c = int(i - IDX(r) * per_row), h = c / vph, v = c - h * vph;
     __nv_bfloat16* p = qkv + r * ld + (long long)h * hd + v * 8;
     float f[8];
     ld8(p, f);
@@ -463,10 +463,14 @@ int lt_rope_append(void* qkv, long long ld, const float* cos_t, const float* sin
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   auto X = static_cast<__nv_bfloat16*>(qkv);
   auto Q = static_cast<__nv_bfloat16*>(q_out);
-  if (kv_fp8)
-    LT_RETURN_IF_CUDA(launch_chained(rope_append_kernel<true>, grid_for(work, 256), 256, 0, st, X, ld, cos_t, sin_t, pos, slots, Q, k_cache, v_cache, rows, Hq, Hkv, hd, block_size, 1.f / k_scale, 1.f / v_scale));
-  else
-    LT_RETURN_IF_CUDA(launch_chained(rope_append_kernel<false>, grid_for(work, 256), 256, 0, st, X, ld, cos_t, sin_t, pos, slots, Q, k_cache, v_cache, rows, Hq, Hkv, hd, block_size, 1.f, 1.f));
+  const int grid = grid_for(work, 256);
+  const bool small = work + (long long)grid * 256 < (1ll << 32);     // (see rope_kernel)
+  const float ki = kv_fp8 ? 1.f / k_scale : 1.f, vi = kv_fp8 ? 1.f / v_scale : 1.f;
+#define LT_ROPE_APPEND(F8, IDX) \
+  LT_RETURN_IF_CUDA(launch_chained(rope_append_kernel<F8, IDX>, grid, 256, 0, st, X, ld, cos_t, sin_t, pos, slots, Q, k_cache, v_cache, rows, Hq, Hkv, hd, block_size, ki, vi))
+  if (kv_fp8) { if (small) LT_ROPE_APPEND(true, unsigned); else LT_ROPE_APPEND(true, long long); }
+  else { if (small) LT_ROPE_APPEND(false, unsigned); else LT_ROPE_APPEND(false, long long); }
+#undef LT_ROPE_APPEND
   LT_LAUNCH_CHECK();
   return 0;
 }

@@ -36,10 +36,10 @@ class RavenexModel(ServingModel):
         """The output on its way into the residual (arguments of `residual_norm`)."""
         K, f = self.e.K, lay.mlp
         if not isinstance(lay.cfg.mlp, MoeConfig):
-            return dict(y=K.glu_mlp(h, f.gu, f.down, "gelu"))
+            return dict(y=K.glu_mlp(h, f.gu, f.down, "gelu", constant=True))
         out = dict(experts=K.moe_experts(h, f.router, f.correction, f.cfg.top, f.gu, f.down, "silu"))
         if f.shared is not None:
-            out["y"] = K.glu_mlp(h, f.shared.gu, f.shared.down, "silu")
+            out["y"] = K.glu_mlp(h, f.shared.gu, f.shared.down, "silu", constant=True)
         return out
 
     def _layers(self, tok: torch.Tensor, attention):
@@ -51,15 +51,15 @@ class RavenexModel(ServingModel):
         pending = dict(tokens=tok, embed=e.embed)
         for i, lay in enumerate(e.layers):
             h = K.residual_norm(x, cfg.eps, norm=lay.norm1, **opt, **pending)
-            o = attention(i, lay, K.linear(h, lay.mix.w_in))
-            pending = dict(y=K.linear(o, lay.mix.o), y_norm=lay.norm1b)
+            o = attention(i, lay, K.linear(h, lay.mix.w_in, constant=True))
+            pending = dict(y=K.linear(o, lay.mix.o, constant=True), y_norm=lay.norm1b)
             if lay.mlp is not None:
                 h = K.residual_norm(x, cfg.eps, norm=lay.norm2, **opt, **pending)
                 pending = dict(self._feed_forward(lay, h), y_norm=lay.norm2b)
             if cfg.side_dim:
                 h = K.residual_norm(x, cfg.eps, **opt, **pending)
-                g = K.token_gate(K.linear(h, lay.side_gate), tok, e.side_embed, i * cfg.side_dim, cfg.side_dim)
-                pending = dict(y=K.linear(g, lay.side_proj), y_norm=lay.side_norm)
+                g = K.token_gate(K.linear(h, lay.side_gate, constant=True), tok, e.side_embed, i * cfg.side_dim, cfg.side_dim)
+                pending = dict(y=K.linear(g, lay.side_proj, constant=True), y_norm=lay.side_norm)
         return x, pending
 
     def _logits(self, hidden, rows: Optional[List[int]] = None) -> torch.Tensor:
@@ -70,7 +70,7 @@ class RavenexModel(ServingModel):
             rows = (torch.tensor(rows, dtype=torch.int32, device=e.device) if run is None else      # (a copy that is waited for)
                     torch.arange(run.start, run.stop, dtype=torch.int32, device=e.device))
         h = K.residual_norm(x, e.cfg.eps, norm=e.final_norm, dtype=e.dtype, mult=e.cfg.residual_mult, rows=rows, write=False, **pending)
-        return K.linear(h, e.head, out_dtype=torch.float32)
+        return K.linear(h, e.head, out_dtype=torch.float32, constant=True)
 
     def _rope(self, i: int, lay, proj, pos, slots, q_out=None, lin=None):
         """Rotates the queries (in place, or into q_out) and writes the layer's own latents, if it has any, to the pages."""

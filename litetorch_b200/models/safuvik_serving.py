@@ -54,14 +54,14 @@ class SafuvikModel(ServingModel):
         for i, lay in enumerate(e.layers):
             h = K.hyper_norm(x, lay.norm1, cfg.eps, dtype=e.dtype, inn=lay.hc1.inn, **pending)
             if isinstance(lay.cfg.mixer, ParallelConfig):
-                left, right = parallel(i, lay, K.linear(h, lay.w_in))
-                pending = dict(y=K.linear(left, lay.left_o), y_norm=lay.left_out, y2=K.linear(right, lay.right_o), y2_norm=lay.right_out)
+                left, right = parallel(i, lay, K.linear(h, lay.w_in, constant=True))
+                pending = dict(y=K.linear(left, lay.left_o, constant=True), y_norm=lay.left_out, y2=K.linear(right, lay.right_o, constant=True), y2_norm=lay.right_out)
             else:
-                pending = dict(y=K.linear(mlstm(i, lay, K.linear(h, lay.w_in), K.rows_dot(h, lay.w_if)), lay.o))
+                pending = dict(y=K.linear(mlstm(i, lay, K.linear(h, lay.w_in, constant=True), K.rows_dot(h, lay.w_if)), lay.o, constant=True))
             pending.update(mix=lay.hc1.mix, out=lay.hc1.out)
             if lay.cfg.mlp is not None:
                 h = K.hyper_norm(x, lay.norm2, cfg.eps, dtype=e.dtype, inn=lay.hc2.inn, **pending)
-                y = K.linear(K.clamped_glu(K.linear(h, lay.w_gu), lay.cfg.mlp.limit), lay.w_down)
+                y = K.linear(K.clamped_glu(K.linear(h, lay.w_gu, constant=True), lay.cfg.mlp.limit), lay.w_down, constant=True)
                 pending = dict(y=y, mix=lay.hc2.mix, out=lay.hc2.out)
         return x, pending
 

@@ -985,20 +985,21 @@ def _f32(t) -> int:
     return 0
 
 
-def linear(x: torch.Tensor, w: torch.Tensor, out_dtype=None, alpha: float = 1.0) -> torch.Tensor:
+def linear(x: torch.Tensor, w: torch.Tensor, out_dtype=None, alpha: float = 1.0, constant: bool = False) -> torch.Tensor:
     """alpha * x[M, K] @ w[N, K]^T.  bf16 goes to the tensor-core GEMMs of `gemm`; fp32, and bf16 operands that TMA cannot
-    describe (K or a pitch not a multiple of 8), to the CUDA-core kernel."""
+    describe (K or a pitch not a multiple of 8), to the CUDA-core kernel.  constant: no kernel of the pass writes w, see `product_of_constants`."""
     out_dtype = out_dtype or x.dtype
     assert x.stride(1) == 1 and w.is_contiguous() and x.dtype == w.dtype and x.shape[1] == w.shape[1]
     (M, Kd), N = x.shape, w.shape[0]
     if M == 0:
         return torch.empty((0, N), dtype=out_dtype, device=x.device)
     if x.dtype == torch.bfloat16 and Kd % 8 == 0 and (M == 1 or x.stride(0) % 8 == 0) and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0:
-        if M <= 16 and out_dtype == torch.float32 and alpha == 1.0 and (M == 1 or x.stride(0) >= Kd):
+        f32 = out_dtype == torch.float32
+        if alpha == 1.0 and (M == 1 or x.stride(0) >= Kd) and ((f32 and M <= 16) or (constant and M <= 64 and out_dtype == torch.bfloat16)):
             # few rows with 32-bit results (a head): the matrix is read once (16 x 32000 x 2048: 33 us on tiles of 128 rows, 21 here)
             y = torch.empty((M, N), dtype=out_dtype, device=x.device)
-            rc = _fn("lt_weight_stream_norm")(x.data_ptr(), x.stride(0) if M > 1 else Kd, None, 0.0, w.data_ptr(), Kd, y.data_ptr(), N, 1, None, 0, M, N, Kd, 0, 0,
-                                              _stream())
+            rc = _fn("lt_weight_stream_norm")(x.data_ptr(), x.stride(0) if M > 1 else Kd, None, 0.0, w.data_ptr(), Kd, y.data_ptr(), N, 1 if f32 else 0, None, 0, M,
+                                              N, Kd, 0, 1 if constant else 0, _stream())
             _check(rc, "lt_weight_stream_norm")
             return y
         return gemm(x, w, out_dtype=out_dtype, alpha=alpha)
@@ -1313,10 +1314,12 @@ def gemm_staged(a, b, *, act: str = "", alpha: float = 1.0, block_n: int = 0):
     return y
 
 
-def glu_rows(x, gu, act: str):
-    """act(gate @ x) * (up @ x) with gu = [gate; up]; bf16 gates in the product's epilogue."""
+def glu_rows(x, gu, act: str, constant: bool = False):
+    """act(gate @ x) * (up @ x) with gu = [gate; up]; bf16 gates in the product's epilogue.  constant: as in `linear`."""
     M, Kd = x.shape
     F = gu.shape[0] // 2
+    if constant and x.dtype == torch.bfloat16 and 0 < M <= 64 and Kd % 8 == 0 and gu.is_contiguous() and x.stride(0) % 8 == 0 and x.stride(0) >= Kd and _aligned(x, gu):
+        return product_of_constants(x, gu, act=act)
     if x.dtype == torch.bfloat16 and 0 < M <= 128 and Kd % 32 == 0 and F % 8 == 0 and x.stride(0) % 8 == 0 and _aligned(x, gu):
         h = torch.empty((M, F), dtype=x.dtype, device=x.device)
         rc = _fn("lt_gemm_skinny_glu")(x.data_ptr(), x.stride(0), gu.data_ptr(), h.data_ptr(), M, F, Kd, _ACT[act], _stream())
@@ -1327,9 +1330,9 @@ def glu_rows(x, gu, act: str):
     return act_glu(linear(x, gu), act)
 
 
-def glu_mlp(x, gu, down, act: str):
+def glu_mlp(x, gu, down, act: str, constant: bool = False):
     """down @ glu_rows(x)."""
-    return linear(glu_rows(x, gu, act), down)
+    return linear(glu_rows(x, gu, act, constant), down, constant=constant)
 
 
 def moe_plan(logits, correction, top: int, block_rows: int, x=None):

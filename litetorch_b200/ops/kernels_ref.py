@@ -319,7 +319,7 @@ def clamped_glu(gu, limit, slope=1.702):
     return (g * torch.sigmoid(slope * g) * (u + 1)).to(gu.dtype)
 
 
-def linear(x, w, out_dtype=None, alpha=1.0):
+def linear(x, w, out_dtype=None, alpha=1.0, constant=False):
     return (x.float() @ w.float().t() * alpha).to(out_dtype or x.dtype)
 
 
@@ -561,11 +561,11 @@ def act_glu(gu, act):
     return (_ACT[act](g) * u).to(gu.dtype)
 
 
-def glu_rows(x, gu, act):
+def glu_rows(x, gu, act, constant=False):
     return act_glu(linear(x, gu), act)
 
 
-def glu_mlp(x, gu, down, act):
+def glu_mlp(x, gu, down, act, constant=False):
     return linear(glu_rows(x, gu, act), down)
 
 

@@ -53,3 +53,25 @@ def test_32_bit_results(M, N, Kd):
     want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
     assert y.dtype == torch.float32 and ((y.double() - want).abs() <= size * 2.0 ** -20).all()
     assert K.status_fetch() == 0
+
+
+@pytest.mark.parametrize("M,N,Kd", [(1, 1, 8), (1, 1000, 72), (7, 129, 1024), (17, 96, 200), (64, 257, 512), (65, 96, 512)])
+@pytest.mark.parametrize("strided", [False, True])
+def test_products_with_constant_matrices(M, N, Kd, strided):
+    from litetorch_b200.ops import kernels as K
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.randn(M, Kd + (24 if strided else 0), device="cuda", generator=g).bfloat16()[:, :Kd]
+    w = (torch.randn(2 * N, Kd, device="cuda", generator=g) * Kd ** -0.5).bfloat16()
+    want = x.double() @ w.double().t()
+    # 32-bit sums of exact products, one rounding to bf16
+    slack = (x.double().abs() @ w.double().abs().t()) * (Kd * 2.0 ** -24)
+    for dtype, unit in ((torch.bfloat16, 2.0 ** -8), (torch.float32, 2.0 ** -23)):
+        got = K.linear(x, w, out_dtype=dtype, constant=True).double()
+        assert ((got - want).abs() <= want.abs() * unit + slack).all()
+    gate, up = want[:, :N], want[:, N:]
+    for act, f in (("silu", torch.nn.functional.silu), ("gelu", lambda v: torch.nn.functional.gelu(v, approximate="tanh"))):
+        got = K.glu_rows(x, w, act, constant=True).double()
+        # 1.13: the steepest that either gate is; more than 64 rows round gate and up to bf16 first
+        e = (2.0 ** -8 if M > 64 else 0) + 2.0 ** -18
+        assert ((got - f(gate) * up).abs() <= (f(gate) * up).abs() * 2.0 ** -8 + 1.13 * (gate.abs() * up.abs() * 2 * e + slack[:, :N] * up.abs() + slack[:, N:] * gate.abs()) + 1e-6).all()
+    assert K.status_fetch() == 0
