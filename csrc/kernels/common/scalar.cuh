@@ -92,6 +92,19 @@ __device__ __forceinline__ float2 block_sum2(float a, float b, float* red) {
   return make_float2(sa, sb);
 }
 
+// Sum of v over the W warps of a group, given to all of them.  `sums` alternates between two arrays from call to call: what is read here is
+// overwritten only after the next call's barrier.
+__device__ __forceinline__ float row_sum(float v, float* sums, int W, int group, int warp, int lane) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (W == 1) return v;
+  if (lane == 0) sums[warp] = v;
+  asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(W * 32) : "memory");
+  v = 0.f;
+  for (int k = 0; k < W; ++k) v += sums[group * W + k];
+  return v;
+}
+
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + expf(-x)); }
 // SiLU for results that leave as bf16: the quick exponential and quotient (a few units in the last place of fp32).  The divisor is between 1
 // and 2: the quick quotient gives zero once it passes 2^126, which 1 + e^-x does for x from -88.8 to -87.3.

@@ -8,6 +8,7 @@
 #include "lt_cuda.h"
 #include "common/host.h"
 #include "common/ptx.cuh"
+#include "common/scalar.cuh"
 
 #include <mutex>
 
@@ -45,19 +46,6 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
   u.x = pack_bf16x2(f[0], f[1]); u.y = pack_bf16x2(f[2], f[3]);
   u.z = pack_bf16x2(f[4], f[5]); u.w = pack_bf16x2(f[6], f[7]);
   *reinterpret_cast<uint4*>(p) = u;
-}
-
-// Sum of v over the W warps of a group, given to all of them.  `sums` alternates between two arrays from call to call: what is read here is
-// overwritten only after the next call's barrier.
-__device__ __forceinline__ float row_sum(float v, float* sums, int W, int group, int warp, int lane) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if (W == 1) return v;
-  if (lane == 0) sums[warp] = v;
-  asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(W * 32) : "memory");
-  v = 0.f;
-  for (int k = 0; k < W; ++k) v += sums[group * W + k];
-  return v;
 }
 
 // y = norm(x (+ res)) * w (+ b).  RMS: mean unused.  If sum_out != nullptr the pre-norm sum is stored.

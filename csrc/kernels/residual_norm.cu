@@ -169,6 +169,91 @@ __global__ void __launch_bounds__(max_threads(V)) residual_norm_kernel(const Res
   }
 }
 
+// Many rows (bf16, width = 512 * W, no expert rows): W warps of a CTA share a row, a lane owns 16 of its columns.  The norms' weights are read
+// once, the next row is fetched while this one is worked on, and each of a row's two sums costs one barrier of its warps alone.  Bound by HBM.
+// A CTA a row / this: 296 x 2048 6.3 / 3.6 us, 1337 x 2048 12.7 / 9.5, 4096 x 2048 25.9 / 20.7, 4096 x 1024 14.4 / 11.7, 2048 x 4096 28.6 / 22.7,
+// 8192 x 2048 47.0 / 39.9 (bytes at the copy rate: 1.1, 4.9, 15.1, 7.6, 15.1, 30.3).
+__global__ void __launch_bounds__(256, 2) residual_norm_wide_kernel(const ResidualParams p, int n, int W) {
+  __shared__ float sums[2][8];
+  constexpr int IT = 4;                         // pieces of 4 columns a lane
+  const int D = 128 * IT * W;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, group = warp / W, sub = warp - group * W;
+  const int groups = (blockDim.x >> 5) / W, step = gridDim.x * groups;
+  const int c0 = (sub * IT * 32 + lane) * 4;    // column of piece i: c0 + 128 i
+  using bf16 = __nv_bfloat16;
+  float4 wy[IT], wn[IT];
+  pdl_launch_dependents();
+  pdl_wait();
+#pragma unroll
+  for (int i = 0; i < IT; ++i) {
+    wy[i] = p.y_norm ? ldf4(p.y_norm + c0 + i * 128) : make_float4(1.f, 1.f, 1.f, 1.f);
+    wn[i] = p.norm ? ldf4(p.norm + c0 + i * 128) : make_float4(1.f, 1.f, 1.f, 1.f);
+  }
+  float4 nx[IT];                                // the next row of this group: residual (or embedding) and output
+  uint2 ny[IT];
+  auto fetch = [&](int r) {
+    const long long row = p.rows ? p.rows[r] : r;
+    if (p.embed) {
+      const bf16* e = static_cast<const bf16*>(p.embed) + (long long)p.tokens[row] * D + c0;
+#pragma unroll
+      for (int i = 0; i < IT; ++i) nx[i] = ldf4(e + i * 128);
+    } else {
+#pragma unroll
+      for (int i = 0; i < IT; ++i) nx[i] = ldf4(p.x + row * D + c0 + i * 128);
+    }
+    if (p.y) {
+      const bf16* y = static_cast<const bf16*>(p.y) + row * p.ldy + c0;
+#pragma unroll
+      for (int i = 0; i < IT; ++i) ny[i] = *reinterpret_cast<const uint2*>(y + i * 128);
+    }
+  };
+  int r = blockIdx.x * groups + group, turn = 0;
+  if (r < n) fetch(r);
+  for (; r < n; r += step) {
+    float4 x[IT];
+    uint2 y[IT];
+#pragma unroll
+    for (int i = 0; i < IT; ++i) { x[i] = nx[i]; y[i] = ny[i]; }
+    if (r + step < n) fetch(r + step);
+    if (p.y) {
+      float f = p.mult;
+      if (p.y_norm) {
+        float ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < IT; ++i) {
+          const float2 a = unpack_bf16x2(y[i].x), b = unpack_bf16x2(y[i].y);
+          ss = fmaf(a.x, a.x, ss); ss = fmaf(a.y, a.y, ss); ss = fmaf(b.x, b.x, ss); ss = fmaf(b.y, b.y, ss);
+        }
+        f *= 1.f / sqrtf(row_sum(ss, sums[turn], W, group, warp, lane) / D + p.eps);
+        turn ^= 1;
+      }
+#pragma unroll
+      for (int i = 0; i < IT; ++i) {
+        const float2 a = unpack_bf16x2(y[i].x), b = unpack_bf16x2(y[i].y);
+        x[i].x = fmaf(f, a.x * wy[i].x, x[i].x); x[i].y = fmaf(f, a.y * wy[i].y, x[i].y);
+        x[i].z = fmaf(f, b.x * wy[i].z, x[i].z); x[i].w = fmaf(f, b.y * wy[i].w, x[i].w);
+      }
+    }
+    if (p.write_x) {
+      float* xw = p.x + (p.rows ? p.rows[r] : r) * (long long)D + c0;
+#pragma unroll
+      for (int i = 0; i < IT; ++i) stf4(xw + i * 128, x[i]);
+    }
+    float inv = 1.f;
+    if (p.norm) {
+      float ss = 0.f;
+#pragma unroll
+      for (int i = 0; i < IT; ++i) { ss = fmaf(x[i].x, x[i].x, ss); ss = fmaf(x[i].y, x[i].y, ss); ss = fmaf(x[i].z, x[i].z, ss); ss = fmaf(x[i].w, x[i].w, ss); }
+      inv = 1.f / sqrtf(row_sum(ss, sums[turn], W, group, warp, lane) / D + p.eps);
+      turn ^= 1;
+    }
+    bf16* h = static_cast<bf16*>(p.h) + (long long)r * D + c0;
+#pragma unroll
+    for (int i = 0; i < IT; ++i)
+      stf4(h + i * 128, make_float4(x[i].x * inv * wn[i].x, x[i].y * inv * wn[i].y, x[i].z * inv * wn[i].z, x[i].w * inv * wn[i].w));
+  }
+}
+
 template <typename T, int V>
 static int launch_residual(const ResidualParams& p, int rows, cudaStream_t st) {
   const int pieces = (p.width + V - 1) / V;
@@ -201,6 +286,14 @@ int lt_residual_norm(int fp32, float* x, const int* tokens, const void* embed, c
   auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   const bool vec = width % 4 == 0 && ldy % 4 == 0 && al(x) && al(embed) && al(y) && al(z) && al(h);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // Two rows an SM and more (below that a CTA a row has more loads in flight), four pieces a lane (with two, 4096 x 768 took 14.8 us, a CTA a row 11.9).
+  const int wide = width / 512;
+  if (!fp32 && vec && !z && n_rows >= 2 * sm_count() && width % 512 == 0 && wide <= 8 && al(y_norm) && al(norm)) {
+    const int groups = 8 / wide, need = (n_rows + groups - 1) / groups, full = 2 * sm_count();
+    LT_RETURN_IF_CUDA(launch_chained(residual_norm_wide_kernel, need < full ? need : full, wide * groups * 32, 0, st, p, n_rows, wide));
+    LT_LAUNCH_CHECK();
+    return 0;
+  }
   if (fp32) return vec ? launch_residual<float, 4>(p, n_rows, st) : launch_residual<float, 1>(p, n_rows, st);
   return vec ? launch_residual<__nv_bfloat16, 4>(p, n_rows, st) : launch_residual<__nv_bfloat16, 1>(p, n_rows, st);
 }
