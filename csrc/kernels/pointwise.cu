@@ -194,16 +194,30 @@ __global__ void act_glu_kernel(const T* __restrict__ gu, T* __restrict__ h, long
   }
 }
 
-// out[n, c] = gelu(g[n, c]) * table[tokens[n], off + c] for c < dim, zero up to ld: a token's own input, gated.
-template <typename T>
+// out[n, c] = gelu(g[n, c]) * table[tokens[n], off + c] for c < dim, zero up to ld: a token's own input, gated.  A thread takes V columns (8 where all
+// pieces are aligned: one load each instead of eight, and a division a piece; 4096 x 256: 5.8 us a column at a time, 3.4 so).
+template <typename T, int V>
 __global__ void token_gate_kernel(const T* __restrict__ g, const int* __restrict__ tokens, const T* __restrict__ table, long long ldt,
                                   int off, int dim, int ld, T* __restrict__ out, long long total) {
   pdl_launch_dependents();
   pdl_wait();
+  const int pieces = ld / V;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long n = i / ld;
-    const int c = int(i - n * ld);
-    stf(out + i, c < dim ? gelu_tanh_f(ldf(g + i)) * ldf(table + tokens[n] * ldt + off + c) : 0.f);
+    const long long n = total < (1ll << 31) ? int(i) / pieces : i / pieces;
+    const int c = int(i - n * pieces) * V;
+    if constexpr (V == 8) {
+      float a[8], t[8];
+      if (c < dim) {
+        ldf8(table + tokens[n] * ldt + off + c, t);
+        ldf8(g + i * 8, a);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) a[j] = c < dim ? gelu_tanh_f(a[j]) * t[j] : 0.f;
+      stf4(out + i * 8, make_float4(a[0], a[1], a[2], a[3]));
+      stf4(out + i * 8 + 4, make_float4(a[4], a[5], a[6], a[7]));
+    } else {
+      stf(out + i, c < dim ? gelu_tanh_f(ldf(g + i)) * ldf(table + tokens[n] * ldt + off + c) : 0.f);
+    }
   }
 }
 
@@ -513,12 +527,17 @@ int lt_token_gate(int fp32, const void* g, const int* tokens, const void* table,
                   int n, void* stream) {
   using namespace lt;
   if (dim > ld) return -int(kStatusBadArgument);
-  const long long total = (long long)n * ld;
-  if (total == 0) return 0;
+  if ((long long)n * ld == 0) return 0;
+  const bool wide = ((dim | ld | off | ldt) & 7) == 0 &&
+                    ((reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  const long long total = (long long)n * (wide ? ld / 8 : ld);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   using bf = __nv_bfloat16;
-  if (fp32) LT_RETURN_IF_CUDA(launch_chained(token_gate_kernel<float>, grid_for(total, 256), 256, 0, st, static_cast<const float*>(g), tokens, static_cast<const float*>(table), ldt, off, dim, ld, static_cast<float*>(out), total));
-  else LT_RETURN_IF_CUDA(launch_chained(token_gate_kernel<bf>, grid_for(total, 256), 256, 0, st, static_cast<const bf*>(g), tokens, static_cast<const bf*>(table), ldt, off, dim, ld, static_cast<bf*>(out), total));
+#define LT_TOKEN_GATE(T, V) \
+  LT_RETURN_IF_CUDA(launch_chained(token_gate_kernel<T, V>, grid_for(total, 256), 256, 0, st, static_cast<const T*>(g), tokens, static_cast<const T*>(table), ldt, off, dim, ld, static_cast<T*>(out), total))
+  if (fp32) { if (wide) LT_TOKEN_GATE(float, 8); else LT_TOKEN_GATE(float, 1); }
+  else { if (wide) LT_TOKEN_GATE(bf, 8); else LT_TOKEN_GATE(bf, 1); }
+#undef LT_TOKEN_GATE
   LT_LAUNCH_CHECK();
   return 0;
 }
