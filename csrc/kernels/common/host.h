@@ -69,6 +69,25 @@ inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, s
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// The same with CTAs in clusters of `cluster` along x.
+template <class... P, class... A>
+inline cudaError_t launch_chained_clusters(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, int cluster, cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr[2]{};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 inline int cuda_ok(cudaError_t e) { return e == cudaSuccess ? 0 : int(e); }
 
 }  // namespace lt

@@ -239,6 +239,12 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The word at the same shared-memory offset in CTA `cta` of the cluster.
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr, int cta) {
+  float v;
+  asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.f32 %0, [ra];\n\t}" : "=f"(v) : "r"(addr), "r"(cta) : "memory");
+  return v;
+}
 // Arrive on the barrier at the same shared-memory offset in CTA `cta` of the cluster.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar, uint32_t cta) {
   asm volatile(

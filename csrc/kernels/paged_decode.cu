@@ -488,11 +488,6 @@ __device__ __forceinline__ long long pd_newest_at(const PdStep& f, int s, int hk
   if (slot < 0 || lane >= D / 4) return -1;
   return (((long long)(slot / block_size) * Hkv + hkv) * block_size + slot % block_size) * D + (lane % (D / 8)) * 8;
 }
-__device__ __forceinline__ float ld_cluster_f32(uint32_t addr, int cta) {
-  float v;
-  asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.f32 %0, [ra];\n\t}" : "=f"(v) : "r"(addr), "r"(cta) : "memory");
-  return v;
-}
 // The cluster's splits (their rows [G][D + 2] at `mine` in each one's shared memory) merged and written, every CTA a share of the G * D results.
 template <int D>
 __device__ __forceinline__ void pd_merge_cluster(const float* mine, __nv_bfloat16* out, int G, int splits, int sp) {
@@ -1158,20 +1153,8 @@ static int launch_clustered(K kernel, int warps, int smem, OncePerDevice& config
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     configured.finish();
   }
-  cudaLaunchAttribute attr[2]{};
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = cluster;
-  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(ctas);
-  cfg.blockDim = dim3(warps * 32);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = attr;
-  cfg.numAttrs = cluster > 1 ? 2 : 1;
-  LT_RETURN_IF_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+  LT_RETURN_IF_CUDA(launch_chained_clusters(kernel, ctas, warps * 32, smem, cluster, st, args...));
+  LT_LAUNCH_CHECK();
   return 0;
 }
 template <bool STEP, int D, int NT>

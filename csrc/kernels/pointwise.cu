@@ -319,41 +319,48 @@ __device__ __forceinline__ bool goes_before(T a, int i, T b, int j) {
   if (na || nb) return na && (!nb || i < j);
   return a > b || (a == b && i < j);
 }
-// Index of the largest element of every row, a CTA a row.  (A conversion to fp32 and a library reduction took 13 us of a decode step; 16 rows of
-// 32000 here 4.)
+// Index of the largest element of every row.  (A conversion to fp32 and a library reduction took 13 us of a decode step.)  A cluster of 1 << log_parts CTAs
+// takes a row and its first one compares their candidates: few long rows leave a CTA a row waiting for one load after the other.  A CTA a row / this:
+// 8 x 32000 5.1 / 3.6 us, 8 x 128256 14.1 / 5.0, 64 x 128256 21.3 / 7.2; more rows than that keep a CTA a row (256 x 32000 7.7 / 5.1: one
+// comparison an element instead of three).
 template <bool F32>
-__global__ void __launch_bounds__(1024) argmax_rows_kernel(const void* __restrict__ x, long long* __restrict__ out, int V, long long ld) {
+__global__ void __launch_bounds__(1024) argmax_rows_kernel(const void* __restrict__ x, long long* __restrict__ out, int V, long long ld, int log_parts) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float bv[32];
   __shared__ int bi[32];
-  const long long row = blockIdx.x;
+  const int parts = 1 << log_parts, part = blockIdx.x & (parts - 1);
+  const long long row = blockIdx.x >> log_parts;
+  const int len = log_parts ? (V / parts + 8) / 8 * 8 : V;
+  const int from = part * len, end = from + len < V ? from + len : V;      // (from beyond V: nothing)
   float best = -INFINITY;
   int at = V;
+  // a thread's elements come in order: a later one goes before only if it is larger, or the first NaN
+  auto see = [&](float v, int i) { if (!(v <= best) && best == best) { best = v; at = i; } };
   auto take = [&](float v, int i) { if (goes_before(v, i, best, at)) { best = v; at = i; } };
   if (F32) {
     const float* r = static_cast<const float*>(x) + row * ld;
     if ((reinterpret_cast<uintptr_t>(r) & 15) == 0) {
-      for (int c = threadIdx.x * 4; c + 3 < V; c += 4096) {
+      for (int c = from + threadIdx.x * 4; c + 3 < end; c += 4096) {
         const float4 f = *reinterpret_cast<const float4*>(r + c);
-        take(f.x, c); take(f.y, c + 1); take(f.z, c + 2); take(f.w, c + 3);
+        see(f.x, c); see(f.y, c + 1); see(f.z, c + 2); see(f.w, c + 3);
       }
-      for (int c = V / 4 * 4 + threadIdx.x; c < V; c += 1024) take(r[c], c);
+      for (int c = end / 4 * 4 + threadIdx.x; c < end; c += 1024) see(r[c], c);
     } else {
-      for (int c = threadIdx.x; c < V; c += 1024) take(r[c], c);
+      for (int c = from + threadIdx.x; c < end; c += 1024) see(r[c], c);
     }
   } else {
     const __nv_bfloat16* r = static_cast<const __nv_bfloat16*>(x) + row * ld;
     if ((reinterpret_cast<uintptr_t>(r) & 15) == 0) {
-      for (int c = threadIdx.x * 8; c + 7 < V; c += 8192) {
+      for (int c = from + threadIdx.x * 8; c + 7 < end; c += 8192) {
         float f[8];
         ld8(r + c, f);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) take(f[j], c + j);
+        for (int j = 0; j < 8; ++j) see(f[j], c + j);
       }
-      for (int c = V / 8 * 8 + threadIdx.x; c < V; c += 1024) take(__bfloat162float(r[c]), c);
+      for (int c = end / 8 * 8 + threadIdx.x; c < end; c += 1024) see(__bfloat162float(r[c]), c);
     } else {
-      for (int c = threadIdx.x; c < V; c += 1024) take(__bfloat162float(r[c]), c);
+      for (int c = from + threadIdx.x; c < end; c += 1024) see(__bfloat162float(r[c]), c);
     }
   }
   auto reduce = [&]() {
@@ -371,8 +378,15 @@ __global__ void __launch_bounds__(1024) argmax_rows_kernel(const void* __restric
     best = bv[threadIdx.x];
     at = bi[threadIdx.x];
     reduce();
-    if (threadIdx.x == 0) out[row] = at < V ? at : 0;
+    if (threadIdx.x == 0) { bv[0] = best; bi[0] = at; }
   }
+  if (parts > 1) {
+    cluster_sync_all();
+    if (part == 0 && threadIdx.x == 0)
+      for (int i = 1; i < parts; ++i) take(ld_cluster_f32(smem_u32(bv), i), __float_as_int(ld_cluster_f32(smem_u32(bi), i)));
+    cluster_sync_all();                  // a CTA's shared memory is read until here
+  }
+  if (part == 0 && threadIdx.x == 0) out[row] = at < V ? at : 0;
 }
 
 // ---------------------------------------------------------------------------------------------- embedding
@@ -612,8 +626,12 @@ int lt_argmax_rows(const void* x, int fp32, long long* out, int rows, int V, lon
   if (rows == 0) return 0;
   if (V < 1) return -int(kStatusBadArgument);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (fp32) LT_RETURN_IF_CUDA(launch_chained(argmax_rows_kernel<true>, rows, 1024, 0, st, x, out, V, ld));
-  else LT_RETURN_IF_CUDA(launch_chained(argmax_rows_kernel<false>, rows, 1024, 0, st, x, out, V, ld));
+  // two CTAs of 1024 threads fit an SM; a part of 4096 elements is one load a thread (fp32)
+  int parts = 3;
+  while (parts > 0 && (((long long)rows << parts) > 2 * sm_count() || (V >> parts) < 4096)) --parts;
+  auto kernel = fp32 ? argmax_rows_kernel<true> : argmax_rows_kernel<false>;
+  if (parts > 0) LT_RETURN_IF_CUDA(launch_chained_clusters(kernel, rows << parts, 1024, 0, 1 << parts, st, x, out, V, ld, parts));
+  else LT_RETURN_IF_CUDA(launch_chained(kernel, rows, 1024, 0, st, x, out, V, ld, 0));
   return 0;
 }
 int lt_embedding_bwd(const long long* idx, const void* dout, void* dtable, long long n_tok, int D, int V, void* stream) {

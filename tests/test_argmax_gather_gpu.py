@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("rows,V", [(1, 1), (3, 7), (2, 1024), (5, 4097), (1, 32000), (7, 32003), (2, 128256)])
+@pytest.mark.parametrize("rows,V", [(1, 1), (3, 7), (2, 1024), (5, 4097), (3, 8192), (40, 16390), (1, 32000), (7, 32003), (70, 32001), (200, 9000), (2, 128256)])
 @pytest.mark.parametrize("odd", [False, True])
 def test_argmax(dtype, rows, V, odd):
     from litetorch_b200.ops import kernels as K
