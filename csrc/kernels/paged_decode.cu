@@ -245,8 +245,9 @@ paged_decode_gqa_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         const float nm = fmaxf(m[g], mx);
+        const float top = nm == -INFINITY ? 0.f : nm;      // (no score above minus infinity: weights of zero, or of NaN for NaN scores)
         const float a = (m[g] == -INFINITY) ? 0.f : __expf(m[g] - nm);
-        const float pv = live ? __expf(sc[g] - nm) : 0.f;
+        const float pv = live ? __expf(sc[g] - top) : 0.f;
         float ps = pv;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, o);
@@ -303,14 +304,14 @@ paged_decode_gqa_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
     float lsum = 0.f, o = 0.f;
 #pragma unroll
     for (int w = 0; w < kPdWarps; ++w) {
-      const float mw = red_m[w * kPdMaxG + g];
-      if (mw == -INFINITY) continue;
-      const float a = __expf(mw - gm);
-      lsum += red_l[w * kPdMaxG + g] * a;
+      const float lw = red_l[w * kPdMaxG + g];
+      if (lw == 0.f) continue;                           // no keys; a NaN goes on
+      const float a = __expf(red_m[w * kPdMaxG + g] - gm);
+      lsum += lw * a;
       o += red_o[(w * kPdMaxG + g) * D + d] * a;
     }
     float* out = part + (((long long)s * Hq + hkv * G + g) * splits + sp) * (D + 2);
-    out[d] = lsum > 0.f ? o / lsum : 0.f;
+    out[d] = lsum == 0.f ? 0.f : o / lsum;
     if (d == 0) { out[D] = gm; out[D + 1] = lsum; }
   }
 }
@@ -405,14 +406,15 @@ __device__ __forceinline__ void pd_softmax(float (&s)[NT][2][4], const float (&f
       }
 #pragma unroll
       for (int o = 4; o <= 16; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      const float nm = fmaxf(m[n][e], mx);   // finite: every chunk has a live key (the first one ends after `lo`)
+      const float nm = fmaxf(m[n][e], mx);   // (fmaxf passes NaN over: a NaN score shows in the sum alone)
+      const float top = nm == -INFINITY ? 0.f : nm;
       a[n][e] = m[n][e] == -INFINITY ? 0.f : __expf(m[n][e] - nm);
       m[n][e] = nm;
       float sum = 0.f;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         float& x = s[n][i >> 1][(i & 1) * 2 + e];
-        x = __expf(x - nm);
+        x = __expf(x - top);
         sum += x;
       }
       l[n][e] = l[n][e] * a[n][e] + sum;
@@ -433,14 +435,14 @@ __device__ __forceinline__ void pd_write_partial(uint8_t* smem, float* part, int
     float lsum = 0.f, o = 0.f;
 #pragma unroll
     for (int w = 0; w < W; ++w) {
-      const float mw = red_m[w * kPdMmaMaxG + gg];
-      if (mw == -INFINITY) continue;
-      const float a = __expf(mw - gm);
-      lsum += red_l[w * kPdMmaMaxG + gg] * a;
+      const float lw = red_l[w * kPdMmaMaxG + gg];
+      if (lw == 0.f) continue;                                     // no keys; a NaN goes on
+      const float a = __expf(red_m[w * kPdMmaMaxG + gg] - gm);
+      lsum += lw * a;
       o += red_o[(w * kPdMmaMaxG + gg) * D + d] * a;
     }
     float* out = part + ((long long)gg * splits + sp) * (D + 2);   // (in shared memory: splits 1, sp 0)
-    out[d] = lsum > 0.f ? o / lsum * out_scale : 0.f;
+    out[d] = lsum == 0.f ? 0.f : o / lsum * out_scale;
     if (d == 0) { out[D] = gm; out[D + 1] = lsum; }
   }
 }
@@ -519,7 +521,7 @@ __device__ __forceinline__ void pd_merge_cluster(const float* mine, __nv_bfloat1
         acc += w * o[i];
       }
     }
-    out[e] = __float2bfloat16(sum > 0.f ? acc / sum : 0.f);
+    out[e] = __float2bfloat16(sum == 0.f ? 0.f : acc / sum);       // zeros only where there is no key at all: a NaN goes out as one
   }
   cluster_sync_all();   // nobody leaves while its rows are read
 }

@@ -96,3 +96,62 @@ def test_not_a_number_past_the_context():
             t[int(bt[s, (n - 1) // 16]), :, (n - 1) % 16:] = math.nan
     b = K.decode_step(qkv, cos, sin, pos, slots, 8, 2, 128, kc, vc, bt, ctx, 16, 2)
     assert torch.equal(a, b) and bool(torch.isfinite(b.float()).all())
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("G,Hkv,D,bs", [(4, 2, 64, 16), (9, 2, 128, 32), (4, 2, 128, 4), (12, 2, 64, 4)])
+@pytest.mark.parametrize("longest,splits", [(20, 0), (20, 2), (700, 0), (700, 1), (700, 8), (3000, 0)])
+def test_not_a_number_inside_the_context(G, Hkv, D, bs, longest, splits, fp8):
+    """A NaN in a query makes its head's results NaN, one in a key that is seen those of the key's group, however the keys are cut into splits and
+    whichever kernel takes the shape; the other results stay as they are."""
+    from litetorch_b200.ops import kernels as K
+    H = G * Hkv
+    qkv, cos, sin, pos, slots, kc, vc, bt, ctx, lens = _case(3, G, Hkv, D, bs, longest, fp8, longest + D)
+    run = lambda q, k, v: K.decode_step(q, cos, sin, pos, slots, H, Hkv, D, k, v, bt, ctx, bs, splits)                       # noqa: E731
+    parts = lambda q, k, v: K.paged_decode(K.rope_append(q.clone(), cos, sin, pos, slots, H, Hkv, D, k, v, bs, fp8), k, v, bt, ctx, bs,   # noqa: E731
+                                           max(1, splits), D ** -0.5)
+    for attend in (run, parts):
+        base = attend(qkv, kc.clone(), vc.clone())
+        assert bool(torch.isfinite(base.float()).all())
+        q = qkv.clone()
+        q[1, 2 * D + 5] = math.nan                                      # head 2 of sequence 1
+        want = torch.zeros_like(base, dtype=torch.bool)
+        want[1, 2] = True
+        got = attend(q, kc.clone(), vc.clone())
+        assert torch.equal(torch.isnan(got), want) and torch.equal(got[~want], base[~want])
+        # an older key of sequence 0's second group, and the newest of sequence 2's first
+        k = kc.clone()
+        at = lens[0] // 2
+        k[int(bt[0, at // bs]), 1, at % bs, 3] = math.nan
+        q = qkv.clone()
+        q[2, H * D + 7] = math.nan
+        want = torch.zeros_like(base, dtype=torch.bool)
+        want[0, G:] = True
+        want[2, :G] = True
+        got = attend(q, k, vc.clone())
+        assert torch.equal(torch.isnan(got), want) and torch.equal(got[~want], base[~want])
+    assert K.status_fetch() == 0
+
+
+@pytest.mark.parametrize("D,bs", [(64, 16), (128, 16), (128, 4)])
+@pytest.mark.parametrize("longest,splits", [(700, 0), (700, 8), (3000, 0)])
+def test_scores_of_minus_infinity(D, bs, longest, splits):
+    """Keys whose scores are too far below zero for 32 bits have weights of zero, chunks of nothing else included."""
+    from litetorch_b200.ops import kernels as K
+    G, Hkv = 4, 2
+    qkv, cos, sin, pos, slots, kc, vc, bt, ctx, lens = _case(2, G, Hkv, D, bs, longest, False, longest + D)
+    cos.fill_(1.0)
+    sin.zero_()
+    qkv[:, :G * Hkv * D].abs_().add_(0.5)
+    n, dead = lens[0], 256
+    at = torch.arange(n, device="cuda")
+    cells = bt[0].long()[at // bs], at % bs
+    kc[cells[0][:dead], :, cells[1][:dead]] = -3e38
+    o = K.decode_step(qkv, cos, sin, pos, slots, G * Hkv, Hkv, D, kc, vc, bt, ctx, bs, splits)
+    kk, vv = kc[cells[0], :, cells[1]].double(), vc[cells[0], :, cells[1]].double()
+    p = torch.softmax(torch.einsum("hgd,nhd->hgn", qkv[0, :G * Hkv * D].double().view(Hkv, G, D), kk) * D ** -0.5, -1)
+    assert float(p[..., :dead].abs().max()) == 0.0
+    ref, size = (torch.einsum("hgn,nhd->hgd", p, v).reshape(G * Hkv, D) for v in (vv, vv.abs()))
+    # roundings of the result and of the weights, each within 2^-9 of itself
+    assert ((o[0].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + size * 2.0 ** -8 + 1e-4).all()
+    assert K.status_fetch() == 0
