@@ -568,7 +568,7 @@ __global__ void __launch_bounds__(128) latent_merge_kernel(const float* __restri
     m = warp_max(m);
     for (int i = threadIdx.x; i < splits; i += 32) {
       const float2 v = st[i];
-      const float f = v.y > 0.f ? exp2f(v.x - m) : 0.f;
+      const float f = v.y == 0.f ? 0.f : exp2f(v.x - m);        // zero: no keys; a NaN goes on
       share[i] = f;
       l = fmaf(v.y, f, l);
     }
@@ -585,11 +585,11 @@ __global__ void __launch_bounds__(128) latent_merge_kernel(const float* __restri
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         f[i] = i0 + i < splits ? share[i0 + i] : 0.f;
-        if (f[i] > 0.f) v[i] = ldf4(src + (long long)(i0 + i) * c);    // a split without keys has written no outputs
+        if (f[i] != 0.f) v[i] = ldf4(src + (long long)(i0 + i) * c);   // a split without keys has written no outputs
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i)
-        if (f[i] > 0.f) {
+        if (f[i] != 0.f) {
           a.x = fmaf(f[i], v[i].x, a.x); a.y = fmaf(f[i], v[i].y, a.y); a.z = fmaf(f[i], v[i].z, a.z); a.w = fmaf(f[i], v[i].w, a.w);
         }
     }

@@ -58,3 +58,33 @@ def test_gates(dtype, N, F, dim, off, width):
     err = want.abs() * 2.0 ** -8 if dtype == torch.bfloat16 else 0
     assert ((o[:, :dim].double() - want).abs() <= err + 2.0 ** -20 * t.abs() * (1 + x[:, :dim].double().abs())).all()
     assert not bool(o[:, dim:].any())
+
+
+@pytest.mark.parametrize("H,rank,w,window", [(4, 128, 192, 0), (17, 512, 576, 0), (16, 512, 576, 300)])
+@pytest.mark.parametrize("splits", [1, 2, 7])
+def test_not_a_number_in_latent_attention(H, rank, w, window, splits):
+    """A NaN in a query makes its head's results NaN, one in a row that is seen those of all heads, and no others."""
+    from litetorch_b200.ops import kernels as K
+    bs, lens = 16, [700, 33, 501]
+    g = torch.Generator(device="cuda").manual_seed(w + splits)
+    width = (max(lens) + bs - 1) // bs
+    tables = torch.randperm(len(lens) * width, generator=torch.Generator().manual_seed(w)).to(torch.int32).view(len(lens), width).cuda()
+    cache = torch.randn(len(lens) * width, 1, bs, w, device="cuda", generator=g).bfloat16()
+    q = torch.randn(len(lens), H, w, device="cuda", generator=g).bfloat16()
+    ctx = torch.tensor(lens, dtype=torch.int32, device="cuda")
+
+    def run(q, cache):
+        return K.latent_decode(q, cache, tables, ctx, rank=rank, window=window, scale=w ** -0.5, max_keys=max(lens), splits=splits)
+
+    base = run(q, cache)
+    assert bool(torch.isfinite(base.float()).all())
+    q, cache = q.clone(), cache.clone()
+    q[2, 3, 5] = float("nan")
+    at = lens[0] - 100                                      # its place among the keys, not the values
+    cache[int(tables[0, at // bs]), 0, at % bs, w - 1] = float("nan")
+    want = torch.zeros_like(base, dtype=torch.bool)
+    want[0] = True
+    want[2, 3] = True
+    got = run(q, cache)
+    assert torch.equal(torch.isnan(got), want) and torch.equal(got[~want], base[~want])
+    assert K.status_fetch() == 0
