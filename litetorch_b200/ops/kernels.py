@@ -596,10 +596,14 @@ def axpby(a, b=None, alpha=1.0, beta=1.0, out=None):
     return out
 
 
-def embedding_fwd(idx: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
+def _dense_index(idx: torch.Tensor, *dtypes) -> torch.Tensor:
+    """The indexes one after another in one of the types (else the first).  (`reshape` alone gives a view of a column, or of one that is repeated.)"""
     idx = idx.reshape(-1)
-    if idx.dtype != torch.int32:
-        idx = idx.to(torch.int64)
+    return (idx if idx.dtype in dtypes else idx.to(dtypes[0])).contiguous()
+
+
+def embedding_fwd(idx: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
+    idx = _dense_index(idx, torch.int64, torch.int32)
     V, D = table.shape
     out = torch.empty((idx.numel(), D), dtype=table.dtype, device=table.device)
     _check(_fn("lt_embedding_fwd_idx")(idx.data_ptr(), 1 if idx.dtype == torch.int32 else 0, table.data_ptr(), out.data_ptr(), idx.numel(), D, V, _stream()),
@@ -617,7 +621,7 @@ def argmax_rows(x: torch.Tensor) -> torch.Tensor:
 
 
 def embedding_bwd(idx: torch.Tensor, dout: torch.Tensor, dtable: torch.Tensor):
-    idx = idx.reshape(-1).to(torch.int64)
+    idx = _dense_index(idx, torch.int64)
     V, D = dtable.shape
     _check(_fn("lt_embedding_bwd")(idx.data_ptr(), dout.data_ptr(), dtable.data_ptr(), idx.numel(), D, V, _stream()), "lt_embedding_bwd")
     return dtable
@@ -638,6 +642,7 @@ def cast_to_f32(x: torch.Tensor, out=None):
 # ------------------------------------------------------------------------------------------------ loss
 def ce_stats(logits: torch.Tensor, targets: torch.Tensor, vocab_start: int = 0) -> torch.Tensor:
     N, V = logits.shape
+    targets = _dense_index(targets, torch.int64)
     stats = torch.empty((N, 3), dtype=torch.float32, device=logits.device)
     _check(_fn("lt_ce_stats")(logits.data_ptr(), logits.stride(0), targets.data_ptr(), vocab_start, N, V, stats.data_ptr(), _stream()), "lt_ce_stats")
     return stats
@@ -646,6 +651,7 @@ def ce_stats(logits: torch.Tensor, targets: torch.Tensor, vocab_start: int = 0) 
 def ce_finish(logits, targets, gstats, *, vocab_start=0, grad_scale=1.0, ignore_index=-100, write_grad=True):
     """Per-row losses; overwrites `logits` with d(loss)/d(logits) * grad_scale when write_grad."""
     N, V = logits.shape
+    targets = _dense_index(targets, torch.int64)
     loss = torch.empty(N, dtype=torch.float32, device=logits.device)
     _check(_fn("lt_ce_finish")(logits.data_ptr(), logits.stride(0), targets.data_ptr(), vocab_start, N, V, gstats.data_ptr(),
                                loss.data_ptr(), float(grad_scale), ignore_index, 1 if write_grad else 0, _stream()), "lt_ce_finish")
@@ -814,7 +820,7 @@ def rs_adamw(grad_ptrs, mc_grads, master, m, v, param_shard, segs, *, lr, beta1,
 
 
 def embedding_fwd_sharded(idx, table_ptrs, V, D, rows_per_rank, world, dtype=torch.bfloat16):
-    idx = idx.reshape(-1).to(torch.int64)
+    idx = _dense_index(idx, torch.int64)
     out = torch.empty((idx.numel(), D), dtype=dtype, device=idx.device)
     rc = _fn("lt_embedding_fwd_sharded")(idx.data_ptr(), ctypes.cast(_ptr_array(table_ptrs), c_void_p), out.data_ptr(),
                                          idx.numel(), D, V, rows_per_rank, world, _stream())
