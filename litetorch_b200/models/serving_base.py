@@ -19,6 +19,7 @@ for, ends when everything before it has run.
 from __future__ import annotations
 
 from itertools import chain
+from operator import index
 from typing import List, Optional, Sequence
 
 import numpy as np
@@ -69,14 +70,14 @@ class ServingModel:
         x = self._prompt_hidden(tokens, start, block_ids, slot)
         if not want_token:
             return -1
-        return int(self._pick(self._logits(x, [len(tokens) - 1])).item())
+        return int(self._pick(self._logits(x, self._places([-1], len(tokens)))).item())
 
     @torch.no_grad()
     def score_chunk(self, tokens: Sequence[int], start: int, block_ids: Sequence[int], rows: Sequence[int], slot: int = 0) -> torch.Tensor:
-        """The same pass; returns the fp32 logits [len(rows), vocab] at the given places among `tokens`."""
+        """The same pass; returns the fp32 logits [len(rows), vocab] at the given places among `tokens` (negative ones count from the end)."""
         self.prefill_tokens_computed += len(tokens)
         x = self._prompt_hidden(tokens, start, block_ids, slot)
-        return self._logits(x, list(rows)).float()
+        return self._logits(x, self._places(rows, len(tokens))).float()
 
     # ------------------------------------------------------------------ one token for every running sequence
     def _decode_body(self, d: torch.Tensor, S: int, width: int):
@@ -166,6 +167,15 @@ class ServingModel:
         h[3 * n:] = table
         d = host.to(self.e.device, non_blocking=True)
         return d[:n], d[n:2 * n], d[2 * n:3 * n], d[3 * n:]
+
+    @staticmethod
+    def _places(rows: Sequence[int], n: int) -> List[int]:
+        """The rows as places among n.  (Checked here: a slice ends where there are no more rows, and the kernels that pick rows read where they are told.)"""
+        rows = [index(r) for r in rows]
+        for r in rows:
+            if not -n <= r < n:
+                raise IndexError("row %d is not among %d tokens" % (r, n))
+        return [r + n if r < 0 else r for r in rows]
 
     @staticmethod
     def _run_of(rows: Sequence[int]) -> Optional[slice]:

@@ -1,4 +1,6 @@
 """Inputs of prompt portions and decode steps as they are packed on the host."""
+import numpy as np
+import pytest
 import torch
 
 
@@ -41,3 +43,31 @@ def test_runs_of_rows():
     near = dict(rtol=0, atol=64 * 2.0 ** -24 * 8 * 0.3)
     assert float(m.e.w.p("lm_head").float().norm(dim=1).max()) < 0.3
     assert torch.allclose(m._logits(x, [3, 4]), m._logits(x)[3:5], **near) and torch.allclose(m._logits(x, [4, 1]), m._logits(x)[[4, 1]], **near)
+
+
+def _family(name):
+    """(serving model, vocabulary) of a small model."""
+    import os
+    import sys
+    sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
+    if name == "llama":
+        return _model(), 64
+    suite = __import__(name + "_suite")
+    cfg = suite.CONFIGS["odd"]
+    from decoder_suite import server
+    return server(suite.engine(cfg, suite.weights(cfg), "cpu", torch.float32), block_size=4)[0], cfg["vocab"]
+
+
+@pytest.mark.parametrize("name", ["llama", "ravenex", "safuvik"])
+def test_rows_that_are_not_there_are_refused(name):
+    m, vocab = _family(name)
+    tokens, table = [3, 1, 4], [7, 2]
+    every = m.score_chunk(tokens, 0, table, [0, 1, 2])
+    assert every.shape == (3, vocab)
+    for rows in ([2, 3], [3], [1, 5], [-4], [-4, -3], range(1, 4)):
+        with pytest.raises(IndexError):
+            m.score_chunk(tokens, 0, table, rows)
+    for rows in ([1, 2], [2], [-1], [-3, -2], [2, 0], (1,), range(0, 2), torch.tensor([1, 2]), np.array([0, 2])):
+        at = [int(r) for r in rows]
+        assert torch.allclose(m.score_chunk(tokens, 0, table, rows), every[at], atol=1e-5)
+    assert m.score_chunk(tokens, 0, table, []).shape == (0, vocab)
