@@ -14,11 +14,12 @@ from __future__ import annotations
 from collections import OrderedDict
 from typing import List, Sequence
 
+import numpy as np
 import torch
 
 from ..serving import PagedKVCache
 from .llama import LlamaEngine
-from .serving_base import Sampler, ServingModel, generate          # noqa: F401  (their names live here as well)
+from .serving_base import Sampler, ServingModel, _ints, generate          # noqa: F401  (their names live here as well)
 
 
 class LlamaKVModel(ServingModel):
@@ -43,6 +44,13 @@ class LlamaKVModel(ServingModel):
         if self.prefix_cache_bytes > 0:
             from ..serving import PrefixCache
             self._index = PrefixCache()
+
+    def _tokens(self, tokens, n):
+        # the embedding takes a token past the vocabulary for the nearest one it has, one past 32 bits too
+        try:
+            return super()._tokens(tokens, n)
+        except OverflowError:
+            return np.clip(_ints(tokens, n, np.int64), -1 << 31, (1 << 31) - 1)
 
     # ------------------------------------------------------------------ shared layer body
     def _layers(self, x, attend):

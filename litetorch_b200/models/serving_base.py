@@ -18,12 +18,20 @@ for, ends when everything before it has run.
 """
 from __future__ import annotations
 
-from itertools import chain
 from operator import index
 from typing import List, Optional, Sequence
 
 import numpy as np
 import torch
+
+
+def _ints(values: Sequence[int], n: int, dtype=np.int32) -> np.ndarray:
+    """n whole numbers as an array.  They may be a tensor, or tensors of one element, on the device too (what a step returns)."""
+    if isinstance(values, torch.Tensor):
+        values = values.tolist()
+    elif n and isinstance(values[0], torch.Tensor):
+        values = map(int, values)
+    return np.fromiter(values, dtype, n)
 
 
 class ServingModel:
@@ -91,19 +99,20 @@ class ServingModel:
         dev = self.e.device
         S = len(last_tokens)
         bs = self.block_size
+        positions = [int(p) for p in positions]
         width = max((p + bs) // bs for p in positions)
         use_graph = self.graphs and dev.type == "cuda"
         if use_graph:
             width = (width + 15) // 16 * 16                     # fewer distinct graphs: table widths in steps of 16 blocks
         host = self._host(5 + width, S)
         h = host.numpy()
-        h[0] = last_tokens
+        h[0] = self._tokens(last_tokens, S)
         h[1] = positions
-        h[2] = [block_tables[s][p // bs] * bs + p % bs for s, p in enumerate(positions)]
+        h[2] = [int(t[p // bs]) * bs + p % bs for t, p in zip(block_tables, positions)]
         h[3] = h[1] + 1
-        h[4] = 0 if slots is None else list(slots)
+        h[4] = 0 if slots is None else _ints(slots, S)
         n = [min(len(t), width) for t in block_tables]
-        flat = np.fromiter(chain.from_iterable(t if len(t) <= width else t[:width] for t in block_tables), np.int32, sum(n))
+        flat = np.concatenate([_ints(t if len(t) <= width else t[:width], k) for t, k in zip(block_tables, n)])
         table = np.zeros((S, width), np.int32)
         table[np.arange(width) < np.array(n)[:, None]] = flat
         h[5:] = table.T
@@ -153,6 +162,9 @@ class ServingModel:
         """Host memory for 32-bit inputs, pinned where there is a GPU."""
         return torch.empty(shape, dtype=torch.int32, pin_memory=self.e.device.type == "cuda")
 
+    def _tokens(self, tokens: Sequence[int], n: int) -> np.ndarray:
+        return _ints(tokens, n)
+
     def _prompt_inputs(self, tokens: Sequence[int], start: int, block_ids: Sequence[int]):
         """(tokens, positions, cache slots, block table) of a portion on the device, int32, through one copy."""
         n, bs = len(tokens), self.block_size
@@ -160,8 +172,8 @@ class ServingModel:
         host = self._host(3 * n + nb)
         h = host.numpy()
         p = np.arange(start, start + n, dtype=np.int32)
-        table = np.fromiter(block_ids[:nb], np.int32, nb)
-        h[:n] = np.fromiter(tokens, np.int32, n)
+        table = _ints(block_ids[:nb], nb)
+        h[:n] = self._tokens(tokens, n)
         h[n:2 * n] = p
         h[2 * n:3 * n] = table[p // bs] * bs + p % bs
         h[3 * n:] = table

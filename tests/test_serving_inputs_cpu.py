@@ -71,3 +71,19 @@ def test_rows_that_are_not_there_are_refused(name):
         at = [int(r) for r in rows]
         assert torch.allclose(m.score_chunk(tokens, 0, table, rows), every[at], atol=1e-5)
     assert m.score_chunk(tokens, 0, table, []).shape == (0, vocab)
+
+
+def test_inputs_that_are_tensors_and_tokens_past_32_bits():
+    m = _model()
+    tables = [[5, 9, 2], [1, 3, 8]]
+    for t in tables:
+        m.prefill_chunk(list(range(6)), 0, t, False)
+    want = m.decode_logits([7, 63], [6, 6], tables)
+    for tok, pos, bt in ((torch.tensor([7, 63]), torch.tensor([6, 6]), [torch.tensor(t) for t in tables]),
+                         ((np.int64(7), 63), np.array([6, 6]), [np.array(t) for t in tables]),
+                         ([torch.tensor(7), torch.tensor(63)], (6, 6), tables), ([7, 1 << 40], [6, 6], tables)):
+        assert torch.equal(m.decode_logits(tok, pos, bt, slots=torch.tensor([0, 0])), want)
+    one = m.score_chunk([1, 63], 0, tables[0], [1])
+    assert torch.equal(m.score_chunk(torch.tensor([1, 63]), 0, torch.tensor(tables[0]), [1]), one)
+    assert torch.equal(m.score_chunk([1, 1 << 40], 0, tables[0], [1]), one)
+    assert torch.equal(m.score_chunk([1, -1 << 40], 0, tables[0], [1]), m.score_chunk([1, -3], 0, tables[0], [1]))
