@@ -18,6 +18,7 @@ for, ends when everything before it has run.
 """
 from __future__ import annotations
 
+import gc
 from operator import index
 from typing import List, Optional, Sequence
 
@@ -127,14 +128,7 @@ class ServingModel:
                 self._decode_body(static_in, S, width)
             torch.cuda.current_stream().wait_stream(side)
             torch.cuda.synchronize()
-            g = torch.cuda.CUDAGraph()
-            # (not `torch.cuda.graph`: it gives all cached memory back first, which takes a tenth of a second and more after large states)
-            with torch.cuda.stream(side):
-                g.capture_begin()
-                try:
-                    static_out = self._decode_body(static_in, S, width)
-                finally:
-                    g.capture_end()
+            g, static_out = self._record(static_in, S, width, side)
             entry = self._graphs[S, width] = (g, static_in, static_out)
             # the eager pass wrote this step's cache cells already; the replay below rewrites the same ones
         g, static_in, static_out = entry
@@ -142,6 +136,30 @@ class ServingModel:
         g.replay()
         self.last_logits = static_out[0]
         return static_out
+
+    def _record(self, static_in: torch.Tensor, S: int, width: int, side: torch.cuda.Stream):
+        """(graph, outputs) of a decode step, recorded on `side`.  `torch.cuda.graph` gives all cached memory back first, which takes a tenth of a second
+        and more after large states; here that is done where the device has less than 1 GB left (the driver keeps the graph there), and where the
+        recording finds no memory: what lies free in the cache of another stream, or of the common pool, cannot be used, nor given back, while it is
+        under way."""
+        for give_back in (torch.cuda.mem_get_info(side.device)[0] < 1 << 30, True):
+            if give_back:
+                torch.cuda.synchronize()
+                gc.collect()
+                torch.cuda.empty_cache()
+            g, short = torch.cuda.CUDAGraph(), None
+            with torch.cuda.stream(side):
+                g.capture_begin()
+                try:
+                    out = self._decode_body(static_in, S, width)
+                except torch.cuda.OutOfMemoryError as e:
+                    short = e.with_traceback(None)             # (its frames hold what was made so far)
+                finally:
+                    g.capture_end()
+            if short is None:
+                return g, out
+            g.reset()
+        raise short
 
     @torch.no_grad()
     def decode_batch(self, last_tokens: Sequence[int], positions: Sequence[int], block_tables: List[Sequence[int]],
