@@ -181,6 +181,8 @@ class LlamaKVModel(ServingModel):
         bt = d[5:].t().contiguous()
 
         def attend(i, qkv):
-            return K.decode_step(qkv, e.cos, e.sin, pos, slots, cfg.n_heads, cfg.n_kv_heads, cfg.head_dim, c.k[i], c.v[i], bt, ctx, bs, self.num_splits, c.k_scale, c.v_scale)
+            # early: the tables were made, and what earlier passes cached was complete, before the embedding, which starts after everything before it
+            return K.decode_step(qkv, e.cos, e.sin, pos, slots, cfg.n_heads, cfg.n_kv_heads, cfg.head_dim, c.k[i], c.v[i], bt, ctx, bs, self.num_splits, c.k_scale, c.v_scale,
+                                 early=True)
 
         return self._layers(K.embedding_fwd(tok, e.w.p("embed")), attend)

@@ -893,11 +893,14 @@ def _decode_splits(pairs: int, keys: int, head_dim: int, fp8: bool):
 
 
 def decode_step(qkv, cos, sin, positions, slots, heads: int, kv_heads: int, head_dim: int, k_cache, v_cache, block_tables, context_lens, block_size: int,
-                splits: int = 0, k_scale: float = 1.0, v_scale: float = 1.0):
+                splits: int = 0, k_scale: float = 1.0, v_scale: float = 1.0, early: bool = False):
     """Attention of a decode step from the rows [q | k | v] of its product: queries and keys are rotated, the newest keys and values cached, and every
-    sequence attends to its context, whose last token is the row's.  Returns [S, heads, head_dim].  Block tables, lengths and the cached rows
-    before were complete when the step's embedding was launched.  positions, slots, context_lens [S], block_tables [S, width]: int32.
+    sequence attends to its context, whose last token is the row's.  Returns [S, heads, head_dim].  positions, slots, context_lens [S],
+    block_tables [S, width]: int32.
 
+    early: block tables, lengths and every cached row but the newest are read before the kernels in front of this one have ended.  The caller answers
+    for it that no kernel writes them which the stream may still run then: since the last write a kernel of torch, a copy or another launch that
+    starts after everything before it (`embedding_fwd`) was made, not only kernels of this library, which start under one another.
     splits: how many the keys of a (sequence, KV head) are cut into (0: by size).  One launch, or two; caches that it does not take go through
     rope_append and paged_decode."""
     S, D = qkv.shape[0], head_dim
@@ -918,7 +921,7 @@ def decode_step(qkv, cos, sin, positions, slots, heads: int, kv_heads: int, head
         rc = _fn("lt_paged_decode_step")(qkv.data_ptr(), qkv.stride(0), cos.data_ptr(), sin.data_ptr(), positions.data_ptr(), slots.data_ptr(),
                                          k_cache.data_ptr(), v_cache.data_ptr(), block_tables.data_ptr(), context_lens.data_ptr(), _p(part), o.data_ptr(), S, heads,
                                          kv_heads, D, block_size, block_tables.shape[1], k_cache.shape[0], splits, float(D ** -0.5),
-                                         1 if fp8 else 0, float(k_scale), float(v_scale), 1, _stream())
+                                         1 if fp8 else 0, float(k_scale), float(v_scale), 1 if early else 0, _stream())
         _check(rc, "lt_paged_decode_step")
         return o
     q = rope_append(qkv, cos, sin, positions, slots, heads, kv_heads, D, k_cache, v_cache, block_size, fp8, k_scale, v_scale)

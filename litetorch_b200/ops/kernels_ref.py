@@ -141,7 +141,7 @@ def rope_append(qkv, cos, sin, positions, slots, heads, kv_heads, head_dim, k_ca
 
 
 def decode_step(qkv, cos, sin, positions, slots, heads, kv_heads, head_dim, k_cache, v_cache, block_tables, context_lens, block_size, splits=0, k_scale=1.0,
-                v_scale=1.0):
+                v_scale=1.0, early=False):
     from ..serving import paged_attention
     q = rope_append(qkv, cos, sin, positions, slots, heads, kv_heads, head_dim, k_cache, v_cache, block_size, k_cache.dtype == torch.float8_e4m3fn, k_scale,
                     v_scale)

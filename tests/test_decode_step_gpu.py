@@ -155,3 +155,65 @@ def test_scores_of_minus_infinity(D, bs, longest, splits):
     # roundings of the result and of the weights, each within 2^-9 of itself
     assert ((o[0].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + size * 2.0 ** -8 + 1e-4).all()
     assert K.status_fetch() == 0
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("G,Hkv,D", [(8, 4, 64), (4, 8, 128)])
+def test_rows_cached_by_the_kernel_in_front(G, Hkv, D, fp8):
+    """A step right behind the launch that caches the rows it attends to, and, with the cached rows complete before the step's embedding, behind that
+    and a product: both start while the kernel in front of them runs."""
+    from litetorch_b200.ops import kernels as K
+    H, bs, n, S = G * Hkv, 16, 6000, 2
+    g = torch.Generator(device="cuda").manual_seed(D)
+    dt = torch.float8_e4m3fn if fp8 else torch.bfloat16
+    blocks = n // bs + 1
+    kc, vc = (torch.zeros(S * blocks, Hkv, bs, D, device="cuda", dtype=torch.bfloat16).to(dt) for _ in range(2))
+    bt = torch.arange(S * blocks, dtype=torch.int32, device="cuda").view(S, blocks)
+    ang = torch.arange(n + 1, device="cuda", dtype=torch.float64)[:, None] * 1e4 ** (-torch.arange(0, D, 2, device="cuda", dtype=torch.float64) / D)[None]
+    cos, sin = ang.cos().float().contiguous(), ang.sin().float().contiguous()
+    rows = torch.randn(S * n, (H + 2 * Hkv) * D, device="cuda", generator=g).bfloat16()          # the earlier tokens of both sequences
+    at = torch.arange(n, dtype=torch.int32, device="cuda").repeat(S)
+    cells = torch.cat([torch.arange(n, dtype=torch.int32, device="cuda") + s * blocks * bs for s in range(S)])
+    pos = torch.full((S,), n, dtype=torch.int32, device="cuda")
+    slots = torch.tensor([s * blocks * bs + n for s in range(S)], dtype=torch.int32, device="cuda")
+    tok = torch.tensor([3, 1], dtype=torch.int32, device="cuda")
+    table = torch.randn(5, 256, device="cuda", generator=g).bfloat16()
+    w = torch.randn((H + 2 * Hkv) * D, 256, device="cuda", generator=g).bfloat16() / 16
+    step = K.product_of_constants(K.embedding_fwd(tok, table), w)
+    ctx = pos + 1
+    K.rope_append(rows, cos, sin, at, cells, H, Hkv, D, kc, vc, bs, fp8)
+    torch.cuda.synchronize()
+    want = K.decode_step(step, cos, sin, pos, slots, H, Hkv, D, kc, vc, bt, ctx, bs)
+    assert bool(want.float().abs().max() > 0)
+    for _ in range(5):
+        for t in (kc, vc):
+            t.view(torch.uint8).zero_()
+        K.rope_append(rows, cos, sin, at, cells, H, Hkv, D, kc, vc, bs, fp8)
+        o = K.decode_step(step, cos, sin, pos, slots, H, Hkv, D, kc, vc, bt, ctx, bs)
+        assert torch.equal(o, want)
+        for t in (kc, vc):
+            t.view(torch.uint8).zero_()
+        K.rope_append(rows, cos, sin, at, cells, H, Hkv, D, kc, vc, bs, fp8)
+        qkv = K.product_of_constants(K.embedding_fwd(tok, table), w)
+        o = K.decode_step(qkv, cos, sin, pos, slots, H, Hkv, D, kc, vc, bt, ctx, bs, early=True)
+        assert torch.equal(o, want)
+    assert K.status_fetch() == 0
+
+
+def test_early_reads_are_asked_for(monkeypatch):
+    """`early` is off unless the caller says so; the served model does."""
+    from litetorch_b200.models.llama import LlamaConfig, LlamaEngine
+    from litetorch_b200.models.registry import new_serving
+    from litetorch_b200.ops import kernels as K
+    real, seen = K._fn, []
+
+    def fn(name):
+        return (lambda *a: seen.append(a[-2]) or real(name)(*a)) if name == "lt_paged_decode_step" else real(name)
+
+    monkeypatch.setattr(K, "_fn", fn)
+    qkv, cos, sin, pos, slots, kc, vc, bt, ctx, lens = _case(2, 4, 2, 64, 16, 40, False, 3)
+    K.decode_step(qkv, cos, sin, pos, slots, 8, 2, 64, kc, vc, bt, ctx, 16)
+    m = new_serving(LlamaEngine(LlamaConfig(vocab_size=64, n_layers=2, d_model=128, n_heads=2, n_kv_heads=1, head_dim=64, ffn=256, max_seq=64), "cuda", seed=1),
+                    num_blocks=4, block_size=16, max_num_seqs=1, graphs=False)
+    m.decode_logits([3], [0], [[2]])
+    assert seen == [0, 1, 1]
