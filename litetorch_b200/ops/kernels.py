@@ -510,7 +510,7 @@ def product_of_constants(x, w, residual=None, act: str = "", norm=None):
     if gain is not None:
         assert gain.dtype == x.dtype and gain.shape == (Kd,) and gain.is_contiguous()
         if not (few and M <= 16 and Kd <= 8192 and _aligned(gain)):
-            return product_of_constants(norm_fwd(x, gain, eps=eps)[0], w, residual, act)
+            return product_of_constants(norm_fwd(x.contiguous(), gain, eps=eps)[0], w, residual, act)
     if few:
         y = torch.empty((M, N), dtype=x.dtype, device=x.device)
         rc = _fn("lt_weight_stream_norm")(x.data_ptr(), x.stride(0), _p(gain), float(eps), w.data_ptr(), Kd, y.data_ptr(), N, 0, _p(residual),

@@ -75,3 +75,14 @@ def test_products_with_constant_matrices(M, N, Kd, strided):
         e = (2.0 ** -8 if M > 64 else 0) + 2.0 ** -18
         assert ((got - f(gate) * up).abs() <= (f(gate) * up).abs() * 2.0 ** -8 + 1.13 * (gate.abs() * up.abs() * 2 * e + slack[:, :N] * up.abs() + slack[:, N:] * gate.abs()) + 1e-6).all()
     assert K.status_fetch() == 0
+
+
+@pytest.mark.parametrize("M,N,Kd,act", [(3, 40, 256, ""), (17, 40, 256, ""), (200, 512, 256, "silu"), (9, 7112, 512, "silu"), (2, 40, 8200, "")])
+def test_rows_with_a_pitch(M, N, Kd, act):
+    """Rows out of a wider matrix give what dense ones give."""
+    from litetorch_b200.ops import kernels as K
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.randn(M, Kd + 24, device="cuda", generator=g).bfloat16()[:, 8:Kd + 8]
+    gain, w = torch.ones(Kd, device="cuda").bfloat16(), torch.randn((2 if act else 1) * N, Kd, device="cuda", generator=g).bfloat16()
+    assert torch.equal(K.product_of_constants(x, w, None, act, norm=(gain, 1e-6)), K.product_of_constants(x.contiguous(), w, None, act, norm=(gain, 1e-6)))
+    assert K.status_fetch() == 0
