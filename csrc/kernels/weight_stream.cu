@@ -262,6 +262,10 @@ weight_stream_kernel(const __grid_constant__ CUtensorMap tw, const __grid_consta
     for (int spin = 0; spin < 2000; ++spin) __nanosleep(100);  // bounded grace period for copies in flight
 }
 
+// Shared memory that normalising takes beside kSmem: sums of squares and gains.
+template <class Cfg>
+static int norm_bytes(int K) { return Cfg::kWarps * 64 + (K + 63) / 64 * 128; }
+
 template <int XR, int R, bool GLU, bool NORM = false>
 static int launch_ws(const StreamProduct& p, cudaStream_t st) {
   using Cfg = WsCfg<XR, R>;
@@ -270,9 +274,9 @@ static int launch_ws(const StreamProduct& p, cudaStream_t st) {
   }
   static OncePerDevice configured;
   auto kern = weight_stream_kernel<XR, R, GLU, NORM>;
-  const int smem = Cfg::kSmem + (NORM ? Cfg::kWarps * 64 + (p.K + 63) / 64 * 128 : 0);
+  const int smem = Cfg::kSmem + (NORM ? norm_bytes<Cfg>(p.K) : 0);
   if (configured.pending()) {
-    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem + (NORM ? Cfg::kWarps * 64 + kStreamNormK * 2 : 0)));
+    LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem + (NORM ? norm_bytes<Cfg>(kStreamNormK) : 0)));
     configured.finish();
   }
   // As many tiles as CTAs, or a multiple of that, so that none ends in a round of a few tiles: tiles get as wide as that takes, and
@@ -293,14 +297,16 @@ static int launch_ws(const StreamProduct& p, cudaStream_t st) {
 
 // Tiles of 16 rows where they give every SM one, else of 32: 2048 columns 4.3 against 4.7 us, 4096 columns 13.9 against 8.3.  Up to
 // 8 rows of x and more columns than SMs have tiles, two CTAs an SM and a stage for 8 rows of x (28672 x 4096, 8 rows: 39 against 42 us); with
-// 17 to 32 rows and that many columns, tiles of 64, which read x half as often (53 against 55 us, 32000 x 2048 34.7 against 37.7).
+// 17 to 32 rows and that many columns, tiles of 64, which read x half as often (53 against 55 us, 32000 x 2048 34.7 against 37.7).  Gains of more than 7808
+// columns leave no room for the second CTA: its tiles would come after the first one's (10240 x 8192, 8 rows: 49 us, with 16 rows of x 31).
 template <bool GLU>
 static int stream_by_size(const StreamProduct& p, cudaStream_t st) {
   const long long rows = GLU ? 2ll * p.N : p.N, sms = sm_count();
   const bool narrow = rows <= 16 * sms, wide = rows > 32 * sms;
   if (p.M <= 16) {
     if (narrow) return launch_ws<16, 16, GLU>(p, st);
-    return wide && p.M <= 8 ? launch_ws<8, 32, GLU>(p, st) : launch_ws<16, 32, GLU>(p, st);
+    const bool two = !p.gain || 2 * (WsCfg<8, 32>::kSmem + norm_bytes<WsCfg<8, 32>>(p.K) + 1024) <= 228 * 1024;
+    return wide && p.M <= 8 && two ? launch_ws<8, 32, GLU>(p, st) : launch_ws<16, 32, GLU>(p, st);
   }
   if (p.M <= 32) {
     if (narrow) return launch_ws<32, 16, GLU>(p, st);

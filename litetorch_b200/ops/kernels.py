@@ -496,9 +496,20 @@ def rope_(x2d: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, T: int, heads
     return x2d
 
 
+def _norm_on_the_way(M: int, N: int, Kd: int, gated: bool) -> bool:
+    """Whether the product of M rows normalises them itself.  It does so again for every tile of its CTA, which shows where a CTA has an SM to itself
+    (more than 8 rows, or gains that leave no room for two) and many tiles, two products each.  On the way / by a kernel in front (us, in a recorded graph):
+    8 rows 14336 x 4096 gated 38.8 / 40.5, 16 rows 41.6 / 38.7; 16 rows 5632 x 2048 gated 11.4 / 11.4, 14336 x 2048 24.5 / 21.8; 32000 x 4096 41.0 /
+    43.9; 8 rows 28672 x 7168 gated 117 / 120, 28672 x 8192 146 / 138, 10240 x 8192 30.6 / 34.1, 128256 x 8192 301 to 323 / 300 to 310."""
+    if M > 16 or Kd > 8192:
+        return False
+    alone = Kd > 7808                                # (csrc/kernels/weight_stream.cu, stream_by_size)
+    return not ((M > 8 or alone) and gated and N > 48 * sm_count()) and not (alone and N > 40000)
+
+
 def product_of_constants(x, w, residual=None, act: str = "", norm=None):
     """x @ w^T (+ residual), or with `act` glu_rows(x, w), for weights that no kernel of the pass writes: with up to 64 rows the kernel starts
-    under the one before it and fetches weights meanwhile.  norm (gains, eps): x is RMS-normalised first, with up to 16 rows in the same kernel."""
+    under the one before it and fetches weights meanwhile.  norm (gains, eps): x is RMS-normalised first, mostly in the same kernel (`_norm_on_the_way`)."""
     M, Kd = x.shape
     N = w.shape[0] // 2 if act else w.shape[0]
     assert x.dtype == w.dtype and w.dim() == 2 and w.shape[1] == Kd, "operands do not match: %s and %s" % (tuple(x.shape), tuple(w.shape))
@@ -509,7 +520,7 @@ def product_of_constants(x, w, residual=None, act: str = "", norm=None):
     gain, eps = norm or (None, 0.0)
     if gain is not None:
         assert gain.dtype == x.dtype and gain.shape == (Kd,) and gain.is_contiguous()
-        if not (few and M <= 16 and Kd <= 8192 and _aligned(gain)):
+        if not (few and _norm_on_the_way(M, N, Kd, bool(act)) and _aligned(gain)):
             return product_of_constants(norm_fwd(x.contiguous(), gain, eps=eps)[0], w, residual, act)
     if few:
         y = torch.empty((M, N), dtype=x.dtype, device=x.device)

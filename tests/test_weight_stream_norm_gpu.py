@@ -77,6 +77,27 @@ def test_products_with_constant_matrices(M, N, Kd, strided):
     assert K.status_fetch() == 0
 
 
+@pytest.mark.parametrize("M,Kd", [(8, 512), (9, 512), (16, 2048), (1, 7808), (8, 7816), (1, 8192), (9, 8192)])
+@pytest.mark.parametrize("N,act", [(7104, "silu"), (7112, "silu"), (40000, ""), (40002, "")])
+def test_norm_on_the_way_or_in_front(M, Kd, N, act):
+    """Both sides of the lines between them, against 64 bits."""
+    from litetorch_b200.ops import kernels as K
+    g = torch.Generator(device="cuda").manual_seed(M + Kd + N)
+    x = torch.randn(M, Kd, device="cuda", generator=g).bfloat16()
+    gain = (1 + 0.1 * torch.randn(Kd, device="cuda", generator=g)).bfloat16()
+    w = torch.empty((2 if act else 1) * N, Kd, device="cuda").normal_(0.0, Kd ** -0.5, generator=g).bfloat16()
+    y = K.product_of_constants(x, w, None, act, norm=(gain, 1e-5))
+    x64 = x.double()
+    z = (x64 * torch.rsqrt((x64 ** 2).mean(-1, keepdim=True) + 1e-5) * gain.double()) @ w.double().t()
+    want = torch.nn.functional.silu(z[:, :N]) * z[:, N:] if act else z
+    assert float((y.double() - want).norm() / want.norm()) < 6e-3            # factors and result rounded to bf16, as above
+    first = K.product_of_constants(K.norm_fwd(x, gain, eps=1e-5)[0], w, None, act)
+    assert float((first.double() - want).norm() / want.norm()) < 6e-3
+    if not K._norm_on_the_way(M, N, Kd, bool(act)):
+        assert torch.equal(y, first)
+    assert K.status_fetch() == 0
+
+
 @pytest.mark.parametrize("M,N,Kd,act", [(3, 40, 256, ""), (17, 40, 256, ""), (200, 512, 256, "silu"), (9, 7112, 512, "silu"), (2, 40, 8200, "")])
 def test_rows_with_a_pitch(M, N, Kd, act):
     """Rows out of a wider matrix give what dense ones give."""
