@@ -51,7 +51,9 @@ class OncePerDevice {
 
 // Launch of a kernel that calls pdl_wait() ahead of its first access to global memory: it may take its place on the SMs and set up its shared and
 // tensor memory while the kernel ahead of it in the stream ends (from that one's pdl_launch_dependents() on; a kernel with tensor memory calls that
-// after its own allocation, so that a successor cannot take the columns that it still needs).  Between kernels of a stream 2.2 us pass otherwise, 0.4 in
+// after its own allocation, so that a successor cannot take the columns that it still needs).  What the kernels ahead may have written it reads by plain
+// loads: no __ldg, ld.global.nc or inputs declared "const ... __restrict__", which are for memory that nobody writes while the kernel lives, and which the
+// compiler may move across the wait.  Between kernels of a stream 2.2 us pass otherwise, 0.4 in
 // a recorded graph, and set-up comes on top.  Training step of 1.1B layers over 2 x 2000 tokens (506 kernels) 18.4 -> 17.7 ms, four 8B layers over 8192
 // tokens 82.9 -> 80.5 (1 % of it the norms), prompt of 4096 tokens 11.7 -> 11.4, decode step of the 1.1B model 1038 -> 956 us, latent decode step 510 -> 470.
 template <class... P, class... A>

@@ -411,6 +411,12 @@ __device__ __forceinline__ uint4 ld_nc_v4(const void* p) {
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
+// The same by a plain load, for kernels that lie on the SMs while the one before them still writes.
+__device__ __forceinline__ uint4 ld_stream_v4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
 // Plain (coherent at system scope after an acquire) 16-byte load, used for peer memory.
 __device__ __forceinline__ uint4 ld_relaxed_sys_v4(const void* p) {
   uint4 v;

@@ -110,7 +110,7 @@ __device__ __forceinline__ void turn_back(float (&v)[8], const float* cos_row, c
 
 // delta[b,h,t] = sum_d O * dO ; D/8 threads per (b,t,h) row, 16 bytes each.  They also zero their columns of the dQ accumulator [B, Tq, Hq, D] (nullptr: the
 // caller has).
-__global__ void flash_bwd_delta_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __restrict__ dO,
+__global__ void flash_bwd_delta_kernel(const __nv_bfloat16* O, const __nv_bfloat16* dO,
                                        float* __restrict__ delta, float* __restrict__ dq_acc, int B, int Tq, int Hq, int D, long long so_b,
                                        long long so_t, long long sdo_b, long long sdo_t) {
   pdl_launch_dependents();
@@ -146,7 +146,7 @@ __global__ void flash_bwd_delta_kernel(const __nv_bfloat16* __restrict__ O, cons
 
 // dQ leaves its accumulator as bf16, eight columns a thread; with tables [., D / 2] of cosines and sines (nullptr: as it is) turned back by the angles of
 // its row's position t, pairs of neighbouring columns together.
-__global__ void __launch_bounds__(256) flash_bwd_convert_dq_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, long long rows, int Tq,
+__global__ void __launch_bounds__(256) flash_bwd_convert_dq_kernel(const float* acc, __nv_bfloat16* __restrict__ dq, long long rows, int Tq,
                                                                    int HD, int D, long long sdq_b, long long sdq_t, const float* __restrict__ cos_t,
                                                                    const float* __restrict__ sin_t) {
   pdl_launch_dependents();

@@ -139,7 +139,7 @@ gemm_skinny_kernel(const SkinnyParams p) {
       const int cc = c + u * kSkWarps;
 #pragma unroll
       for (int f = 0; f < 4; ++f)
-        wv[u][f] = (cc < c_end && wok[f]) ? ld_nc_v4(wrow[f] + (long long)cc * 32) : make_uint4(0u, 0u, 0u, 0u);
+        wv[u][f] = (cc < c_end && wok[f]) ? ld_stream_v4(wrow[f] + (long long)cc * 32) : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -152,8 +152,8 @@ gemm_skinny_kernel(const SkinnyParams p) {
         const __nv_bfloat16 *x0, *x1;
         if constexpr (MODE == kSkGrouped) { x0 = xrow[m][0]; x1 = xrow[m][1]; }
         else { x0 = xbase + (long long)r0 * ldx; x1 = xbase + (long long)r1 * ldx; }
-        const uint4 xlo = r0 < M ? __ldg(reinterpret_cast<const uint4*>(x0 + cc * 32)) : zero;
-        const uint4 xhi = r1 < M ? __ldg(reinterpret_cast<const uint4*>(x1 + cc * 32)) : zero;
+        const uint4 xlo = r0 < M ? *reinterpret_cast<const uint4*>(x0 + cc * 32) : zero;
+        const uint4 xhi = r1 < M ? *reinterpret_cast<const uint4*>(x1 + cc * 32) : zero;
 #pragma unroll
         for (int f = 0; f < 4; ++f) {
           // physical k = q * 8 + j * 4 + {0, 1} plays logical k = q * 2 + {0, 1}, physical + 2 plays logical + 8, for A and B alike

@@ -170,7 +170,7 @@ __device__ __forceinline__ void epilogue_store_chunk(const GemmParams& p, int ro
   const bool full = (col0 + 32 <= p.N);
   const int ncols = full ? 32 : (p.N - col0);
   if (p.a_scale) {
-    const float as = __ldg(p.a_scale + row);
+    const float as = p.a_scale[row];
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] *= as;
   }
@@ -179,12 +179,12 @@ __device__ __forceinline__ void epilogue_store_chunk(const GemmParams& p, int ro
       const float4* b4 = reinterpret_cast<const float4*>(p.b_scale + col0);
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        const float4 f = __ldg(b4 + q);
+        const float4 f = b4[q];
         v[q * 4 + 0] *= f.x; v[q * 4 + 1] *= f.y; v[q * 4 + 2] *= f.z; v[q * 4 + 3] *= f.w;
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) if (j < ncols) v[j] *= __ldg(p.b_scale + col0 + j);
+      for (int j = 0; j < 32; ++j) if (j < ncols) v[j] *= p.b_scale[col0 + j];
     }
   }
   if (p.bias) {
@@ -192,7 +192,7 @@ __device__ __forceinline__ void epilogue_store_chunk(const GemmParams& p, int ro
       const uint4* b4 = reinterpret_cast<const uint4*>(p.bias + col0);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        uint4 u = __ldg(b4 + q);
+        uint4 u = b4[q];
         float2 f;
         f = unpack_bf16x2(u.x); v[q * 8 + 0] += f.x; v[q * 8 + 1] += f.y;
         f = unpack_bf16x2(u.y); v[q * 8 + 2] += f.x; v[q * 8 + 3] += f.y;

@@ -555,7 +555,7 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap tmap, const LatentDecod
 }
 
 // out[row, :] from the splits of one (sequence, head): a thread per four columns, eight splits in flight.
-__global__ void __launch_bounds__(128) latent_merge_kernel(const float* __restrict__ part, const float* __restrict__ stat,
+__global__ void __launch_bounds__(128) latent_merge_kernel(const float* part, const float* stat,
                                                            __nv_bfloat16* __restrict__ out, int splits, int c) {
   pdl_launch_dependents();
   pdl_wait();

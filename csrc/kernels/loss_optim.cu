@@ -27,7 +27,7 @@ __device__ __forceinline__ void ce_ld8(const __nv_bfloat16* p, float (&f)[8]) {
 
 // stats[row] = {max, sum exp(l - max), target logit if the target falls in [vocab_start, vocab_start+V) else 0}
 __global__ void __launch_bounds__(kCeThreads)
-ce_stats_kernel(const __nv_bfloat16* __restrict__ logits, long long ldl, const long long* __restrict__ targets,
+ce_stats_kernel(const __nv_bfloat16* logits, long long ldl, const long long* targets,
                 int vocab_start, int N, int V, float* __restrict__ stats, int vec_ok) {
   pdl_launch_dependents();
   pdl_wait();
@@ -92,8 +92,8 @@ ce_stats_kernel(const __nv_bfloat16* __restrict__ logits, long long ldl, const l
 // gstats[row] = {global max, global sum-exp, target logit}.  loss[row] = log(sum) + max - target (0 if ignored);
 // logits are overwritten by dlogits = (softmax - onehot) * grad_scale when write_grad != 0.
 __global__ void __launch_bounds__(kCeThreads)
-ce_finish_kernel(__nv_bfloat16* __restrict__ logits, long long ldl, const long long* __restrict__ targets,
-                 int vocab_start, int N, int V, const float* __restrict__ gstats, float* __restrict__ loss,
+ce_finish_kernel(__nv_bfloat16* __restrict__ logits, long long ldl, const long long* targets,
+                 int vocab_start, int N, int V, const float* gstats, float* __restrict__ loss,
                  float grad_scale, long long ignore_index, int write_grad, int vec_ok) {
   pdl_launch_dependents();
   pdl_wait();

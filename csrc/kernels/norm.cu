@@ -51,8 +51,8 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
 // y = norm(x (+ res)) * w (+ b).  RMS: mean unused.  If sum_out != nullptr the pre-norm sum is stored.
 template <bool kLayerNorm>
 __global__ void __launch_bounds__(kNormThreads)
-norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
-                const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
+norm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* res,
+                const __nv_bfloat16* w, const __nv_bfloat16* b,
                 __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ sum_out, float* __restrict__ mean_out,
                 float* __restrict__ rstd_out, int M, int D, float eps) {
   pdl_launch_dependents();
@@ -120,7 +120,7 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 // 34.0 -> 29.0, 4096 x 2048 12.5 -> 10.5, 1337 x 4096 9.4 -> 8.4 (bytes at the copy rate: 10.2, 20.5, 5.1, 3.3).
 template <int IT>
 __global__ void __launch_bounds__(kNormThreads)
-rmsnorm_fwd_wide_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
+rmsnorm_fwd_wide_kernel(const __nv_bfloat16* x, const __nv_bfloat16* w, __nv_bfloat16* __restrict__ y,
                         float* __restrict__ rstd_out, int M, int W, float eps) {
   __shared__ float sums[2][8];
   const int D = 256 * IT * W;
@@ -174,9 +174,9 @@ rmsnorm_fwd_wide_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
 // dx (+= dres) and per-CTA partial dw/db.  ITERS = ceil(D / (threads*8)).
 template <bool kLayerNorm, int ITERS>
 __global__ void __launch_bounds__(kNormThreads)
-norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                const __nv_bfloat16* __restrict__ w, const float* __restrict__ mean_in,
-                const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
+norm_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
+                const __nv_bfloat16* w, const float* mean_in,
+                const float* rstd_in, const __nv_bfloat16* dres,
                 __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_part, float* __restrict__ db_part, int M, int D) {
   pdl_launch_dependents();
   pdl_wait();
@@ -260,8 +260,8 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
 // the copy rate: 20.5, 41.0, 15.4, 41.0, 1.5).
 template <int IT>
 __global__ void __launch_bounds__(kNormThreads, IT == 2 ? 2 : 1)
-rmsnorm_bwd_wide_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                        const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
+rmsnorm_bwd_wide_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w,
+                        const float* rstd_in, const __nv_bfloat16* dres, __nv_bfloat16* __restrict__ dx,
                         float* __restrict__ dw_part, int M, int W) {
   pdl_launch_dependents();
   pdl_wait();
@@ -358,9 +358,9 @@ rmsnorm_bwd_wide_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat1
 // dgamma is accumulated per lane over all rows of the warp and folded to one partial row per CTA at the end.
 template <int ITERS>
 __global__ void __launch_bounds__(kNormThreads)
-rmsnorm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                        const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in,
-                        const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
+rmsnorm_bwd_warp_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
+                        const __nv_bfloat16* w, const float* rstd_in,
+                        const __nv_bfloat16* dres, __nv_bfloat16* __restrict__ dx,
                         float* __restrict__ dw_part, int M) {
   pdl_launch_dependents();
   pdl_wait();
@@ -435,7 +435,7 @@ rmsnorm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat1
 }
 
 // out[c] (+)= sum_p part[p, c]; out is bf16 or fp32.  A block owns 32 columns; its 32 warps split the partial rows.
-__global__ void __launch_bounds__(1024) fold_partials_kernel(const float* __restrict__ part, void* __restrict__ out, int P, int D,
+__global__ void __launch_bounds__(1024) fold_partials_kernel(const float* part, void* __restrict__ out, int P, int D,
                                      int out_fp32, int accumulate) {
   pdl_launch_dependents();
   pdl_wait();

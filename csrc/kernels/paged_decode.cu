@@ -532,8 +532,8 @@ __device__ __forceinline__ void pd_merge_cluster(const float* mine, __nv_bfloat1
 template <int D, int NT, bool STEP>
 __global__ void __launch_bounds__(PdMmaCfg<D>::kWarps * 32)
 paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-                        const __nv_bfloat16* __restrict__ q, const int* __restrict__ block_tables,
-                        const int* __restrict__ context_lens, float* __restrict__ part, int S, int Hq, int Hkv, int block_size,
+                        const __nv_bfloat16* q, const int* block_tables,
+                        const int* context_lens, float* __restrict__ part, int S, int Hq, int Hkv, int block_size,
                         int max_blocks, int splits, float scale, int window, int* status, const __grid_constant__ PdStep step) {
   using Cfg = PdMmaCfg<D>;
   constexpr int ST = Cfg::kStages;
@@ -814,8 +814,8 @@ __device__ __forceinline__ void split_f16x2(float x0, float x1, uint32_t& hi, ui
 template <int D, int NT, bool STEP>
 __global__ void __launch_bounds__(PdF8Cfg<D>::kWarps * 32)
 paged_decode_f8_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-                       const __nv_bfloat16* __restrict__ q, const int* __restrict__ block_tables,
-                       const int* __restrict__ context_lens, float* __restrict__ part, int S, int Hq, int Hkv, int block_size,
+                       const __nv_bfloat16* q, const int* block_tables,
+                       const int* context_lens, float* __restrict__ part, int S, int Hq, int Hkv, int block_size,
                        int max_blocks, int splits, float scale, float v_scale, int window, int* status, const __grid_constant__ PdStep step) {
   using Cfg = PdF8Cfg<D>;
   constexpr int ST = Cfg::kStages;
@@ -1082,8 +1082,8 @@ paged_decode_f8_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
 }
 
 template <int D>
-__global__ void paged_decode_merge_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ o, int rows, int splits,
-                                          const __nv_bfloat16* __restrict__ gate, long long ldg, int Hq, int vdim) {
+__global__ void paged_decode_merge_kernel(const float* part, __nv_bfloat16* __restrict__ o, int rows, int splits,
+                                          const __nv_bfloat16* gate, long long ldg, int Hq, int vdim) {
   pdl_launch_dependents();
   pdl_wait();
   const int row = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);

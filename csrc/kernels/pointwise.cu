@@ -35,7 +35,7 @@ __device__ __forceinline__ void st8(__nv_bfloat16* p, const float (&f)[8]) {
 // IDX: 32 bits where the count of 8-element pieces fits (64-bit divisions cost more than the bytes: 8192 rows of 32 heads of 64, 20 us).
 template <typename IDX>
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ cos_t,
-                            const float* __restrict__ sin_t, const int* __restrict__ pos, IDX rows, IDX T,
+                            const float* __restrict__ sin_t, const int* pos, IDX rows, IDX T,
                             IDX heads, IDX hd, long long row_stride, float sign) {
   pdl_launch_dependents();
   pdl_wait();
@@ -67,7 +67,7 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restri
 // in 32 bits where they fit: three 64-bit divisions an item were most of a prompt's time here (12 us a layer of 4096 tokens, 8 without).
 template <bool FP8, typename IDX>
 __global__ void rope_append_kernel(__nv_bfloat16* __restrict__ qkv, long long ld, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
-                                   const int* __restrict__ pos, const int* __restrict__ slots, __nv_bfloat16* __restrict__ q_out,
+                                   const int* pos, const int* slots, __nv_bfloat16* __restrict__ q_out,
                                    void* __restrict__ k_cache, void* __restrict__ v_cache, IDX rows, int Hq, int Hkv, int hd, int block_size,
                                    float k_inv, float v_inv) {
   pdl_launch_dependents();
@@ -114,7 +114,7 @@ __global__ void rope_append_kernel(__nv_bfloat16* __restrict__ qkv, long long ld
 
 // ---------------------------------------------------------------------------------------------- SwiGLU
 // gu: [M, 2F] with gate in columns [0,F) and up in [F,2F).  h = silu(gate) * up.
-__global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h, long long M, int F) {
+__global__ void swiglu_fwd_kernel(const __nv_bfloat16* gu, __nv_bfloat16* __restrict__ h, long long M, int F) {
   pdl_launch_dependents();
   pdl_wait();
   const int vpr = F / 8;
@@ -197,7 +197,7 @@ __global__ void act_glu_kernel(const T* __restrict__ gu, T* __restrict__ h, long
 // out[n, c] = gelu(g[n, c]) * table[tokens[n], off + c] for c < dim, zero up to ld: a token's own input, gated.  A thread takes V columns (8 where all
 // pieces are aligned: one load each instead of eight, and a division a piece; 4096 x 256: 5.8 us a column at a time, 3.4 so).
 template <typename T, int V>
-__global__ void token_gate_kernel(const T* __restrict__ g, const int* __restrict__ tokens, const T* __restrict__ table, long long ldt,
+__global__ void token_gate_kernel(const T* g, const int* tokens, const T* table, long long ldt,
                                   int off, int dim, int ld, T* __restrict__ out, long long total) {
   pdl_launch_dependents();
   pdl_wait();
@@ -221,7 +221,7 @@ __global__ void token_gate_kernel(const T* __restrict__ g, const int* __restrict
   }
 }
 
-__global__ void swiglu_bwd_kernel(const __nv_bfloat16* gu, const __nv_bfloat16* __restrict__ dh, __nv_bfloat16* dgu,
+__global__ void swiglu_bwd_kernel(const __nv_bfloat16* gu, const __nv_bfloat16* dh, __nv_bfloat16* dgu,
                                   long long M, int F) {
   pdl_launch_dependents();
   pdl_wait();
@@ -293,8 +293,8 @@ __global__ void axpby_kernel(const __nv_bfloat16* a, const __nv_bfloat16* b, __n
 
 // ---------------------------------------------------------------------------------------------- cached rows
 // Rows [pos0, pos0 + n) of one sequence out of its blocks into [n, G, D] arrays.
-__global__ void kv_gather_kernel(const uint4* __restrict__ k_cache, const uint4* __restrict__ v_cache, uint4* __restrict__ k_lin,
-                                 uint4* __restrict__ v_lin, const int* __restrict__ table, int pos0, int G, int ku, int vu,
+__global__ void kv_gather_kernel(const uint4* k_cache, const uint4* v_cache, uint4* __restrict__ k_lin,
+                                 uint4* __restrict__ v_lin, const int* table, int pos0, int G, int ku, int vu,
                                  int block_size) {
   pdl_launch_dependents();
   pdl_wait();
@@ -324,7 +324,7 @@ __device__ __forceinline__ bool goes_before(T a, int i, T b, int j) {
 // 8 x 32000 5.1 / 3.6 us, 8 x 128256 14.1 / 5.0, 64 x 128256 21.3 / 7.2; more rows than that keep a CTA a row (256 x 32000 7.7 / 5.1: one
 // comparison an element instead of three).
 template <bool F32>
-__global__ void __launch_bounds__(1024) argmax_rows_kernel(const void* __restrict__ x, long long* __restrict__ out, int V, long long ld, int log_parts) {
+__global__ void __launch_bounds__(1024) argmax_rows_kernel(const void* x, long long* __restrict__ out, int V, long long ld, int log_parts) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float bv[32];
@@ -406,7 +406,7 @@ __global__ void embedding_fwd_kernel(const IDX* __restrict__ idx, const __nv_bfl
   }
 }
 // dtable[idx[r]] += dout[r]   (bf16x2 atomics; dtable must be zeroed or hold the running gradient)
-__global__ void embedding_bwd_kernel(const long long* __restrict__ idx, const __nv_bfloat16* __restrict__ dout,
+__global__ void embedding_bwd_kernel(const long long* idx, const __nv_bfloat16* dout,
                                      __nv_bfloat16* __restrict__ dtable, long long n_tok, int D, int V) {
   pdl_launch_dependents();
   pdl_wait();
