@@ -385,6 +385,8 @@ __device__ __forceinline__ float* pd_row_sums(uint8_t* smem, int warp, int lane,
   }
   return red_l + W * kPdMmaMaxG;
 }
+// What the maxima start from: below all scores but those of minus infinity, whose weights are zero then.
+constexpr float kPdLowest = -3.402823466e38f;
 // Scores of a chunk of 32 keys, [16-key block][fragment] for every 8 heads: rows are keys g and g + 8, columns heads 2 qd and 2 qd + 1.  They become
 // weights; maxima m and sums l go on, and `a` is what the outputs so far are multiplied by.  factor: of the scores of this lane's heads.
 template <int NT>
@@ -406,15 +408,14 @@ __device__ __forceinline__ void pd_softmax(float (&s)[NT][2][4], const float (&f
       }
 #pragma unroll
       for (int o = 4; o <= 16; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      const float nm = fmaxf(m[n][e], mx);   // (fmaxf passes NaN over: a NaN score shows in the sum alone)
-      const float top = nm == -INFINITY ? 0.f : nm;
-      a[n][e] = m[n][e] == -INFINITY ? 0.f : __expf(m[n][e] - nm);
+      const float nm = fmaxf(m[n][e], mx);   // finite from the start (kPdLowest); fmaxf passes NaN over: a NaN score shows in the sum alone
+      a[n][e] = __expf(m[n][e] - nm);
       m[n][e] = nm;
       float sum = 0.f;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         float& x = s[n][i >> 1][(i & 1) * 2 + e];
-        x = __expf(x - top);
+        x = __expf(x - nm);
         sum += x;
       }
       l[n][e] = l[n][e] * a[n][e] + sum;
@@ -600,7 +601,7 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
 #pragma unroll
   for (int n = 0; n < NT; ++n) {
 #pragma unroll
-    for (int e = 0; e < 2; ++e) { m[n][e] = -INFINITY; l[n][e] = 0.f; factor[n][e] = scale; }
+    for (int e = 0; e < 2; ++e) { m[n][e] = kPdLowest; l[n][e] = 0.f; factor[n][e] = scale; }
 #pragma unroll
     for (int u = 0; u < NU; ++u)
 #pragma unroll
@@ -881,7 +882,7 @@ paged_decode_f8_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
 #pragma unroll
   for (int n = 0; n < NT; ++n) {
 #pragma unroll
-    for (int e = 0; e < 2; ++e) { m[n][e] = -INFINITY; l[n][e] = 0.f; }
+    for (int e = 0; e < 2; ++e) { m[n][e] = kPdLowest; l[n][e] = 0.f; }
 #pragma unroll
     for (int u = 0; u < NU; ++u)
 #pragma unroll
