@@ -123,6 +123,11 @@ struct SplitWs {
   unsigned* flags = nullptr;
 };
 constexpr int kSplitSlots = 160;                                   // >= SM count: at most one partial per CTA
+constexpr int kSplitFlags = 640;                                   // a flag per epilogue warp of a cut tile: 592 at 148 SMs (37 tiles of pairs, 16 each)
+// Whether the workspace holds the parts and flags of `tiles` tiles, cut into `split` parts, on `ctas` CTAs of `warps` epilogue warps each.
+static bool split_fits(int tiles, int split, int ctas, int warps) {
+  return tiles * (split - 1) * ctas <= kSplitSlots && tiles * ctas * warps <= kSplitFlags;
+}
 constexpr size_t kSplitSlotBytes = size_t(kBlockM) * 256 * 4;      // one 128 x 256 fp32 partial
 static std::mutex g_split_mu;
 static std::map<std::pair<int, cudaStream_t>, SplitWs> g_split_ws;
@@ -142,14 +147,14 @@ static bool get_split_ws(cudaStream_t st, SplitWs* out) {
   }
   SplitWs w;
   void* base = nullptr;
-  if (cudaMalloc(&base, kSplitSlots * kSplitSlotBytes + kSplitSlots * 4 * sizeof(unsigned)) != cudaSuccess) {
+  if (cudaMalloc(&base, kSplitSlots * kSplitSlotBytes + kSplitFlags * sizeof(unsigned)) != cudaSuccess) {
     cudaGetLastError();
     g_split_ws[key] = SplitWs{};
     return false;
   }
   w.ws = static_cast<float*>(base);
   w.flags = reinterpret_cast<unsigned*>(static_cast<char*>(base) + kSplitSlots * kSplitSlotBytes);
-  if (cudaMemsetAsync(w.flags, 0, kSplitSlots * 4 * sizeof(unsigned), st) != cudaSuccess) {
+  if (cudaMemsetAsync(w.flags, 0, kSplitFlags * sizeof(unsigned), st) != cudaSuccess) {
     cudaGetLastError();
     cudaFree(base);
     g_split_ws[key] = SplitWs{};
@@ -357,7 +362,7 @@ static int gemm_launch(int kind, const void* A, const void* B, void* C, int M, i
       if (split_on) {
         const int split = tail_split(q.num_tiles, q.k_blocks, sms / 2);
         SplitWs w;
-        if (split > 1 && get_split_ws(st, &w)) {
+        if (split > 1 && split_fits(q.num_tiles % (sms / 2), split, 2, stage ? 8 : 4) && get_split_ws(st, &w)) {
           q.dp_tiles = q.num_tiles / (sms / 2) * (sms / 2);
           q.sk_tiles = q.num_tiles - q.dp_tiles;
           if (q.dp_tiles == 0) pairs = q.sk_tiles * split;
@@ -427,7 +432,7 @@ static int gemm_launch(int kind, const void* A, const void* B, void* C, int M, i
   if (split_on) {
     const int split = tail_split(p.num_tiles, p.k_blocks, slots);
     SplitWs w;
-    if (split > 1 && get_split_ws(st, &w)) {
+    if (split > 1 && split_fits(p.num_tiles % slots, split, 1, 4) && get_split_ws(st, &w)) {
       p.dp_tiles = p.num_tiles / slots * slots;
       p.sk_tiles = p.num_tiles - p.dp_tiles;
       if (p.dp_tiles == 0) grid = p.sk_tiles * split;

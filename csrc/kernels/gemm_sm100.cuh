@@ -71,11 +71,11 @@ struct GemmParams {
   float* acc_ptrs[8];
   // Split tail: tiles [0, dp_tiles) are computed whole, one per CTA per wave; when the last wave would leave most SMs
   // idle, each of the remaining sk_tiles tiles is cut along K into sk_split parts that run on different CTAs.  Parts
-  // 1..sk_split-1 dump their fp32 accumulators into sk_ws and bump sk_flags[tile * 4 + lane quarter]; part 0 waits for
+  // 1..sk_split-1 dump their fp32 accumulators into sk_ws and bump the flag of their epilogue warp; part 0 waits for
   // them (bounded), adds them to its own accumulator and runs the normal epilogue.  sk_split <= 1: no split.
   int dp_tiles, sk_tiles, sk_split;
   float* sk_ws;          // [sk_tiles][sk_split - 1][BLOCK_N / 32][8][128 rows][4]
-  unsigned* sk_flags;    // [sk_tiles][4], zero between launches
+  unsigned* sk_flags;    // [sk_tiles][CTAs of a tile][epilogue warps of a CTA: 4, staged 8], zero between launches
   // Dequantisation of 8-bit operands, applied to the accumulator before bias / residual: row r times a_scale[r], column c
   // times b_scale[c] (fp32, nullptr: 1).
   const float* a_scale;
