@@ -352,11 +352,9 @@ rmsnorm_bwd_wide_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const _
   }
 }
 
-// RMSNorm backward with ONE WARP PER ROW (D = 256 * ITERS, ITERS in {1, 2}): dy and x of the row stay in
-// registers between the reduction and the dx pass, the row sums are warp shuffles (no block barrier per row), and a
-// lane has 16 * ITERS bytes x 2 of loads in flight, so a CTA of 8 warps keeps 8 rows moving instead of one.
-// dgamma is accumulated per lane over all rows of the warp and folded to one partial row per CTA at the end.
-template <int ITERS>
+// RMSNorm backward of 256 columns, a warp a row: dy and x of the row stay in registers between the reduction and the dx pass, the row's sum is a warp
+// shuffle (no block barrier per row), so a CTA of 8 warps keeps 8 rows moving.  dgamma is accumulated per lane over all rows of the warp and folded to one
+// partial row per CTA at the end.
 __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_bwd_warp_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
                         const __nv_bfloat16* w, const float* rstd_in,
@@ -364,74 +362,48 @@ rmsnorm_bwd_warp_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
                         float* __restrict__ dw_part, int M) {
   pdl_launch_dependents();
   pdl_wait();
-  constexpr int D = 256 * ITERS;
+  constexpr int D = 256;
   constexpr int kWarps = kNormThreads / 32;
-  __shared__ float fold[kWarps][256];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float dw_acc[ITERS][8];
+  __shared__ float fold[kWarps][D];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = lane * 8;
+  float dw_acc[8];
 #pragma unroll
-  for (int i = 0; i < ITERS; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) dw_acc[i][j] = 0.f;
+  for (int j = 0; j < 8; ++j) dw_acc[j] = 0.f;
 
   for (int row = blockIdx.x * kWarps + warp; row < M; row += gridDim.x * kWarps) {
-    const long long off = (long long)row * D;
-    uint4 gq[ITERS], xq[ITERS];
-#pragma unroll
-    for (int i = 0; i < ITERS; ++i) {
-      const int c = (i * 32 + lane) * 8;
-      gq[i] = *reinterpret_cast<const uint4*>(dy + off + c);
-      xq[i] = *reinterpret_cast<const uint4*>(x + off + c);
-    }
+    const long long off = (long long)row * D + c;
+    float g[8], xv[8], wv[8], o[8];
+    load8(dy + off, g);
+    load8(x + off, xv);
+    load8(w + c, wv);
     const float rstd = rstd_in[row];
     float s_gx = 0.f;
 #pragma unroll
-    for (int i = 0; i < ITERS; ++i) {
-      const int c = (i * 32 + lane) * 8;
-      float g[8], xv[8], wv[8];
-      unpack8(gq[i], g);
-      unpack8(xq[i], xv);
-      load8(w + c, wv);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float xh = xv[j] * rstd;
-        dw_acc[i][j] += g[j] * xh;
-        s_gx += g[j] * wv[j] * xh;
-      }
+    for (int j = 0; j < 8; ++j) {
+      const float xh = xv[j] * rstd;
+      dw_acc[j] += g[j] * xh;
+      s_gx += g[j] * wv[j] * xh;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s_gx += __shfl_xor_sync(0xffffffffu, s_gx, o);
     const float m_gx = s_gx / D;
 #pragma unroll
-    for (int i = 0; i < ITERS; ++i) {
-      const int c = (i * 32 + lane) * 8;
-      float g[8], xv[8], wv[8], o[8];
-      unpack8(gq[i], g);
-      unpack8(xq[i], xv);
-      load8(w + c, wv);
+    for (int j = 0; j < 8; ++j) o[j] = rstd * (g[j] * wv[j] - xv[j] * rstd * m_gx);
+    if (dres) {
+      float r[8];
+      load8(dres + off, r);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = rstd * (g[j] * wv[j] - xv[j] * rstd * m_gx);
-      if (dres) {
-        float r[8];
-        load8(dres + off + c, r);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] += r[j];
-      }
-      store8(dx + off + c, o);
+      for (int j = 0; j < 8; ++j) o[j] += r[j];
     }
+    store8(dx + off, o);
   }
-  // one partial dgamma row per CTA: 256 columns at a time through shared memory
 #pragma unroll
-  for (int i = 0; i < ITERS; ++i) {
+  for (int j = 0; j < 8; ++j) fold[warp][c + j] = dw_acc[j];
+  __syncthreads();
+  float sum = 0.f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) fold[warp][lane * 8 + j] = dw_acc[i][j];
-    __syncthreads();
-    float sum = 0.f;
-#pragma unroll
-    for (int k = 0; k < kWarps; ++k) sum += fold[k][threadIdx.x];
-    dw_part[(long long)blockIdx.x * D + i * 256 + threadIdx.x] = sum;
-    __syncthreads();
-  }
+  for (int k = 0; k < kWarps; ++k) sum += fold[k][threadIdx.x];
+  dw_part[(long long)blockIdx.x * D + threadIdx.x] = sum;
 }
 
 // out[c] (+)= sum_p part[p, c]; out is bf16 or fp32.  A block owns 32 columns; its 32 warps split the partial rows.
@@ -523,7 +495,7 @@ int lt_norm_bwd(int layer_norm, const void* dy, const void* x, const void* w, co
     int g2 = (M + 7) / 8;
     if (g2 > grid) g2 = grid;
     if (g2 > sm_count()) g2 = sm_count();
-    LT_RETURN_IF_CUDA(launch_chained(rmsnorm_bwd_warp_kernel<1>, g2, kNormThreads, 0, st, DY, X, W, rstd, DR, DX, dw_part, M));
+    LT_RETURN_IF_CUDA(launch_chained(rmsnorm_bwd_warp_kernel, g2, kNormThreads, 0, st, DY, X, W, rstd, DR, DX, dw_part, M));
     LT_LAUNCH_CHECK();
     LT_RETURN_IF_CUDA(launch_chained(fold_partials_kernel, (D + 31) / 32, 1024, 0, st, dw_part, dw, g2, D, grads_fp32, accumulate));
     LT_LAUNCH_CHECK();

@@ -3,10 +3,11 @@
 //
 // Reference: paged_attention_forward runs one THREAD per (sequence, head) with a 2048-float local score
 // array and float block tables (src/backend/gpu_native/nn/nn_kernels.cu:1256-1312), flash-decoding exists
-// only on the CPU (src/ops/flash_decoding.cpp:13-115), and nothing writes the cache.  Here a warp owns one
-// (sequence, query head, split): lanes span the head dimension, keys stream through an online softmax, and a
-// second kernel merges the per-split (max, sum, partial output) triples.  Decode is bandwidth bound (each
-// K/V byte is used once per query head of its group), so the kernel is plain CUDA-core code.
+// only on the CPU (src/ops/flash_decoding.cpp:13-115), and nothing writes the cache.  Here a CTA owns a
+// (sequence, KV head, split) and its warps stream chunks of 32 keys through an online softmax, each byte read once
+// for the whole group of query heads: on the warp-level tensor-core instruction for caches in blocks of 8 keys or more (bf16 and
+// e4m3), on CUDA cores for bf16 caches in smaller blocks, and, where neither applies, a warp a query head.  The splits' (max, sum,
+// partial output) triples meet in a cluster or in a merge kernel.  Decode is bound by the cache's bytes.
 // Cache layout: [num_blocks, Hkv, block_size, D] as in the reference.
 #include "lt_cuda.h"
 #include <cuda_fp8.h>
@@ -319,7 +320,7 @@ paged_decode_gqa_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
 // ------------------------------------------------------------------------------------------------------------
 // Grouped-query decode with the scores and the P V product on the warp-level tensor-core instruction.
 //
-// Same split of the work as paged_decode_gqa_kernel (one CTA of four warps per sequence, KV head and context split;
+// Same split of the work as paged_decode_gqa_kernel (one CTA of four warps, or six, per sequence, KV head and context split;
 // a warp streams chunks of 32 keys through its own shared-memory stages), but the tiles arrive as TMA tensor copies in
 // the 128-byte-swizzled layout, so that ldmatrix reads them without bank conflicts.  Both products are made transposed: keys (and then
 // value columns) are the 16 rows of mma.sync m16n8k16, the group's query heads its 8 columns, so that groups of up to 8 heads, which is
@@ -361,7 +362,7 @@ __device__ __forceinline__ uint32_t movmatrix(uint32_t a) {
 }
 
 // End of a CTA of the tensor-core decode kernels: shared memory (the tile area: every requested copy has been waited for) takes
-// the four warps' maxima, sums and outputs, [warps][16], [warps][16] and [warps][16][D] floats; the last one is returned.  m, l: of heads
+// the warps' maxima, sums and outputs, [warps][16], [warps][16] and [warps][16][D] floats; the last one is returned.  m, l: of heads
 // 8 n + 2 (lane % 4) + e, l this lane's share.
 template <int W, int NT>
 __device__ __forceinline__ float* pd_row_sums(uint8_t* smem, int warp, int lane, bool ok, const float (&m)[NT][2], float (&l)[NT][2]) {
@@ -569,7 +570,7 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
   const int t0 = base + sp * per, t1 = min(ctx, t0 + per);
   const int* bt = block_tables + (long long)s * max_blocks;
   const int n_chunks = t1 > t0 ? (t1 - t0 + 31) / 32 : 0;
-  const int my_n = n_chunks > warp ? (n_chunks - warp + Cfg::kWarps - 1) / Cfg::kWarps : 0;   // chunks warp, warp + 4, ...
+  const int my_n = n_chunks > warp ? (n_chunks - warp + Cfg::kWarps - 1) / Cfg::kWarps : 0;   // chunks warp, warp + kWarps, ...
   const int run = block_size < 32 ? block_size : 32;                 // rows per tensor copy
 
   // The copies of a chunk, a lane for every run of rows; its block, read from the table a chunk ahead, is in `next_blk`.
@@ -738,9 +739,9 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         for (int n = 0; n < NT; ++n) mma_16816(oacc[n][u], va, pb[n][2 * ks], pb[n][2 * ks + 1]);
       }
     }
-    __syncwarp();            // every lane is done with this stage before lane 0 requests into it again
+    __syncwarp();            // every lane is done with this stage before the next copies into it are requested
   }
-  // ---- merge the four warps (the tile area is free now: every requested copy has been waited for), write the partial result
+  // ---- merge the warps (the tile area is free now: every requested copy has been waited for), write the partial result
   float* red_o = pd_row_sums<Cfg::kWarps, NT>(pd_smem, warp, lane, ok, m, l);
 #pragma unroll
   for (int n = 0; n < NT; ++n)
@@ -853,7 +854,7 @@ paged_decode_f8_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
   const int t0 = base + sp * per, t1 = min(ctx, t0 + per);
   const int* bt = block_tables + (long long)s * max_blocks;
   const int n_chunks = t1 > t0 ? (t1 - t0 + 31) / 32 : 0;
-  const int my_n = n_chunks > warp ? (n_chunks - warp + Cfg::kWarps - 1) / Cfg::kWarps : 0;   // chunks warp, warp + 4, ...
+  const int my_n = n_chunks > warp ? (n_chunks - warp + Cfg::kWarps - 1) / Cfg::kWarps : 0;   // chunks warp, warp + kWarps, ...
   const int run = block_size < 32 ? block_size : 32;                 // rows per tensor copy
 
   // The copies of a chunk, a lane for every run of rows; its block, read from the table a chunk ahead, is in `next_blk`.
@@ -1063,7 +1064,7 @@ paged_decode_f8_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
 #pragma unroll
           for (int r = 0; r < 4; ++r) oacc[n][u2 * 2 + uu][r] = fmaf(oacc[n][u2 * 2 + uu][r], a[n][r & 1], pv[n][uu][r]);
     }
-    __syncwarp();            // every lane is done with this stage before lane 0 requests into it again
+    __syncwarp();            // every lane is done with this stage before the next copies into it are requested
   }
   float* red_o = pd_row_sums<Cfg::kWarps, NT>(pd_smem, warp, lane, ok, m, l);
 #pragma unroll

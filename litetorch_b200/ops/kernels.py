@@ -54,7 +54,6 @@ _SIGS = {
     "lt_set_wait_budget_cycles": [_ll, _ll],
     "lt_gemm_bf16": [_vp, _vp, _vp, _i, _i, _i, _ll, _ll, _ll, _i, _i, _i, _vp, _vp, _ll, _i, _i, _f, _i, _i, _vp],
     "lt_gemm_typed": [_i, _vp, _vp, _vp, _i, _i, _i, _ll, _ll, _ll, _i, _i, _i, _vp, _vp, _ll, _i, _i, _f, _vp],
-    "lt_weight_stream": [_vp, _ll] * 4 + [_i] * 5 + [_vp],
     "lt_weight_stream_norm": [_vp, _ll, _vp, _f, _vp, _ll, _vp, _ll, _i, _vp, _ll] + [_i] * 5 + [_vp],
     "lt_rope_append": [_vp, _ll] + [_vp] * 7 + [_ll, _i, _i, _i, _i, _i, _f, _f, _vp],
     "lt_gemv_bf16": [_vp, _ll, _vp, _ll, _vp, _ll, _vp, _ll, _i, _i, _i, _vp],
@@ -91,7 +90,6 @@ _SIGS = {
     "lt_gelu_fwd": [_vp, _vp, _ll, _vp],
     "lt_gelu_bwd": [_vp, _vp, _vp, _ll, _vp],
     "lt_axpby": [_vp, _vp, _vp, _f, _f, _ll, _vp],
-    "lt_embedding_fwd": [_vp, _vp, _vp, _ll, _i, _i, _vp],
     "lt_embedding_fwd_idx": [_vp, _i, _vp, _vp, _ll, _i, _i, _vp],
     "lt_argmax_rows": [_vp, _i, _vp, _i, _i, _ll, _vp],
     "lt_embedding_bwd": [_vp, _vp, _vp, _ll, _i, _i, _vp],
@@ -934,6 +932,7 @@ def decode_step(qkv, cos, sin, positions, slots, heads: int, kv_heads: int, head
                                          kv_heads, D, block_size, block_tables.shape[1], k_cache.shape[0], splits, float(D ** -0.5),
                                          1 if fp8 else 0, float(k_scale), float(v_scale), 1 if early else 0, _stream())
         _check(rc, "lt_paged_decode_step")
+        _launches[0] += part is not None                    # the merge
         return o
     q = rope_append(qkv, cos, sin, positions, slots, heads, kv_heads, D, k_cache, v_cache, block_size, fp8, k_scale, v_scale)
     return paged_decode(q, k_cache, v_cache, block_tables, context_lens, block_size, splits, D ** -0.5, k_scale, v_scale)

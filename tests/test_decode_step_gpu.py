@@ -217,3 +217,12 @@ def test_early_reads_are_asked_for(monkeypatch):
                     num_blocks=4, block_size=16, max_num_seqs=1, graphs=False)
     m.decode_logits([3], [0], [[2]])
     assert seen == [0, 1, 1]
+
+
+def test_launches_are_counted():
+    from litetorch_b200.ops import kernels as K
+    qkv, cos, sin, pos, slots, kc, vc, bt, ctx, lens = _case(2, 4, 2, 64, 16, 600, False, 3)
+    for splits, launches in ((0, 1), (1, 1), (4, 2)):           # splits that meet in a cluster, one, and a merge kernel
+        before = K.launch_count()
+        K.decode_step(qkv, cos, sin, pos, slots, 8, 2, 64, kc, vc, bt, ctx, 16, splits)
+        assert K.launch_count() - before == launches
