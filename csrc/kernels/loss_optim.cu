@@ -439,7 +439,8 @@ int lt_ce_stats(const void* logits, long long ldl, const long long* targets, int
   if (N == 0) return 0;
   const int vec_ok = (ldl % 8 == 0) && ((reinterpret_cast<uintptr_t>(logits) & 15) == 0);
   const int grid = N < sm_count() * 8 ? N : sm_count() * 8;
-  LT_RETURN_IF_CUDA(launch_chained(ce_stats_kernel, grid, kCeThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(logits), ldl, targets, vocab_start, N, V, stats, vec_ok));
+  // (ordinary launches, here and below: see lt_norm_bwd.  300 x 32000, chained / ordinary: 11.7 / 8.6 us, with the gradient 12.3 / 9.4)
+  ce_stats_kernel<<<grid, kCeThreads, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const __nv_bfloat16*>(logits), ldl, targets, vocab_start, N, V, stats, vec_ok);
   LT_LAUNCH_CHECK();
   return 0;
 }
@@ -450,7 +451,8 @@ int lt_ce_finish(void* logits, long long ldl, const long long* targets, int voca
   if (N == 0) return 0;
   const int vec_ok = (ldl % 8 == 0) && ((reinterpret_cast<uintptr_t>(logits) & 15) == 0);
   const int grid = N < sm_count() * 8 ? N : sm_count() * 8;
-  LT_RETURN_IF_CUDA(launch_chained(ce_finish_kernel, grid, kCeThreads, 0, static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(logits), ldl, targets, vocab_start, N, V, gstats, loss, grad_scale, ignore_index, write_grad, vec_ok));
+  ce_finish_kernel<<<grid, kCeThreads, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<__nv_bfloat16*>(logits), ldl, targets, vocab_start, N, V, gstats, loss, grad_scale, ignore_index,
+                                                                               write_grad, vec_ok);
   LT_LAUNCH_CHECK();
   return 0;
 }
