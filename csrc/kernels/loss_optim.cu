@@ -439,7 +439,7 @@ int lt_ce_stats(const void* logits, long long ldl, const long long* targets, int
   if (N == 0) return 0;
   const int vec_ok = (ldl % 8 == 0) && ((reinterpret_cast<uintptr_t>(logits) & 15) == 0);
   const int grid = N < sm_count() * 8 ? N : sm_count() * 8;
-  // (ordinary launches, here and below: see lt_norm_bwd.  300 x 32000, chained / ordinary: 11.7 / 8.6 us, with the gradient 12.3 / 9.4)
+  // (ordinary launches, here and below: see lt_norm_bwd.  300 x 32000, chained / ordinary: 11.7 / 8.7 us, with the gradient 12.3 / 9.5)
   ce_stats_kernel<<<grid, kCeThreads, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const __nv_bfloat16*>(logits), ldl, targets, vocab_start, N, V, stats, vec_ok);
   LT_LAUNCH_CHECK();
   return 0;

@@ -512,8 +512,8 @@ int lt_norm_bwd(int layer_norm, const void* dy, const void* x, const void* w, co
     return 0;
   }
   // An ordinary launch: two CTAs an SM with room for more, which go where there is room if they come while the kernels ahead lie on some of the SMs, and
-  // each of them has many rows (in a recorded chain, chained / ordinary, us: LayerNorm of 4096 x 2048 42.0 / 30.0, of 1337 x 4096 36.5 / 29.0, RMSNorm of
-  // 100 x 8192 15.8 / 10.8, of 4096 x 768 18.9 / 15.2).
+  // each of them has many rows (in a recorded chain, chained / ordinary, us: LayerNorm of 4096 x 2048 42.0 / 26.3, of 1337 x 4096 36.5 / 25.3, RMSNorm of
+  // 100 x 8192 15.8 / 10.6, of 4096 x 768 18.9 / 13.8).
 #define LT_NORM_BWD(LN, IT) \
   norm_bwd_kernel<LN, IT><<<grid, kNormThreads, 0, st>>>(DY, X, W, mean, rstd, DR, DX, dw_part, db_part, M, D)
   if (layer_norm) {
