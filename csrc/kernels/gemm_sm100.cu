@@ -338,10 +338,14 @@ static int gemm_launch(int kind, const void* A, const void* B, void* C, int M, i
   // bf16 results with nothing but a residual (or C itself) added leave through shared memory and TMA
   const bool stage = kind == 0 && !out_fp32 && !bias && !act && !(accumulate && residual) && !(ldc & 7) && !(N & 7) &&
                      !(residual && (ldr & 7)) && ((reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(residual)) & 15) == 0;
-  if (pair_mode > 0 && block_n != 128 && (max_ctas <= 0 || max_ctas >= sms)) {
-    const double c256 = wave_cost(M, N, K, sms, 256, split_on && !stage), c128 = wave_cost(M, N, K, sms, 128, split_on && !stage);
-    const double single = c256 < c128 ? c256 : c128;
-    if (pair_mode == 2 || pair_cost(M, N, K, sms, split_on) < single) {
+  const int slots = max_ctas > 0 && max_ctas < sms ? max_ctas : sms;
+  const GemmTimes& times = stage ? (a_major && b_major ? kTimeStagedTurned : kTimeStaged) : act ? kTimeDirectAct : kTimeDirect;
+  const GemmForm f128 = gemm_form(times.narrow, M, N, K, kBlockM, 128, slots, split_on && !stage);
+  const GemmForm f256 = gemm_form(times.wide, M, N, K, kBlockM, 256, slots, split_on && !stage);
+  const bool narrow = block_n == 128 || (block_n != 256 && f128.us < f256.us);
+  if (pair_mode > 0 && block_n != 128 && slots == sms) {
+    const GemmForm pair = gemm_form(times.pair, M, N, K, kPairBlockM, kPairBlockN, sms / 2, split_on);
+    if (pair_mode == 2 || pair.us < (narrow ? f128 : f256).us) {
       GemmParams q{};
       q.kind = kind;
       q.M = M; q.N = N; q.K = K;
@@ -359,17 +363,14 @@ static int gemm_launch(int kind, const void* A, const void* B, void* C, int M, i
       int pairs = sms / 2;
       if (pairs > q.num_tiles) pairs = q.num_tiles;
       cudaStream_t st = static_cast<cudaStream_t>(stream);
-      if (split_on) {
-        const int split = tail_split(q.num_tiles, q.k_blocks, sms / 2);
-        SplitWs w;
-        if (split > 1 && split_fits(q.num_tiles % (sms / 2), split, 2, stage ? 8 : 4) && get_split_ws(st, &w)) {
-          q.dp_tiles = q.num_tiles / (sms / 2) * (sms / 2);
-          q.sk_tiles = q.num_tiles - q.dp_tiles;
-          if (q.dp_tiles == 0) pairs = q.sk_tiles * split;
-          q.sk_split = split;
-          q.sk_ws = w.ws;
-          q.sk_flags = w.flags;
-        }
+      SplitWs w;
+      if (pair.split > 1 && split_fits(q.num_tiles % (sms / 2), pair.split, 2, stage ? 8 : 4) && get_split_ws(st, &w)) {
+        q.dp_tiles = q.num_tiles / (sms / 2) * (sms / 2);
+        q.sk_tiles = q.num_tiles - q.dp_tiles;
+        if (q.dp_tiles == 0) pairs = q.sk_tiles * pair.split;
+        q.sk_split = pair.split;
+        q.sk_ws = w.ws;
+        q.sk_flags = w.flags;
       }
       if (kind == 2) return launch_gemm_pair<0, 0, 2>(tmA, tmB, q, 2 * pairs, st);   // tf32: both operands K-major
       if (kind == 4) return launch_gemm_pair<0, 0, 4>(tmA, tmB, q, 2 * pairs, st);   // e4m3: both operands K-major
@@ -394,7 +395,7 @@ static int gemm_launch(int kind, const void* A, const void* B, void* C, int M, i
       }
     }
   }
-  if (block_n != 128 && block_n != 256) block_n = split_on && !stage ? pick_block_n_split(M, N, K, sms) : pick_block_n(M, N, sms);
+  block_n = narrow ? 128 : 256;
   GemmParams p{};
   p.kind = kind;
   p.M = M; p.N = N; p.K = K;
@@ -408,10 +409,7 @@ static int gemm_launch(int kind, const void* A, const void* B, void* C, int M, i
   CUtensorMap tmA, tmB;
   int r = make_operand_maps(&tmA, &tmB, A, B, M, N, K, lda, ldb, a_major, b_major, block_n);
   if (r) return r;
-  int grid = sms;
-  if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
-  const int slots = grid;
-  if (grid > p.num_tiles) grid = p.num_tiles;
+  int grid = slots < p.num_tiles ? slots : p.num_tiles;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (stage) {
     if (accumulate) { p.residual = static_cast<const __nv_bfloat16*>(C); p.ldr = ldc; }
@@ -429,17 +427,15 @@ static int gemm_launch(int kind, const void* A, const void* B, void* C, int M, i
       default: return launch_staged<256, 1, 1>(tmA, tmB, tmC, p, grid, st);
     }
   }
-  if (split_on) {
-    const int split = tail_split(p.num_tiles, p.k_blocks, slots);
-    SplitWs w;
-    if (split > 1 && split_fits(p.num_tiles % slots, split, 1, 4) && get_split_ws(st, &w)) {
-      p.dp_tiles = p.num_tiles / slots * slots;
-      p.sk_tiles = p.num_tiles - p.dp_tiles;
-      if (p.dp_tiles == 0) grid = p.sk_tiles * split;
-      p.sk_split = split;
-      p.sk_ws = w.ws;
-      p.sk_flags = w.flags;
-    }
+  const int split = (narrow ? f128 : f256).split;
+  SplitWs w;
+  if (split > 1 && split_fits(p.num_tiles % slots, split, 1, 4) && get_split_ws(st, &w)) {
+    p.dp_tiles = p.num_tiles / slots * slots;
+    p.sk_tiles = p.num_tiles - p.dp_tiles;
+    if (p.dp_tiles == 0) grid = p.sk_tiles * split;
+    p.sk_split = split;
+    p.sk_ws = w.ws;
+    p.sk_flags = w.flags;
   }
   if (kind == 2) return block_n == 256 ? launch_gemm<256, 0, 0, 2>(tmA, tmB, p, grid, st) : launch_gemm<128, 0, 0, 2>(tmA, tmB, p, grid, st);
   if (kind == 3) return block_n == 256 ? launch_gemm<256, 0, 0, 3>(tmA, tmB, p, grid, st) : launch_gemm<128, 0, 0, 3>(tmA, tmB, p, grid, st);

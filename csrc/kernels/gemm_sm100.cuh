@@ -692,21 +692,39 @@ inline int tail_split(int num_tiles, int k_blocks, int slots) {
   int s = slots / rem;
   return s < 1 ? 1 : s > 4 ? 4 : s;
 }
-// Time of `num_tiles` tiles in waves of `slots`; parts of a cut tile cost about five K blocks more (their sums go through L2).
-inline double waves(int num_tiles, int k_blocks, int slots, bool split_on) {
-  const int s = split_on ? tail_split(num_tiles, k_blocks, slots) : 1;
-  const int rem = num_tiles % slots;
-  return double(num_tiles / slots) + (rem == 0 ? 0.0 : s > 1 ? 1.0 / s + 5.0 / k_blocks : 1.0);
-}
+// What a kernel is expected to take (us), and by that the choice between one CTA a tile, 128 or 256 columns wide, and CTA pairs, with the last wave cut
+// along K or not: start, a K block of a full wave, the share of that which a last wave of a single tile takes (few tiles have L2 and the clock to
+// themselves), the results of a wave, and every further part of a cut tile.  Fitted to 830 products of 129 .. 8192 rows, 256 .. 12000 columns and K of 192 ..
+// 14336 in each form (5 to 9 % off, root mean square).  Against the best form of each the choice loses 0.1 to 0.5 % on average and 10 to 17 % at most; counting
+// waves, with a pair's at 0.88 and one of 128 columns at 0.6 of a wave of 256, lost 1.1 % (16-bit results) and 4.1 % (32-bit), and 24 and 60 % at most.
+struct GemmTime {
+  double start, k_block, partial, wave, part;
+};
+struct GemmTimes {
+  GemmTime narrow, wide, pair;
+};
+// staged results; these where both operands are turned on the way (weight gradients), which are mostly added to; results from registers; these behind an activation
+constexpr GemmTimes kTimeStaged{{3.2, 0.302, 0.90, 0.49, 0.0}, {3.7, 0.413, 0.75, 0.75, 0.0}, {5.0, 0.364, 0.69, 1.23, 4.0}};
+constexpr GemmTimes kTimeStagedTurned{{3.7, 0.322, 0.82, 1.76, 0.0}, {4.4, 0.438, 0.76, 2.71, 0.0}, {5.5, 0.357, 0.75, 3.40, 3.5}};
+constexpr GemmTimes kTimeDirect{{3.2, 0.313, 0.86, 3.1, 2.8}, {2.3, 0.428, 0.60, 6.7, 4.9}, {3.6, 0.351, 0.73, 7.2, 5.0}};
+constexpr GemmTimes kTimeDirectAct{{4.5, 0.281, 1.00, 5.1, 3.0}, {5.2, 0.364, 0.78, 9.9, 5.2}, {5.9, 0.309, 0.89, 14.2, 5.4}};
 
-// Time of a GEMM in units of one full 128 x 256 tile wave, used to pick the tile width.
-inline double wave_cost(int M, int N, int K, int sms, int bn, bool split_on = true) {
-  const int tiles = ((M + kBlockM - 1) / kBlockM) * ((N + bn - 1) / bn);
-  return waves(tiles, (K + kBlockK - 1) / kBlockK, sms, split_on) * (bn == 256 ? 1.0 : 0.5 / 0.84);   // measured: the 128-wide tile runs at ~0.84 of the 256-wide one
+inline double gemm_us(const GemmTime& t, int tiles, int k_blocks, int slots, int split) {
+  const int full = tiles / slots, rem = tiles % slots;
+  const double last = rem == 0 ? 0.0 : (t.partial + (1.0 - t.partial) * split * rem / slots) / split;
+  return t.start + t.k_block * k_blocks * (full + last) + t.wave * (full + (rem > 0)) + t.part * (split - 1);
 }
-
-inline int pick_block_n_split(int M, int N, int K, int sms) {
-  return wave_cost(M, N, K, sms, 256) <= wave_cost(M, N, K, sms, 128) ? 256 : 128;
+struct GemmForm {
+  double us;
+  int split;
+};
+// A form's time with the better of cutting its last wave and not.
+inline GemmForm gemm_form(const GemmTime& t, int M, int N, int K, int tile_m, int tile_n, int slots, bool may_split) {
+  const int tiles = ((M + tile_m - 1) / tile_m) * ((N + tile_n - 1) / tile_n), kb = (K + kBlockK - 1) / kBlockK;
+  const GemmForm whole{gemm_us(t, tiles, kb, slots, 1), 1};
+  const int s = may_split ? tail_split(tiles, kb, slots) : 1;
+  const GemmForm cut{gemm_us(t, tiles, kb, slots, s), s};
+  return cut.us < whole.us ? cut : whole;
 }
 
 // Host: the output map of a staged epilogue.

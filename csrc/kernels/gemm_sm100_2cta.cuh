@@ -55,14 +55,6 @@ inline void fill_pair_tiles(GemmParams& p) {
   p.group_m = 8;
 }
 
-// Time of the GEMM on CTA pairs in the unit of wave_cost (one wave of 128 x 256 tiles on every SM).
-inline double pair_cost(int M, int N, int K, int sms, bool split_on) {
-  const int tiles = ((M + kPairBlockM - 1) / kPairBlockM) * ((N + kPairBlockN - 1) / kPairBlockN);
-  const int kb = (K + kBlockK - 1) / kBlockK;
-  // a pair wave does the work of one single-CTA wave, measured 10-14 % faster (operand sharing); start and end of a pair cost about five K blocks more
-  return waves(tiles, kb, sms / 2, split_on) * 0.88 + 5.0 / kb;
-}
-
 // p.m_blocks / p.n_blocks / p.num_tiles count 256 x 256 tiles; everything else as in gemm_body.
 // `gate(m_chunk, n_blk, kb, status)` and `done(m_chunk, n_blk)` are the hooks of gemm_body; m_chunk counts 128-row
 // blocks (the rows one CTA of the pair loads and writes), n_blk counts 256-column blocks.  CTAs [0, cta_first) of
