@@ -873,6 +873,11 @@ def paged_decode(q, k_cache, v_cache, block_tables, context_lens, block_size: in
     return o
 
 
+def _merged_splits(pairs: int, keys: int) -> int:
+    """Splits of the keys of every (sequence, KV head) that a kernel merges: about four CTAs an SM, at least 256 keys each."""
+    return max(1, min(32, keys // 256, (sm_count() * 4 + pairs - 1) // pairs))
+
+
 def _decode_splits(pairs: int, keys: int, head_dim: int, fp8: bool):
     """(how the splits of a (sequence, KV head) meet, how many there are) for a decode step's attention over contexts of up to `keys`:
 
@@ -886,7 +891,7 @@ def _decode_splits(pairs: int, keys: int, head_dim: int, fp8: bool):
     a_sm = (3 if head_dim == 64 else 2) if fp8 else (2 if head_dim == 64 else 1)      # CTAs, by shared memory
     slots = sm_count() * a_sm
     places = slots * 9 // 10
-    many = max(1, min(32, keys // 256, (sm_count() * 4 + pairs - 1) // pairs))
+    many = _merged_splits(pairs, keys)
     if pairs <= 8 and many > 8:
         if keys <= (8192 if head_dim == 64 else 32768):
             return "cluster", 16 if head_dim == 64 else 8
@@ -914,9 +919,6 @@ def decode_step(qkv, cos, sin, positions, slots, heads: int, kv_heads: int, head
     rope_append and paged_decode."""
     S, D = qkv.shape[0], head_dim
     fp8 = k_cache.dtype == torch.float8_e4m3fn
-    how = "part"
-    if splits <= 0:
-        how, splits = _decode_splits(max(1, S * kv_heads), block_tables.shape[1] * block_size, D, fp8)
     if (qkv.dtype == torch.bfloat16 and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0 and D in (64, 128) and heads % kv_heads == 0 and heads // kv_heads <= 16
             and block_size % 8 == 0 and (32 % block_size == 0 or block_size % 32 == 0) and k_cache.is_contiguous() and v_cache.is_contiguous()
             and _aligned(qkv, cos, sin, k_cache, v_cache)):
@@ -925,6 +927,9 @@ def decode_step(qkv, cos, sin, positions, slots, heads: int, kv_heads: int, head
         assert positions.numel() == slots.numel() == context_lens.numel() == block_tables.shape[0] == S
         assert all(t.dtype == torch.float32 and t.is_contiguous() and t.shape[-1] == D // 2 for t in (cos, sin))
         assert all(t.shape[1:] == (kv_heads, block_size, D) for t in (k_cache, v_cache)) and k_cache.shape[0] == v_cache.shape[0]
+        how = "part"
+        if splits <= 0:
+            how, splits = _decode_splits(max(1, S * kv_heads), block_tables.shape[1] * block_size, D, fp8)
         part = torch.empty((S, heads, splits, D + 2), dtype=torch.float32, device=qkv.device) if how == "part" and splits > 1 else None
         o = torch.empty((S, heads, D), dtype=qkv.dtype, device=qkv.device)
         rc = _fn("lt_paged_decode_step")(qkv.data_ptr(), qkv.stride(0), cos.data_ptr(), sin.data_ptr(), positions.data_ptr(), slots.data_ptr(),
@@ -935,6 +940,7 @@ def decode_step(qkv, cos, sin, positions, slots, heads: int, kv_heads: int, head
         _launches[0] += part is not None                    # the merge
         return o
     q = rope_append(qkv, cos, sin, positions, slots, heads, kv_heads, D, k_cache, v_cache, block_size, fp8, k_scale, v_scale)
+    splits = splits if splits > 0 else _merged_splits(max(1, S * kv_heads), block_tables.shape[1] * block_size)
     return paged_decode(q, k_cache, v_cache, block_tables, context_lens, block_size, splits, D ** -0.5, k_scale, v_scale)
 
 

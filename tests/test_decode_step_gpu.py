@@ -226,3 +226,18 @@ def test_launches_are_counted():
         before = K.launch_count()
         K.decode_step(qkv, cos, sin, pos, slots, 8, 2, 64, kc, vc, bt, ctx, 16, splits)
         assert K.launch_count() - before == launches
+
+
+@pytest.mark.parametrize("S,longest,bs", [(1, 6000, 4), (2, 3000, 12), (40, 600, 4)])
+def test_splits_of_caches_that_go_through_the_parts(S, longest, bs, monkeypatch):
+    """As many as a merge kernel takes, not as a cluster holds."""
+    from litetorch_b200.ops import kernels as K
+    real, seen = K.paged_decode, []
+    monkeypatch.setattr(K, "paged_decode", lambda *a: seen.append(a[6]) or real(*a))
+    qkv, cos, sin, pos, slots, kc, vc, bt, ctx, lens = _case(S, 4, 2, 64, bs, longest, False, 5)
+    k2, v2 = kc.clone(), vc.clone()
+    o = K.decode_step(qkv, cos, sin, pos, slots, 8, 2, 64, kc, vc, bt, ctx, bs)
+    many = max(1, min(32, bt.shape[1] * bs // 256, -(-4 * K.sm_count() // (2 * S))))
+    assert seen == [many]
+    q = K.rope_append(qkv, cos, sin, pos, slots, 8, 2, 64, k2, v2, bs, False)
+    assert torch.equal(o, real(q, k2, v2, bt, ctx, bs, many, 64 ** -0.5)) and K.status_fetch() == 0
