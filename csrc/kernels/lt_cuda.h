@@ -266,6 +266,7 @@ int lt_head_norm_gate(int fp32, const float* o, const float* w, const void* gate
 int lt_paged_decode_step(const void* qkv, long long ld, const float* cos_t, const float* sin_t, const int* pos, const int* slots, void* k_cache, void* v_cache,
                          const int* block_tables, const int* context_lens, float* part, void* o, int S, int Hq, int Hkv, int D, int block_size,
                          int max_blocks, int num_blocks, int splits, float scale, int kv_fp8, float k_scale, float v_scale, int early, void* stream);
+int lt_paged_decode_places(int Hq, int Hkv, int D, int kv_fp8, int cluster);
 int lt_paged_decode(const void* q, const void* k_cache, const void* v_cache, const int* block_tables,
                     const int* context_lens, float* part, void* o, int S, int Hq, int Hkv, int D, int block_size,
                     int max_blocks, int num_blocks, int splits, float scale, int kv_fp8, float k_scale, float v_scale,

@@ -1149,14 +1149,38 @@ __global__ void kv_append_kernel(const __nv_bfloat16* __restrict__ k_new, const 
   }
 }
 
-// One of the tensor-core decode kernels, by cache type, head size and heads of a group; cluster: CTAs of a cluster.
-template <class K, class... A>
-static int launch_clustered(K kernel, int warps, int smem, OncePerDevice& configured, int ctas, int cluster, cudaStream_t st, A... args) {
+template <class K>
+static int configure_clustered(K kernel, int smem, OncePerDevice& configured) {
   if (configured.pending()) {
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     LT_RETURN_IF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     configured.finish();
   }
+  return 0;
+}
+// Clusters of `cluster` CTAs that an empty GPU holds at once; negative: an error.
+template <class K>
+static int clusters_at_once(K kernel, int warps, int smem, int cluster) {
+  OncePerDevice configured;
+  if (const int rc = configure_clustered(kernel, smem, configured)) return -rc;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = cluster;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(cluster);
+  cfg.blockDim = dim3(warps * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
+  return e == cudaSuccess ? n : -int(e);
+}
+// One of the tensor-core decode kernels, by cache type, head size and heads of a group; cluster: CTAs of a cluster.
+template <class K, class... A>
+static int launch_clustered(K kernel, int warps, int smem, OncePerDevice& configured, int ctas, int cluster, cudaStream_t st, A... args) {
+  if (const int rc = configure_clustered(kernel, smem, configured)) return rc;
   LT_RETURN_IF_CUDA(launch_chained_clusters(kernel, ctas, warps * 32, smem, cluster, st, args...));
   LT_LAUNCH_CHECK();
   return 0;
@@ -1291,6 +1315,18 @@ int lt_paged_decode_step(const void* qkv, long long ld, const float* cos_t, cons
                                             kv_fp8 ? scale * k_scale : scale, kv_fp8, v_scale, 0, device_status_word(), step, S * Hkv * splits, part ? 1 : splits, st);
   if (rc) return rc;
   return part ? merge_splits(part, static_cast<__nv_bfloat16*>(o), S * Hq, splits, D, nullptr, 0, Hq, D, st) : 0;
+}
+
+// How many clusters of `cluster` CTAs (1 .. 16) of the step's kernel for these heads the current GPU holds at once; negative: an error.
+int lt_paged_decode_places(int Hq, int Hkv, int D, int kv_fp8, int cluster) {
+  using namespace lt;
+  if ((D != 64 && D != 128) || Hkv < 1 || Hq % Hkv != 0 || Hq / Hkv > kPdMmaMaxG || cluster < 1 || cluster > kPdMaxCluster) return -int(kStatusBadArgument);
+#define LT_PLACES(DD, NT) \
+  (kv_fp8 ? clusters_at_once(paged_decode_f8_kernel<DD, NT, true>, PdF8Cfg<DD>::kWarps, PdF8Cfg<DD>::kSmemBytes, cluster) \
+          : clusters_at_once(paged_decode_mma_kernel<DD, NT, true>, PdMmaCfg<DD>::kWarps, PdMmaCfg<DD>::kSmemBytes, cluster))
+  if (Hq / Hkv <= 8) return D == 64 ? LT_PLACES(64, 1) : LT_PLACES(128, 1);
+  return D == 64 ? LT_PLACES(64, 2) : LT_PLACES(128, 2);
+#undef LT_PLACES
 }
 
 int lt_kv_append(const void* k_new, const void* v_new, void* k_cache, void* v_cache, const int* slots, long long n_tok, int Hkv,

@@ -7,6 +7,7 @@ tensors.  No autograd here: `litetorch_b200.ops.functional` wraps these into aut
 from __future__ import annotations
 
 import ctypes
+import functools
 from ctypes import c_void_p, c_int, c_longlong, c_float
 
 import torch
@@ -114,6 +115,7 @@ _SIGS = {
     "lt_gemm_num_tiles": [_i, _i, _i],
     "lt_paged_decode": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _f, _f, _vp],
     "lt_paged_decode_step": [_vp, _ll] + [_vp] * 10 + [_i] * 8 + [_f, _i, _f, _f, _i, _vp],
+    "lt_paged_decode_places": [_i] * 5,
     "lt_kv_append": [_vp, _vp, _vp, _vp, _vp, _ll, _i, _i, _i, _i, _f, _f, _vp],
     "lt_gemm_rs_bf16": [_vp, _vp, _i, _i, _i, _ll, _ll, _i, _vp, _vp, ctypes.c_uint, _i, _i, _i, _vp, _ll, _vp, _vp, _ll, _vp],
     "lt_flash_fwd": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _ll, _f, _i, _vp],
@@ -139,7 +141,7 @@ class LlamaLayer(ctypes.Structure):
 _bound = {}
 
 # Kernels launched per native call; `launch_count()` is what bench.py reports as "gpu_launches".
-_LAUNCHES_PER_CALL = {"lt_gemm_num_tiles": 0, "lt_gemm_skinny_set_target": 0, "lt_adam_q8": 3, "lt_set_wait_budget_cycles": 0, "lt_norm_bwd": 2, "lt_paged_decode": 2, "lt_paged_decode_window": 2, "lt_mlstm_prefill": 4, "lt_rglru_scan": 3, "lt_rglru_step": 2, "lt_flash_bwd": 3, "lt_flash_bwd_rope": 3, "lt_llama_layer_fwd": 8, "lt_llama_layer_bwd": 16, "lt_status_fetch": 0, "lt_sm_count": 0, "lt_gemm_set_tail_split": 0, "lt_reduce_parts": 0, "lt_reduce_all": 2, "lt_gemm_set_pair_mode": 0, "lt_flash_bwd_set_trace": 0, "lt_flash_fwd_set_trace": 0, "lt_norm_bwd_ctas": 0,
+_LAUNCHES_PER_CALL = {"lt_gemm_num_tiles": 0, "lt_gemm_skinny_set_target": 0, "lt_adam_q8": 3, "lt_set_wait_budget_cycles": 0, "lt_norm_bwd": 2, "lt_paged_decode": 2, "lt_paged_decode_window": 2, "lt_mlstm_prefill": 4, "lt_rglru_scan": 3, "lt_rglru_step": 2, "lt_flash_bwd": 3, "lt_flash_bwd_rope": 3, "lt_llama_layer_fwd": 8, "lt_llama_layer_bwd": 16, "lt_status_fetch": 0, "lt_sm_count": 0, "lt_gemm_set_tail_split": 0, "lt_reduce_parts": 0, "lt_reduce_all": 2, "lt_gemm_set_pair_mode": 0, "lt_flash_bwd_set_trace": 0, "lt_flash_fwd_set_trace": 0, "lt_norm_bwd_ctas": 0, "lt_paged_decode_places": 0,
                       "lt_adam_chunk_elems": 0}
 _launches = [0]
 
@@ -878,32 +880,43 @@ def _merged_splits(pairs: int, keys: int) -> int:
     return max(1, min(32, keys // 256, (sm_count() * 4 + pairs - 1) // pairs))
 
 
+@functools.lru_cache(maxsize=1024)
+def _decode_places(device: int, head_dim: int, fp8: bool, cluster: int) -> int:
+    """How many clusters of so many CTAs of a decode step's attention the GPU holds at once."""
+    n = _fn("lt_paged_decode_places")(1, 1, head_dim, 1 if fp8 else 0, cluster)
+    if n <= 0:
+        raise KernelError("lt_paged_decode_places: %d" % n)
+    return n if cluster == 1 else n * 19 // 20               # (they find their places while the kernel in front still lies on some SMs)
+
+
+# us a key and CTA, with all places taken
+_DECODE_KEY_US = {(64, False): 0.0105, (64, True): 0.0145, (128, False): 0.0095, (128, True): 0.0145}
+
+
 def _decode_splits(pairs: int, keys: int, head_dim: int, fp8: bool):
     """(how the splits of a (sequence, KV head) meet, how many there are) for a decode step's attention over contexts of up to `keys`:
 
-    cluster  they merge in a cluster, as many as fill the SMs in one or two rounds (a cluster wants its places together: nine tenths of them).
-             Four layers of a model (us, clusters of 1, 2, 4, 8 / as many splits as give every SM four CTAs, with a merge kernel): 1.1b 16 x 2000
-             247, 208, 192, 226 / 215; 8b 8 x 9000 on 8 bits 832, 614, 497, 528 / 542; 8b 3 x 3000 454, 416, 397, 420 / 419 (of 5: 398); 8b 16 x 2000
-             463, 483, 529, 634 / 524; 8b 32 x 4096 736, 752, 835, . / 751.  One sequence: 8b 1 x 4096 484, 428, 398, 388 / 397, of 16 412; 1.1b
-             1 x 4096 300, 238, 200, 181 / 180, of 16 (which heads of 64 find places for) 173.
-    part     more splits than a cluster holds, and a merge kernel: a few very long sequences (1.1b 1 x 16384 199, clusters of 16 202), and batches
-             that would leave the SMs with a last round of few."""
-    a_sm = (3 if head_dim == 64 else 2) if fp8 else (2 if head_dim == 64 else 1)      # CTAs, by shared memory
-    slots = sm_count() * a_sm
-    places = slots * 9 // 10
-    many = _merged_splits(pairs, keys)
-    if pairs <= 8 and many > 8:
-        if keys <= (8192 if head_dim == 64 else 32768):
-            return "cluster", 16 if head_dim == 64 else 8
-        return "part", many
+    cluster  they merge in a cluster: as many as find places in one round (a second round costs as much as the first: 16 pairs of 2000 keys, heads of 128,
+             clusters of 6 11.2 us, of 8, of which 15 fit, 17.3; 96 pairs of 700 keys, heads of 64, of 2 12.7, of 5 16.8).
+    part     as many as fill one round, and a merge kernel, where the shorter splits gain more than that costs: few pairs and long contexts (8 pairs of
+             32000 8-bit keys 29 us in 32 parts, 60 in clusters of 8); and more pairs than clusters of two find places for, if 2 to 4 parts fill
+             the last round better (384 pairs of 4000 8-bit keys 127 us whole, 104 in 2).
 
-    def rounds(n):
-        return -(-pairs * n // (places if n > 1 else slots))
+    Over 416 shapes (1 to 64 sequences, 40 to 32000 keys) the choice loses 1.1 % on average against the best number of splits."""
+    device = torch.cuda.current_device()
+    slots, key_us = _decode_places(device, head_dim, fp8, 1), _DECODE_KEY_US[head_dim, fp8]
+    clusters = [n for n in range(2, 9) if keys // n >= 128 and pairs <= _decode_places(device, head_dim, fp8, n)]
+    if head_dim == 64 and keys // 16 >= 128 and pairs * 16 <= sm_count() and pairs <= _decode_places(device, head_dim, fp8, 16):
+        clusters.append(16)
+    if clusters:
+        n, parts = clusters[-1], min(32, keys // 256, slots // pairs)
+        return ("part", parts) if parts > n and key_us * keys * (1 / n - 1 / parts) > 6.0 else ("cluster", n)
 
-    n = min((n for n in range(1, max(1, min(8, keys // 128)) + 1) if n == 1 or rounds(n) <= 2), key=lambda n: (rounds(n) / n, n))
-    if many > 1 and 1.5 * -(-pairs * many // slots) / many < rounds(n) / n:           # (the merge costs a launch)
-        return "part", many
-    return "cluster", n
+    def us(n):
+        return -(-pairs * n // slots) * (4.5 + key_us * keys / n) + (3.5 if n > 1 else 0.0)
+
+    n = min((n for n in (1, 2, 3, 4) if n == 1 or keys // n >= 256), key=us)
+    return ("cluster", 1) if n == 1 else ("part", n)
 
 
 def decode_step(qkv, cos, sin, positions, slots, heads: int, kv_heads: int, head_dim: int, k_cache, v_cache, block_tables, context_lens, block_size: int,
@@ -916,10 +929,13 @@ def decode_step(qkv, cos, sin, positions, slots, heads: int, kv_heads: int, head
     for it that no kernel writes them which the stream may still run then: since the last write a kernel of torch, a copy or another launch that
     starts after everything before it (`embedding_fwd`) was made, not only kernels of this library, which start under one another.
     splits: how many the keys of a (sequence, KV head) are cut into (0: by size).  One launch, or two; caches that it does not take go through
-    rope_append and paged_decode."""
+    rope_append and paged_decode, and so do many short contexts with heads of 128 (more pairs than CTAs find places, each of which would turn its queries
+    and wait for them with one or two chunks of keys to read: 64 sequences of 40 tokens, 8 KV heads, 34.8 us against 28.3; of 300 tokens 42.7 against 45.7)."""
     S, D = qkv.shape[0], head_dim
     fp8 = k_cache.dtype == torch.float8_e4m3fn
-    if (qkv.dtype == torch.bfloat16 and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0 and D in (64, 128) and heads % kv_heads == 0 and heads // kv_heads <= 16
+    pairs, keys = max(1, S * kv_heads), block_tables.shape[1] * block_size
+    apart = splits <= 0 and D == 128 and keys <= 256 and pairs > _decode_places(torch.cuda.current_device(), D, fp8, 1)
+    if (not apart and qkv.dtype == torch.bfloat16 and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0 and D in (64, 128) and heads % kv_heads == 0 and heads // kv_heads <= 16
             and block_size % 8 == 0 and (32 % block_size == 0 or block_size % 32 == 0) and k_cache.is_contiguous() and v_cache.is_contiguous()
             and _aligned(qkv, cos, sin, k_cache, v_cache)):
         assert qkv.dim() == 2 and qkv.shape[1] >= (heads + 2 * kv_heads) * D and k_cache.dtype == v_cache.dtype and (fp8 or k_cache.dtype == torch.bfloat16)
@@ -929,7 +945,7 @@ def decode_step(qkv, cos, sin, positions, slots, heads: int, kv_heads: int, head
         assert all(t.shape[1:] == (kv_heads, block_size, D) for t in (k_cache, v_cache)) and k_cache.shape[0] == v_cache.shape[0]
         how = "part"
         if splits <= 0:
-            how, splits = _decode_splits(max(1, S * kv_heads), block_tables.shape[1] * block_size, D, fp8)
+            how, splits = _decode_splits(pairs, keys, D, fp8)
         part = torch.empty((S, heads, splits, D + 2), dtype=torch.float32, device=qkv.device) if how == "part" and splits > 1 else None
         o = torch.empty((S, heads, D), dtype=qkv.dtype, device=qkv.device)
         rc = _fn("lt_paged_decode_step")(qkv.data_ptr(), qkv.stride(0), cos.data_ptr(), sin.data_ptr(), positions.data_ptr(), slots.data_ptr(),
@@ -940,7 +956,7 @@ def decode_step(qkv, cos, sin, positions, slots, heads: int, kv_heads: int, head
         _launches[0] += part is not None                    # the merge
         return o
     q = rope_append(qkv, cos, sin, positions, slots, heads, kv_heads, D, k_cache, v_cache, block_size, fp8, k_scale, v_scale)
-    splits = splits if splits > 0 else _merged_splits(max(1, S * kv_heads), block_tables.shape[1] * block_size)
+    splits = splits if splits > 0 else _merged_splits(pairs, keys)
     return paged_decode(q, k_cache, v_cache, block_tables, context_lens, block_size, splits, D ** -0.5, k_scale, v_scale)
 
 

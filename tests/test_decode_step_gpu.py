@@ -241,3 +241,39 @@ def test_splits_of_caches_that_go_through_the_parts(S, longest, bs, monkeypatch)
     assert seen == [many]
     q = K.rope_append(qkv, cos, sin, pos, slots, 8, 2, 64, k2, v2, bs, False)
     assert torch.equal(o, real(q, k2, v2, bt, ctx, bs, many, 64 ** -0.5)) and K.status_fetch() == 0
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("S,longest", [(37, 250), (38, 250), (75, 256), (75, 270)])
+def test_many_short_contexts(S, longest, fp8, monkeypatch):
+    """Both sides of the line beyond which queries are turned and rows cached by a launch of their own."""
+    from litetorch_b200.ops import kernels as K
+    seen, real = [], K._fn
+    monkeypatch.setattr(K, "_fn", lambda name: seen.append(name) or real(name))
+    G, Hkv, D, bs = 2, 4, 128, 16
+    qkv, cos, sin, pos, slots, kc, vc, bt, ctx, lens = _case(S, G, Hkv, D, bs, longest, fp8, S)
+    bt = bt[:, :(longest + bs - 1) // bs].contiguous()
+    k2, v2 = kc.clone(), vc.clone()
+    o = K.decode_step(qkv, cos, sin, pos, slots, G * Hkv, Hkv, D, kc, vc, bt, ctx, bs)
+    apart = S * Hkv > K._decode_places(0, D, fp8, 1) and bt.shape[1] * bs <= 256
+    assert ("lt_paged_decode_step" in seen) == (not apart) and apart == (longest <= 256 and S * Hkv > K.sm_count() * (2 if fp8 else 1))
+    q = K.rope_append(qkv, cos, sin, pos, slots, G * Hkv, Hkv, D, k2, v2, bs, fp8)
+    want = K.paged_decode(q, k2, v2, bt, ctx, bs, 1, D ** -0.5)
+    bits = torch.uint8 if fp8 else torch.int16
+    assert torch.equal(kc.view(bits), k2.view(bits)) and torch.equal(vc.view(bits), v2.view(bits))
+    assert ((o.float() - want.float()).abs() <= want.float().abs() * 2.0 ** -7 + 2e-3).all() and K.status_fetch() == 0
+
+
+def test_one_round_of_clusters():
+    """Clusters are as large as they all find places at once, parts as many as fill one round."""
+    from litetorch_b200.ops import kernels as K
+    for D in (64, 128):
+        for fp8 in (False, True):
+            for pairs in (1, 4, 8, 16, 24, 32, 48, 64, 96, 128, 256):
+                for keys in (256, 1024, 2048, 8192, 32768):
+                    how, n = K._decode_splits(pairs, keys, D, fp8)
+                    if how == "cluster" and n > 1:
+                        assert pairs <= K._decode_places(0, D, fp8, n)
+                        assert n >= 8 or keys // (n + 1) < 128 or pairs > K._decode_places(0, D, fp8, n + 1)
+                    if how == "part" and pairs <= K._decode_places(0, D, fp8, 2):
+                        assert pairs * n <= K._decode_places(0, D, fp8, 1)
