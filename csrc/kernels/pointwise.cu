@@ -323,8 +323,8 @@ __device__ __forceinline__ bool goes_before(T a, int i, T b, int j) {
 // takes a row and its first one compares their candidates: few long rows leave a CTA a row waiting for one load after the other.  A CTA a row / this:
 // 8 x 32000 5.1 / 3.6 us, 8 x 128256 14.1 / 5.0, 64 x 128256 21.3 / 7.2; more rows than that keep a CTA a row (256 x 32000 7.7 / 5.1: one
 // comparison an element instead of three).
-template <bool F32>
-__global__ void __launch_bounds__(1024) argmax_rows_kernel(const void* x, long long* __restrict__ out, int V, long long ld, int log_parts) {
+template <bool F32, int NT>
+__global__ void __launch_bounds__(NT) argmax_rows_kernel(const void* x, long long* __restrict__ out, int V, long long ld, int log_parts) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float bv[32];
@@ -341,26 +341,26 @@ __global__ void __launch_bounds__(1024) argmax_rows_kernel(const void* x, long l
   if (F32) {
     const float* r = static_cast<const float*>(x) + row * ld;
     if ((reinterpret_cast<uintptr_t>(r) & 15) == 0) {
-      for (int c = from + threadIdx.x * 4; c + 3 < end; c += 4096) {
+      for (int c = from + threadIdx.x * 4; c + 3 < end; c += 4 * NT) {
         const float4 f = *reinterpret_cast<const float4*>(r + c);
         see(f.x, c); see(f.y, c + 1); see(f.z, c + 2); see(f.w, c + 3);
       }
-      for (int c = end / 4 * 4 + threadIdx.x; c < end; c += 1024) see(r[c], c);
+      for (int c = end / 4 * 4 + threadIdx.x; c < end; c += NT) see(r[c], c);
     } else {
-      for (int c = from + threadIdx.x; c < end; c += 1024) see(r[c], c);
+      for (int c = from + threadIdx.x; c < end; c += NT) see(r[c], c);
     }
   } else {
     const __nv_bfloat16* r = static_cast<const __nv_bfloat16*>(x) + row * ld;
     if ((reinterpret_cast<uintptr_t>(r) & 15) == 0) {
-      for (int c = from + threadIdx.x * 8; c + 7 < end; c += 8192) {
+      for (int c = from + threadIdx.x * 8; c + 7 < end; c += 8 * NT) {
         float f[8];
         ld8(r + c, f);
 #pragma unroll
         for (int j = 0; j < 8; ++j) see(f[j], c + j);
       }
-      for (int c = end / 8 * 8 + threadIdx.x; c < end; c += 1024) see(__bfloat162float(r[c]), c);
+      for (int c = end / 8 * 8 + threadIdx.x; c < end; c += NT) see(__bfloat162float(r[c]), c);
     } else {
-      for (int c = from + threadIdx.x; c < end; c += 1024) see(__bfloat162float(r[c]), c);
+      for (int c = from + threadIdx.x; c < end; c += NT) see(__bfloat162float(r[c]), c);
     }
   }
   auto reduce = [&]() {
@@ -375,8 +375,9 @@ __global__ void __launch_bounds__(1024) argmax_rows_kernel(const void* x, long l
   if ((threadIdx.x & 31) == 0) { bv[threadIdx.x >> 5] = best; bi[threadIdx.x >> 5] = at; }
   __syncthreads();
   if (threadIdx.x < 32) {
-    best = bv[threadIdx.x];
-    at = bi[threadIdx.x];
+    const bool there = threadIdx.x * 32 < NT;
+    best = there ? bv[threadIdx.x] : -INFINITY;
+    at = there ? bi[threadIdx.x] : V;
     reduce();
     if (threadIdx.x == 0) { bv[0] = best; bi[0] = at; }
   }
@@ -629,9 +630,12 @@ int lt_argmax_rows(const void* x, int fp32, long long* out, int rows, int V, lon
   // two CTAs of 1024 threads fit an SM; a part of 4096 elements is one load a thread (fp32)
   int parts = 3;
   while (parts > 0 && (((long long)rows << parts) > 2 * sm_count() || (V >> parts) < 4096)) --parts;
-  auto kernel = fp32 ? argmax_rows_kernel<true> : argmax_rows_kernel<false>;
-  if (parts > 0) LT_RETURN_IF_CUDA(launch_chained_clusters(kernel, rows << parts, 1024, 0, 1 << parts, st, x, out, V, ld, parts));
-  else LT_RETURN_IF_CUDA(launch_chained(kernel, rows, 1024, 0, st, x, out, V, ld, 0));
+  // short rows: fewer threads that have nothing to load (1024 x 512 fp32: 1024 threads a row 7.6 us, 256 2.8)
+  const bool few = V >> parts <= (fp32 ? 2048 : 4096);
+  const int threads = few ? 256 : 1024;
+  auto kernel = few ? (fp32 ? argmax_rows_kernel<true, 256> : argmax_rows_kernel<false, 256>) : (fp32 ? argmax_rows_kernel<true, 1024> : argmax_rows_kernel<false, 1024>);
+  if (parts > 0) LT_RETURN_IF_CUDA(launch_chained_clusters(kernel, rows << parts, threads, 0, 1 << parts, st, x, out, V, ld, parts));
+  else LT_RETURN_IF_CUDA(launch_chained(kernel, rows, threads, 0, st, x, out, V, ld, 0));
   return 0;
 }
 int lt_embedding_bwd(const long long* idx, const void* dout, void* dtable, long long n_tok, int D, int V, void* stream) {

@@ -69,3 +69,16 @@ def test_logits_and_loss_of_columns(dtype):
     part, target = tokens[:, 3:4], tokens[:, 4:5]
     assert torch.equal(eng.forward_logits(part), eng.forward_logits(part.long().contiguous()))
     assert torch.equal(eng.eval_loss(part, target), eng.eval_loss(part.long().contiguous(), target.long().contiguous()))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows", [1, 400])
+@pytest.mark.parametrize("V", [31, 255, 257, 2047, 2048, 2049, 4095, 4096, 4098, 16384, 16388])
+def test_argmax_of_few_and_many_threads(dtype, rows, V):
+    from litetorch_b200.ops import kernels as K
+    x = torch.randn(rows, V, device="cuda", generator=torch.Generator(device="cuda").manual_seed(V)).to(dtype)
+    x[:, V - 1] = 9.0
+    assert bool((K.argmax_rows(x) == V - 1).all())
+    x[:, V // 3] = 9.0
+    assert bool((K.argmax_rows(x) == V // 3).all())
+    assert K.status_fetch() == 0
